@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/dvg.h"
+#include "cells.cuh"
 #include "kernels.cuh"
 #include "prepare.hpp"
 
@@ -66,6 +67,34 @@ struct DevBuf {
     }
 };
 
+// Device memory of one scene, stream-ordered from its context's pool: a program that uploads a
+// scene per call reuses the freed blocks of the one before instead of mapping memory again.
+struct SceneBuf {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    ~SceneBuf() {
+        if (ptr) cudaFreeAsync(ptr, stream);
+    }
+    cudaError_t reserve(size_t n) {
+        if (n <= bytes) return cudaSuccess;
+        if (ptr) cudaFreeAsync(ptr, stream);
+        ptr = nullptr;
+        bytes = 0;
+        cudaError_t e = cudaMallocFromPoolAsync(&ptr, n, pool, stream);
+        if (e == cudaSuccess) bytes = n;
+        else ptr = nullptr;
+        return e;
+    }
+    template <typename T>
+    T* as() const {
+        return static_cast<T*>(ptr);
+    }
+};
+// Bytes of freed scene memory that a context keeps for its next uploads.
+constexpr uint64_t kScenePoolKeep = 256ull << 20;
+
 // Packs several host arrays into one blob with 256-byte aligned offsets.
 struct Blob {
     std::vector<char> data;
@@ -96,7 +125,9 @@ struct dvg_context {
     std::vector<ProfEvent> pending;
     std::vector<ProfStat> stats;
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;  // scene memory (SceneBuf)
     unsigned* status = nullptr;  // device word
+    L2Acc* l2acc = nullptr;
     DevBuf accum, wsum, image, d_render, target, loss, bg_grad, trans_grad;
     DevBuf bsamples, bkey, border, bcounts;  // boundary-pass scratch
     DevBuf sdf, positions, dvalues;          // signed-distance host calls
@@ -126,10 +157,12 @@ struct dvg_scene {
     dvg_context* ctx = nullptr;
     HostScene host;
     DevScene dev{};
-    DevBuf arena;
-    DevBuf tiles;    // counts, offsets
-    DevBuf entries;  // tile entries
-    DevBuf grads;    // gradient arena (device)
+    SceneBuf arena;
+    SceneBuf tiles;    // counts, offsets
+    SceneBuf entries;  // tile entries
+    SceneBuf cells;    // per-cell lists (cell_table)
+    CellTable cell_table{};
+    SceneBuf grads;    // gradient arena (device)
     size_t grad_off[11] = {0};
     size_t grad_floats = 0;
     size_t arena_bytes = 0;  // bytes of prepared tables in `arena`
@@ -138,6 +171,32 @@ struct dvg_scene {
 };
 
 namespace {
+
+// Sizes a scene's per-cell lists for `total` tile entries and points its tables at them: at
+// most one cell entry per tile entry and cell, and four items for each (what finds no room
+// keeps the full query).
+dvg_status reserve_cells(dvg_scene* sc, size_t total) {
+    DevScene& S = sc->dev;
+    const size_t cells = (size_t)S.tiles_x * S.tiles_y * CELLS;
+    const size_t ents = std::min<size_t>(std::max<size_t>(total, 1) * CELLS, (size_t)1 << 30);
+    const size_t items = std::min<size_t>(ents * 4, (size_t)1 << 30);
+    const size_t o_ent = (cells * sizeof(int2) + 255) & ~(size_t)255, o_item = o_ent + ents * 2 * sizeof(int4);
+    const size_t o_cnt = (o_item + items * sizeof(int4) + 255) & ~(size_t)255;
+    CK(sc->cells.reserve(o_cnt + 2 * sizeof(int)));
+    char* b = sc->cells.as<char>();
+    sc->cell_table = CellTable{(int2*)b, (int4*)(b + o_ent), (int4*)(b + o_item), (int*)(b + o_cnt), (int)ents, (int)items};
+    S.cell_info = sc->cell_table.info;
+    S.cell_entries = sc->cell_table.entries;
+    S.cell_items = sc->cell_table.items;
+    return DVG_OK;
+}
+// Builds the lists on the context's stream (after the tile lists).
+dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
+    CK(cudaMemsetAsync(sc->cell_table.counters, 0, 2 * sizeof(int), ctx->stream));
+    ctx->launches += launch_cells(sc->dev, sc->cell_table, ctx->stream);
+    CK(cudaGetLastError());
+    return DVG_OK;
+}
 
 // Offsets of each gradient part inside the scene's gradient arena (in floats).
 void layout_grads(dvg_scene* sc) {
@@ -357,7 +416,15 @@ dvg_status dvg_context_create(int device, dvg_context** out) {
     ctx->device = device;
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    CK(cudaMemPoolCreate(&ctx->pool, &props));
+    uint64_t keep = kScenePoolKeep;
+    CK(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     CK(cudaMalloc(&ctx->status, sizeof(unsigned)));
+    CK(cudaMalloc(&ctx->l2acc, sizeof(L2Acc)));
     CK(cudaMemsetAsync(ctx->status, 0, sizeof(unsigned), ctx->stream));
     *out = ctx.release();
     return DVG_OK;
@@ -381,6 +448,8 @@ void dvg_context_destroy(dvg_context* ctx) {
     ctx->kept = nullptr;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->status) cudaFree(ctx->status);
+    if (ctx->l2acc) cudaFree(ctx->l2acc);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -394,6 +463,10 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
     CK(cudaSetDevice(ctx->device));
     std::unique_ptr<dvg_scene> sc(new dvg_scene());
     sc->ctx = ctx;
+    for (SceneBuf* b : {&sc->arena, &sc->tiles, &sc->entries, &sc->cells, &sc->grads}) {
+        b->pool = ctx->pool;
+        b->stream = ctx->stream;
+    }
     std::string err;
     dvg_status st = prepare_scene(desc, &sc->host, &err);
     if (st != DVG_OK) return fail(st, err);
@@ -496,6 +569,9 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
         S.tile_entries = sc->entries.as<int>();
         ctx->launches += launch_binning(S, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
         CK(cudaGetLastError());
+        st = reserve_cells(sc.get(), (size_t)std::max(total, 0));
+        if (st == DVG_OK) st = build_cells(ctx, sc.get());
+        if (st != DVG_OK) return st;
     }
     layout_grads(sc.get());
     CK(sc->grads.reserve(sizeof(float) * std::max<size_t>(sc->grad_floats, 64)));
@@ -909,10 +985,10 @@ dvg_status dvg_fwd_bwd_l2_device(dvg_context* ctx, dvg_scene* scene, const dvg_r
     st = render_into(ctx, scene, opts, img, &frag);
     if (st != DVG_OK) return st;
     CK(ctx->d_render.reserve(npix * 4 * sizeof(float)));
-    if (loss_out) CK(cudaMemsetAsync(loss_out, 0, sizeof(float), ctx->stream));
     {
         Prof prof_(ctx, "l2_loss");
-        ctx->launches += launch_l2(img, target_rgba, npix * 4, ctx->d_render.as<float>(), loss_out, ctx->stream);
+        ctx->launches += launch_l2(img, target_rgba, npix * 4, ctx->d_render.as<float>(), loss_out, ctx->l2acc,
+                                   ctx->stream);
     }
     CK(cudaGetLastError());
     GradPtrs G = grads_from_user(grads);
@@ -1018,10 +1094,12 @@ dvg_status dvg_l2_device(dvg_context* ctx, const float* image, const float* targ
                          float* loss) {
     if (!ctx || !image || !target || !d_render) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     CK(cudaSetDevice(ctx->device));
-    if (loss) CK(cudaMemsetAsync(loss, 0, sizeof(float), ctx->stream));
-    if (n == 0) return DVG_OK;
+    if (n == 0) {
+        if (loss) CK(cudaMemsetAsync(loss, 0, sizeof(float), ctx->stream));
+        return DVG_OK;
+    }
     Prof prof_(ctx, "l2_loss");
-    ctx->launches += launch_l2(image, target, (size_t)n, d_render, loss, ctx->stream);
+    ctx->launches += launch_l2(image, target, (size_t)n, d_render, loss, ctx->l2acc, ctx->stream);
     CK(cudaGetLastError());
     return DVG_OK;
 }
@@ -1203,6 +1281,8 @@ dvg_status batch_enqueue(dvg_batch* b) {
             int* offsets = counts + sc->dev.tiles_x * sc->dev.tiles_y;
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, nullptr, ctx->stream);
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
+            const dvg_status st = build_cells(ctx, sc);
+            if (st != DVG_OK) return st;
         }
     }
     CK(cudaGetLastError());
@@ -1463,8 +1543,19 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, nullptr, ctx->stream);
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
             CK(cudaGetLastError());
+            // room for four times the cell entries that the present geometry takes: a step that
+            // moves more than that into view walks the tile lists instead
+            int total = 0;
+            CK(cudaMemcpyAsync(&total, offsets + tiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+            dvg_status st = reserve_cells(sc, std::min<size_t>(need, 4 * (size_t)std::max(total, 0) + 1024));
+            if (st == DVG_OK) st = build_cells(ctx, sc);
+            if (st != DVG_OK) return st;
         }
         b->host_entries[i].S.tile_entries = sc->dev.tile_entries;
+        b->host_entries[i].S.cell_info = sc->dev.cell_info;
+        b->host_entries[i].S.cell_entries = sc->dev.cell_entries;
+        b->host_entries[i].S.cell_items = sc->dev.cell_items;
     }
     // Adam moments and sort scratch, one block per scene.
     std::vector<size_t> st_off(n), so_off(n);

@@ -1,0 +1,311 @@
+// cell_classify.cuh — what a segment contributes to the sample points of a small box.
+//
+// The render kernels look at the scene through lists kept for every 4x4-pixel cell of the
+// canvas (cells.cu).  A list holds, per group, only the segments that come near the cell; the
+// winding contribution of the others is summed beforehand, up to a few comparisons of the
+// sample's row with the rows where it steps.  The functions here decide which is which, for a
+// box that holds every point the cell's samples can have in shape space (their f32 rounding
+// included).
+//
+// Certainty.  The crate adds, per segment, the sign of y'(t) of each computed root t in [0, 1]
+// of y(t) = py with x(t) > px (winding.rs:118-192).  Let m be the largest coordinate of the
+// segment and the box.  The polynomial that it solves has f32-rounded coefficients and lies
+// within 4.6e-6 m of the curve on [0, 1]; its f64 roots carry the error of its root formula.
+// Take the monotone pieces of y(t) that meet the box's rows, and the parameter range in which
+// each is inside them (bracketed by evaluation).  When every such range of the curve lies
+// left of the box by more than M = 1e-4 (1 + m), the segment adds nothing; where it lies right
+// of the box by more than M, the piece from level l0 to l1 adds [py > l0] - [py > l1].  At an
+// extremum between two such pieces that cancels; what remains is a constant and a step at each
+// end point inside the rows.  A piece that crosses all of the rows near the box is replaced by
+// a parabola x = c0 + c1 y + c2 y^2 through three of its points, with a bound on the distance in
+// x between the two: it counts where px lies left of the parabola by more than the bound, and
+// not where it lies right of it by as much.  The crate's computed sum is this number when
+//  * py is farther than T = 1e-5 (1 + m) from every level inside the rows (end points and
+//    extrema): the sample loop compares, and runs the full query otherwise;
+//  * |y'| >= M at an inflection, so that |y'| is small near extrema only;
+//  * a cubic is well conditioned: |b|, |c|, |d| <= 64 |a|, so that the crate's normalised
+//    coefficients are at most 64, or its a is below the 1e-6 at which the crate solves a
+//    quadratic.
+// Then with D = T - 4.6e-6 m > 5e-6 m the distance in y to the next level of the crate's own
+// polynomial, its roots are off by p / |y'| with p = 24 m 64^2 eps < 1.1e-11 m from the rounding
+// of its normalised coefficients.  Next to an extremum, |y'| dt = 2 D for the distance dt to it,
+// so the error is below 1.1e-6 dt; next to an end point the root is at least D / |y'| away from
+// it, 4e5 times the error.  The trigonometric formula adds 4 sqrt(q) 8 eps / sqrt(1 - x^2), below
+// 1e-7 for roots that are sqrt(2 D / 24 m) apart.  So every computed root is on the same side of
+// 0, of 1, of px (M against 6 m times the error) and of every extremum as the exact one.
+// A parabola's bound holds the interpolation error (the third derivative of X - c0 - c1 Y - c2 Y^2
+// over the bracket) and T moved in y and in x, for the rounded coefficients and the root.
+// Anything else is left to the per-sample test.  A segment whose control points miss the rays
+// of the whole box by the per-sample culling margin (ray_misses_segment in device.cuh)
+// contributes nothing, as there.
+//
+// Host and device share this code: oracle/cell_stress.cpp runs it against the oracle's f64
+// decisions at random points of random boxes.
+#pragma once
+#include <cmath>
+
+#ifdef __CUDACC__
+#define DVG_CC_HD __host__ __device__ __forceinline__
+#else
+#define DVG_CC_HD inline
+#endif
+
+namespace dvgb {
+
+struct CellBox {
+    float x0, y0, x1, y1;
+};
+
+DVG_CC_HD float cc_max8(const float* q) {
+    float m = 0.0f;
+    for (int k = 0; k < 8; ++k) m = std::fmax(m, std::fabs(q[k]));
+    return m;
+}
+DVG_CC_HD float cc_poly(float a, float b, float c, float d, float t) { return ((a * t + b) * t + c) * t + d; }
+
+// The box as seen through an affine map (rows m[0..2], m[3..5]), grown by the f32 rounding of
+// the map at its points.
+DVG_CC_HD CellBox cc_map_box(const float* m, CellBox b) {
+    const float cx = 0.5f * (b.x0 + b.x1), cy = 0.5f * (b.y0 + b.y1);
+    const float hx = 0.5f * (b.x1 - b.x0), hy = 0.5f * (b.y1 - b.y0);
+    const float ax = std::fmax(std::fabs(b.x0), std::fabs(b.x1)), ay = std::fmax(std::fabs(b.y0), std::fabs(b.y1));
+    CellBox r;
+    float v = m[0] * cx + m[1] * cy + m[2];
+    float h = std::fabs(m[0]) * hx + std::fabs(m[1]) * hy;
+    h += 2.0e-6f * (std::fabs(m[0]) * ax + std::fabs(m[1]) * ay + std::fabs(m[2])) + 1.0e-30f;
+    r.x0 = v - h;
+    r.x1 = v + h;
+    v = m[3] * cx + m[4] * cy + m[5];
+    h = std::fabs(m[3]) * hx + std::fabs(m[4]) * hy;
+    h += 2.0e-6f * (std::fabs(m[3]) * ax + std::fabs(m[4]) * ay + std::fabs(m[5])) + 1.0e-30f;
+    r.y0 = v - h;
+    r.y1 = v + h;
+    return r;
+}
+
+// A segment's winding contribution over a box: base + start [py > y(0)] - end [py > y(1)] for
+// rows farther than `tol` from y(0) (if start), y(1) (if end) and ext[0 .. ne).
+// Each of the nc parabolas adds its sign where px < c0 + (c1 + c2 v) v - band, v = py - yc with yc
+// the middle of the box's rows, and nothing where px > c0 + (c1 + c2 v) v + band.
+struct CellCurve {
+    float c0, c1, c2, band;
+    int sign;
+};
+struct CellSeg {
+    int base, start, end, ne, nc;
+    float ext[2];
+    CellCurve curve[3];
+    float tol;
+    int twice;  // the crate counts each crossing twice
+};
+DVG_CC_HD double cc_polyd(float a, float b, float c, float d, double t) {
+    return (((double)a * t + (double)b) * t + (double)c) * t + (double)d;
+}
+DVG_CC_HD float cc_row_centre(CellBox b) { return 0.5f * (b.y0 + b.y1); }
+// The parabola through the piece's points at u0, the middle and v1 (y monotone between them).
+DVG_CC_HD bool cell_curve(float a, float b, float c, float d, float ax, float bx, float cx, float dx, float u0, float v1,
+                          float T, CellBox box, CellCurve* r) {
+    const float yc = cc_row_centre(box);
+    const double t1 = 0.5 * ((double)u0 + (double)v1);
+    const double y0 = cc_polyd(a, b, c, d, u0) - (double)yc, y1 = cc_polyd(a, b, c, d, t1) - (double)yc,
+                 y2 = cc_polyd(a, b, c, d, v1) - (double)yc;
+    const double x0 = cc_polyd(ax, bx, cx, dx, u0), x1 = cc_polyd(ax, bx, cx, dx, t1), x2 = cc_polyd(ax, bx, cx, dx, v1);
+    const double d01 = (x1 - x0) / (y1 - y0), d12 = (x2 - x1) / (y2 - y1);
+    const double g = (d12 - d01) / (y2 - y0);
+    const double be = d01 - g * (y0 + y1), al = x0 - (be + g * y0) * y0;
+    r->c0 = (float)al;
+    r->c1 = (float)be;
+    r->c2 = (float)g;
+    // third derivative of X - be Y - g Y^2 over the bracket (Y relative to yc)
+    const float H = 0.5f * (v1 - u0), tm = (float)t1;
+    const float yb = std::fmax(std::fabs((float)y0), std::fabs((float)y2));
+    const float d3 = 6.0f * std::fabs(a), d2 = std::fabs(6.0f * a * tm + 2.0f * b) + d3 * H;
+    const float d1 = std::fabs((3.0f * a * tm + 2.0f * b) * tm + c) + d2 * H;
+    const float fb = std::fabs(r->c1), fg = std::fabs(r->c2);
+    const float R3 = 6.0f * std::fabs(ax) + fb * d3 + fg * (2.0f * yb * d3 + 6.0f * d1 * d2);
+    const float fit = 0.0642f * H * H * H * R3 * 1.01f;
+    const float slope = fb + 2.0f * fg * yb;
+    r->band = fit + T * (1.0f + slope) + 1.0e-6f * (std::fabs(r->c0) + fb * yb + fg * yb * yb);
+    // worth it while most of the box lies outside the band
+    return r->band < 0.25f * (box.x1 - box.x0);  // (NaN: no)
+}
+// Fills *r for a segment (kind 0 line, 1 quadratic, 2 cubic; q: four control points, lines and
+// quadratics repeat their last one), or returns false: test it per sample.
+DVG_CC_HD bool cell_winding(int kind, const float* q, CellBox bx, CellSeg* r) {
+    r->base = r->start = r->end = r->ne = r->nc = r->twice = 0;
+    const float m = std::fmax(std::fmax(cc_max8(q), std::fmax(std::fabs(bx.x0), std::fabs(bx.x1))),
+                              std::fmax(std::fabs(bx.y0), std::fabs(bx.y1)));
+    if (!(m < 1.0e6f)) return false;  // also NaN and infinities
+    const float M1 = 1.0e-3f * (1.0f + m), M = 1.0e-4f * (1.0f + m);
+    r->tol = 1.0e-5f * (1.0f + m);
+    const float ymin = std::fmin(std::fmin(q[1], q[3]), std::fmin(q[5], q[7]));
+    const float ymax = std::fmax(std::fmax(q[1], q[3]), std::fmax(q[5], q[7]));
+    const float xmin = std::fmin(std::fmin(q[0], q[2]), std::fmin(q[4], q[6]));
+    const float xmax = std::fmax(std::fmax(q[0], q[2]), std::fmax(q[4], q[6]));
+    if (bx.y1 < ymin - M1 || bx.y0 > ymax + M1 || bx.x0 > xmax + M1) return true;
+    const bool hull_right = xmin > bx.x1 + M;
+    const float lo = bx.y0 - M, hi = bx.y1 + M;
+    // power coefficients of y(t) and x(t), as the crate forms them
+    float a = 0.0f, b = 0.0f, c, d = q[1], ax = 0.0f, bxc = 0.0f, cx, dx = q[0];
+    if (kind == 0) {
+        c = q[3] - q[1];
+        cx = q[2] - q[0];
+    } else if (kind == 1) {
+        b = q[1] - 2.0f * q[3] + q[5];
+        c = -2.0f * q[1] + 2.0f * q[3];
+        bxc = q[0] - 2.0f * q[2] + q[4];
+        cx = -2.0f * q[0] + 2.0f * q[2];
+    } else {
+        a = -q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7];
+        b = 3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5];
+        c = -3.0f * q[1] + 3.0f * q[3];
+        ax = -q[0] + 3.0f * q[2] - 3.0f * q[4] + q[6];
+        bxc = 3.0f * q[0] - 6.0f * q[2] + 3.0f * q[4];
+        cx = -3.0f * q[0] + 3.0f * q[2];
+        if (std::fabs(a) < 0.9e-6f) {
+            a = 0.0f;  // the crate solves the quadratic
+            // ... and below 1e-12 the linear equation, whose root its quadratic solver returns twice
+            r->twice = std::fabs(b) < 1.0e-12f ? 1 : 0;
+        } else {
+            const float dm = std::fmax(std::fabs(d - bx.y0), std::fabs(d - bx.y1));
+            const float k = std::fmax(std::fmax(std::fabs(b), std::fabs(c)), dm);
+            if (!(std::fabs(a) > 1.1e-6f && k <= 64.0f * std::fabs(a))) return false;
+        }
+    }
+    // extrema of y in (0, 1): roots of 3a t^2 + 2b t + c
+    float e1 = 2.0f, e2 = 2.0f;
+    const float disc = b * b - 3.0f * a * c;
+    if (a != 0.0f) {
+        const float ti = -b / (3.0f * a);
+        if (ti > -0.05f && ti < 1.05f && !(std::fabs(disc) >= 3.0f * std::fabs(a) * M)) return false;
+    }
+    if (disc > 0.0f) {
+        const float s = -(b + (b < 0.0f ? -std::sqrt(disc) : std::sqrt(disc)));
+        if (a != 0.0f) e1 = s / (3.0f * a);
+        if (s != 0.0f) e2 = c / s;
+        if (!(e1 > 0.0f && e1 < 1.0f)) e1 = 2.0f;
+        if (!(e2 > 0.0f && e2 < 1.0f)) e2 = 2.0f;
+        if (e2 < e1) {
+            const float t = e1;
+            e1 = e2;
+            e2 = t;
+        }
+    }
+    float t0 = 0.0f, l0 = d;
+    for (int i = 0; i < 3; ++i) {
+        const float te = i == 0 ? e1 : (i == 1 ? e2 : 1.0f);
+        if (te > 1.0f) continue;  // no such extremum
+        const float ts = t0, t1 = te, ls = l0;
+        // an extremum's level in f64: the sample rows are compared with it
+        const float l1 = i == 2 ? q[7]
+                                : (float)((((double)a * (double)te + (double)b) * (double)te + (double)c) * (double)te +
+                                          (double)d);
+        t0 = t1;
+        l0 = l1;
+        if (std::fmax(ls, l1) < lo || std::fmin(ls, l1) > hi) continue;
+        const bool up = l1 > ls;
+        const bool in0 = ls >= lo && ls <= hi, in1 = l1 >= lo && l1 <= hi;
+        if (!hull_right) {
+            // the parameter range inside the rows: a piece end, or the outer end of a bracket
+            // around the row limit that the piece crosses
+            float u0 = ts, u1 = in0 ? ts : t1, v0 = in1 ? t1 : ts, v1 = t1;
+            const float lin = up ? lo : hi, lout = up ? hi : lo;
+            for (int it = 0; it < 11; ++it) {
+                const float tu = 0.5f * (u0 + u1), tv = 0.5f * (v0 + v1);
+                const float yu = cc_poly(a, b, c, d, tu), yv = cc_poly(a, b, c, d, tv);
+                if ((yu < lin) == up) u0 = tu; else u1 = tu;
+                if ((yv < lout) == up) v0 = tv; else v1 = tv;
+            }
+            if (in0) u0 = ts;
+            if (in1) v1 = t1;
+            const float tm = 0.5f * (u0 + v1), h = 0.5f * (v1 - u0) + 1.0e-6f;
+            const float x = cc_poly(ax, bxc, cx, dx, tm);
+            const float dxx = (3.0f * ax * tm + 2.0f * bxc) * tm + cx, ddx = 6.0f * ax * tm + 2.0f * bxc;
+            const float rx = ((std::fabs(ax) * h + 0.5f * std::fabs(ddx)) * h + std::fabs(dxx)) * h * 1.0001f;
+            if (x + rx < bx.x0 - M) continue;
+            if (!(x - rx > bx.x1 + M)) {
+                if (in0 || in1 ||
+                    !cell_curve(a, b, c, d, ax, bxc, cx, dx, u0, v1, r->tol, bx, &r->curve[r->nc]))
+                    return false;
+                r->curve[r->nc++].sign = up ? 1 : -1;
+                continue;
+            }
+        }
+        // [py > ls] - [py > l1]; an extremum's two halves cancel
+        if (in0) {
+            if (i == 0 || ts == 0.0f) r->start = 1;
+        } else if (ls < lo) {
+            r->base += 1;
+        }
+        if (in1) {
+            if (i == 2) r->end = 1;
+            else r->ext[r->ne++] = l1;
+        } else if (l1 < lo) {
+            r->base -= 1;
+        }
+    }
+    return true;
+}
+
+// Lower bound on the distance from (px, py) to a segment: the distance to its n-chord polyline
+// less the chord deviation, (1 / (8 n^2)) max|B''| (16 chords; a line is its own chord).
+DVG_CC_HD float cell_dist_lower(int kind, const float* q, float px, float py) {
+    const int n = kind == 0 ? 1 : 16;
+    const float ex = kind == 0 ? q[2] : (kind == 1 ? q[4] : q[6]), ey = kind == 0 ? q[3] : (kind == 1 ? q[5] : q[7]);
+    float ax = 0.0f, ay = 0.0f, bx = 0.0f, by = 0.0f, cx, cy, dev = 0.0f;
+    if (kind == 0) {
+        cx = q[2] - q[0];
+        cy = q[3] - q[1];
+    } else if (kind == 1) {
+        bx = q[0] - 2.0f * q[2] + q[4];
+        by = q[1] - 2.0f * q[3] + q[5];
+        cx = 2.0f * (q[2] - q[0]);
+        cy = 2.0f * (q[3] - q[1]);
+        dev = (1.0f / 1024.0f) * std::sqrt(bx * bx + by * by);  // |B''| = 2 |b|
+    } else {
+        ax = -q[0] + 3.0f * q[2] - 3.0f * q[4] + q[6];
+        ay = -q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7];
+        bx = 3.0f * q[0] - 6.0f * q[2] + 3.0f * q[4];
+        by = 3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5];
+        cx = 3.0f * (q[2] - q[0]);
+        cy = 3.0f * (q[3] - q[1]);
+        const float s0x = q[0] - 2.0f * q[2] + q[4], s0y = q[1] - 2.0f * q[3] + q[5];
+        const float s1x = q[2] - 2.0f * q[4] + q[6], s1y = q[3] - 2.0f * q[5] + q[7];
+        dev = (3.0f / 1024.0f) * std::sqrt(std::fmax(s0x * s0x + s0y * s0y, s1x * s1x + s1y * s1y));
+    }
+    float best = INFINITY, vx = q[0] - px, vy = q[1] - py;
+    const float step = 1.0f / (float)n;
+    for (int k = 1; k <= n; ++k) {
+        const float t = (float)k * step;
+        const float wx = (k == n ? ex : cc_poly(ax, bx, cx, q[0], t)) - px;
+        const float wy = (k == n ? ey : cc_poly(ay, by, cy, q[1], t)) - py;
+        const float dx = wx - vx, dy = wy - vy, ee = dx * dx + dy * dy, de = -(vx * dx + vy * dy);
+        float d2;
+        if (de <= 0.0f || ee <= 0.0f) d2 = vx * vx + vy * vy;
+        else if (de >= ee) d2 = wx * wx + wy * wy;
+        else d2 = std::fmax(vx * vx + vy * vy - de * (de / ee), 0.0f);
+        best = std::fmin(best, d2);
+        vx = wx;
+        vy = wy;
+    }
+    return std::sqrt(best) - dev;
+}
+// Whether every point of the box is farther than r from the segment's control hull (hull_only)
+// or curve, by the culling margin of the per-sample tests; NaN: no.
+DVG_CC_HD bool cell_far(int kind, const float* q, float r, CellBox b, bool hull_only) {
+    const float m = std::fmax(std::fmax(cc_max8(q), std::fmax(std::fabs(b.x0), std::fabs(b.x1))),
+                              std::fmax(std::fabs(b.y0), std::fabs(b.y1)));
+    if (!(m < 1.0e6f)) return false;
+    const float rm = r + 1.0e-3f * (1.0f + m) + 1.0e-5f * std::fabs(r);
+    const float xmin = std::fmin(std::fmin(q[0], q[2]), std::fmin(q[4], q[6]));
+    const float xmax = std::fmax(std::fmax(q[0], q[2]), std::fmax(q[4], q[6]));
+    const float ymin = std::fmin(std::fmin(q[1], q[3]), std::fmin(q[5], q[7]));
+    const float ymax = std::fmax(std::fmax(q[1], q[3]), std::fmax(q[5], q[7]));
+    if (b.x1 < xmin - rm || b.x0 > xmax + rm || b.y1 < ymin - rm || b.y0 > ymax + rm) return true;
+    if (hull_only) return false;
+    const float hx = 0.5f * (b.x1 - b.x0), hy = 0.5f * (b.y1 - b.y0);
+    const float hd = std::sqrt(hx * hx + hy * hy) * 1.00001f;
+    return cell_dist_lower(kind, q, 0.5f * (b.x0 + b.x1), 0.5f * (b.y0 + b.y1)) > rm + hd;
+}
+
+}  // namespace dvgb

@@ -102,6 +102,10 @@ struct DevScene {
     int tiles_x, tiles_y;
     const int* tile_offsets;
     const int* tile_entries;
+    // per-cell lists (cells.cuh); NULL: not built
+    const int2* cell_info;
+    const int4* cell_entries;
+    const int4* cell_items;
 };
 
 // ------------------------------------------------------------------ small math
@@ -1434,9 +1438,10 @@ static __device__ void d_gradient_paint_warp(const DevScene& S, const GradPtrs& 
 
 // ------------------------------------------------------------------ filtered splat / gather
 // Adds the sample's premultiplied colour times the filter weight (and the weight)
-// to every pixel of its (2*ri+1)^2 footprint: into the CTA's shared tile+halo
-// accumulator when it fits, else straight to global memory.
-__device__ __forceinline__ void splat_sample(const DevScene& S, int x, int y, int tx, int ty, int ri, int HW,
+// to every pixel of its (2*ri+1)^2 footprint: into the CTA's shared accumulator (its
+// pixels and their halo, origin (ox, oy), HW pixels wide) when it fits, else straight to
+// global memory.
+__device__ __forceinline__ void splat_sample(const DevScene& S, int x, int y, int ox, int oy, int ri, int HW,
                                              bool use_sm, float2 pt, float4 acc, float* sm, float* accum,
                                              float* wsum) {
     for (int dy = -ri; dy <= ri; ++dy)
@@ -1446,7 +1451,7 @@ __device__ __forceinline__ void splat_sample(const DevScene& S, int x, int y, in
             float w = filter_weight(S.filter_type, S.filter_radius, (float)xx + 0.5f - pt.x, (float)yy + 0.5f - pt.y);
             if (!(w > 0.0f)) continue;
             if (use_sm) {
-                int li = (yy - (ty * TILE - ri)) * HW + (xx - (tx * TILE - ri));
+                int li = (yy - oy) * HW + (xx - ox);
                 float* c = sm + 5 * li;
                 atomicAdd(c + 0, acc.x * w);
                 atomicAdd(c + 1, acc.y * w);
@@ -1463,13 +1468,13 @@ __device__ __forceinline__ void splat_sample(const DevScene& S, int x, int y, in
             }
         }
 }
-// Flushes the CTA's tile+halo accumulator to global memory (one atomic per value).
-__device__ __forceinline__ void flush_splat(const DevScene& S, int tx, int ty, int ri, int HW, const float* sm,
-                                            float* accum, float* wsum) {
+// Flushes the CTA's pixels+halo accumulator (origin (ox, oy)) to global memory (one atomic per value).
+__device__ __forceinline__ void flush_splat(const DevScene& S, int ox, int oy, int HW, const float* sm, float* accum,
+                                            float* wsum) {
     for (int i = threadIdx.x; i < HW * HW; i += blockDim.x) {
         const float* c = sm + 5 * i;
         if (c[4] == 0.0f) continue;
-        int xx = tx * TILE - ri + i % HW, yy = ty * TILE - ri + i / HW;
+        int xx = ox + i % HW, yy = oy + i / HW;
         if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
         size_t p = (size_t)yy * S.width + xx;
         atomicAdd(accum + 4 * p + 0, c[0]);

@@ -13,6 +13,7 @@
 // Built with -fmad=false (see device.cuh).
 #include <algorithm>
 
+#include "cells.cuh"
 #include "device.cuh"
 #include "kernels.cuh"
 
@@ -180,65 +181,66 @@ __global__ void __launch_bounds__(256) k_bin_write(DevScene S, const float4* g_b
 }
 
 // ------------------------------------------------------------------ forward
-// One CTA = one 16x16 tile at one sub-sample (sx, sy); thread = pixel.  Every
-// thread of the CTA walks the same group list, so group data loads are uniform.
+// One CTA = 256 samples of one 16x16 tile.  Pixels are numbered cell by cell (pix_xy), so a
+// warp's samples share one cell list (or two): entry loads are uniform.  When the CTA's
+// samples lie in one cell (layout 1, spp a power of two from 16 to 256), its splat
+// accumulator covers that cell and its halo only.
 __device__ __forceinline__ void forward_body(const DevScene& S, const SampleParams& sp, int tile, int round,
                                              float* accum, float* wsum, float* sm) {
     const int ri = S.filter_ri;
-    const int HW = TILE + 2 * ri;
     const bool use_sm = ri <= MAX_SMEM_RI;
     const int tx = tile % S.tiles_x, ty = tile / S.tiles_x;
     const int spp = sp.sxn * sp.syn;
     const int s_in_tile = round * 256 + (int)threadIdx.x;
     const int pix = sp.layout ? s_in_tile / spp : (int)threadIdx.x, sub = sp.layout ? s_in_tile % spp : round;
-    const int x = tx * TILE + (pix % TILE), y = ty * TILE + (pix / TILE);
+    const int2 pxy = pix_xy(pix);
+    const int x = tx * TILE + pxy.x, y = ty * TILE + pxy.y;
+    const bool one_cell = sp.layout && spp >= 16 && 256 % spp == 0;
+    const int HW = (one_cell ? CELL : TILE) + 2 * ri;
+    const int ox = (one_cell ? x & ~(CELL - 1) : tx * TILE) - ri, oy = (one_cell ? y & ~(CELL - 1) : ty * TILE) - ri;
     if (use_sm)
         for (int i = threadIdx.x; i < HW * HW * 5; i += blockDim.x) sm[i] = 0.0f;
     __syncthreads();
-    const int off = S.tile_offsets[tile];
-    const int n = S.tile_offsets[tile + 1] - off;
-    const int* list = S.tile_entries + off;
     if (x < S.width && y < S.height) {
         const int sx = sub % sp.sxn, sy = sub / sp.sxn;
         const float2 pt = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, S.width, sp.seed, sp.jitter);
+        const CellWalk walk = cell_walk(S, tile, cell_of_pix(pix));
         // Fragment cache (see SampleParams): kept only where the interior pass, which
         // normalises the sample point by the canvas size and scales it back
         // (src/backward/render.rs:111, src/backward/sampling.rs:91), tests the same point.
         const size_t fstride = (size_t)S.tiles_x * S.tiles_y * spp * 256;
         const size_t sid = ((size_t)tile * spp + round) * 256 + threadIdx.x;
-        const bool cache = sp.frag != nullptr && n <= FRAG_MAX_ENTRIES &&
+        const bool cache = sp.frag != nullptr &&
+                           S.tile_offsets[tile + 1] - S.tile_offsets[tile] <= FRAG_MAX_ENTRIES &&
                            (pt.x / (float)S.width) * (float)S.width == pt.x &&
                            (pt.y / (float)S.height) * (float)S.height == pt.y;
         int nf = 0;
         float4 acc = background_premul(S, y * S.width + x);
-        for (int e = 0; e < n; ++e) {
-            const int g = __ldg(&list[e]);
+        for (int k = 0; k < walk.n; ++k) {
             // stroke first, then fill; one paint call site for both
-            const int4 gi = __ldg(&S.g_info[g]);
-            const float2 lp = xf9(S.g_c2s + 9 * g, pt);
-            int hitp[2];
-            hitp[0] = gi.y >= 0 && group_within(S, g, lp) ? gi.y : -1;
-            hitp[1] = gi.x >= 0 && group_inside(S, g, lp, gi.z) ? gi.x : -1;
+            const int4 A = cell_entry(S, walk, k);
+            bool hit[2];
+            cell_hits(S, walk, k, A, pt, &hit[0], &hit[1]);
 #pragma unroll 1
             for (int which = 0; which < 2; ++which)
-                if (hitp[which] >= 0) {
-                    over(acc, paint_color(S, hitp[which], pt));
+                if (which ? hit[1] : hit[0]) {
+                    over(acc, paint_color(S, which ? A.z : A.w, pt));
                     if (cache) {
-                        if (nf < sp.frag_slots) sp.frag[(size_t)nf * fstride + sid] = (uint16_t)(2 * e + which);
+                        if (nf < sp.frag_slots) sp.frag[(size_t)nf * fstride + sid] = (uint16_t)(2 * (A.x >> 8) + which);
                         ++nf;
                     }
                 }
         }
         if (sp.frag) sp.frag_n[sid] = cache && nf <= sp.frag_slots ? (uint8_t)nf : FRAG_NONE;
-        splat_sample(S, x, y, tx, ty, ri, HW, use_sm, pt, acc, sm, accum, wsum);
+        splat_sample(S, x, y, ox, oy, ri, HW, use_sm, pt, acc, sm, accum, wsum);
     }
     if (!use_sm) return;
     __syncthreads();
-    flush_splat(S, tx, ty, ri, HW, sm, accum, wsum);
+    flush_splat(S, ox, oy, HW, sm, accum, wsum);
 }
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k_forward(DevScene S, SampleParams sp, float* accum, float* wsum,
-                                                       unsigned* status) {
+__global__ void __launch_bounds__(256, MINB) k_forward(const __grid_constant__ DevScene S, SampleParams sp, float* accum,
+                                                       float* wsum, unsigned* status) {
     extern __shared__ float sm[];
     (void)status;
     forward_body(S, sp, sp.tile_base + blockIdx.x, blockIdx.y, accum, wsum, sm);
@@ -317,7 +319,8 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
     const int spp = sp.sxn * sp.syn;
     const int s_in_tile = round * 256 + (int)threadIdx.x;
     const int pix = sp.layout ? s_in_tile / spp : (int)threadIdx.x, sub = sp.layout ? s_in_tile % spp : round;
-    const int x = tx * TILE + (pix % TILE), y = ty * TILE + (pix / TILE);
+    const int2 pxy = pix_xy(pix);
+    const int x = tx * TILE + pxy.x, y = ty * TILE + pxy.y;
     const size_t fstride = (size_t)S.tiles_x * S.tiles_y * spp * 256;
     const size_t sid = ((size_t)tile * spp + round) * 256 + threadIdx.x;
     const bool inside = x < S.width && y < S.height;
@@ -325,9 +328,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
     const bool valid = inside && (LEAN ? cn != (int)FRAG_NONE : cn == (int)FRAG_NONE);
     if (!__syncthreads_or(valid)) return;  // uniform per CTA
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int off = S.tile_offsets[tile];
-    const int n = S.tile_offsets[tile + 1] - off;
-    const int* list = S.tile_entries + off;
+    const int* list = S.tile_entries + S.tile_offsets[tile];
     const int W = S.width, H = S.height;
 
     float2 ps = make_float2(0.0f, 0.0f), pt = make_float2(0.0f, 0.0f);
@@ -350,8 +351,10 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
     float4 acc = bg;
     if (valid) {
         // Either the forward's cached fragment codes (one fragment per step) or the
-        // tile's group list with both hit tests (up to two fragments per step).
-        const int steps = LEAN ? cn : n;
+        // cell's entries with both hit tests (up to two fragments per step).
+        CellWalk walk{};
+        if constexpr (!LEAN) walk = cell_walk(S, tile, cell_of_pix(pix));
+        const int steps = LEAN ? cn : walk.n;
         for (int k = 0; k < steps; ++k) {
             int e, hitp[2];
             if constexpr (LEAN) {
@@ -361,12 +364,12 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
                 hitp[0] = (c0 & 1) ? -1 : gi.y;
                 hitp[1] = (c0 & 1) ? gi.x : -1;
             } else {
-                e = k;
-                const int g = __ldg(&list[e]);
-                const int4 gi = __ldg(&S.g_info[g]);
-                const float2 lp = xf9(S.g_c2s + 9 * g, pt);
-                hitp[0] = gi.y >= 0 && group_within(S, g, lp) ? gi.y : -1;
-                hitp[1] = gi.x >= 0 && group_inside(S, g, lp, gi.z) ? gi.x : -1;
+                const int4 A = cell_entry(S, walk, k);
+                bool st, fi;
+                cell_hits(S, walk, k, A, pt, &st, &fi);
+                e = A.x >> 8;
+                hitp[0] = st ? A.w : -1;
+                hitp[1] = fi ? A.z : -1;
             }
 #pragma unroll 1
             for (int which = 0; which < 2; ++which) {
@@ -503,7 +506,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
     }
 }
 
-__global__ void __launch_bounds__(256, DVG_MINB_INT) k_interior(DevScene S, SampleParams sp, const float* d_render,
+__global__ void __launch_bounds__(256, DVG_MINB_INT) k_interior(const __grid_constant__ DevScene S, SampleParams sp, const float* d_render,
                                                                 const float* wsum, GradPtrs G, unsigned* status) {
     interior_body<false>(S, sp, sp.tile_base + blockIdx.x, blockIdx.y, d_render, wsum, G, status);
 }
@@ -535,32 +538,34 @@ __global__ void __launch_bounds__(256, DVG_MINB_LEAN) k_interior_cached_batch(co
 }
 
 // ------------------------------------------------------------------ boundary sampling
+// The queried shape's own tests, out of line (run where no fragment decides the hit).
+static __device__ __noinline__ bool within_shape_any(const DevScene& S, int s, float2 lp, float r) {
+    return within_shape(S, s, lp, r);
+}
+static __device__ __noinline__ int winding_shape_any(const DevScene& S, int s, float2 sp) {
+    return winding_shape(S, s, sp, true);
+}
 // sample_color with an EdgeQuery (sampling.rs:76-224, 485-552) at canvas point pt.
 // Returns the un-premultiplied colour (or the premultiplied background when no
 // fragment covers pt) and whether the queried shape is the visible boundary.
-__device__ float4 edge_color(const DevScene& S, int tile, float2 pt, float4 bg, int eq_group, int eq_shape,
+__device__ float4 edge_color(const DevScene& S, int tile, int cell, float2 pt, float4 bg, int eq_group, int eq_shape,
                              bool* hit_out) {
-    const int off = S.tile_offsets[tile];
-    const int n = S.tile_offsets[tile + 1] - off;
-    const int* list = S.tile_entries + off;
+    const CellWalk walk = cell_walk(S, tile, cell);
     float4 acc = bg;
     int nfrag = 0, ev = 0;  // ev: 0 none, 1 last event sets the hit, 2 last event clears it
-    for (int e = 0; e < n; ++e) {
-        const int g = __ldg(&list[e]);
+    for (int k = 0; k < walk.n; ++k) {
         // stroke first, then fill; one paint call site for both
-        const int4 gi = __ldg(&S.g_info[g]);
-        const float2 lp = xf9(S.g_c2s + 9 * g, pt);
-        int hitp[2];
-        hitp[0] = gi.y >= 0 && group_within(S, g, lp) ? gi.y : -1;
-        hitp[1] = gi.x >= 0 && group_inside(S, g, lp, gi.z) ? gi.x : -1;
+        const int4 A = cell_entry(S, walk, k);
+        bool hit[2];
+        cell_hits(S, walk, k, A, pt, &hit[0], &hit[1]);
 #pragma unroll 1
         for (int which = 0; which < 2; ++which) {
-            if (hitp[which] < 0) continue;
-            const float4 c = paint_color(S, hitp[which], pt);
+            if (!(which ? hit[1] : hit[0])) continue;
+            const float4 c = paint_color(S, which ? A.z : A.w, pt);
             over(acc, c);
             ++nfrag;
             if (c.w >= 1.0f) ev = 2;
-            if (g == eq_group) ev = 1;
+            if (A.y == eq_group) ev = 1;
         }
     }
     if (ev != 0) {
@@ -572,11 +577,11 @@ __device__ float4 edge_color(const DevScene& S, int tile, float2 pt, float4 bg, 
         const float2 lp = xf9(S.g_c2s + 9 * eq_group, pt);
         if (gi.y >= 0) {
             float sw = __ldg(&S.s_stroke[eq_shape]);
-            if (sw > 0.0f && within_shape(S, eq_shape, lp, sw)) hit0 = true;
+            if (sw > 0.0f && within_shape_any(S, eq_shape, lp, sw)) hit0 = true;
         }
         if (gi.x >= 0) {
             float2 sp = shape_local_bwd(S, eq_shape, lp);
-            if (fill_hit(gi.z, winding_shape(S, eq_shape, sp, true))) hit0 = true;
+            if (fill_hit(gi.z, winding_shape_any(S, eq_shape, sp))) hit0 = true;
         }
         *hit_out = hit0;
     }
@@ -1330,10 +1335,12 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
     float4 bg = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (valid) {
         bg = background_premul(S, r.pixel);
-        const int tile = ((r.pixel / S.width) / TILE) * S.tiles_x + ((r.pixel % S.width) / TILE);
+        const int bx = r.pixel % S.width, by = r.pixel / S.width;
+        const int tile = (by / TILE) * S.tiles_x + bx / TILE;
+        const int cell = (by % TILE) / CELL * (TILE / CELL) + (bx % TILE) / CELL;
         const float o = side == 0 ? -1.0e-4f : 1.0e-4f;
         const float2 q = make_float2(r.bx + r.nx * o, r.by + r.ny * o);
-        cs = edge_color(S, tile, make_float2(q.x * W, q.y * H), bg, r.group, r.shape, &hs);
+        cs = edge_color(S, tile, cell, make_float2(q.x * W, q.y * H), bg, r.group, r.shape, &hs);
     }
     float4 co;
     co.x = __shfl_xor_sync(0xffffffffu, cs.x, 1);
@@ -1398,7 +1405,7 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
 }
 // Two threads per sample (boundary_eval_pair): launch 2 * samples threads.
 template <bool STYLED>
-__global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval(DevScene S, const BSample* samples,
+__global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval(const __grid_constant__ DevScene S, const BSample* samples,
                                                                      const int* order, const int* offsets, int tiles,
                                                                      const float* d_render, const float* wsum,
                                                                      GradPtrs G) {
@@ -1456,21 +1463,29 @@ __global__ void k_fill_background(DevScene S, float* out) {
 }
 
 // ------------------------------------------------------------------ L2 loss
-__global__ void k_l2(const float* img, const float* target, size_t n, float* d_render, float* loss) {
-    __shared__ float red[8];
-    float s = 0.0f;
+// Block sums are added in f64 (acc, zeroed before the launch) and the last block rounds the
+// total once: an f32 accumulator rounds at every block's addition, in whatever order they come.
+__global__ void k_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, L2Acc* acc) {
+    __shared__ double red[8];
+    double s = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float d = img[i] - target[i];
         d_render[i] = 2.0f * d;
-        s += d * d;
+        s += (double)(d * d);
     }
-    s = warp_sum(s);
+    if (!loss) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x == 0 && loss) {
-        float t = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-        atomicAdd(loss, t);
+    if (threadIdx.x != 0) return;
+    double t = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+    atomicAdd(&acc->sum, t);
+    __threadfence();
+    if (atomicAdd(&acc->done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        *loss = (float)atomicAdd(&acc->sum, 0.0);
     }
 }
 
@@ -1696,11 +1711,13 @@ int launch_fill_background(const DevScene& S, float* out, cudaStream_t stream) {
     k_fill_background<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(S, out);
     return 1;
 }
-int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, cudaStream_t stream) {
+int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, L2Acc* acc,
+              cudaStream_t stream) {
+    if (loss) cudaMemsetAsync(acc, 0, sizeof(L2Acc), stream);
     unsigned blocks = (unsigned)((n + 255) / 256);
-    if (blocks > 4096) blocks = 4096;
+    if (blocks > 1184) blocks = 1184;  // 8 per SM: the loop takes the rest
     if (blocks == 0) blocks = 1;
-    k_l2<<<blocks, 256, 0, stream>>>(img, target, n, d_render, loss);
+    k_l2<<<blocks, 256, 0, stream>>>(img, target, n, d_render, loss, acc);
     return 1;
 }
 

@@ -214,6 +214,12 @@ int launch_positions_backward(const DevScene& S, const float2* pos, uint64_t n, 
 // Linear BVH over n boxes into L (leaf_item[k] = item_map[box index], or the box
 // index without a map).
 int launch_lbvh_build(const float4* boxes, int n, const int* item_map, LbvhBufs& L, cudaStream_t stream);
-int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, cudaStream_t stream);
+// Loss accumulator (context scratch) of launch_l2.
+struct L2Acc {
+    double sum;
+    unsigned done;  // blocks that have added theirs
+};
+int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, L2Acc* acc,
+              cudaStream_t stream);
 
 }  // namespace dvgb

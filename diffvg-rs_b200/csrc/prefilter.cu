@@ -16,6 +16,7 @@
 #endif
 #include <algorithm>
 
+#include "cells.cuh"
 #include "device.cuh"
 #include "kernels.cuh"
 // Minimum resident CTAs per SM of the prefiltered forward and interior kernels, by
@@ -530,10 +531,10 @@ __device__ __forceinline__ void forward_prefilter_body(const DevScene& S, const 
         }
     }
     __syncthreads();  // the splat tile is cleared even without groups
-    if (valid) splat_sample(S, x, y, tx, ty, ri, HW, use_sm, pt, acc, sm, accum, wsum);
+    if (valid) splat_sample(S, x, y, tx * TILE - ri, ty * TILE - ri, ri, HW, use_sm, pt, acc, sm, accum, wsum);
     if (!use_sm) return;
     __syncthreads();
-    flush_splat(S, tx, ty, ri, HW, sm, accum, wsum);
+    flush_splat(S, tx * TILE - ri, ty * TILE - ri, HW, sm, accum, wsum);
 }
 // The prefiltered forward kernels and their launchers are compiled in prefilter_fwd.cu
 // (DVG_PREFILTER_FORWARD, with the crate's root formulas); everything else here.
