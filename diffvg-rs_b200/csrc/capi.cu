@@ -129,7 +129,7 @@ struct dvg_context {
     unsigned* status = nullptr;  // device word
     L2Acc* l2acc = nullptr;
     DevBuf accum, wsum, image, d_render, target, loss, bg_grad, trans_grad;
-    DevBuf bsamples, bkey, border, bcounts;  // boundary-pass scratch
+    DevBuf bsamples, bkey, border, bcounts, bsegs;  // boundary-pass scratch
     DevBuf sdf, positions, dvalues;          // signed-distance host calls
     DevBuf frag;                             // fragment cache of the fused calls
     uint64_t launches = 0;
@@ -497,6 +497,7 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
     S.num_shapes = (int)h.num_shapes;
     S.num_paints = (int)h.num_paints;
     S.num_paths = (int)h.num_paths;
+    S.num_segs = (int)(h.seg_meta.size() / 4);
     S.filter_type = (int)h.filter_type;
     S.filter_radius = h.filter_radius;
     {
@@ -727,13 +728,14 @@ static dvg_status backward_core(dvg_context* ctx, dvg_scene* sc, const dvg_rende
             const uint64_t cap = std::max<uint64_t>(std::min<uint64_t>(bp.num_samples - bp.sample_base, (uint64_t)1 << 24), 1);
             const int tiles = S.tiles_x * S.tiles_y;
             CK(ctx->bsamples.reserve(cap * sizeof(BSample)));
-            CK(ctx->bkey.reserve(cap * sizeof(int)));
-            CK(ctx->border.reserve(cap * sizeof(int)));
+            CK(ctx->bkey.reserve(cap * sizeof(int2)));
+            CK(ctx->border.reserve(2 * cap * sizeof(int)));
             CK(ctx->bcounts.reserve(bnd_count_ints((size_t)tiles) * sizeof(int)));
+            CK(ctx->bsegs.reserve(bnd_scan_ints((size_t)S.num_segs + S.num_shapes) * sizeof(int)));
+            const BoundaryScratch sc_{ctx->bsamples.as<BSample>(),   ctx->bkey.as<int2>(),    ctx->border.as<int>(),
+                                      ctx->border.as<int>() + cap,   ctx->bcounts.as<int>(), ctx->bsegs.as<int>()};
             Prof prof_(ctx, "boundary");
-            ctx->launches += launch_boundary(S, bp, d_render, wsum_now(), G, ctx->bsamples.as<BSample>(),
-                                             ctx->bkey.as<int>(), ctx->bcounts.as<int>(), ctx->border.as<int>(), cap,
-                                             ctx->stream);
+            ctx->launches += launch_boundary(S, bp, d_render, wsum_now(), G, sc_, cap, ctx->stream);
             CK(cudaGetLastError());
         }
     } else if (d_render && S.num_groups == 0) {
@@ -1218,9 +1220,9 @@ struct dvg_batch {
     std::vector<size_t> wpix_off;     // float offset of each scene's 1-channel region
     std::vector<size_t> grad_base;    // float offset of each scene's gradient block
     size_t total_pix4 = 0, total_pix = 0, total_grads = 0, max_pixels = 0;
-    int items = 0, total_tiles = 0, max_ri = 0;
+    int items = 0, total_tiles = 0, total_segs = 0, max_ri = 0;
     uint64_t total_bsamples = 0;
-    DevBuf entries, work, queue, accum, wsum, image, target, d_render, loss, grads, bsamples, bkey, border, bcounts;
+    DevBuf entries, work, queue, accum, wsum, image, target, d_render, loss, grads, bsamples, bkey, border, bcounts, bsegs;
     DevBuf frag;  // per-scene fragment caches (forward -> interior)
     bool any_styled = false;  // some scene strokes with non-round joins or caps
     cudaGraph_t graph = nullptr;
@@ -1265,11 +1267,12 @@ dvg_status batch_enqueue(dvg_batch* b) {
         ctx->launches += launch_interior_batch(B, b->work.as<int2>(), b->items, queue ? queue + 1 : nullptr,
                                                ctx->status, ctx->stream);
     if (!pre)
-        ctx->launches += launch_boundary_batch(B, n, b->total_bsamples, b->total_tiles, (int)b->tune.boundary_cell,
-                                               b->any_styled,
-                                               b->bsamples.as<BSample>(),
-                                               b->bkey.as<int>(), b->bcounts.as<int>(), b->border.as<int>(),
-                                               ctx->stream);
+        ctx->launches += launch_boundary_batch(
+            B, n, b->total_bsamples, b->total_tiles, b->total_segs, (int)b->tune.boundary_cell, b->any_styled,
+            BoundaryScratch{b->bsamples.as<BSample>(), b->bkey.as<int2>(), b->border.as<int>(),
+                            b->border.as<int>() + std::max<uint64_t>(b->total_bsamples, 1), b->bcounts.as<int>(),
+                            b->bsegs.as<int>()},
+            ctx->stream);
     ctx->launches += launch_pixels_batch(B, n, b->max_pixels, 2, ctx->stream);
     if (b->adam) {
         BatchEntry* Bm = b->entries.as<BatchEntry>();
@@ -1364,6 +1367,8 @@ extern "C" dvg_status dvg_batch_create(dvg_context* ctx, dvg_scene* const* scene
         e.item_off = b->items;
         const int tiles = S.tiles_x * S.tiles_y;
         e.tile_off = b->total_tiles;
+        e.seg_off = b->total_segs;
+        b->total_segs += S.num_segs + S.num_shapes;
         const uint64_t spp = (uint64_t)sp.sxn * sp.syn;
         e.nb = b->bopts.boundary_samples ? b->bopts.boundary_samples : (uint64_t)npix * spp;
         // (scenes without boundary tables draw no samples: the generator checks the flag,
@@ -1396,8 +1401,9 @@ extern "C" dvg_status dvg_batch_create(dvg_context* ctx, dvg_scene* const* scene
     CK(b->work.reserve(work2.size() * sizeof(int2)));
     const uint64_t nbs = std::max<uint64_t>(b->total_bsamples, 1);
     CK(b->bsamples.reserve(nbs * sizeof(BSample)));
-    CK(b->bkey.reserve(nbs * sizeof(int)));
-    CK(b->border.reserve(nbs * sizeof(int)));
+    CK(b->bkey.reserve(nbs * sizeof(int2)));
+    CK(b->border.reserve(2 * nbs * sizeof(int)));
+    CK(b->bsegs.reserve(bnd_scan_ints((size_t)b->total_segs) * sizeof(int)));
     CK(b->bcounts.reserve(bnd_count_ints((size_t)b->total_tiles) * sizeof(int)));
     CK(cudaMemsetAsync(b->target.ptr, 0, b->total_pix4 * sizeof(float), ctx->stream));
     float* acc = b->accum.as<float>();

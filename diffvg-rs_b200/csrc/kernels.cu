@@ -1213,9 +1213,10 @@ __device__ void accumulate_boundary(const DevScene& S, const GradPtrs& G, int sh
 // Boundary pass, stage 1: draw every edge sample (boundary.rs:141-175), keep
 // the valid ones with the tile of their boundary pixel as sort key.
 __device__ __forceinline__ void boundary_gen_one(const DevScene& S, uint64_t idx, uint64_t slot, uint32_t seed,
-                                                 int rng_kind, int tile_off, int scene, int cell, float pdf_scale,
-                                                 BSample* out, int* key, int* tile_counts) {
-    key[slot] = -1;
+                                                 int rng_kind, int tile_off, int seg_off, int scene, int cell,
+                                                 float pdf_scale, BSample* out, int2* key, int* tile_counts,
+                                                 int* seg_counts) {
+    key[slot] = make_int2(-1, -1);
     float u, t;
     if (rng_kind == 1) {
         uint4 r = philox4x32_10(make_uint4((uint32_t)idx, (uint32_t)(idx >> 32), 0u, 0u), make_uint2(seed, 0u));
@@ -1280,21 +1281,27 @@ __device__ __forceinline__ void boundary_gen_one(const DevScene& S, uint64_t idx
     const int cls = (bd.is_stroke ? 2 : 0) + (__ldg(&S.s_info[shape]).x == K_PATH ? 1 : 0);
     const int bucket =
         (tile * (per_row * per_row) + ((by % TILE) / cell) * per_row + (bx % TILE) / cell) * BND_CLASSES + cls;
-    key[slot] = bucket;
+    // second bucket: the path segment, or the shape, whose parameters the sample's gradient goes to
+    const int4 si = __ldg(&S.s_info[shape]);
+    const int2 ps = si.x == K_PATH && si.z >= 0 ? make_int2(__ldg(&S.p_info[2 * si.z].x), __ldg(&S.p_info[2 * si.z].y))
+                                                : make_int2(0, 0);
+    const int seg = bd.base_point_id >= 0 && bd.base_point_id < ps.y ? ps.x + bd.base_point_id : S.num_segs + shape;
+    key[slot] = make_int2(bucket, seg_off + seg);
     atomicAdd(tile_counts + bucket, 1);
+    atomicAdd(seg_counts + seg_off + seg, 1);
 }
-__global__ void __launch_bounds__(256) k_boundary_gen(DevScene S, BoundaryParams bp, BSample* out, int* key,
-                                                      int* tile_counts) {
+__global__ void __launch_bounds__(256) k_boundary_gen(const __grid_constant__ DevScene S, BoundaryParams bp, BSample* out,
+                                                      int2* key, int* tile_counts, int* seg_counts) {
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x + bp.sample_base;
     if (idx >= bp.num_samples) return;
-    boundary_gen_one(S, idx, idx - bp.slot_base, bp.seed, bp.rng, 0, 0, bp.cell, bp.pdf_scale, out, key,
-                     tile_counts);
+    boundary_gen_one(S, idx, idx - bp.slot_base, bp.seed, bp.rng, 0, 0, 0, bp.cell, bp.pdf_scale, out, key,
+                     tile_counts, seg_counts);
 }
 // Batched stage 1: one flat index over all scenes' boundary samples; the scene is
 // found by binary search over the per-scene sample offsets.
 __global__ void __launch_bounds__(256) k_boundary_gen_batch(const BatchEntry* __restrict__ B, int nscenes,
-                                                            uint64_t total, int cell, BSample* out, int* key,
-                                                            int* tile_counts) {
+                                                            uint64_t total, int cell, BSample* out, int2* key,
+                                                            int* tile_counts, int* seg_counts) {
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total) return;
     int lo = 0, hi = nscenes - 1;
@@ -1306,17 +1313,20 @@ __global__ void __launch_bounds__(256) k_boundary_gen_batch(const BatchEntry* __
             hi = mid - 1;
     }
     const BatchEntry& E = B[lo];
-    key[g] = -1;
+    key[g] = make_int2(-1, -1);
     if (!E.S.boundary_ok || g - E.b_off >= E.nb) return;
-    boundary_gen_one(E.S, g - E.b_off, g, E.bseed, E.rng, E.tile_off, lo, cell, E.bscale, out, key, tile_counts);
+    boundary_gen_one(E.S, g - E.b_off, g, E.bseed, E.rng, E.tile_off, E.seg_off, lo, cell, E.bscale, out, key,
+                     tile_counts, seg_counts);
 }
-// Stage 2: counting-sort scatter of sample slots by tile.
-__global__ void k_boundary_scatter(const int* key, uint64_t n, int* cursor, int* order) {
+// Stage 2: counting-sort scatter of sample slots, by cell and by segment.
+__global__ void k_boundary_scatter(const int2* key, uint64_t n, int* cursor, int* order, int* seg_cursor,
+                                   int* seg_order) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int k = key[i];
-    if (k < 0) return;
-    order[atomicAdd(cursor + k, 1)] = (int)i;
+    const int2 k = key[i];
+    if (k.x < 0) return;
+    order[atomicAdd(cursor + k.x, 1)] = (int)i;
+    seg_order[atomicAdd(seg_cursor + k.y, 1)] = (int)i;
 }
 // Stage 3: evaluate both sides of every edge sample in tile order, so that the
 // lanes of a warp share one group list (render_edge_sample, boundary.rs:845-967).
@@ -1324,10 +1334,12 @@ __global__ void k_boundary_scatter(const int* key, uint64_t n, int* cursor, int*
 // the colour outside.  The two points are 2e-4 of the canvas apart, so a pair walks
 // the same BVH nodes and segment tests in lockstep; the even lane receives the odd
 // lane's colour and hit by shuffle and finishes the sample alone.  Every lane of the
-// warp reaches the shuffles (`valid` false: a pair past the last sample).
-template <bool STYLED>
+// warp reaches the shuffles (`valid` false: a pair past the last sample).  The sample's
+// contribution goes back into its record (pdf), with the normal turned outwards: stage 4
+// adds it to the gradients.
 __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSample& r, bool valid,
-                                                   const float* d_render, const float* wsum, const GradPtrs& G) {
+                                                   const float* d_render, const float* wsum, float* d_translation,
+                                                   BSample* out) {
     const float W = (float)S.width, H = (float)S.height;
     const int side = threadIdx.x & 1;
     float4 cs = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -1352,9 +1364,14 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
     float2 nc = make_float2(r.nx, r.ny);
     float4 ci = cs;
     const bool hi = hs;
-    if (!hi && !ho) return;
+    if (!hi && !ho) {
+        out->pdf = 0.0f;
+        return;
+    }
     if (!hi) {
         nc = make_float2(nc.x * -1.0f, nc.y * -1.0f);
+        out->nx = nc.x;
+        out->ny = nc.y;
         float4 tmp = ci;
         ci = co;
         co = tmp;
@@ -1391,40 +1408,234 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
     }
     const float contrib =
         ((ci.x - co.x) * dc.x + (ci.y - co.y) * dc.y + (ci.z - co.z) * dc.z + (ci.w - co.w) * dc.w) / r.pdf;
-    if (!isfinite(contrib)) return;
-    BData bd;
-    bd.base_point_id = r.base_point_id;
-    bd.point_id = r.point_id;
-    bd.t = r.bt;
-    bd.is_stroke = r.is_stroke != 0;
-    accumulate_boundary<STYLED>(S, G, r.shape, r.group, contrib, r.t, nc, bd, make_float2(r.lx, r.ly));
-    if (G.d_translation) {
-        add_if(G.d_translation + 2 * (size_t)r.pixel, nc.x * contrib);
-        add_if(G.d_translation + 2 * (size_t)r.pixel + 1, nc.y * contrib);
+    out->pdf = isfinite(contrib) ? contrib : 0.0f;
+    if (d_translation && isfinite(contrib)) {
+        add_if(d_translation + 2 * (size_t)r.pixel, nc.x * contrib);
+        add_if(d_translation + 2 * (size_t)r.pixel + 1, nc.y * contrib);
     }
 }
 // Two threads per sample (boundary_eval_pair): launch 2 * samples threads.
-template <bool STYLED>
-__global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval(const __grid_constant__ DevScene S, const BSample* samples,
-                                                                     const int* order, const int* offsets, int tiles,
+__global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval(const __grid_constant__ DevScene S,
+                                                                     BSample* samples, const int* order,
+                                                                     const int* offsets, int tiles,
                                                                      const float* d_render, const float* wsum,
-                                                                     GradPtrs G) {
+                                                                     float* d_translation) {
     const int64_t i = (int64_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1);
     const bool valid = i < offsets[tiles];
     BSample r{};
-    if (valid) r = samples[order[i]];
-    boundary_eval_pair<STYLED>(S, r, valid, d_render, wsum, G);
+    const int at = valid ? order[i] : 0;
+    if (valid) r = samples[at];
+    boundary_eval_pair(S, r, valid, d_render, wsum, d_translation, samples + at);
 }
-template <bool STYLED>
 __global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval_batch(const BatchEntry* __restrict__ B,
-                                                                           const BSample* samples, const int* order,
+                                                                           BSample* samples, const int* order,
                                                                            const int* offsets, int tiles) {
     const int64_t i = (int64_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1);
     const bool valid = i < offsets[tiles];
     BSample r{};
-    if (valid) r = samples[order[i]];
+    const int at = valid ? order[i] : 0;
+    if (valid) r = samples[at];
     const BatchEntry& E = B[valid ? r.scene : 0];
-    boundary_eval_pair<STYLED>(E.S, r, valid, E.d_render, E.wsum, E.G);
+    boundary_eval_pair(E.S, r, valid, E.d_render, E.wsum, E.G.d_translation, samples + at);
+}
+
+// Stage 4: the samples' gradients (accumulate_boundary), in segment order.  A warp takes
+// ACC_SAMPLES consecutive samples, 32 at a time.  While they share a segment, group and side,
+// every lane keeps its own sums of the terms below; the sums are transposed over the warp (31
+// shuffles, lane i receives term i) and added with one atomic per parameter, instead of some
+// thirty per sample on the same few addresses.  The group's and the shape's transform gradient
+// are both linear in the nine entries of dm, so dm is what is summed.
+constexpr int ACC_SAMPLES = 128;
+enum : int { ACC_DM = 0, ACC_PTS = 9, ACC_RAD = 17, ACC_PRM = 21, ACC_TERMS = 32 };
+struct AccKey {
+    int shape, group, base_point_id, point_id, is_stroke, scene;
+    __device__ __forceinline__ bool operator==(const AccKey& o) const {
+        return shape == o.shape && group == o.group && base_point_id == o.base_point_id &&
+               point_id == o.point_id && is_stroke == o.is_stroke && scene == o.scene;
+    }
+};
+// The terms of one sample (the formulas of accumulate_boundary).
+__device__ __forceinline__ void boundary_terms(const DevScene& S, const BSample& r, float* v) {
+    const float contrib = r.pdf;
+    const float2 n = make_float2(r.nx, r.ny);
+    const int4 si = __ldg(&S.s_info[r.shape]);
+    int co = 0, pflags = 0, nc = 0;
+    const bool path = si.x == K_PATH;
+    if (path && si.z >= 0) {
+        const int4 pi2 = __ldg(&S.p_info[2 * si.z + 1]);
+        co = pi2.z;
+        pflags = pi2.w;
+    }
+    if (path) nc = r.base_point_id < __ldg(&S.path_cdf_info[r.shape].y) ? S.ncp[co + r.base_point_id] : 0;
+    const float t2 = r.bt, tt = 1.0f - t2;
+    float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (path) {
+        if (nc == 0) {
+            w[0] = 1.0f - t2;
+            w[1] = t2;
+        } else if (nc == 1) {
+            w[0] = tt * tt;
+            w[1] = 2.0f * tt * t2;
+            w[2] = t2 * t2;
+        } else if (nc == 2) {
+            w[0] = tt * tt * tt;
+            w[1] = 3.0f * tt * tt * t2;
+            w[2] = 3.0f * tt * t2 * t2;
+            w[3] = t2 * t2 * t2;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[ACC_PTS + 2 * j] += n.x * (w[j] * contrib);
+            v[ACC_PTS + 2 * j + 1] += n.y * (w[j] * contrib);
+        }
+    }
+    if (r.is_stroke) {
+        if (path && (pflags & PF_THICK)) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[ACC_RAD + j] += w[j] * contrib;
+        } else {
+            v[ACC_RAD] += contrib;
+        }
+    }
+    if (si.x == K_CIRCLE) {
+        v[ACC_PRM] += n.x * contrib;
+        v[ACC_PRM + 1] += n.y * contrib;
+        v[ACC_PRM + 2] += contrib;
+    } else if (si.x == K_ELLIPSE) {
+        const float ang = 2.0f * PI_F * r.t;
+        v[ACC_PRM] += n.x * contrib;
+        v[ACC_PRM + 1] += n.y * contrib;
+        v[ACC_PRM + 2] += dvg_cosf(ang) * n.x * contrib;
+        v[ACC_PRM + 3] += dvg_sinf(ang) * n.y * contrib;
+    } else if (si.x == K_RECT) {
+        if (n.x == -1.0f && n.y == 0.0f) v[ACC_PRM] -= contrib;
+        else if (n.x == 1.0f && n.y == 0.0f) v[ACC_PRM + 2] += contrib;
+        else if (n.x == 0.0f && n.y == -1.0f) v[ACC_PRM + 1] -= contrib;
+        else if (n.x == 0.0f && n.y == 1.0f) v[ACC_PRM + 3] += contrib;
+    }
+    float m[9];
+    mul33(S.g_s2c + 9 * r.group, S.s_xform + 9 * r.shape, m);
+    const float2 dout = make_float2(n.x * contrib, n.y * contrib);
+    const float px = r.lx, py = r.ly;
+    const float t0 = m[0] * px + m[1] * py + m[2], t1 = m[3] * px + m[4] * py + m[5], tw = m[6] * px + m[7] * py + m[8];
+    const float d0 = dout.x / tw, d1 = dout.y / tw, d2 = -(dout.x * (t0 / tw) + dout.y * (t1 / tw)) / tw;
+    const float dm[9] = {d0 * px, d0 * py, d0, d1 * px, d1 * py, d1, d2 * px, d2 * py, d2};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[ACC_DM + k] += dm[k];
+}
+// Adds the warp's sums of one key to the gradients and clears them.
+__device__ __forceinline__ void boundary_flush(const DevScene& S, const GradPtrs& G, const AccKey& k, float* v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+        for (int i = 0; i < s; ++i) {
+            const float keep = lane & s ? v[i + s] : v[i], send = lane & s ? v[i] : v[i + s];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+        }
+    const float sum = v[0];
+    float dm[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) dm[i] = __shfl_sync(0xffffffffu, sum, ACC_DM + i);
+#pragma unroll
+    for (int i = 0; i < ACC_TERMS; ++i) v[i] = 0.0f;
+    const int4 si = __ldg(&S.s_info[k.shape]);
+    int po = 0, pc = 0, pflags = 0, pid = 0, np = 0;
+    const bool path = si.x == K_PATH;
+    if (path && si.z >= 0) {
+        const int4 pi2 = __ldg(&S.p_info[2 * si.z + 1]);
+        po = pi2.x;
+        pc = pi2.y;
+        pflags = pi2.w;
+        np = 2 + (k.base_point_id < __ldg(&S.path_cdf_info[k.shape].y) ? S.ncp[pi2.z + k.base_point_id] : 0);
+        pid = k.point_id;
+    }
+    // lanes 0-17: the two transforms
+    if (lane < 18) {
+        const int o = lane < 9 ? lane : lane - 9, r = o / 3, c = o % 3;
+        const float* gs = S.g_s2c + 9 * k.group;
+        const float* sx = S.s_xform + 9 * k.shape;
+        float a = 0.0f;
+        if (lane < 9)
+            a = (r == 0 ? dm[0] : r == 1 ? dm[3] : dm[6]) * sx[3 * c] + (r == 0 ? dm[1] : r == 1 ? dm[4] : dm[7]) * sx[3 * c + 1] +
+                (r == 0 ? dm[2] : r == 1 ? dm[5] : dm[8]) * sx[3 * c + 2];
+        else
+            a = gs[r] * (c == 0 ? dm[0] : c == 1 ? dm[1] : dm[2]) + gs[3 + r] * (c == 0 ? dm[3] : c == 1 ? dm[4] : dm[5]) +
+                gs[6 + r] * (c == 0 ? dm[6] : c == 1 ? dm[7] : dm[8]);
+        add_if(lane < 9 ? G.d_group_transform + 9 * k.group + o : G.d_shape_transform + 9 * k.shape + o, a);
+    }
+    // lanes 9-24: points, radius or thickness, shape parameters
+    if (lane >= ACC_PTS && lane < ACC_RAD) {
+        const int j = (lane - ACC_PTS) >> 1;
+        if (path && j < np && pc > 0) {
+            const bool closed = pflags & PF_CLOSED;
+            const int i = closed ? (pid + j) % pc : pid + j;
+            if (i < pc) add_if(G.d_points + 2 * (po + i) + ((lane - ACC_PTS) & 1), sum);
+        }
+    } else if (lane >= ACC_RAD && lane < ACC_PRM) {
+        const int j = lane - ACC_RAD;
+        if (path && (pflags & PF_THICK)) {
+            // the last point of a closed path's segment wraps around, as the points do
+            const int i = (pflags & PF_CLOSED) && j == np - 1 ? (pid + j) % pc : pid + j;
+            if (j < np && i < pc) add_if(G.d_thickness + po + i, sum);
+        } else if (j == 0) {
+            add_if(G.d_shape_stroke_width + k.shape, sum);
+        }
+    } else if (lane >= ACC_PRM && lane < ACC_PRM + 4) {
+        add_if(G.d_shape_params + 4 * k.shape + (lane - ACC_PRM), sum);
+    }
+}
+template <bool STYLED, typename SceneOf, typename GradsOf>
+__device__ __forceinline__ void boundary_accum(const BSample* samples, const int* order, int64_t n, SceneOf&& scene,
+                                               GradsOf&& grads) {
+    const int lane = threadIdx.x & 31;
+    const int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * ACC_SAMPLES;
+    float v[ACC_TERMS];
+#pragma unroll
+    for (int i = 0; i < ACC_TERMS; ++i) v[i] = 0.0f;
+    AccKey run{-1, 0, 0, 0, 0, 0};
+#pragma unroll 1
+    for (int64_t i0 = base; i0 < base + ACC_SAMPLES && i0 < n; i0 += 32) {
+        const bool in = i0 + lane < n;
+        BSample r{};
+        if (in) r = samples[order[i0 + lane]];
+        const bool has = in && r.pdf != 0.0f;
+        const AccKey mine{r.shape, r.group, r.base_point_id, r.point_id, r.is_stroke, r.scene};
+        const unsigned m = __ballot_sync(0xffffffffu, has);
+        if (!m) continue;
+        const int l = __ffs(m) - 1;
+        const AccKey key{__shfl_sync(0xffffffffu, mine.shape, l), __shfl_sync(0xffffffffu, mine.group, l),
+                         __shfl_sync(0xffffffffu, mine.base_point_id, l), __shfl_sync(0xffffffffu, mine.point_id, l),
+                         __shfl_sync(0xffffffffu, mine.is_stroke, l), __shfl_sync(0xffffffffu, mine.scene, l)};
+        const bool join = STYLED && key.base_point_id < 0;
+        if (__all_sync(0xffffffffu, !has || mine == key) && !join) {
+            if (run.shape >= 0 && !(run == key)) boundary_flush(scene(run.scene), grads(run.scene), run, v);
+            run = key;
+            if (has) boundary_terms(scene(r.scene), r, v);
+        } else if (has) {  // the warp spans segments: each lane adds its own
+            BData bd;
+            bd.base_point_id = r.base_point_id;
+            bd.point_id = r.point_id;
+            bd.t = r.bt;
+            bd.is_stroke = r.is_stroke != 0;
+            accumulate_boundary<STYLED>(scene(r.scene), grads(r.scene), r.shape, r.group, r.pdf, r.t,
+                                        make_float2(r.nx, r.ny), bd, make_float2(r.lx, r.ly));
+        }
+    }
+    if (run.shape >= 0) boundary_flush(scene(run.scene), grads(run.scene), run, v);
+}
+template <bool STYLED>
+__global__ void __launch_bounds__(256) k_boundary_accum(const __grid_constant__ DevScene S, const BSample* samples,
+                                                        const int* order, const int* total,
+                                                        const __grid_constant__ GradPtrs G) {
+    boundary_accum<STYLED>(samples, order, *total, [&](int) -> const DevScene& { return S; },
+                           [&](int) -> const GradPtrs& { return G; });
+}
+template <bool STYLED>
+__global__ void __launch_bounds__(256) k_boundary_accum_batch(const BatchEntry* __restrict__ B, const BSample* samples,
+                                                              const int* order, const int* total) {
+    boundary_accum<STYLED>(samples, order, *total, [&](int k) -> const DevScene& { return B[k].S; },
+                           [&](int k) -> const GradPtrs& { return B[k].G; });
 }
 
 // ------------------------------------------------------------------ background finalisation (background.rs:29-61)
@@ -1601,11 +1812,29 @@ int launch_interior(const DevScene& S, const SampleParams& sp, const float* d_re
     k_interior<<<grid, 256, 0, stream>>>(S, sp, d_render, wsum, G, status);
     return sp.frag ? 2 : 1;
 }
+// Stages 2 to 4 for the n drawn samples in sc (counts filled by stage 1).
+template <typename Eval, typename Accum>
+static int boundary_stages(const BoundaryScratch& sc, uint64_t n, int tiles, int segs, cudaStream_t stream, Eval eval,
+                           Accum accum) {
+    int* offsets = sc.counts + tiles;  // tiles + 1 entries
+    int* seg_counts = sc.seg_counts;
+    int* seg_offsets = seg_counts + segs;
+    int launches = launch_scan(sc.counts, tiles, offsets, sc.counts + 2 * (size_t)tiles + 1, stream);
+    launches += launch_scan(seg_counts, segs, seg_offsets, seg_counts + 2 * (size_t)segs + 1, stream);
+    // reuse the count arrays as the scatter cursors (copies of the exclusive offsets)
+    cudaMemcpyAsync(sc.counts, offsets, sizeof(int) * (size_t)tiles, cudaMemcpyDeviceToDevice, stream);
+    cudaMemcpyAsync(seg_counts, seg_offsets, sizeof(int) * (size_t)segs, cudaMemcpyDeviceToDevice, stream);
+    k_boundary_scatter<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(sc.key, n, sc.counts, sc.order, seg_counts,
+                                                                       sc.seg_order);
+    eval(offsets, (unsigned)((2 * n + 127) / 128));
+    accum(seg_offsets + segs, (unsigned)((n + 8 * ACC_SAMPLES - 1) / (8 * ACC_SAMPLES)));
+    return launches + 3;
+}
 int launch_boundary(const DevScene& S, const BoundaryParams& bp, const float* d_render, const float* wsum,
-                    const GradPtrs& G, BSample* samples, int* key, int* counts, int* order, uint64_t capacity,
-                    cudaStream_t stream) {
+                    const GradPtrs& G, const BoundaryScratch& sc, uint64_t capacity, cudaStream_t stream) {
     const uint64_t n = bp.num_samples;  // samples [bp.sample_base, n)
     const int tiles = S.tiles_x * S.tiles_y * bnd_buckets(bp.cell);  // sort buckets
+    const int segs = S.num_segs + S.num_shapes;
     int launches = 0;
     for (uint64_t base = bp.sample_base; base < n; base += capacity) {
         const uint64_t cnt = base + capacity < n ? capacity : n - base;
@@ -1613,20 +1842,22 @@ int launch_boundary(const DevScene& S, const BoundaryParams& bp, const float* d_
         b.sample_base = base;
         b.slot_base = base;
         b.num_samples = base + cnt;
-        cudaMemsetAsync(counts, 0, sizeof(int) * (2 * (size_t)tiles + 1), stream);
-        k_boundary_gen<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(S, b, samples, key, counts);
-        int* offsets = counts + tiles;  // tiles + 1 entries
-        launches += launch_scan(counts, tiles, offsets, counts + 2 * (size_t)tiles + 1, stream);
-        // reuse the count array as the scatter cursor (a copy of the exclusive offsets)
-        cudaMemcpyAsync(counts, offsets, sizeof(int) * (size_t)tiles, cudaMemcpyDeviceToDevice, stream);
-        k_boundary_scatter<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(key, cnt, counts, order);
-        if (S.styled)
-            k_boundary_eval<true><<<(unsigned)((2 * cnt + 127) / 128), 128, 0, stream>>>(S, samples, order, offsets,
-                                                                                      tiles, d_render, wsum, G);
-        else
-            k_boundary_eval<false><<<(unsigned)((2 * cnt + 127) / 128), 128, 0, stream>>>(S, samples, order, offsets,
-                                                                                       tiles, d_render, wsum, G);
-        launches += 3;
+        cudaMemsetAsync(sc.counts, 0, sizeof(int) * (2 * (size_t)tiles + 1), stream);
+        cudaMemsetAsync(sc.seg_counts, 0, sizeof(int) * (2 * (size_t)segs + 1), stream);
+        k_boundary_gen<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(S, b, sc.samples, sc.key, sc.counts,
+                                                                         sc.seg_counts);
+        launches += 1 + boundary_stages(
+            sc, cnt, tiles, segs, stream,
+            [&](const int* offsets, unsigned grid) {
+                k_boundary_eval<<<grid, 128, 0, stream>>>(S, sc.samples, sc.order, offsets, tiles, d_render, wsum,
+                                                          G.d_translation);
+            },
+            [&](const int* total, unsigned grid) {
+                if (S.styled)
+                    k_boundary_accum<true><<<grid, 256, 0, stream>>>(S, sc.samples, sc.seg_order, total, G);
+                else
+                    k_boundary_accum<false><<<grid, 256, 0, stream>>>(S, sc.samples, sc.seg_order, total, G);
+            });
     }
     return launches;
 }
@@ -1686,24 +1917,25 @@ int launch_interior_batch(const BatchEntry* B, const int2* work, int items, int*
                                                                                                   status);
     return 2;
 }
-int launch_boundary_batch(const BatchEntry* B, int nscenes, uint64_t total, int total_tiles, int cell, bool styled,
-                          BSample* samples, int* key, int* counts, int* order, cudaStream_t stream) {
+int launch_boundary_batch(const BatchEntry* B, int nscenes, uint64_t total, int total_tiles, int total_segs, int cell,
+                          bool styled, const BoundaryScratch& sc, cudaStream_t stream) {
     if (total == 0) return 0;
     total_tiles *= bnd_buckets(cell);  // sort buckets
-    cudaMemsetAsync(counts, 0, sizeof(int) * (2 * (size_t)total_tiles + 1), stream);
-    k_boundary_gen_batch<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(B, nscenes, total, cell, samples,
-                                                                              key, counts);
-    int* offsets = counts + total_tiles;
-    const int scans = launch_scan(counts, total_tiles, offsets, counts + 2 * (size_t)total_tiles + 1, stream);
-    cudaMemcpyAsync(counts, offsets, sizeof(int) * (size_t)total_tiles, cudaMemcpyDeviceToDevice, stream);
-    k_boundary_scatter<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(key, total, counts, order);
-    if (styled)
-        k_boundary_eval_batch<true><<<(unsigned)((2 * total + 127) / 128), 128, 0, stream>>>(B, samples, order,
-                                                                                         offsets, total_tiles);
-    else
-        k_boundary_eval_batch<false><<<(unsigned)((2 * total + 127) / 128), 128, 0, stream>>>(B, samples, order,
-                                                                                          offsets, total_tiles);
-    return 3 + scans;
+    cudaMemsetAsync(sc.counts, 0, sizeof(int) * (2 * (size_t)total_tiles + 1), stream);
+    cudaMemsetAsync(sc.seg_counts, 0, sizeof(int) * (2 * (size_t)total_segs + 1), stream);
+    k_boundary_gen_batch<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(B, nscenes, total, cell, sc.samples,
+                                                                              sc.key, sc.counts, sc.seg_counts);
+    return 1 + boundary_stages(
+        sc, total, total_tiles, total_segs, stream,
+        [&](const int* offsets, unsigned grid) {
+            k_boundary_eval_batch<<<grid, 128, 0, stream>>>(B, sc.samples, sc.order, offsets, total_tiles);
+        },
+        [&](const int* tot, unsigned grid) {
+            if (styled)
+                k_boundary_accum_batch<true><<<grid, 256, 0, stream>>>(B, sc.samples, sc.seg_order, tot);
+            else
+                k_boundary_accum_batch<false><<<grid, 256, 0, stream>>>(B, sc.samples, sc.seg_order, tot);
+        });
 }
 
 int launch_fill_background(const DevScene& S, float* out, cudaStream_t stream) {

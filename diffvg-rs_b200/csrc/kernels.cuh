@@ -23,10 +23,8 @@ constexpr int BND_MAX_BUCKETS = (16 / 2) * (16 / 2) * BND_CLASSES;
 inline int bnd_buckets(int cell) { return (16 / cell) * (16 / cell) * BND_CLASSES; }
 // Ints of boundary-sort scratch for `tiles` tiles: counts, offsets (+1) and the
 // two-level scan's chunk totals, bases and grand total.
-inline size_t bnd_count_ints(size_t tiles) {
-    const size_t b = tiles * BND_MAX_BUCKETS;
-    return 2 * b + 1 + 2 * ((b + 4095) / 4096) + 1;
-}
+inline size_t bnd_scan_ints(size_t buckets) { return 2 * buckets + 1 + 2 * ((buckets + 4095) / 4096) + 1; }
+inline size_t bnd_count_ints(size_t tiles) { return bnd_scan_ints(tiles * BND_MAX_BUCKETS); }
 
 // Fragment cache of the fused forward -> interior paths: the forward stores, per
 // pixel sample, the codes (2 * tile-list entry + 0 stroke / 1 fill) of the fragments
@@ -107,6 +105,15 @@ struct BSample {
     float bt;
     int is_stroke, scene;  // scene: index in a batch (0 for single-scene calls)
 };
+// Scratch of the boundary stages for up to a given number of samples.
+struct BoundaryScratch {
+    BSample* samples;
+    int2* key;        // per sample: cell bucket, segment bucket (-1: not drawn)
+    int* order;       // samples by cell
+    int* seg_order;   // samples by segment
+    int* counts;      // bnd_count_ints(tiles)
+    int* seg_counts;  // bnd_scan_ints(segments + shapes)
+};
 // One scene of a batch: its tables, options, gradient pointers, per-scene
 // output buffers and its ranges in the batch-wide work numbering.
 struct BatchEntry {
@@ -121,6 +128,7 @@ struct BatchEntry {
     float* loss;
     int item_off;    // first (tile, sub-sample) work item
     int tile_off;    // first tile in the batch-wide tile numbering
+    int seg_off;     // first segment bucket (segments, then shapes) in the batch-wide numbering
     uint64_t b_off;  // first boundary sample in the batch-wide numbering
     uint64_t nb;     // boundary samples of this scene
     uint32_t bseed;
@@ -171,11 +179,9 @@ int launch_interior(const DevScene& S, const SampleParams& sp, const float* d_re
                     const GradPtrs& G, unsigned* status, cudaStream_t stream);
 int launch_interior_prefilter(const DevScene& S, const SampleParams& sp, const float* d_render, const float* wsum,
                               const GradPtrs& G, unsigned* status, cudaStream_t stream);
-// Boundary pass in chunks of at most `capacity` samples; scratch: samples[capacity],
-// key[capacity], order[capacity], counts[2*tiles*BND_MAX_BUCKETS+1].
+// Boundary pass in chunks of at most `capacity` samples (the size of the scratch).
 int launch_boundary(const DevScene& S, const BoundaryParams& bp, const float* d_render, const float* wsum,
-                    const GradPtrs& G, BSample* samples, int* key, int* counts, int* order, uint64_t capacity,
-                    cudaStream_t stream);
+                    const GradPtrs& G, const BoundaryScratch& sc, uint64_t capacity, cudaStream_t stream);
 int launch_finalize_background(const DevScene& S, const GradPtrs& G, cudaStream_t stream);
 int launch_fill_background(const DevScene& S, float* out, cudaStream_t stream);
 // Batched launchers: B (device) holds one BatchEntry per scene; work[i] = (scene, tile +
@@ -192,8 +198,8 @@ int launch_interior_batch(const BatchEntry* B, const int2* work, int items, int*
                           cudaStream_t stream);
 int launch_interior_prefilter_batch(const BatchEntry* B, const int2* work, int items, int* counter, unsigned* status,
                                     cudaStream_t stream);
-int launch_boundary_batch(const BatchEntry* B, int nscenes, uint64_t total, int total_tiles, int cell, bool styled,
-                          BSample* samples, int* key, int* counts, int* order, cudaStream_t stream);
+int launch_boundary_batch(const BatchEntry* B, int nscenes, uint64_t total, int total_tiles, int total_segs, int cell,
+                          bool styled, const BoundaryScratch& sc, cudaStream_t stream);
 // Optimisation step: Adam on the selected parameters of every scene, then the
 // scene tables that depend on path points are rebuilt in place (segments, path and
 // group BVHs, group canvas boxes, boundary-sampling tables).  Tile binning is

@@ -90,3 +90,23 @@ def test_transforms_and_groups(renderer, scale):
     sc.shapes[3].transform = Mat3.scale(1.0, 0.0)  # singular: sampled untransformed
     sc.groups[1].shape_indices = [1, 2]  # several shapes in one group
     _check(renderer, sc)
+
+
+@pytest.mark.parametrize("samples", [1, 31, 33, 127, 129, 5000, 60000])
+def test_edge_sample_counts(renderer, samples):
+    """The edge pass's segment-ordered sums around a warp's share of 128 samples, on every
+    primitive (circle, ellipse, rectangle, mixed path, per-point thickness)."""
+    import pyoracle
+    from dvg import synth
+
+    sc = synth.primitives_scene()
+    opts = RenderOptions(samples_x=2, samples_y=2, seed=5, jitter=True, use_prefiltering=False)
+    d = np.random.default_rng(2).uniform(-1.0, 1.0, (sc.height, sc.width, 4)).astype(np.float32)
+    bo = BackwardOptions(boundary_samples=samples)
+    g = renderer.render_backward(sc, opts, bo, d)
+    _, gref = pyoracle.render_backward(sc, opts, bo, d)
+    for name in ("d_points", "d_thickness", "d_shape_params", "d_shape_stroke_width", "d_shape_transform",
+                 "d_group_transform"):
+        a, b = g.buffers[name], gref[name]
+        scale = float(np.max(np.abs(b))) + 1e-6
+        assert float(np.max(np.abs(a - b))) <= 1e-4 * scale + 1e-6, name
