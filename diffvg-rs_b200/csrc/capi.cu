@@ -127,7 +127,6 @@ struct dvg_context {
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;  // scene memory (SceneBuf)
     unsigned* status = nullptr;  // device word
-    L2Acc* l2acc = nullptr;
     DevBuf accum, wsum, image, d_render, target, loss, bg_grad, trans_grad;
     DevBuf bsamples, bkey, border, bcounts, bsegs;  // boundary-pass scratch
     DevBuf sdf, positions, dvalues;          // signed-distance host calls
@@ -296,7 +295,6 @@ dvg_status check_options(const dvg_render_options* o) {
 SampleParams sample_params(const dvg_render_options* o, const dvg_tuning& tune) {
     SampleParams sp;
     sp.layout = (int)tune.sample_layout;
-    sp.fwd_occ = (int)tune.forward_occupancy;
     sp.sxn = o->samples_x > 0 ? (int)o->samples_x : 1;
     sp.syn = o->samples_y > 0 ? (int)o->samples_y : 1;
     sp.seed = o->seed;
@@ -424,7 +422,6 @@ dvg_status dvg_context_create(int device, dvg_context** out) {
     uint64_t keep = kScenePoolKeep;
     CK(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     CK(cudaMalloc(&ctx->status, sizeof(unsigned)));
-    CK(cudaMalloc(&ctx->l2acc, sizeof(L2Acc)));
     CK(cudaMemsetAsync(ctx->status, 0, sizeof(unsigned), ctx->stream));
     *out = ctx.release();
     return DVG_OK;
@@ -448,7 +445,6 @@ void dvg_context_destroy(dvg_context* ctx) {
     ctx->kept = nullptr;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->status) cudaFree(ctx->status);
-    if (ctx->l2acc) cudaFree(ctx->l2acc);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -626,8 +622,7 @@ static dvg_status render_into(dvg_context* ctx, dvg_scene* sc, const dvg_render_
             ctx->launches += launch_forward_prefilter(S, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->status,
                                                       ctx->stream);
         else
-            ctx->launches += launch_forward(S, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->status,
-                                            ctx->stream);
+            ctx->launches += launch_forward(S, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->stream);
     }
     CK(cudaGetLastError());
     {
@@ -987,10 +982,10 @@ dvg_status dvg_fwd_bwd_l2_device(dvg_context* ctx, dvg_scene* scene, const dvg_r
     st = render_into(ctx, scene, opts, img, &frag);
     if (st != DVG_OK) return st;
     CK(ctx->d_render.reserve(npix * 4 * sizeof(float)));
+    if (loss_out) CK(cudaMemsetAsync(loss_out, 0, sizeof(float), ctx->stream));
     {
         Prof prof_(ctx, "l2_loss");
-        ctx->launches += launch_l2(img, target_rgba, npix * 4, ctx->d_render.as<float>(), loss_out, ctx->l2acc,
-                                   ctx->stream);
+        ctx->launches += launch_l2(img, target_rgba, npix * 4, ctx->d_render.as<float>(), loss_out, ctx->stream);
     }
     CK(cudaGetLastError());
     GradPtrs G = grads_from_user(grads);
@@ -1063,7 +1058,7 @@ dvg_status dvg_shard_forward(dvg_context* ctx, dvg_scene* scene, const dvg_rende
         if (opts->use_prefiltering)
             ctx->launches += launch_forward_prefilter(S, sp, accum_rgba, wsum, ctx->status, ctx->stream);
         else
-            ctx->launches += launch_forward(S, sp, accum_rgba, wsum, ctx->status, ctx->stream);
+            ctx->launches += launch_forward(S, sp, accum_rgba, wsum, ctx->stream);
     }
     CK(cudaGetLastError());
     ctx->shard_scene = scene;
@@ -1096,12 +1091,10 @@ dvg_status dvg_l2_device(dvg_context* ctx, const float* image, const float* targ
                          float* loss) {
     if (!ctx || !image || !target || !d_render) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     CK(cudaSetDevice(ctx->device));
-    if (n == 0) {
-        if (loss) CK(cudaMemsetAsync(loss, 0, sizeof(float), ctx->stream));
-        return DVG_OK;
-    }
+    if (loss) CK(cudaMemsetAsync(loss, 0, sizeof(float), ctx->stream));
+    if (n == 0) return DVG_OK;
     Prof prof_(ctx, "l2_loss");
-    ctx->launches += launch_l2(image, target, (size_t)n, d_render, loss, ctx->l2acc, ctx->stream);
+    ctx->launches += launch_l2(image, target, (size_t)n, d_render, loss, ctx->stream);
     CK(cudaGetLastError());
     return DVG_OK;
 }
@@ -1201,7 +1194,7 @@ extern "C" dvg_status dvg_render_device_noalloc(dvg_context* ctx, dvg_scene* sce
     if (opts->use_prefiltering)
         ctx->launches += launch_forward_prefilter(S, sp, accum, wsum, ctx->status, ctx->stream);
     else
-        ctx->launches += launch_forward(S, sp, accum, wsum, ctx->status, ctx->stream);
+        ctx->launches += launch_forward(S, sp, accum, wsum, ctx->stream);
     ctx->launches += launch_resolve(S, accum, wsum, out_rgba, ctx->stream);
     CK(cudaGetLastError());
     return DVG_OK;
@@ -1256,8 +1249,8 @@ dvg_status batch_enqueue(dvg_batch* b) {
         ctx->launches += launch_forward_prefilter_batch(B, b->work.as<int2>(), b->items, queue, b->max_ri,
                                                         ctx->status, ctx->stream);
     else
-        ctx->launches += launch_forward_batch(B, b->work.as<int2>(), b->items, queue, b->max_ri,
-                                              (int)b->tune.forward_occupancy, ctx->stream);
+        ctx->launches += launch_forward_batch(B, b->host_entries[0].sp, b->work.as<int2>(), b->items, queue, b->max_ri,
+                                              ctx->stream);
     ctx->launches += launch_pixels_batch(B, n, b->max_pixels, 0, ctx->stream);
     ctx->launches += launch_pixels_batch(B, n, b->max_pixels, 1, ctx->stream);
     if (pre)
@@ -1305,7 +1298,6 @@ dvg_status batch_apply_tuning(dvg_batch* b) {
     for (size_t i = 0; i < b->host_entries.size(); ++i) {
         BatchEntry& e = b->host_entries[i];
         e.sp.layout = (int)b->tune.sample_layout;
-        e.sp.fwd_occ = (int)b->tune.forward_occupancy;
         e.sp.frag = nullptr;
         e.sp.frag_n = nullptr;
         e.sp.frag_slots = 0;
@@ -1910,8 +1902,7 @@ bool tuning_valid(const dvg_tuning* t) {
 // The candidates: both warp layouts with the default cell and cache, then every cell
 // with the better layout (the boundary pass does not depend on the layout), then the
 // fragment-cache sizes (`try_slots`: only where the cache is used, non-prefiltered),
-// then persistent CTAs for the batch stages (`try_queue`), then the forward kernel at
-// 3 and at 2 CTAs per SM.
+// then persistent CTAs for the batch stages (`try_queue`).
 template <typename Apply, typename Run>
 dvg_status autotune_loop(dvg_context* ctx, dvg_tuning* tune, bool try_slots, Apply apply, Run run,
                          bool try_queue = false) {
@@ -1961,11 +1952,6 @@ dvg_status autotune_loop(dvg_context* ctx, dvg_tuning* tune, bool try_slots, App
         for (int k = 0; k < 3; ++k) consider(dvg_tuning{b2.sample_layout, b2.boundary_cell, slots[k]});
     }
     if (try_queue) consider(dvg_tuning{best.sample_layout, best.boundary_cell, best.fragment_slots, 1, 0});
-    {
-        const dvg_tuning b3 = best;
-        for (uint32_t occ = 1; occ <= 2; ++occ)
-            consider(dvg_tuning{b3.sample_layout, b3.boundary_cell, b3.fragment_slots, b3.work_queue, occ});
-    }
     *tune = best;
     if (st == DVG_OK) st = apply();
     cudaEventDestroy(e0);

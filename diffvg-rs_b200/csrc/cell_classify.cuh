@@ -247,65 +247,148 @@ DVG_CC_HD bool cell_winding(int kind, const float* q, CellBox bx, CellSeg* r) {
     return true;
 }
 
-// Lower bound on the distance from (px, py) to a segment: the distance to its n-chord polyline
-// less the chord deviation, (1 / (8 n^2)) max|B''| (16 chords; a line is its own chord).
-DVG_CC_HD float cell_dist_lower(int kind, const float* q, float px, float py) {
-    const int n = kind == 0 ? 1 : 16;
-    const float ex = kind == 0 ? q[2] : (kind == 1 ? q[4] : q[6]), ey = kind == 0 ? q[3] : (kind == 1 ? q[5] : q[7]);
-    float ax = 0.0f, ay = 0.0f, bx = 0.0f, by = 0.0f, cx, cy, dev = 0.0f;
+// A segment's 16-chord polyline (a line is its own chord), within `dev` of the curve at equal
+// parameters: (1 / (8 n^2)) max|B''|.
+struct CellChords {
+    float ax, ay, bx, by, cx, cy, dx, dy, ex, ey;  // power coefficients, end point
+    float dev;
+    int n;
+};
+DVG_CC_HD CellChords cell_chords(int kind, const float* q) {
+    CellChords c{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, q[0], q[1], q[6], q[7], 0.0f, 16};
     if (kind == 0) {
-        cx = q[2] - q[0];
-        cy = q[3] - q[1];
+        c.cx = q[2] - q[0];
+        c.cy = q[3] - q[1];
+        c.n = 1;
     } else if (kind == 1) {
-        bx = q[0] - 2.0f * q[2] + q[4];
-        by = q[1] - 2.0f * q[3] + q[5];
-        cx = 2.0f * (q[2] - q[0]);
-        cy = 2.0f * (q[3] - q[1]);
-        dev = (1.0f / 1024.0f) * std::sqrt(bx * bx + by * by);  // |B''| = 2 |b|
+        c.bx = q[0] - 2.0f * q[2] + q[4];
+        c.by = q[1] - 2.0f * q[3] + q[5];
+        c.cx = 2.0f * (q[2] - q[0]);
+        c.cy = 2.0f * (q[3] - q[1]);
+        c.dev = (1.0f / 1024.0f) * std::sqrt(c.bx * c.bx + c.by * c.by);  // |B''| = 2 |b|
     } else {
-        ax = -q[0] + 3.0f * q[2] - 3.0f * q[4] + q[6];
-        ay = -q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7];
-        bx = 3.0f * q[0] - 6.0f * q[2] + 3.0f * q[4];
-        by = 3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5];
-        cx = 3.0f * (q[2] - q[0]);
-        cy = 3.0f * (q[3] - q[1]);
+        c.ax = -q[0] + 3.0f * q[2] - 3.0f * q[4] + q[6];
+        c.ay = -q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7];
+        c.bx = 3.0f * q[0] - 6.0f * q[2] + 3.0f * q[4];
+        c.by = 3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5];
+        c.cx = 3.0f * (q[2] - q[0]);
+        c.cy = 3.0f * (q[3] - q[1]);
         const float s0x = q[0] - 2.0f * q[2] + q[4], s0y = q[1] - 2.0f * q[3] + q[5];
         const float s1x = q[2] - 2.0f * q[4] + q[6], s1y = q[3] - 2.0f * q[5] + q[7];
-        dev = (3.0f / 1024.0f) * std::sqrt(std::fmax(s0x * s0x + s0y * s0y, s1x * s1x + s1y * s1y));
+        c.dev = (3.0f / 1024.0f) * std::sqrt(std::fmax(s0x * s0x + s0y * s0y, s1x * s1x + s1y * s1y));
     }
-    float best = INFINITY, vx = q[0] - px, vy = q[1] - py;
-    const float step = 1.0f / (float)n;
-    for (int k = 1; k <= n; ++k) {
-        const float t = (float)k * step;
-        const float wx = (k == n ? ex : cc_poly(ax, bx, cx, q[0], t)) - px;
-        const float wy = (k == n ? ey : cc_poly(ay, by, cy, q[1], t)) - py;
-        const float dx = wx - vx, dy = wy - vy, ee = dx * dx + dy * dy, de = -(vx * dx + vy * dy);
-        float d2;
-        if (de <= 0.0f || ee <= 0.0f) d2 = vx * vx + vy * vy;
-        else if (de >= ee) d2 = wx * wx + wy * wy;
-        else d2 = std::fmax(vx * vx + vy * vy - de * (de / ee), 0.0f);
-        best = std::fmin(best, d2);
+    return c;
+}
+DVG_CC_HD void cell_chord_point(const CellChords& c, int k, float px, float py, float* x, float* y) {
+    const float t = (float)k * (1.0f / 16.0f);
+    *x = (k == c.n ? c.ex : cc_poly(c.ax, c.bx, c.cx, c.dx, t)) - px;
+    *y = (k == c.n ? c.ey : cc_poly(c.ay, c.by, c.cy, c.dy, t)) - py;
+}
+// Squared distance of the origin to the chord v -> w.
+DVG_CC_HD float cell_chord_d2(float vx, float vy, float wx, float wy) {
+    const float dx = wx - vx, dy = wy - vy, ee = dx * dx + dy * dy, de = -(vx * dx + vy * dy);
+    if (de <= 0.0f || ee <= 0.0f) return vx * vx + vy * vy;
+    if (de >= ee) return wx * wx + wy * wy;
+    const float cr = vx * dy - vy * dx;
+    return cr * cr / ee;
+}
+// Squared distance from (px, py) to chords k0 .. k1 - 1.
+DVG_CC_HD float cell_chords_d2(const CellChords& c, float px, float py, int k0, int k1) {
+    float best = INFINITY, vx, vy;
+    cell_chord_point(c, k0, px, py, &vx, &vy);
+    for (int k = k0 + 1; k <= k1; ++k) {
+        float wx, wy;
+        cell_chord_point(c, k, px, py, &wx, &wy);
+        best = std::fmin(best, cell_chord_d2(vx, vy, wx, wy));
         vx = wx;
         vy = wy;
     }
-    return std::sqrt(best) - dev;
+    return best;
 }
-// Whether every point of the box is farther than r from the segment's control hull (hull_only)
-// or curve, by the culling margin of the per-sample tests; NaN: no.
-DVG_CC_HD bool cell_far(int kind, const float* q, float r, CellBox b, bool hull_only) {
+
+// A stroke segment over a box: the samples' tests on chords k0 .. k1 - 1 (the others are out of
+// every point's reach; k1 = 0: no chord test), on their squared distance d2.
+//   d2 > miss: the crate's closest point is farther than the radius, by the culling margin of
+//     the per-sample tests and the chord deviation;
+//   d2 <= hit: the crate finds a point nearer than the radius (hit < 0: never taken).
+// For `hit` the curve has a point within sqrt(d2) + dev, and the crate's closest point is at
+// most a little farther than the true one.  A quadratic's comes from f64 roots (within 1e-6 of
+// the coordinates).  A cubic's parameter comes from a bracketed Newton iteration that stops at
+// |p(t)| < 1e-5 of the normalised quintic p, and d(dist^2)/dt = 2 a p with a = 3 |A|^2 (A the
+// curve's leading coefficient), so dist^2 is at most 2e-5 a too large, given that the brackets
+// isolate the roots; `hit` is left out for segments where they may not: |A| small against the
+// other coefficients (9 |A|^2 < |B|^2 or |C|^2), nearly straight ones (the sine between A and B
+// or C below 0.1), and those symmetric about t = 1/2 (whose isolating point is a root).
+// oracle/cell_stress.cpp counts no exception on random segments, and one in 10^7 on integer
+// coordinates, where the crate misses its nearest root.
+struct CellStroke {
+    bool far;   // no point of the box is in reach
+    bool full;  // every point of the box is a hit
+    float key;  // distance of the box centre less the radius
+    float miss, hit;
+    int k0, k1;
+};
+DVG_CC_HD CellStroke cell_stroke(int kind, const float* q, const float* rad, CellBox b, bool approx) {
+    CellStroke s{false, false, 0.0f, INFINITY, -1.0f, 0, 0};
     const float m = std::fmax(std::fmax(cc_max8(q), std::fmax(std::fabs(b.x0), std::fabs(b.x1))),
                               std::fmax(std::fabs(b.y0), std::fabs(b.y1)));
-    if (!(m < 1.0e6f)) return false;
+    if (!(m < 1.0e6f)) return s;
+    const float r = std::fmax(std::fmax(rad[0], rad[1]), std::fmax(rad[2], rad[3]));
     const float rm = r + 1.0e-3f * (1.0f + m) + 1.0e-5f * std::fabs(r);
     const float xmin = std::fmin(std::fmin(q[0], q[2]), std::fmin(q[4], q[6]));
     const float xmax = std::fmax(std::fmax(q[0], q[2]), std::fmax(q[4], q[6]));
     const float ymin = std::fmin(std::fmin(q[1], q[3]), std::fmin(q[5], q[7]));
     const float ymax = std::fmax(std::fmax(q[1], q[3]), std::fmax(q[5], q[7]));
-    if (b.x1 < xmin - rm || b.x0 > xmax + rm || b.y1 < ymin - rm || b.y0 > ymax + rm) return true;
-    if (hull_only) return false;
+    s.far = b.x1 < xmin - rm || b.x0 > xmax + rm || b.y1 < ymin - rm || b.y0 > ymax + rm;
+    if (s.far || (kind == 2 && approx)) return s;  // (approximate cubic: the hull test only)
+    const CellChords c = cell_chords(kind, q);
+    const float px = 0.5f * (b.x0 + b.x1), py = 0.5f * (b.y0 + b.y1);
     const float hx = 0.5f * (b.x1 - b.x0), hy = 0.5f * (b.y1 - b.y0);
     const float hd = std::sqrt(hx * hx + hy * hy) * 1.00001f;
-    return cell_dist_lower(kind, q, 0.5f * (b.x0 + b.x1), 0.5f * (b.y0 + b.y1)) > rm + hd;
+    const float reach = rm + c.dev + hd;
+    float best = INFINITY, vx, vy;
+    int k0 = 16, k1 = 0;
+    cell_chord_point(c, 0, px, py, &vx, &vy);
+    for (int k = 1; k <= c.n; ++k) {
+        float wx, wy;
+        cell_chord_point(c, k, px, py, &wx, &wy);
+        const float d2 = cell_chord_d2(vx, vy, wx, wy);
+        best = std::fmin(best, d2);
+        if (!(d2 > reach * reach)) {
+            if (k0 == 16) k0 = k - 1;
+            k1 = k;
+        }
+        vx = wx;
+        vy = wy;
+    }
+    const float d = std::sqrt(best);
+    s.key = d - r;
+    if (k1 == 0) {
+        s.far = true;
+        return s;
+    }
+    if (kind == 0 || approx) return s;
+    s.k0 = k0;
+    s.k1 = k1;
+    s.miss = (rm + c.dev) * (rm + c.dev) * 1.00001f;
+    if (!(rad[0] > 0.0f && rad[0] == rad[1] && rad[0] == rad[2] && rad[0] == rad[3])) return s;
+    float slack = 2.0e-4f * (1.0f + m) * r;
+    if (kind == 2) {
+        const float A = c.ax * c.ax + c.ay * c.ay, B = c.bx * c.bx + c.by * c.by, C = c.cx * c.cx + c.cy * c.cy;
+        const float ab = c.ax * c.by - c.ay * c.bx, ac = c.ax * c.cy - c.ay * c.cx;
+        const float tq = -(c.ax * c.bx + c.ay * c.by) / (3.0f * A);
+        if (!(9.0f * A >= B && 9.0f * A >= C && ab * ab >= 0.01f * A * B && ac * ac >= 0.01f * A * C && C > 0.0f &&
+              B > 0.0f && std::fabs(tq - 0.5f) >= 1.0e-3f))
+            return s;
+        slack += 6.3e-5f * A;
+    }
+    const float in = r * r - slack;
+    const float h = in > 0.0f ? std::sqrt(in) - c.dev : -1.0f;
+    if (h > 0.0f) {
+        s.hit = h * h * 0.99999f;
+        s.full = d + hd <= h;
+    }
+    return s;
 }
 
 }  // namespace dvgb

@@ -57,7 +57,8 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
     __shared__ int2 lev[CELLS][CELL_MAX_ITEMS];
     __shared__ int4 cur[CELLS][CELL_MAX_ITEMS];
     __shared__ short hard[CELLS][CELL_MAX_ITEMS], soft[CELLS][CELL_MAX_ITEMS], str[CELLS][CELL_MAX_ITEMS];
-    __shared__ float str_key[CELLS][CELL_MAX_ITEMS];
+    __shared__ float str_key[CELLS][CELL_MAX_ITEMS], str_miss[CELLS][CELL_MAX_ITEMS], str_hit[CELLS][CELL_MAX_ITEMS];
+    __shared__ int full[CELLS];
     const int tile = blockIdx.x, tid = threadIdx.x;
     const int tx = tile % S.tiles_x, ty = tile / S.tiles_x;
     const int off = S.tile_offsets[tile], n = S.tile_offsets[tile + 1] - off;
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
             const CellBox lb = cc_map_box(S.g_c2s + 9 * g, cbox[tid]);
             state[tid] = box_state(lb, __ldg(&S.gn_bounds[gb.x]));
             pbox[tid] = single && (si.y & (SF_IDENTITY | SF_INVERTIBLE)) == SF_INVERTIBLE ? cc_map_box(S.s_inv + 6 * s, lb) : lb;
-            base[tid] = base_slow[tid] = n_lev[tid] = n_cur[tid] = n_hard[tid] = n_soft[tid] = n_str[tid] = 0;
+            full[tid] = base[tid] = base_slow[tid] = n_lev[tid] = n_cur[tid] = n_hard[tid] = n_soft[tid] = n_str[tid] = 0;
         }
         if (listed)
             for (int nd = pi.z + tid; nd < pi.z + pi.w; nd += blockDim.x) {
@@ -151,12 +152,16 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
             }
             levels_of[sidx - pi.x][c] = lv;
             if (list_stroke && box_state(b, lb) != BOX_OUT) {
-                const float r = fmaxf(fmaxf(sg.r[0], sg.r[1]), fmaxf(sg.r[2], sg.r[3]));
-                if (!cell_far(sg.kind, sg.q, r, b, sg.kind == 2 && (pflags & PF_APPROX))) {
+                const CellStroke st = cell_stroke(sg.kind, sg.q, sg.r, b, pflags & PF_APPROX);
+                if (!st.far) {
+                    if (st.full && box_state(b, lb) == BOX_IN && state[c] == BOX_IN) full[c] = 1;
                     const int o = atomicAdd(&n_str[c], 1);
                     if (o < CELL_MAX_ITEMS) {
                         str[c][o] = (short)k;
-                        str_key[c][o] = cell_dist_lower(sg.kind, sg.q, 0.5f * (b.x0 + b.x1), 0.5f * (b.y0 + b.y1)) - r;
+                        str_key[c][o] = st.key;
+                        // (rounded up and down to make room for the chord range)
+                        str_miss[c][o] = __int_as_float(((__float_as_int(st.miss) + 15) & ~15) | st.k0);
+                        str_hit[c][o] = __int_as_float((__float_as_int(st.hit) & ~31) | st.k1);
                     }
                 }
             }
@@ -229,7 +234,9 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
                         flags |= CE_FILL;
                 }
             }
-            if (list_stroke && n_str[c] <= CELL_MAX_ITEMS) {
+            if (full[c]) {
+                flags |= CE_STROKE;
+            } else if (list_stroke && n_str[c] <= CELL_MAX_ITEMS) {
                 ns = n_str[c];
                 if (ns > 0) flags |= CE_STROKE_TEST;
             } else if (want_stroke && !(single && si.x == K_PATH && !is_path)) {
@@ -279,10 +286,13 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
             for (int i = j + 1; i < ns; ++i)
                 if (str_key[c][i] < str_key[c][best]) best = i;
             const int k = str[c][best], leaf = pi.z + leaf_of[k];
+            const bool all = box_state(b, __ldg(&S.pn_bounds[leaf])) == BOX_IN;
+            T.items[o++] = make_int4(all ? -1 : leaf, __ldg(&S.pl_segs[k0 + k]), __float_as_int(str_miss[c][best]),
+                                     __float_as_int(str_hit[c][best]));
             str[c][best] = str[c][j];
             str_key[c][best] = str_key[c][j];
-            const bool all = box_state(b, __ldg(&S.pn_bounds[leaf])) == BOX_IN;
-            T.items[o++] = make_int4(all ? -1 : leaf, __ldg(&S.pl_segs[k0 + k]), 0, 0);
+            str_miss[c][best] = str_miss[c][j];
+            str_hit[c][best] = str_hit[c][j];
         }
         int4* E = T.entries + 2 * ((size_t)ent_base + (size_t)c * n + kept[c]);
         E[0] = make_int4((e << 8) | flags, g, gi.x, gi.y);

@@ -26,7 +26,8 @@ enum : int {
     CE_STROKE_TEST = 8,  // the entry's stroke segments
     CE_STROKE_ANY = 16,  // full query (group_within)
     CE_BOX = 32,         // the tests hold inside the group's root box only
-    CE_ODD = 64          // even-odd rule
+    CE_ODD = 64,         // even-odd rule
+    CE_STROKE = 128      // the stroke covers every sample point of the cell
 };
 // Two int4 per entry: {index << 8 | flags, group, fill paint, stroke paint} and {shape,
 // winding base of the fast tests | base of the slow ones << 16, first item, counts}.  The items
@@ -38,7 +39,8 @@ enum : int {
 //   segments {path BVH leaf whose box is to be tested or -1, segment}: the first `hard` are
 //     solved for every sample, all of them (with the slow base, without levels and parabolas)
 //     for a sample within a tolerance or a band,
-//   stroke segments {leaf or -1, segment}.
+//   stroke segments {leaf or -1, segment, miss, hit}: a CellStroke, with k0 in the low four bits
+//     of miss and k1 in the low five of hit.
 // counts: level pairs, parabolas, hard segments, segments, stroke segments, six bits each.
 constexpr int CELL_MAX_ITEMS = 48;  // of each kind
 struct CellCounts {
@@ -95,9 +97,9 @@ __device__ __forceinline__ int4 cell_entry(const DevScene& S, const CellWalk& w,
 __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, int k, int4 A, float2 pt, bool* stroke,
                                           bool* fill) {
     const int flags = A.x & 255;
-    *stroke = false;
+    *stroke = (flags & CE_STROKE) != 0;
     *fill = (flags & CE_FILL) != 0;
-    if (!(flags & ~CE_FILL)) return;
+    if (!(flags & ~(CE_FILL | CE_STROKE))) return;
     const float2 lp = xf9(S.g_c2s + 9 * A.y, pt);
     if (flags & CE_STROKE_ANY) *stroke = group_within_any(S, A.y, lp);
     if (flags & CE_FILL_ANY) *fill = group_inside_any(S, A.y, lp);
@@ -156,8 +158,17 @@ __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, 
             }
             SegGeom sg;
             load_seg(S, it.y, sg);
-            if (stroke_misses_segment(sg, p)) continue;
-            if (sg.kind == 2 && !approx && stroke_far_from_cubic(sg, p)) continue;
+            const int k1 = it.w & 31;
+            if (k1) {
+                const float d2 = cell_chords_d2(cell_chords(sg.kind, sg.q), p.x, p.y, it.z & 15, k1);
+                if (d2 > __int_as_float(it.z & ~15)) continue;
+                if (d2 <= __int_as_float(it.w & ~31)) {
+                    *stroke = true;
+                    break;
+                }
+            } else if (stroke_misses_segment(sg, p)) {
+                continue;
+            }
             const CPRes c = seg_closest(sg, p, approx);
             if (c.dist < seg_radius(sg, c.t)) {
                 *stroke = true;

@@ -1468,6 +1468,51 @@ __device__ __forceinline__ void splat_sample(const DevScene& S, int x, int y, in
             }
         }
 }
+// The same splat into shared memory for warps whose lanes hold the G = 4 or 16 samples of 32 / G
+// pixels, all 32 lanes calling it (`valid`: this lane has a sample).  For each pixel of the
+// footprint the five values are summed over the G lanes by a transposing exchange (6 or 8
+// shuffles) and added by 8 / G or one lane each, in place of G atomics on one address for every
+// value; pixels that no lane's filter reaches are skipped (the box filter's whole halo).
+template <int G>
+__device__ __forceinline__ void splat_group(const DevScene& S, int x, int y, int ox, int oy, int ri, int HW, bool valid,
+                                            float2 pt, float4 acc, float* sm) {
+    const int lane = threadIdx.x & (G - 1);
+#pragma unroll 1
+    for (int k = 0; k < (2 * ri + 1) * (2 * ri + 1); ++k) {
+        const int xx = x + k % (2 * ri + 1) - ri, yy = y + k / (2 * ri + 1) - ri;
+        const bool in = valid && xx >= 0 && yy >= 0 && xx < S.width && yy < S.height;
+        float w = in ? filter_weight(S.filter_type, S.filter_radius, (float)xx + 0.5f - pt.x, (float)yy + 0.5f - pt.y)
+                     : 0.0f;
+        if (!(w > 0.0f)) w = 0.0f;
+        if (!__any_sync(0xffffffffu, w > 0.0f)) continue;
+        // (a sample that the filter does not reach adds nothing, whatever its colour)
+        float v[8] = {w > 0.0f ? acc.x * w : 0.0f, w > 0.0f ? acc.y * w : 0.0f, w > 0.0f ? acc.z * w : 0.0f,
+                      w > 0.0f ? acc.w * w : 0.0f, w, 0.0f, 0.0f, 0.0f};
+        constexpr int TOP = G >= 8 ? 8 : G;  // lanes that end with different values
+        // halve the values over the lane pairs G/2, G/4, ... apart, then sum the rest plainly
+        int n = 8;
+#pragma unroll
+        for (int s = G / 2; s >= G / TOP; s >>= 1) {
+            n >>= 1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < n) {
+                    const float keep = lane & s ? v[i + n] : v[i], send = lane & s ? v[i] : v[i + n];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+                }
+        }
+#pragma unroll
+        for (int s = G / TOP / 2; s > 0; s >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], s);
+        if (in && (G / TOP == 1 || lane % (G / TOP) == 0)) {
+            // a lane's first value: its bits from the top choose halves of the eight
+            const int at = G / TOP > 1 ? lane / (G / TOP) : lane * (8 / TOP);
+            float* c = sm + 5 * ((yy - oy) * HW + (xx - ox));
+#pragma unroll
+            for (int i = 0; i < 8 / TOP; ++i)
+                if (at + i < 5 && v[i] != 0.0f) atomicAdd(c + at + i, v[i]);
+        }
+    }
+}
 // Flushes the CTA's pixels+halo accumulator (origin (ox, oy)) to global memory (one atomic per value).
 __device__ __forceinline__ void flush_splat(const DevScene& S, int ox, int oy, int HW, const float* sm, float* accum,
                                             float* wsum) {
@@ -1505,6 +1550,44 @@ __device__ __forceinline__ float4 gather_d_color(const DevScene& S, const float*
                 out.w += k * d.w;
             }
         }
+    return out;
+}
+// gather_d_color, and in the same pass over the footprint the vector whose dot product with the
+// sample's colour is the filter-radius adjoint (accumulate_filter_gradient below is linear in
+// the colour, and d_filter_weight in its return's adjoint, for every filter but the
+// parabolic one, whose adjoint the crate does not scale): one weight per pixel instead of three.
+__device__ __forceinline__ float4 gather_d_color_radius(const DevScene& S, const float* d_render, const float* wsum,
+                                                        float2 ps, float4* rad) {
+    float4 out = make_float4(0, 0, 0, 0), r4 = out;
+    const int px = f2i(floorf(ps.x)), py = f2i(floorf(ps.y)), ri = S.filter_ri;
+    const float r = S.filter_radius;
+    for (int dy = -ri; dy <= ri; ++dy)
+        for (int dx = -ri; dx <= ri; ++dx) {
+            const int xx = px + dx, yy = py + dy;
+            if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
+            const float fx = (float)xx + 0.5f - ps.x, fy = (float)yy + 0.5f - ps.y;
+            const float w = filter_weight(S.filter_type, r, fx, fy);
+            const size_t q = (size_t)yy * S.width + xx;
+            const float ws = wsum[q];
+            if (!(ws > 0.0f)) continue;
+            const float4 d = reinterpret_cast<const float4*>(d_render)[q];
+            const float k = w / ws;
+            out.x += k * d.x;
+            out.y += k * d.y;
+            out.z += k * d.z;
+            out.w += k * d.w;
+            if (w <= 0.0f) continue;
+            const float denom = ws * ws;
+            const float dw = denom > 0.0f ? (ws - w * (ws - w)) / denom : 0.0f;
+            const float g = S.filter_type == F_GAUSSIAN
+                                ? (r != 0.0f ? dw * w * (4.0f * (fx * fx + fy * fy) / (r * r * r) - 2.0f / r) : 0.0f)
+                                : d_filter_weight(S.filter_type, r, fx, fy, dw);
+            r4.x += g * d.x;
+            r4.y += g * d.y;
+            r4.z += g * d.z;
+            r4.w += g * d.w;
+        }
+    *rad = r4;
     return out;
 }
 // accumulate_filter_gradient (src/backward/filters.rs:106-156) for one sample; returns d radius.

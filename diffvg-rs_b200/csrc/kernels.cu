@@ -19,7 +19,9 @@
 
 // Minimum resident CTAs per SM for the scene-evaluation kernels (register cap =
 // 65536 / (threads * value)); chosen by measurement on B200.
-// (the non-prefiltered forward is compiled for 2, 3 and 4, see dvg_tuning.forward_occupancy)
+#ifndef DVG_MINB_FWD
+#define DVG_MINB_FWD 4
+#endif
 #ifndef DVG_MINB_INT
 #define DVG_MINB_INT 2
 #endif
@@ -184,7 +186,11 @@ __global__ void __launch_bounds__(256) k_bin_write(DevScene S, const float4* g_b
 // One CTA = 256 samples of one 16x16 tile.  Pixels are numbered cell by cell (pix_xy), so a
 // warp's samples share one cell list (or two): entry loads are uniform.  When the CTA's
 // samples lie in one cell (layout 1, spp a power of two from 16 to 256), its splat
-// accumulator covers that cell and its halo only.
+// accumulator covers that cell and its halo only.  G: the splat's lane groups (splat_group: the
+// samples per pixel, 4 or 16, with layout 1), 0: a shared-memory atomic per sample and value.
+// Gaussian r = 1, 4x4 spp, mixed 512x512 scene: 0.55 of the forward's 1.23 ms were those atomics;
+// 0.93 ms with the groups.
+template <int G>
 __device__ __forceinline__ void forward_body(const DevScene& S, const SampleParams& sp, int tile, int round,
                                              float* accum, float* wsum, float* sm) {
     const int ri = S.filter_ri;
@@ -201,9 +207,12 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
     if (use_sm)
         for (int i = threadIdx.x; i < HW * HW * 5; i += blockDim.x) sm[i] = 0.0f;
     __syncthreads();
-    if (x < S.width && y < S.height) {
+    const bool valid = x < S.width && y < S.height;
+    float2 pt = make_float2(0.0f, 0.0f);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
         const int sx = sub % sp.sxn, sy = sub / sp.sxn;
-        const float2 pt = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, S.width, sp.seed, sp.jitter);
+        pt = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, S.width, sp.seed, sp.jitter);
         const CellWalk walk = cell_walk(S, tile, cell_of_pix(pix));
         // Fragment cache (see SampleParams): kept only where the interior pass, which
         // normalises the sample point by the canvas size and scales it back
@@ -215,7 +224,7 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
                            (pt.x / (float)S.width) * (float)S.width == pt.x &&
                            (pt.y / (float)S.height) * (float)S.height == pt.y;
         int nf = 0;
-        float4 acc = background_premul(S, y * S.width + x);
+        acc = background_premul(S, y * S.width + x);
         for (int k = 0; k < walk.n; ++k) {
             // stroke first, then fill; one paint call site for both
             const int4 A = cell_entry(S, walk, k);
@@ -232,29 +241,32 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
                 }
         }
         if (sp.frag) sp.frag_n[sid] = cache && nf <= sp.frag_slots ? (uint8_t)nf : FRAG_NONE;
-        splat_sample(S, x, y, ox, oy, ri, HW, use_sm, pt, acc, sm, accum, wsum);
     }
+    if constexpr (G > 0)
+        splat_group<G>(S, x, y, ox, oy, ri, HW, valid, pt, acc, sm);
+    else if (valid)
+        splat_sample(S, x, y, ox, oy, ri, HW, use_sm, pt, acc, sm, accum, wsum);
     if (!use_sm) return;
     __syncthreads();
     flush_splat(S, ox, oy, HW, sm, accum, wsum);
 }
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k_forward(const __grid_constant__ DevScene S, SampleParams sp, float* accum,
-                                                       float* wsum, unsigned* status) {
+template <int G>
+__global__ void __launch_bounds__(256, DVG_MINB_FWD) k_forward(const __grid_constant__ DevScene S, SampleParams sp,
+                                                               float* accum, float* wsum) {
     extern __shared__ float sm[];
-    (void)status;
-    forward_body(S, sp, sp.tile_base + blockIdx.x, blockIdx.y, accum, wsum, sm);
+    forward_body<G>(S, sp, sp.tile_base + blockIdx.x, blockIdx.y, accum, wsum, sm);
 }
 // Batched forward: one flat grid over every (scene, tile, sub-sample) work item.
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k_forward_batch(const BatchEntry* __restrict__ B,
-                                                             const int2* __restrict__ work, int items, int* counter) {
+template <int G>
+__global__ void __launch_bounds__(256, DVG_MINB_FWD) k_forward_batch(const BatchEntry* __restrict__ B,
+                                                                     const int2* __restrict__ work, int items,
+                                                                     int* counter) {
     extern __shared__ float sm[];
     for_each_item(items, counter, [&](int i) {
         const int2 wk = work[i];  // (scene, tile + tiles * sub-sample round)
         const BatchEntry& E = B[wk.x];
         const int tiles = E.S.tiles_x * E.S.tiles_y;
-        forward_body(E.S, E.sp, wk.y % tiles, wk.y / tiles, E.accum, E.wsum, sm);
+        forward_body<G>(E.S, E.sp, wk.y % tiles, wk.y / tiles, E.accum, E.wsum, sm);
     });
 }
 
@@ -333,7 +345,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
 
     float2 ps = make_float2(0.0f, 0.0f), pt = make_float2(0.0f, 0.0f);
     int pixel = 0;
-    float4 dcol = make_float4(0, 0, 0, 0), bg = make_float4(0, 0, 0, 0);
+    float4 dcol = make_float4(0, 0, 0, 0), bg = make_float4(0, 0, 0, 0), rad = bg;
     if (valid) {
         const int sx = sub % sp.sxn, sy = sub / sp.sxn;
         ps = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, W, sp.seed, sp.jitter);
@@ -341,7 +353,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
         pt = make_float2(npt.x * (float)W, npt.y * (float)H);       // sampling.rs:91
         pixel = y * W + x;
         bg = background_premul(S, pixel);
-        dcol = gather_d_color(S, d_render, wsum, ps);
+        dcol = gather_d_color_radius(S, d_render, wsum, ps, &rad);
     }
     // Pass 1: fragments in order (stroke before fill within a group).
     int code[MAX_FRAGMENTS];
@@ -489,7 +501,10 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
         }
     }
     // Filter-radius adjoint (filters.rs:106-156) and the constant-background adjoint.
-    const float dradius = active ? filter_radius_adjoint(S, d_render, wsum, ps, ret) : 0.0f;
+    float dradius = 0.0f;
+    if (active)
+        dradius = S.filter_type == F_PARABOLIC ? filter_radius_adjoint(S, d_render, wsum, ps, ret)
+                                               : rad.x * ret.x + rad.y * ret.y + rad.z * ret.z + rad.w * ret.w;
     float v[5] = {dcol.x, dcol.y, dcol.z, dcol.w, dradius};
 #pragma unroll
     for (int k = 0; k < 5; ++k) v[k] = warp_sum(v[k]);
@@ -1674,29 +1689,21 @@ __global__ void k_fill_background(DevScene S, float* out) {
 }
 
 // ------------------------------------------------------------------ L2 loss
-// Block sums are added in f64 (acc, zeroed before the launch) and the last block rounds the
-// total once: an f32 accumulator rounds at every block's addition, in whatever order they come.
-__global__ void k_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, L2Acc* acc) {
-    __shared__ double red[8];
-    double s = 0.0;
+__global__ void k_l2(const float* img, const float* target, size_t n, float* d_render, float* loss) {
+    __shared__ float red[8];
+    float s = 0.0f;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float d = img[i] - target[i];
         d_render[i] = 2.0f * d;
-        s += (double)(d * d);
+        s += d * d;
     }
-    if (!loss) return;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    atomicAdd(&acc->sum, t);
-    __threadfence();
-    if (atomicAdd(&acc->done, 1u) == gridDim.x - 1) {
-        __threadfence();
-        *loss = (float)atomicAdd(&acc->sum, 0.0);
+    if (threadIdx.x == 0 && loss) {
+        float t = 0.0f;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+        atomicAdd(loss, t);
     }
 }
 
@@ -1782,17 +1789,22 @@ int launch_binning(const DevScene& S, const float4* g_bbox, int* counts, int* of
     k_bin_write<<<tiles, 256, 0, stream>>>(S, g_bbox, offsets, entries);
     return 1;
 }
-int launch_forward(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, unsigned* status,
-                   cudaStream_t stream) {
+// Lane groups of the forward's splat: 4 or 16 samples of a pixel next to each other in a warp.
+static int splat_lanes(const SampleParams& sp) {
+    const int spp = sp.sxn * sp.syn;
+    return sp.layout && (spp == 4 || spp == 16) ? spp : 0;
+}
+int launch_forward(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, cudaStream_t stream) {
     const int hw = TILE + 2 * S.filter_ri;
     size_t smem = S.filter_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
     dim3 grid(launch_tiles(S, sp), sp.sxn * sp.syn);
-    if (sp.fwd_occ == 2)
-        k_forward<2><<<grid, 256, smem, stream>>>(S, sp, accum, wsum, status);
-    else if (sp.fwd_occ == 1)
-        k_forward<3><<<grid, 256, smem, stream>>>(S, sp, accum, wsum, status);
+    const int g = smem ? splat_lanes(sp) : 0;
+    if (g == 16)
+        k_forward<16><<<grid, 256, smem, stream>>>(S, sp, accum, wsum);
+    else if (g == 4)
+        k_forward<4><<<grid, 256, smem, stream>>>(S, sp, accum, wsum);
     else
-        k_forward<4><<<grid, 256, smem, stream>>>(S, sp, accum, wsum, status);
+        k_forward<0><<<grid, 256, smem, stream>>>(S, sp, accum, wsum);
     return 1;
 }
 int launch_weights(const DevScene& S, const SampleParams& sp, float* wsum, cudaStream_t stream) {
@@ -1876,20 +1888,20 @@ int persistent_grid(K kernel, size_t smem, int items) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem);
     return std::max(1, std::min(items, std::max(per_sm, 1) * std::max(sms, 1)));
 }
-int launch_forward_batch(const BatchEntry* B, const int2* work, int items, int* counter, int max_ri, int occ,
-                         cudaStream_t stream) {
+int launch_forward_batch(const BatchEntry* B, const SampleParams& sp, const int2* work, int items, int* counter,
+                         int max_ri, cudaStream_t stream) {
     const int hw = TILE + 2 * max_ri;
-    size_t smem = max_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
-    if (occ == 2) {
-        const int grid = counter ? persistent_grid(k_forward_batch<2>, smem, items) : items;
-        k_forward_batch<2><<<grid, 256, smem, stream>>>(B, work, items, counter);
-    } else if (occ == 1) {
-        const int grid = counter ? persistent_grid(k_forward_batch<3>, smem, items) : items;
-        k_forward_batch<3><<<grid, 256, smem, stream>>>(B, work, items, counter);
-    } else {
-        const int grid = counter ? persistent_grid(k_forward_batch<4>, smem, items) : items;
-        k_forward_batch<4><<<grid, 256, smem, stream>>>(B, work, items, counter);
-    }
+    const size_t smem = max_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
+    auto go = [&](auto kernel) {
+        kernel<<<counter ? persistent_grid(kernel, smem, items) : items, 256, smem, stream>>>(B, work, items, counter);
+    };
+    const int g = smem ? splat_lanes(sp) : 0;  // (one set of options, and of a batch one layout, for all its scenes)
+    if (g == 16)
+        go(k_forward_batch<16>);
+    else if (g == 4)
+        go(k_forward_batch<4>);
+    else
+        go(k_forward_batch<0>);
     return 1;
 }
 int launch_pixels_batch(const BatchEntry* B, int nscenes, size_t max_pixels, int which, cudaStream_t stream) {
@@ -1943,13 +1955,11 @@ int launch_fill_background(const DevScene& S, float* out, cudaStream_t stream) {
     k_fill_background<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(S, out);
     return 1;
 }
-int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, L2Acc* acc,
-              cudaStream_t stream) {
-    if (loss) cudaMemsetAsync(acc, 0, sizeof(L2Acc), stream);
+int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, cudaStream_t stream) {
     unsigned blocks = (unsigned)((n + 255) / 256);
-    if (blocks > 1184) blocks = 1184;  // 8 per SM: the loop takes the rest
+    if (blocks > 4096) blocks = 4096;
     if (blocks == 0) blocks = 1;
-    k_l2<<<blocks, 256, 0, stream>>>(img, target, n, d_render, loss, acc);
+    k_l2<<<blocks, 256, 0, stream>>>(img, target, n, d_render, loss);
     return 1;
 }
 

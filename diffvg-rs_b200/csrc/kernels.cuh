@@ -49,7 +49,6 @@ struct SampleParams {
     uint8_t* frag_n; // per-sample code count or FRAG_NONE
     int frag_slots;  // codes kept per sample (<= FRAG_MAX_SLOTS)
     int tile_base, tile_count;  // the tiles a single-scene launch covers (count 0: all)
-    int fwd_occ;  // dvg_tuning.forward_occupancy: k_forward at 4 - fwd_occ CTAs per SM
 };
 // Work items of a batched stage (work[i] = (scene, tile + tiles * sub-sample round),
 // heaviest first).  counter == nullptr: one CTA per item, item = blockIdx.x.  Otherwise
@@ -169,8 +168,7 @@ int lbvh_padded(int n);
 // Launchers (all asynchronous on `stream`).  Each returns the number of kernels launched.
 int launch_binning(const DevScene& S, const float4* g_bbox, int* counts, int* offsets, int* entries_or_null,
                    cudaStream_t stream);
-int launch_forward(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, unsigned* status,
-                   cudaStream_t stream);
+int launch_forward(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, cudaStream_t stream);
 int launch_forward_prefilter(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, unsigned* status,
                              cudaStream_t stream);
 int launch_weights(const DevScene& S, const SampleParams& sp, float* wsum, cudaStream_t stream);
@@ -189,8 +187,8 @@ int launch_fill_background(const DevScene& S, float* out, cudaStream_t stream);
 // heaviest tiles first).  counter(s): null for one CTA per item, else zeroed device ints
 // for persistent CTAs (see for_each_item; launch_interior_batch takes two, one per
 // kernel).  which: 0 resolve, 1 L2, 2 background.
-int launch_forward_batch(const BatchEntry* B, const int2* work, int items, int* counter, int max_ri, int occ,
-                         cudaStream_t stream);
+int launch_forward_batch(const BatchEntry* B, const SampleParams& sp, const int2* work, int items, int* counter,
+                         int max_ri, cudaStream_t stream);
 int launch_forward_prefilter_batch(const BatchEntry* B, const int2* work, int items, int* counter, int max_ri,
                                    unsigned* status, cudaStream_t stream);
 int launch_pixels_batch(const BatchEntry* B, int nscenes, size_t max_pixels, int which, cudaStream_t stream);
@@ -220,12 +218,6 @@ int launch_positions_backward(const DevScene& S, const float2* pos, uint64_t n, 
 // Linear BVH over n boxes into L (leaf_item[k] = item_map[box index], or the box
 // index without a map).
 int launch_lbvh_build(const float4* boxes, int n, const int* item_map, LbvhBufs& L, cudaStream_t stream);
-// Loss accumulator (context scratch) of launch_l2.
-struct L2Acc {
-    double sum;
-    unsigned done;  // blocks that have added theirs
-};
-int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, L2Acc* acc,
-              cudaStream_t stream);
+int launch_l2(const float* img, const float* target, size_t n, float* d_render, float* loss, cudaStream_t stream);
 
 }  // namespace dvgb

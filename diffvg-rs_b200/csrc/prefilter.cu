@@ -1016,14 +1016,14 @@ __device__ __forceinline__ void interior_prefilter_body(const DevScene& S, const
     const int W = S.width, H = S.height;
     float2 ps = make_float2(0.0f, 0.0f), pt = ps;
     int pixel = 0;
-    float4 dcol = make_float4(0, 0, 0, 0), bg = dcol;
+    float4 dcol = make_float4(0, 0, 0, 0), bg = dcol, rad = dcol;
     if (valid) {
         const int sx = sub % sp.sxn, sy = sub / sp.sxn;
         ps = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, W, sp.seed, false);
         pt = make_float2((ps.x / (float)W) * (float)W, (ps.y / (float)H) * (float)H);
         pixel = y * W + x;
         bg = background_premul(S, pixel);
-        dcol = gather_d_color(S, d_render, wsum, ps);
+        dcol = gather_d_color_radius(S, d_render, wsum, ps, &rad);
     }
     // pass 1: fragments with their distance data
     int code[MAX_PF], fshape[MAX_PF], fseg[MAX_PF];
@@ -1197,7 +1197,10 @@ __device__ __forceinline__ void interior_prefilter_body(const DevScene& S, const
             }
         }
     }
-    float dradius = active ? filter_radius_adjoint(S, d_render, wsum, ps, ret) : 0.0f;
+    float dradius = 0.0f;
+    if (active)
+        dradius = S.filter_type == F_PARABOLIC ? filter_radius_adjoint(S, d_render, wsum, ps, ret)
+                                               : rad.x * ret.x + rad.y * ret.y + rad.z * ret.z + rad.w * ret.w;
     float v[5] = {dcol.x, dcol.y, dcol.z, dcol.w, dradius};
 #pragma unroll
     for (int k = 0; k < 5; ++k) v[k] = warp_sum(v[k]);

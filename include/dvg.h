@@ -195,9 +195,9 @@ typedef struct dvg_scene dvg_scene;
  *                work item (scene, tile, sub-sample), heaviest tiles first (default);
  *                1 = they launch as many persistent CTAs as the GPU holds at once, which
  *                take the items from a device counter in the same order.
- * forward_occupancy: the non-prefiltered forward kernel's register budget: 0 = 4 CTAs of
- *                256 threads per SM (64 registers, default), 1 = 3 CTAs (80 registers),
- *                2 = 2 CTAs (128 registers): fewer resident warps, fewer spills. */
+ * forward_occupancy: 0, 1 or 2; accepted and kept, without effect on the launches: the
+ *                forward runs at 4 CTAs of 256 threads per SM (64 registers), which measured
+ *                faster than 3 or 2 on every scene since the per-cell lists. */
 typedef struct dvg_tuning {
     uint32_t sample_layout;
     uint32_t boundary_cell;

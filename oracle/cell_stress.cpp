@@ -158,28 +158,40 @@ extern "C" void cell_winding_stress(int kind, int mode, uint64_t seed, uint64_t 
     }
 }
 
-// The stroke test: boxes, boxes called far, points tested, points of far boxes within r of the
-// segment by the crate's closest point.
-extern "C" void cell_far_stress(int kind, int mode, uint64_t seed, uint64_t n, int points, unsigned long long* out) {
+// The stroke tests: boxes, far boxes, full boxes, points tested, points the chords call a miss
+// or a hit, wrong misses (a far box's or a missed point within r by the crate's closest point),
+// wrong hits (a full box's or a hit point that is not).
+extern "C" void cell_stroke_stress(int kind, int mode, uint64_t seed, uint64_t n, int points,
+                                   unsigned long long* out) {
     SplitMix rng{seed * 0x2545f4914f6cdd1dull + (uint64_t)(mode * 3 + kind) + 77};
-    for (int k = 0; k < 4; ++k) out[k] = 0;
+    for (int k = 0; k < 7; ++k) out[k] = 0;
     for (uint64_t i = 0; i < n; ++i) {
         V2 p[4];
         random_segment(rng, kind, mode, p);
         const dvgb::CellBox b = random_box(rng, kind, p);
         const float q[8] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y, p[3].x, p[3].y};
-        const float r = (float)std::pow(10.0, -1.0 + 2.0 * rng.uni());
+        const float r = (float)std::pow(10.0, -1.0 + 2.0 * rng.uni()), rad[4] = {r, r, r, r};
+        const dvgb::CellStroke s = dvgb::cell_stroke(kind, q, rad, b, false);
+        const dvgb::CellChords ch = dvgb::cell_chords(kind, q);
         out[0] += 1;
-        if (!dvgb::cell_far(kind, q, r, b, false)) continue;
-        out[1] += 1;
+        if (s.far) out[1] += 1;
+        if (s.full) out[2] += 1;
         for (int k = 0; k < points; ++k) {
             const V2 pt = random_point(rng, b, p);
             CP c;
             if (kind == 0) distance_to_segment(pt, p[0], p[1], &c.dist, &c.cp, &c.t);
             else if (kind == 1) c = closest_point_quadratic(pt, p[0], p[1], p[2], false);
             else c = closest_point_cubic(pt, p[0], p[1], p[2], p[3], false);
-            out[2] += 1;
-            if (c.dist < r) out[3] += 1;
+            bool miss = s.far, hit = s.full;
+            if (!s.far && s.k1) {
+                const float d2 = dvgb::cell_chords_d2(ch, pt.x, pt.y, s.k0, s.k1);
+                miss = d2 > s.miss;
+                hit = hit || d2 <= s.hit;
+            }
+            out[3] += 1;
+            if (miss || hit) out[4] += 1;
+            if (miss && c.dist < r) out[5] += 1;
+            if (hit && !(c.dist < r)) out[6] += 1;
         }
     }
 }
