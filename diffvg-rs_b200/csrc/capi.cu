@@ -171,14 +171,13 @@ struct dvg_scene {
 
 namespace {
 
-// Sizes a scene's per-cell lists for `total` tile entries and points its tables at them: at
-// most one cell entry per tile entry and cell, and four items for each (what finds no room
-// keeps the full query).
-dvg_status reserve_cells(dvg_scene* sc, size_t total) {
+// Sizes a scene's per-cell lists for `total` tile entries (at most one cell entry per tile entry
+// and cell) and `items` items, and points its tables at them.
+dvg_status reserve_cells(dvg_scene* sc, size_t total, size_t items) {
     DevScene& S = sc->dev;
     const size_t cells = (size_t)S.tiles_x * S.tiles_y * CELLS;
     const size_t ents = std::min<size_t>(std::max<size_t>(total, 1) * CELLS, (size_t)1 << 30);
-    const size_t items = std::min<size_t>(ents * 4, (size_t)1 << 30);
+    items = std::min<size_t>(std::max<size_t>(items, 1), (size_t)1 << 30);
     const size_t o_ent = (cells * sizeof(int2) + 255) & ~(size_t)255, o_item = o_ent + ents * 2 * sizeof(int4);
     const size_t o_cnt = (o_item + items * sizeof(int4) + 255) & ~(size_t)255;
     CK(sc->cells.reserve(o_cnt + 2 * sizeof(int)));
@@ -195,6 +194,21 @@ dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
     ctx->launches += launch_cells(sc->dev, sc->cell_table, ctx->stream);
     CK(cudaGetLastError());
     return DVG_OK;
+}
+// Reserves and builds, and waits: the item counter runs on past the room there is, so a scene
+// that needs more than the first guess (three per cell entry; the mixed scene takes 1.7, the
+// large one 4) is built once again with what it counted, times `slack`.
+dvg_status make_cells(dvg_context* ctx, dvg_scene* sc, size_t total, int slack) {
+    dvg_status st = reserve_cells(sc, total, 3 * CELLS * total * slack);
+    if (st == DVG_OK) st = build_cells(ctx, sc);
+    if (st != DVG_OK) return st;
+    int used[2] = {0, 0};
+    CK(cudaMemcpyAsync(used, sc->cell_table.counters, sizeof used, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (used[1] <= sc->cell_table.cap_items / slack) return DVG_OK;
+    st = reserve_cells(sc, total, (size_t)used[1] * slack);
+    if (st == DVG_OK) st = build_cells(ctx, sc);
+    return st;
 }
 
 // Offsets of each gradient part inside the scene's gradient arena (in floats).
@@ -566,8 +580,7 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
         S.tile_entries = sc->entries.as<int>();
         ctx->launches += launch_binning(S, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
         CK(cudaGetLastError());
-        st = reserve_cells(sc.get(), (size_t)std::max(total, 0));
-        if (st == DVG_OK) st = build_cells(ctx, sc.get());
+        st = make_cells(ctx, sc.get(), (size_t)std::max(total, 0), 1);
         if (st != DVG_OK) return st;
     }
     layout_grads(sc.get());
@@ -1541,13 +1554,12 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, nullptr, ctx->stream);
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
             CK(cudaGetLastError());
-            // room for four times the cell entries that the present geometry takes: a step that
-            // moves more than that into view walks the tile lists instead
+            // room for twice the entries and items that the present geometry takes: what a step
+            // moves into view beyond that walks the tile lists or keeps the full queries
             int total = 0;
             CK(cudaMemcpyAsync(&total, offsets + tiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
-            dvg_status st = reserve_cells(sc, std::min<size_t>(need, 4 * (size_t)std::max(total, 0) + 1024));
-            if (st == DVG_OK) st = build_cells(ctx, sc);
+            const dvg_status st = make_cells(ctx, sc, std::min<size_t>(need, 2 * (size_t)std::max(total, 0) + 1024), 2);
             if (st != DVG_OK) return st;
         }
         b->host_entries[i].S.tile_entries = sc->dev.tile_entries;

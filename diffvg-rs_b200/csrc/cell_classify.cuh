@@ -17,9 +17,9 @@
 // of the box by more than M, the piece from level l0 to l1 adds [py > l0] - [py > l1].  At an
 // extremum between two such pieces that cancels; what remains is a constant and a step at each
 // end point inside the rows.  A piece that crosses all of the rows near the box is replaced by
-// a parabola x = c0 + c1 y + c2 y^2 through three of its points, with a bound on the distance in
-// x between the two: it counts where px lies left of the parabola by more than the bound, and
-// not where it lies right of it by as much.  The crate's computed sum is this number when
+// a cubic x(y) through four of its points, with a bound on the distance in x between the two:
+// it counts where px lies left of that curve by more than the bound, and not where it lies
+// right of it by as much.  The crate's computed sum is this number when
 //  * py is farther than T = 1e-5 (1 + m) from every level inside the rows (end points and
 //    extrema): the sample loop compares, and runs the full query otherwise;
 //  * |y'| >= M at an inflection, so that |y'| is small near extrema only;
@@ -33,8 +33,8 @@
 // it, 4e5 times the error.  The trigonometric formula adds 4 sqrt(q) 8 eps / sqrt(1 - x^2), below
 // 1e-7 for roots that are sqrt(2 D / 24 m) apart.  So every computed root is on the same side of
 // 0, of 1, of px (M against 6 m times the error) and of every extremum as the exact one.
-// A parabola's bound holds the interpolation error (the third derivative of X - c0 - c1 Y - c2 Y^2
-// over the bracket) and T moved in y and in x, for the rounded coefficients and the root.
+// The bound holds the interpolation error (the fourth derivative of X - Q(Y) over the bracket)
+// and T moved in y and in x, for the rounded coefficients and the root.
 // Anything else is left to the per-sample test.  A segment whose control points miss the rays
 // of the whole box by the per-sample culling margin (ray_misses_segment in device.cuh)
 // contributes nothing, as there.
@@ -43,6 +43,9 @@
 // decisions at random points of random boxes.
 #pragma once
 #include <cmath>
+#ifdef __CUDACC__
+#include <cuda_fp16.h>
+#endif
 
 #ifdef __CUDACC__
 #define DVG_CC_HD __host__ __device__ __forceinline__
@@ -85,10 +88,22 @@ DVG_CC_HD CellBox cc_map_box(const float* m, CellBox b) {
 
 // A segment's winding contribution over a box: base + start [py > y(0)] - end [py > y(1)] for
 // rows farther than `tol` from y(0) (if start), y(1) (if end) and ext[0 .. ne).
-// Each of the nc parabolas adds its sign where px < c0 + (c1 + c2 v) v - band, v = py - yc with yc
-// the middle of the box's rows, and nothing where px > c0 + (c1 + c2 v) v + band.
+// Each of the nc curves adds its sign where px < c0 + (c1 + (c2 + c3 v) v) v - band, v = py - yc
+// with yc the middle of the box's rows, and nothing where px is as far to the other side (c3 is
+// rounded to a half-precision number).
+DVG_CC_HD float cc_round_half(float v) {
+#ifdef __CUDA_ARCH__
+    return __half2float(__float2half_rn(v));
+#else
+    if (!(std::fabs(v) < 65504.0f)) return v;
+    int e;
+    std::frexp(v, &e);
+    const int q = e - 11 < -24 ? -24 : e - 11;
+    return std::ldexp(std::nearbyint(std::ldexp(v, -q)), q);
+#endif
+}
 struct CellCurve {
-    float c0, c1, c2, band;
+    float c0, c1, c2, c3, band;
     int sign;
 };
 struct CellSeg {
@@ -102,32 +117,50 @@ DVG_CC_HD double cc_polyd(float a, float b, float c, float d, double t) {
     return (((double)a * t + (double)b) * t + (double)c) * t + (double)d;
 }
 DVG_CC_HD float cc_row_centre(CellBox b) { return 0.5f * (b.y0 + b.y1); }
-// The parabola through the piece's points at u0, the middle and v1 (y monotone between them).
+// x as a cubic polynomial of the row through the piece's points at the four Chebyshev nodes of
+// [u0, v1] (y monotone there).
 DVG_CC_HD bool cell_curve(float a, float b, float c, float d, float ax, float bx, float cx, float dx, float u0, float v1,
                           float T, CellBox box, CellCurve* r) {
     const float yc = cc_row_centre(box);
-    const double t1 = 0.5 * ((double)u0 + (double)v1);
-    const double y0 = cc_polyd(a, b, c, d, u0) - (double)yc, y1 = cc_polyd(a, b, c, d, t1) - (double)yc,
-                 y2 = cc_polyd(a, b, c, d, v1) - (double)yc;
-    const double x0 = cc_polyd(ax, bx, cx, dx, u0), x1 = cc_polyd(ax, bx, cx, dx, t1), x2 = cc_polyd(ax, bx, cx, dx, v1);
-    const double d01 = (x1 - x0) / (y1 - y0), d12 = (x2 - x1) / (y2 - y1);
-    const double g = (d12 - d01) / (y2 - y0);
-    const double be = d01 - g * (y0 + y1), al = x0 - (be + g * y0) * y0;
-    r->c0 = (float)al;
-    r->c1 = (float)be;
-    r->c2 = (float)g;
-    // third derivative of X - be Y - g Y^2 over the bracket (Y relative to yc)
-    const float H = 0.5f * (v1 - u0), tm = (float)t1;
-    const float yb = std::fmax(std::fabs((float)y0), std::fabs((float)y2));
+    const double mid = 0.5 * ((double)u0 + (double)v1), half = 0.5 * ((double)v1 - (double)u0);
+    const double node[4] = {-0.92387953251128674, -0.38268343236508977, 0.38268343236508977, 0.92387953251128674};
+    double y[4], f[4];
+    for (int k = 0; k < 4; ++k) {
+        const double t = mid + half * node[k];
+        y[k] = cc_polyd(a, b, c, d, t) - (double)yc;
+        f[k] = cc_polyd(ax, bx, cx, dx, t);
+    }
+    for (int j = 1; j < 4; ++j)  // divided differences
+        for (int k = 3; k >= j; --k) f[k] = (f[k] - f[k - 1]) / (y[k] - y[k - j]);
+    // Newton form to powers of the row
+    double p0 = f[3], p1 = 0.0, p2 = 0.0, p3 = 0.0;
+    for (int k = 2; k >= 0; --k) {
+        p3 = p2 - y[k] * p3;
+        p2 = p1 - y[k] * p2;
+        p1 = p0 - y[k] * p1;
+        p0 = f[k] - y[k] * p0;
+    }
+    r->c0 = (float)p0;
+    r->c1 = (float)p1;
+    r->c2 = (float)p2;
+    r->c3 = cc_round_half((float)p3);
+    // fourth derivative of X - c1 Y - c2 Y^2 - c3 Y^3 over the bracket (Y relative to yc)
+    const float H = (float)half, tm = (float)mid;
+    const float yb = std::fmax(std::fabs(box.y1 - yc), std::fmax(std::fabs((float)(cc_polyd(a, b, c, d, u0) - (double)yc)),
+                                                                 std::fabs((float)(cc_polyd(a, b, c, d, v1) - (double)yc))));
     const float d3 = 6.0f * std::fabs(a), d2 = std::fabs(6.0f * a * tm + 2.0f * b) + d3 * H;
     const float d1 = std::fabs((3.0f * a * tm + 2.0f * b) * tm + c) + d2 * H;
-    const float fb = std::fabs(r->c1), fg = std::fabs(r->c2);
-    const float R3 = 6.0f * std::fabs(ax) + fb * d3 + fg * (2.0f * yb * d3 + 6.0f * d1 * d2);
-    const float fit = 0.0642f * H * H * H * R3 * 1.01f;
-    const float slope = fb + 2.0f * fg * yb;
-    r->band = fit + T * (1.0f + slope) + 1.0e-6f * (std::fabs(r->c0) + fb * yb + fg * yb * yb);
-    // worth it while most of the box lies outside the band
-    return r->band < 0.25f * (box.x1 - box.x0);  // (NaN: no)
+    const float fb = std::fabs(r->c1), fg = std::fabs(r->c2), fh = std::fabs((float)p3);
+    const float R4 = fg * (8.0f * d1 * d3 + 6.0f * d2 * d2) +
+                     fh * (24.0f * yb * d1 * d3 + 18.0f * yb * d2 * d2 + 36.0f * d1 * d1 * d2);
+    const float fit = H * H * H * H * (1.0f / 192.0f) * R4 * 1.01f + std::fabs(r->c3 - (float)p3) * yb * yb * yb;
+    const float slope = fb + (2.0f * fg + 3.0f * fh * yb) * yb;
+    const float band = fit + T * (1.0f + slope) + 1.0e-6f * (std::fabs(r->c0) + (fb + (fg + fh * yb) * yb) * yb);
+    // Worth it while few samples fall into the band: one that does costs its warp the solves
+    // that the lists are there to avoid.
+    if (!(band < 0.004f * (box.x1 - box.x0) && fh < 6.0e4f)) return false;  // (NaN: no)
+    r->band = band;
+    return true;
 }
 // Fills *r for a segment (kind 0 line, 1 quadratic, 2 cubic; q: four control points, lines and
 // quadratics repeat their last one), or returns false: test it per sample.
@@ -243,6 +276,122 @@ DVG_CC_HD bool cell_winding(int kind, const float* q, CellBox bx, CellSeg* r) {
         } else if (l1 < lo) {
             r->base -= 1;
         }
+    }
+    return true;
+}
+
+// The extrema of y(t) in (0, 1) for cell_winding_point (2: none), or e1 < 0 when a segment does
+// not meet the conditions on its coefficients (its inflection, its |a| against |b| and |c|).
+DVG_CC_HD void cell_extrema(int kind, const float* q, float m, float* e1, float* e2) {
+    *e1 = *e2 = 2.0f;
+    if (kind == 0) return;
+    float a = 0.0f, b, c;
+    if (kind == 1) {
+        b = q[1] - 2.0f * q[3] + q[5];
+        c = -2.0f * q[1] + 2.0f * q[3];
+    } else {
+        a = -q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7];
+        b = 3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5];
+        c = -3.0f * q[1] + 3.0f * q[3];
+        if (!(std::fabs(a) > 1.1e-6f && std::fmax(std::fabs(b), std::fabs(c)) <= 64.0f * std::fabs(a))) {
+            *e1 = -1.0f;
+            return;
+        }
+    }
+    const float disc = b * b - 3.0f * a * c;
+    if (a != 0.0f) {
+        const float ti = -b / (3.0f * a);
+        if (ti > -0.05f && ti < 1.05f && !(std::fabs(disc) >= 3.0f * std::fabs(a) * 1.0e-4f * (1.0f + m))) {
+            *e1 = -1.0f;
+            return;
+        }
+    }
+    if (!(disc > 0.0f)) return;
+    const float s = -(b + (b < 0.0f ? -std::sqrt(disc) : std::sqrt(disc)));
+    float t1 = a != 0.0f ? s / (3.0f * a) : 2.0f, t2 = s != 0.0f ? c / s : 2.0f;
+    if (!(t1 > 0.0f && t1 < 1.0f)) t1 = 2.0f;
+    if (!(t2 > 0.0f && t2 < 1.0f)) t2 = 2.0f;
+    *e1 = std::fmin(t1, t2);
+    *e2 = std::fmax(t1, t2);
+}
+DVG_CC_HD float cc_quick_div(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fdividef(a, b);
+#else
+    return a / b;
+#endif
+}
+// cell_winding for the box of one point, with the extrema of cell_extrema (e1 >= 0): the
+// winding contribution at (px, py) in *w, or false when it is not certain.  The coefficients
+// are the crate's own (rounded to f32), so its polynomial is met exactly here: a piece that py
+// passes has one root, found by f32 Newton steps kept inside a bracket and two f64 steps.  The
+// crate's root lies within et = 1e-7 + 2e-11 (1 + m) / |y'| of it while py is T from every
+// extremum (the bounds at the top, with 2 D = T); et moves the end-point tests by 2 et |y'| and
+// x by et |x'|.  (Lines are the crate's in f32 throughout: T there.)
+DVG_CC_HD bool cell_winding_point(int kind, const float* q, float e1, float e2, float px, float py, int* w) {
+    *w = 0;
+    const float m = std::fmax(cc_max8(q), std::fmax(std::fabs(px), std::fabs(py)));
+    const float T = 1.0e-5f * (1.0f + m), tiny = 1.0e-9f * (1.0f + m);
+    float a = 0.0f, b = 0.0f, c, ax = 0.0f, bx = 0.0f, cx;
+    const float d = q[1] - py, dx = q[0] - px;
+    if (kind == 0) {
+        c = q[3] - q[1];
+        cx = q[2] - q[0];
+    } else if (kind == 1) {
+        b = q[1] - 2.0f * q[3] + q[5];
+        c = -2.0f * q[1] + 2.0f * q[3];
+        bx = q[0] - 2.0f * q[2] + q[4];
+        cx = -2.0f * q[0] + 2.0f * q[2];
+    } else {
+        a = -q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7];
+        b = 3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5];
+        c = -3.0f * q[1] + 3.0f * q[3];
+        ax = -q[0] + 3.0f * q[2] - 3.0f * q[4] + q[6];
+        bx = 3.0f * q[0] - 6.0f * q[2] + 3.0f * q[4];
+        cx = -3.0f * q[0] + 3.0f * q[2];
+        if (!(std::fabs(d) <= 64.0f * std::fabs(a))) return false;
+    }
+    float t0 = 0.0f, l0 = d;
+    if (!(std::fabs(d) > (kind == 0 ? T : 1.0e-6f * std::fabs(c) + tiny))) return false;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+    for (int i = 0; i < 3; ++i) {
+        const float te = i == 0 ? e1 : (i == 1 ? e2 : 1.0f);
+        if (te > 1.0f) continue;  // no such extremum
+        const float ls = l0, l1 = (float)cc_polyd(a, b, c, d, te);
+        float lo = t0, hi = te;
+        t0 = te;
+        l0 = l1;
+        const float Te = i < 2 || kind == 0 ? T : 1.0e-6f * std::fabs(3.0f * a + 2.0f * b + c) + tiny;
+        if (!(std::fabs(l1) > Te)) return false;
+        if ((ls < 0.0f) == (l1 < 0.0f)) continue;
+        const bool up = l1 > 0.0f;
+        float t = lo + (hi - lo) * cc_quick_div(ls, ls - l1), dy = 0.0f;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+        for (int it = 0; it < 12; ++it) {
+            const float y = cc_poly(a, b, c, d, t);
+            dy = (3.0f * a * t + 2.0f * b) * t + c;
+            if (std::fabs(y) <= 0.3f * T) break;
+            if ((y < 0.0f) == up) lo = t; else hi = t;
+            t = t - cc_quick_div(y, dy);
+            if (!(t > lo && t < hi)) t = 0.5f * (lo + hi);
+        }
+        const float inv = cc_quick_div(1.0f, dy);
+        const double s1 = cc_polyd(a, b, c, d, t) * (double)inv, ta = (double)t - s1;
+        const double s2 = cc_polyd(a, b, c, d, ta) * (double)inv, tr = ta - s2;
+        // the slope within 5 % over the first step, so the second leaves 0.06 |s2| at most
+        const float h = std::fabs((float)s1), ddy = std::fabs(6.0f * a * t + 2.0f * b);
+        if (!((ddy + 6.0f * std::fabs(a) * h) * h <= 0.05f * std::fabs(dy) && std::fabs(s2) <= 1.0e-7)) return false;
+        const float et = (kind == 0 ? 1.0e-6f : 1.1e-7f) + (kind == 0 ? T : 2.0f * 1.0e-2f * tiny) * std::fabs(inv);
+        if (!(tr > 2.0 * (double)et && tr < 1.0 - 2.0 * (double)et)) return false;
+        const double x = cc_polyd(ax, bx, cx, dx, tr);
+        const float tf = (float)tr, xs = std::fabs((3.0f * ax * tf + 2.0f * bx) * tf + cx);
+        const float xss = std::fabs(6.0f * ax * tf + 2.0f * bx) + 6.0f * std::fabs(ax) * et;
+        if (!(std::fabs(x) > (double)((xs + xss * et) * et * 1.01f + (kind == 0 ? T : tiny)))) return false;
+        if (x > 0.0) *w += up ? 1 : -1;
     }
     return true;
 }

@@ -5,8 +5,8 @@
 // classification where the sample loop used to test the segment at each of the cell's
 // 16 * spp sample points.  The sample kernels are bound by instruction issue on those tests
 // (f64 root solves): on the mixed 512x512 scene a sample met 49 segments of 5.3 groups, and
-// with the lists 1.1 segments, 1.7 parabolas and 2.7 rows of 2.2 groups are left (large
-// 1024x1024 scene: 199 -> 16, 8, 26).  Forward 3.43 -> 1.23 ms and edge pass 1.31 -> 0.81 ms on
+// with the lists 1.2 segments, 1.5 curves and 2.7 rows of 2.2 groups are left (large
+// 1024x1024 scene: 199 -> 18, 6, 26).  Forward 3.43 -> 1.23 ms and edge pass 1.31 -> 0.81 ms on
 // the mixed scene at 4x4 spp, 76 -> 34 ms and 216 -> 136 ms on the large one.  4x4 pixels: the
 // 16 samples per pixel of a CTA share one list; cells of a whole tile leave 8 segments.
 #include "cells.cuh"
@@ -45,6 +45,11 @@ __device__ __forceinline__ int primitive_fill(int kind, float4 prm, const CellBo
 }
 // A tolerance (rounded up) with a step of -2 .. 2 in its low bits.
 __device__ __forceinline__ int coded(float tol, int step) { return ((__float_as_int(tol) + 7) & ~7) | (step + 2); }
+// A curve's band (rounded up to its upper half's leading bits), step and c3 in one word.
+__device__ __forceinline__ int coded_curve(const CellCurve& q, int step) {
+    const unsigned band = ((unsigned)__float_as_int(q.band) + 0x7ffffu) & 0xfff80000u;
+    return (int)(band | ((unsigned)(step + 2) << 16) | (unsigned)__half_as_ushort(__float2half_rn(q.c3)));
+}
 }  // namespace
 
 __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene S, const CellTable T) {
@@ -140,7 +145,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
                         const int o = atomicAdd(&n_cur[c], 1);
                         if (o < CELL_MAX_ITEMS)
                             cur[c][o] = make_int4(__float_as_int(q.c0), __float_as_int(q.c1), __float_as_int(q.c2),
-                                                  coded(q.band, mult * q.sign));
+                                                  coded_curve(q, mult * q.sign));
                     }
                     if (r.start || r.end || r.ne || r.nc) {  // not one number over the cell
                         const int o = atomicAdd(&n_soft[c], 1);
@@ -228,10 +233,12 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
                         flags |= in ? CE_FILL : CE_FILL_TEST;
                 } else if (si.x != K_PATH) {
                     const int w = primitive_fill(si.x, __ldg(&S.s_params[s]), pbox[c]);
-                    if (w < 0 || (w == 1 && !in))
-                        flags |= CE_FILL_ANY;
-                    else if (w == 1)
+                    if (w < 0 || (w == 1 && !in)) {
+                        flags |= CE_FILL_TEST;
+                        nh = CELL_PRIMITIVE;
+                    } else if (w == 1 && fill_hit(gi.z, 1)) {
                         flags |= CE_FILL;
+                    }
                 }
             }
             if (full[c]) {
@@ -277,9 +284,17 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
         for (int j = 0; j < nc; ++j) T.items[o++] = cur[c][j];
         for (int j = 0; j < nf; ++j) {
             const int k = j < nh ? hard[c][j] : soft[c][j - nh], leaf = pi.z + leaf_of[k];
+            const int sidx = __ldg(&S.pl_segs[k0 + k]);
             const float4 lb = __ldg(&S.pn_bounds[leaf]);
             const bool all = b.y0 >= lb.y && b.y1 <= lb.w && b.x1 <= lb.z;
-            T.items[o++] = make_int4(all ? -1 : leaf, __ldg(&S.pl_segs[k0 + k]), 0, 0);
+            float e1 = -1.0f, e2 = -1.0f;
+            if (j < nh) {
+                SegGeom sg;
+                load_seg(S, sidx, sg);
+                const float m = fmaxf(fmaxf(fmaxf(fabsf(b.x0), fabsf(b.x1)), fmaxf(fabsf(b.y0), fabsf(b.y1))), cc_max8(sg.q));
+                if (m < 1.0e6f) cell_extrema(sg.kind, sg.q, m, &e1, &e2);
+            }
+            T.items[o++] = make_int4(all ? -1 : leaf, sidx, __float_as_int(e1), __float_as_int(e2));
         }
         for (int j = 0; j < ns; ++j) {  // nearest first: a sample stops at its first hit
             int best = j;

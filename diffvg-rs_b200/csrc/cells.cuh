@@ -3,8 +3,8 @@
 // Each 16x16 tile's group list is split over the tile's sixteen 4x4-pixel cells.  A cell keeps
 // an entry, in group order, for every group that can cover one of its sample points, with the
 // tests that are left there (cell_classify.cuh): none at all when the fill covers the whole
-// cell; else a winding number summed beforehand, the rows at which it steps, the parabolas that
-// stand for curve pieces crossing the cell and the few segments that are solved per sample; and
+// cell; else a winding number summed beforehand, the rows at which it steps, the curves
+// x(y) that stand for pieces crossing the cell and the few segments that are solved per sample; and
 // the segments that a stroke can reach the cell from, the nearest first.  Groups that the lists
 // do not describe (several shapes, styled strokes, strokes of ellipses and rectangles) keep the
 // full query.
@@ -35,14 +35,18 @@ enum : int {
 //   a header {middle row yc} when there are fill tests,
 //   level pairs {row, tolerance, row, tolerance}, each tolerance with (step + 2) in its low three
 //     bits: the winding steps where py passes the row,
-//   parabolas {c0, c1, c2, band}, the band with (sign + 2) in its low three bits,
-//   segments {path BVH leaf whose box is to be tested or -1, segment}: the first `hard` are
-//     solved for every sample, all of them (with the slow base, without levels and parabolas)
-//     for a sample within a tolerance or a band,
+//   curves {c0, c1, c2, c3 as a half | the upper half of the band with (sign + 2) in its low three
+//     bits},
+//   segments {path BVH leaf whose box is to be tested or -1, segment, e1, e2}: the first `hard`
+//     are tested by every sample (cell_winding_point with their extrema, the crate's solve where
+//     that is not certain), all of them solved (with the slow base, without levels and
+//     curves) for a sample within a tolerance or a band,
 //   stroke segments {leaf or -1, segment, miss, hit}: a CellStroke, with k0 in the low four bits
 //     of miss and k1 in the low five of hit.
-// counts: level pairs, parabolas, hard segments, segments, stroke segments, six bits each.
+// counts: level pairs, curves, hard segments, segments, stroke segments, six bits each; hard =
+// CELL_PRIMITIVE: the shape is a circle, an ellipse or a rectangle.
 constexpr int CELL_MAX_ITEMS = 48;  // of each kind
+constexpr int CELL_PRIMITIVE = 63;
 struct CellCounts {
     int pairs, curves, hard, segs, strokes;
     __device__ __forceinline__ explicit CellCounts(int w)
@@ -117,6 +121,7 @@ __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, 
         ++items;
         int wind = (short)(B.y & 0xffff);
         bool close = false;
+#pragma unroll 1
         for (int j = 0; j < n.pairs; ++j) {
             const int4 it = __ldg(&items[j]);
             const float d0 = p.y - __int_as_float(it.x), d1 = p.y - __int_as_float(it.z);
@@ -125,31 +130,45 @@ __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, 
             close = close || fabsf(d0) <= __int_as_float(it.y & ~7) || fabsf(d1) <= __int_as_float(it.w & ~7);
         }
         items += n.pairs;
+#pragma unroll 1
         for (int j = 0; j < n.curves; ++j) {
             const int4 it = __ldg(&items[j]);
             const float c1 = __int_as_float(it.y), c2 = __int_as_float(it.z);
-            const float d = p.x - (__int_as_float(it.x) + (c1 + c2 * v) * v);
-            if (d < 0.0f) wind += (it.w & 7) - 2;
-            close = close || fabsf(d) <= __int_as_float(it.w & ~7);
+            const float c3 = __half2float(__ushort_as_half((unsigned short)(it.w & 0xffff)));
+            const float d = p.x - (__int_as_float(it.x) + (c1 + (c2 + c3 * v) * v) * v);
+            if (d < 0.0f) wind += ((it.w >> 16) & 7) - 2;
+            close = close || fabsf(d) <= __int_as_float(it.w & 0xfff80000);
         }
         items += n.curves;
-        if (close) wind = B.y >> 16;
-        const int solve = close ? n.segs : n.hard;
-        for (int j = 0; j < solve; ++j) {
-            const int4 it = __ldg(&items[j]);
-            if (it.x >= 0) {
-                const float4 b = __ldg(&S.pn_bounds[it.x]);
-                if (p.y < b.y || p.y > b.w || p.x > b.z) continue;
+        if (n.hard == CELL_PRIMITIVE) {
+            wind = winding_primitive(__ldg(&S.s_info[B.x].x), __ldg(&S.s_params[B.x]), p);
+        } else {
+            if (close) wind = B.y >> 16;
+            const int solve = close ? n.segs : n.hard;
+#pragma unroll 1
+            for (int j = 0; j < solve; ++j) {
+                const int4 it = __ldg(&items[j]);
+                if (it.x >= 0) {
+                    const float4 b = __ldg(&S.pn_bounds[it.x]);
+                    if (p.y < b.y || p.y > b.w || p.x > b.z) continue;
+                }
+                SegGeom sg;
+                load_seg(S, it.y, sg);
+                const float e1 = __int_as_float(it.z);
+                int w;
+                if (!close && e1 >= 0.0f &&
+                    cell_winding_point(sg.kind, sg.q, e1, __int_as_float(it.w), p.x, p.y, &w))
+                    wind += w;
+                else if (!ray_misses_segment(sg, p))
+                    wind += winding_segment(sg, p);
             }
-            SegGeom sg;
-            load_seg(S, it.y, sg);
-            if (!ray_misses_segment(sg, p)) wind += winding_segment(sg, p);
         }
         items += n.segs;
         *fill = fill_hit(flags & CE_ODD ? 1 : 0, wind);
     }
     if (flags & CE_STROKE_TEST) {
         const bool approx = __ldg(&S.p_info[2 * __ldg(&S.s_info[B.x].z) + 1].w) & PF_APPROX;
+#pragma unroll 1
         for (int j = 0; j < n.strokes; ++j) {
             const int4 it = __ldg(&items[j]);
             if (it.x >= 0) {
@@ -169,7 +188,7 @@ __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, 
             } else if (stroke_misses_segment(sg, p)) {
                 continue;
             }
-            const CPRes c = seg_closest(sg, p, approx);
+            const CPRes c = seg_closest_plain(sg, p, approx);
             if (c.dist < seg_radius(sg, c.t)) {
                 *stroke = true;
                 break;

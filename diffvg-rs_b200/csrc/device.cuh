@@ -138,6 +138,10 @@ __device__ __forceinline__ float2 shape_local_bwd(const DevScene& S, int s, floa
 
 // ------------------------------------------------------------------ polynomial roots (f64, distance/utils.rs:48-123)
 // Out-of-line wrappers: one copy of each libm body per kernel instead of one per call site.
+// (f64 division and square root too: inlined, each of their two dozen sites here costs some
+// 400 bytes, and the kernels' time depends on their code staying in the instruction cache)
+static __device__ __noinline__ double dvg_div(double a, double b) { return a / b; }
+static __device__ __noinline__ double dvg_sqrt(double x) { return sqrt(x); }
 static __device__ __noinline__ double dvg_acos(double x) { return acos(x); }
 static __device__ __noinline__ double dvg_cos(double x) { return cos(x); }
 static __device__ __noinline__ double dvg_pow(double x, double y) { return pow(x, y); }
@@ -149,28 +153,28 @@ __device__ __forceinline__ bool solve_quadratic(double a, double b, double c, do
     const double eps = 1.0e-12;
     if (fabs(a) < eps) {
         if (fabs(b) < eps) return false;
-        double root = -c / b;
+        double root = dvg_div(-c, b);
         t[0] = root;
         t[1] = root;
         return true;
     }
     double discrim = b * b - 4.0 * a * c;
     if (discrim < 0.0) return false;
-    double root = sqrt(discrim);
+    double root = dvg_sqrt(discrim);
     if (fabs(root) < eps) {
-        double r = -0.5 * b / a;
+        double r = dvg_div(-0.5 * b, a);
         t[0] = r;
         t[1] = r;
         return true;
     }
     double q = (b < 0.0) ? -0.5 * (b - root) : -0.5 * (b + root);
     if (fabs(q) < eps) {
-        double inv = 0.5 / a;
+        double inv = dvg_div(0.5, a);
         t[0] = (-b - root) * inv;
         t[1] = (-b + root) * inv;
     } else {
-        t[0] = q / a;
-        t[1] = c / q;
+        t[0] = dvg_div(q, a);
+        t[1] = dvg_div(c, q);
     }
     if (t[0] > t[1]) {
         double tmp = t[0];
@@ -194,23 +198,25 @@ static __device__ __noinline__ int solve_cubic(double a, double b, double c, dou
         }
         return 0;
     }
-    b = b / a;
-    c = c / a;
-    d = d / a;
-    double q = (b * b - 3.0 * c) / 9.0;
-    double r = (2.0 * b * b * b - 9.0 * b * c + 27.0 * d) / 54.0;
+    b = dvg_div(b, a);
+    c = dvg_div(c, a);
+    d = dvg_div(d, a);
+    double q = dvg_div(b * b - 3.0 * c, 9.0);
+    double r = dvg_div(2.0 * b * b * b - 9.0 * b * c + 27.0 * d, 54.0);
     const double TWO_PI = 6.283185307179586476925286766559;
     if (r * r < q * q * q) {
-        double theta = dvg_acos(r / sqrt(q * q * q));
-        double sq = sqrt(q);
-        t[0] = -2.0 * sq * dvg_cos(theta / 3.0) - b / 3.0;
-        t[1] = -2.0 * sq * dvg_cos((theta + TWO_PI) / 3.0) - b / 3.0;
-        t[2] = -2.0 * sq * dvg_cos((theta - TWO_PI) / 3.0) - b / 3.0;
+        double theta = dvg_acos(dvg_div(r, dvg_sqrt(q * q * q)));
+        double sq = dvg_sqrt(q);
+        const double b3 = dvg_div(b, 3.0);
+        t[0] = -2.0 * sq * dvg_cos(dvg_div(theta, 3.0)) - b3;
+        t[1] = -2.0 * sq * dvg_cos(dvg_div(theta + TWO_PI, 3.0)) - b3;
+        t[2] = -2.0 * sq * dvg_cos(dvg_div(theta - TWO_PI, 3.0)) - b3;
         return 3;
     }
-    double ar = (r > 0.0) ? -cbrt_pow(r + sqrt(r * r - q * q * q)) : cbrt_pow(-r + sqrt(r * r - q * q * q));
-    double br = (fabs(ar) > 1.0e-6) ? q / ar : 0.0;
-    t[0] = (ar + br) - b / 3.0;
+    const double sd = dvg_sqrt(r * r - q * q * q);
+    double ar = (r > 0.0) ? -cbrt_pow(r + sd) : cbrt_pow(-r + sd);
+    double br = (fabs(ar) > 1.0e-6) ? dvg_div(q, ar) : 0.0;
+    t[0] = (ar + br) - dvg_div(b, 3.0);
     return 1;
 }
 
@@ -272,14 +278,18 @@ static __device__ DVG_QUAD_EXACT_ATTR int closest_quad_candidates_exact(double A
     double r[3];
     const int nr = solve_cubic(A, B, C, D, r);
     int n = 0;
+#pragma unroll 1
     for (int i = 0; i < nr; ++i)
         if (r[i] >= 0.0 && r[i] <= 1.0) t32[n++] = (float)r[i];
     return n;
 }
+// PLAIN: the crate's root formula without the certified shortcut (small code).
+template <bool PLAIN>
 static __device__ __noinline__ CPRes closest_quad_v(float2 pt, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, bool approx);
 __device__ __forceinline__ CPRes closest_quad(float2 pt, const float* q, bool approx) {
-    return closest_quad_v(pt, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], approx);
+    return closest_quad_v<DVG_EXACT_CLOSEST_QUAD>(pt, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], approx);
 }
+template <bool PLAIN>
 static __device__ __noinline__ CPRes closest_quad_v(float2 pt, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, bool approx) {
     const float q[8] = {a0, a1, a2, a3, a4, a5, a6, a7};  // curve.rs:26-78
     if (approx) return closest_quad_approx(pt, q);
@@ -305,12 +315,10 @@ static __device__ __noinline__ CPRes closest_quad_v(float2 pt, float a0, float a
     // the crate's candidates t32 = (float)t of the roots in [0, 1]: certified without its
     // acos / cos / pow when their side of 0 and 1 and their f32 rounding provably agree
     float cand[3];
-#if DVG_EXACT_CLOSEST_QUAD
-    const int n = closest_quad_candidates_exact(A, B, Cc, D, cand);
-#else
-    int n = closest_quad_roots_newton(A, B, Cc, D, cand);
+    int n = -1;
+    if constexpr (!PLAIN) n = closest_quad_roots_newton(A, B, Cc, D, cand);
     if (n < 0) n = closest_quad_candidates_exact(A, B, Cc, D, cand);
-#endif
+#pragma unroll 1
     for (int i = 0; i < n; ++i) {
         float t32 = cand[i];
         float tt = 1.0f - t32;
@@ -388,22 +396,24 @@ static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float 
     double d = 3.0 * ((bxx * cx + byy * cy) + (ax * dx + ay * dy));
     double e = (cx * cx + cy * cy) + 2.0 * (dx * bxx + dy * byy);
     double f = dx * cx + dy * cy;
-    b = b / a;
-    c = c / a;
-    d = d / a;
-    e = e / a;
-    f = f / a;
+    b = dvg_div(b, a);
+    c = dvg_div(c, a);
+    d = dvg_div(d, a);
+    e = dvg_div(e, a);
+    f = dvg_div(f, a);
     double p1a = (2.0 / 5.0) * c - (4.0 / 25.0) * b * b;
     double p1b = (3.0 / 5.0) * d - (3.0 / 25.0) * b * c;
     double p1c = (4.0 / 5.0) * e - (2.0 / 25.0) * b * d;
-    double p1d = f - b * e / 25.0;
-    double q_root = -b / 5.0;
+    double p1d = f - dvg_div(b * e, 25.0);
+    double q_root = dvg_div(-b, 5.0);
     double pr[3];
     int num_p = solve_cubic(p1a, p1b, p1c, p1d, pr);
     double iv[4];
     int ni = 0;
     if (q_root >= 0.0 && q_root <= 1.0) iv[ni++] = q_root;
+#pragma unroll 1
     for (int i = 0; i < num_p; ++i) iv[ni++] = pr[i];
+#pragma unroll 1
     for (int j = 1; j < ni; ++j) {
         int k = j;
         while (k > 0 && iv[k - 1] > iv[k]) {
@@ -414,6 +424,7 @@ static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float 
         }
     }
     double lower = 0.0;
+#pragma unroll 1
     for (int j = 0; j <= ni; ++j) {
         if (j < ni && iv[j] < 0.0) continue;
         double upper = (j < ni) ? fmin(iv[j], 1.0) : 1.0;
@@ -430,6 +441,7 @@ static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float 
             ub = t0;
         }
         double t = 0.5 * (lb + ub);
+#pragma unroll 1
         for (int it = 0; it < 20; ++it) {
             if (!(t >= lb && t <= ub)) t = 0.5 * (lb + ub);
             double v = ((((t + b) * t + c) * t + d) * t + e) * t + f;
@@ -439,7 +451,7 @@ static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float 
             else
                 lb = t;
             double dv = (((5.0 * t + 4.0 * b) * t + 3.0 * c) * t + 2.0 * d) * t + e;
-            t -= v / dv;
+            t -= dvg_div(v, dv);
         }
         if (t >= 0.0 && t <= 1.0) {
             float t32 = (float)t;
@@ -500,6 +512,7 @@ static __device__ DVG_WIND_EXACT_ATTR int winding_cubic_exact(double a, double b
     double r[3];
     int nr = solve_cubic(a, b, c, d, r);
     int w = 0;
+#pragma unroll 1
     for (int i = 0; i < nr; ++i) {
         double t = r[i];
         if (t >= 0.0 && t <= 1.0) {
@@ -509,9 +522,10 @@ static __device__ DVG_WIND_EXACT_ATTR int winding_cubic_exact(double a, double b
     }
     return w;
 }
-// winding.rs:118-192
-static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, float2 pt) {
-    const float q[8] = {a0, a1, a2, a3, a4, a5, a6, a7};
+// winding.rs:118-169: lines and quadratics
+static __device__ __noinline__ int winding_segment_low(int kind, float a0, float a1, float a2, float a3, float a4, float a5,
+                                                       float2 pt) {
+    const float q[6] = {a0, a1, a2, a3, a4, a5};
     if (kind == 0) {
         float dy = q[3] - q[1];
         if (fabsf(dy) <= 1.0e-8f) return 0;
@@ -522,7 +536,7 @@ static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a
         }
         return 0;
     }
-    if (kind == 1) {
+    {
         double a = (double)(q[1] - 2.0f * q[3] + q[5]);
         double b = (double)(-2.0f * q[1] + 2.0f * q[3]);
         double c = (double)(q[1] - pt.y);
@@ -530,7 +544,7 @@ static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a
         int nr = 0;
         if (fabs(a) < 1.0e-12) {
             if (fabs(b) > 1.0e-12) {
-                r[0] = -c / b;
+                r[0] = dvg_div(-c, b);
                 nr = 1;
             }
         } else if (solve_quadratic(a, b, c, r)) {
@@ -540,6 +554,7 @@ static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a
         double bx = (double)(-2.0f * q[0] + 2.0f * q[2]);
         double cx = (double)(q[0] - pt.x);
         int w = 0;
+#pragma unroll 1
         for (int i = 0; i < nr; ++i) {
             double t = r[i];
             if (t >= 0.0 && t <= 1.0) {
@@ -549,6 +564,11 @@ static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a
         }
         return w;
     }
+}
+// winding.rs:118-192
+static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, float2 pt) {
+    if (kind < 2) return winding_segment_low(kind, a0, a1, a2, a3, a4, a5, pt);
+    const float q[8] = {a0, a1, a2, a3, a4, a5, a6, a7};
     double a = (double)(-q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7]);
     double b = (double)(3.0f * q[1] - 6.0f * q[3] + 3.0f * q[5]);
     double c = (double)(-3.0f * q[1] + 3.0f * q[3]);
@@ -567,6 +587,16 @@ static __device__ __noinline__ int winding_segment_v(int kind, float a0, float a
 }
 __device__ __forceinline__ int winding_segment(const SegGeom& s, float2 pt) {
     return winding_segment_v(s.kind, s.q[0], s.q[1], s.q[2], s.q[3], s.q[4], s.q[5], s.q[6], s.q[7], pt);
+}
+
+// The crate's own formulas for the strokes that the cell lists' chord tests leave open (a few
+// percent of the samples): small code, since every excursion to it displaces the sample loop's
+// from the instruction cache.  Same results as seg_closest.
+__device__ __forceinline__ CPRes seg_closest_plain(const SegGeom& sg, float2 p, bool approx) {
+    if (sg.kind == 0) return closest_line(p, sg.q[0], sg.q[1], sg.q[2], sg.q[3]);
+    if (sg.kind == 1)
+        return closest_quad_v<true>(p, sg.q[0], sg.q[1], sg.q[2], sg.q[3], sg.q[4], sg.q[5], sg.q[6], sg.q[7], approx);
+    return closest_cubic(p, sg.q, approx);
 }
 
 // ------------------------------------------------------------------ exact-result culling
@@ -719,6 +749,7 @@ static __device__ __forceinline__ bool join_cap_hit_v(const int4* p_info, const 
     const float reach = (join == JOIN_MITER ? limit : 1.0f) * 1.001f;  // join regions lie within reach * r of v
     const float2 p = make_float2(px, py);
     const int off = pi.x, n = pi.y;
+#pragma unroll 1
     for (int k = 0; k < n; ++k) {
         const float4 a = __ldg(&seg_p[2 * (off + k)]), b = __ldg(&seg_p[2 * (off + k) + 1]);
         const float2 v = make_float2(a.x, a.y);
@@ -859,6 +890,7 @@ __device__ __forceinline__ int winding_path(const DevScene& S, int path, float2 
             continue;
         }
         if (m.z > 0) {
+#pragma unroll 1
             for (int k = m.y; k < m.y + m.z; ++k) {
                 SegGeom sg;
                 load_seg(S, __ldg(&S.pl_segs[k]), sg);
@@ -875,6 +907,7 @@ __device__ __forceinline__ int winding_path(const DevScene& S, int path, float2 
 __device__ __forceinline__ int winding_path_list(const DevScene& S, int path, float2 p) {
     int4 pi = __ldg(&S.p_info[2 * path]);
     int w = 0;
+#pragma unroll 1
     for (int k = 0; k < pi.y; ++k) {
         SegGeom sg;
         load_seg(S, pi.x + k, sg);
@@ -895,6 +928,7 @@ __device__ __forceinline__ bool within_path_bvh(const DevScene& S, int path, flo
             continue;
         }
         if (m.z > 0) {
+#pragma unroll 1
             for (int k = m.y; k < m.y + m.z; ++k) {
                 const int sidx = __ldg(&S.pl_segs[k]);
                 SegGeom sg;
@@ -915,6 +949,7 @@ __device__ __forceinline__ bool within_path_list(const DevScene& S, int path, fl
     int4 pi = __ldg(&S.p_info[2 * path]);
     const int pflags = __ldg(&S.p_info[2 * path + 1].w);
     bool approx = pflags & PF_APPROX;
+#pragma unroll 1
     for (int k = 0; k < pi.y; ++k) {
         SegGeom sg;
         load_seg(S, pi.x + k, sg);
@@ -940,6 +975,7 @@ static __device__ __noinline__ float2 closest_point_ellipse(float cx, float cy, 
     dx = fabsf(dx);
     dy = fabsf(dy);
     float t = dvg_atan2f(dy * rx, dx * ry);
+#pragma unroll 1
     for (int i = 0; i < 20; ++i) {
         float s = dvg_sinf(t), c = dvg_cosf(t);
         float g = rx * dx * s - ry * dy * c + (ry * ry - rx * rx) * s * c;
@@ -986,20 +1022,22 @@ __device__ __forceinline__ bool within_shape(const DevScene& S, int s, float2 lp
     return within_path_list(S, si.z, p);
 }
 // winding_number_shape (winding.rs:13-48); sp in shape space.
-__device__ __forceinline__ int winding_shape(const DevScene& S, int s, float2 sp, bool use_bvh) {
-    int4 si = __ldg(&S.s_info[s]);
-    float4 prm = __ldg(&S.s_params[s]);
-    if (si.x == K_CIRCLE) {
+__device__ __forceinline__ int winding_primitive(int kind, float4 prm, float2 sp) {
+    if (kind == K_CIRCLE) {
         float r = fabsf(prm.z);
         float dx = sp.x - prm.x, dy = sp.y - prm.y;
         return (dx * dx + dy * dy) < r * r ? 1 : 0;
     }
-    if (si.x == K_ELLIPSE) {
+    if (kind == K_ELLIPSE) {
         float rx = fmaxf(fabsf(prm.z), 1.0e-6f), ry = fmaxf(fabsf(prm.w), 1.0e-6f);
         float dx = (sp.x - prm.x) / rx, dy = (sp.y - prm.y) / ry;
         return dx * dx + dy * dy < 1.0f ? 1 : 0;
     }
-    if (si.x == K_RECT) return (sp.x > prm.x && sp.x < prm.z && sp.y > prm.y && sp.y < prm.w) ? 1 : 0;
+    return (sp.x > prm.x && sp.x < prm.z && sp.y > prm.y && sp.y < prm.w) ? 1 : 0;  // K_RECT
+}
+__device__ __forceinline__ int winding_shape(const DevScene& S, int s, float2 sp, bool use_bvh) {
+    int4 si = __ldg(&S.s_info[s]);
+    if (si.x != K_PATH) return winding_primitive(si.x, __ldg(&S.s_params[s]), sp);
     if (si.z < 0) return 0;
     int4 pi = __ldg(&S.p_info[2 * si.z]);
     if (use_bvh && pi.w > 0) return winding_path(S, si.z, sp);
@@ -1012,6 +1050,7 @@ __device__ __forceinline__ bool fill_hit(int rule, int w) { return rule == 1 ? (
 __device__ __forceinline__ bool group_within(const DevScene& S, int g, float2 lp) {
     int4 gb = __ldg(&S.g_bvh[g]);
     if (gb.y == 0) {
+#pragma unroll 1
         for (int k = 0; k < gb.w; ++k) {
             int s = __ldg(&S.g_shape_list[gb.z + k]);
             float sw = __ldg(&S.s_stroke[s]);
@@ -1029,6 +1068,7 @@ __device__ __forceinline__ bool group_within(const DevScene& S, int g, float2 lp
             continue;
         }
         if (m.z > 0) {
+#pragma unroll 1
             for (int k = m.y; k < m.y + m.z; ++k) {
                 int s = __ldg(&S.gl_shapes[k]);
                 float sw = __ldg(&S.s_stroke[s]);
@@ -1052,6 +1092,7 @@ __device__ __forceinline__ bool group_inside(const DevScene& S, int g, float2 lp
     int4 gb = __ldg(&S.g_bvh[g]);
     int w = 0;
     if (gb.y == 0) {
+#pragma unroll 1
         for (int k = 0; k < gb.w; ++k) {
             int s = __ldg(&S.g_shape_list[gb.z + k]);
             w += winding_shape(S, s, shape_local_dist(S, s, lp), false);
@@ -1071,6 +1112,7 @@ __device__ __forceinline__ bool group_inside(const DevScene& S, int g, float2 lp
             continue;
         }
         if (m.z > 0) {
+#pragma unroll 1
             for (int k = m.y; k < m.y + m.z; ++k) {
                 int s = __ldg(&S.gl_shapes[k]);
                 w += winding_shape(S, s, shape_local_dist(S, s, lp), true);
@@ -1087,6 +1129,7 @@ __device__ __forceinline__ bool group_inside(const DevScene& S, int g, float2 lp
 __device__ __forceinline__ float4 stops_color(const DevScene& S, int so, int sc, float t) {
     if (sc <= 0) return make_float4(0, 0, 0, 0);
     if (t < __ldg(&S.stop_offsets[so])) return __ldg(&S.stop_colors[so]);
+#pragma unroll 1
     for (int i = 0; i + 1 < sc; ++i) {
         float o0 = __ldg(&S.stop_offsets[so + i]), o1 = __ldg(&S.stop_offsets[so + i + 1]);
         if (t >= o0 && t < o1) {
@@ -1317,6 +1360,7 @@ static __device__ __forceinline__ PaintGradTerms gradient_paint_terms(const DevS
         r.c0 = dc;
         return r;
     }
+#pragma unroll 1
     for (int i = 0; i + 1 < sc; ++i) {
         float o0 = __ldg(&S.stop_offsets[so + i]), o1 = __ldg(&S.stop_offsets[so + i + 1]);
         if (t >= o0 && t < o1) {
@@ -1444,7 +1488,9 @@ static __device__ void d_gradient_paint_warp(const DevScene& S, const GradPtrs& 
 __device__ __forceinline__ void splat_sample(const DevScene& S, int x, int y, int ox, int oy, int ri, int HW,
                                              bool use_sm, float2 pt, float4 acc, float* sm, float* accum,
                                              float* wsum) {
+#pragma unroll 1
     for (int dy = -ri; dy <= ri; ++dy)
+#pragma unroll 1
         for (int dx = -ri; dx <= ri; ++dx) {
             int xx = x + dx, yy = y + dy;
             if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
@@ -1516,6 +1562,7 @@ __device__ __forceinline__ void splat_group(const DevScene& S, int x, int y, int
 // Flushes the CTA's pixels+halo accumulator (origin (ox, oy)) to global memory (one atomic per value).
 __device__ __forceinline__ void flush_splat(const DevScene& S, int ox, int oy, int HW, const float* sm, float* accum,
                                             float* wsum) {
+#pragma unroll 1
     for (int i = threadIdx.x; i < HW * HW; i += blockDim.x) {
         const float* c = sm + 5 * i;
         if (c[4] == 0.0f) continue;
@@ -1534,7 +1581,9 @@ __device__ __forceinline__ float4 gather_d_color(const DevScene& S, const float*
                                                  float2 ps) {
     float4 out = make_float4(0, 0, 0, 0);
     const int px = f2i(floorf(ps.x)), py = f2i(floorf(ps.y)), ri = S.filter_ri;
+#pragma unroll 1
     for (int dy = -ri; dy <= ri; ++dy)
+#pragma unroll 1
         for (int dx = -ri; dx <= ri; ++dx) {
             int xx = px + dx, yy = py + dy;
             if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
@@ -1561,7 +1610,9 @@ __device__ __forceinline__ float4 gather_d_color_radius(const DevScene& S, const
     float4 out = make_float4(0, 0, 0, 0), r4 = out;
     const int px = f2i(floorf(ps.x)), py = f2i(floorf(ps.y)), ri = S.filter_ri;
     const float r = S.filter_radius;
+#pragma unroll 1
     for (int dy = -ri; dy <= ri; ++dy)
+#pragma unroll 1
         for (int dx = -ri; dx <= ri; ++dx) {
             const int xx = px + dx, yy = py + dy;
             if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
@@ -1595,7 +1646,9 @@ __device__ __forceinline__ float filter_radius_adjoint(const DevScene& S, const 
                                                        float2 ps, float4 color) {
     float dradius = 0.0f;
     const int px = f2i(floorf(ps.x)), py = f2i(floorf(ps.y)), ri = S.filter_ri;
+#pragma unroll 1
     for (int dy = -ri; dy <= ri; ++dy)
+#pragma unroll 1
         for (int dx = -ri; dx <= ri; ++dx) {
             int xx = px + dx, yy = py + dy;
             if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;

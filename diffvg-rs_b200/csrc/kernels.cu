@@ -50,6 +50,7 @@ __device__ __forceinline__ bool tile_hits(const DevScene& S, int tile, float4 b)
 __global__ void __launch_bounds__(256) k_bin_count(DevScene S, const float4* g_bbox, int* counts) {
     int tile = blockIdx.x;
     int total = 0;
+#pragma unroll 1
     for (int base = 0; base < S.num_groups; base += blockDim.x) {
         int g = base + threadIdx.x;
         bool hit = false;
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(const int* counts, int n, int
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll 1
     for (int base = 0; base < n; base += 1024) {
         int i = base + threadIdx.x;
         int v = i < n ? counts[i] : 0;
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(256) k_bin_write(DevScene S, const float4* g_b
     int tile = blockIdx.x;
     int cursor = offsets[tile];
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll 1
     for (int base = 0; base < S.num_groups; base += blockDim.x) {
         int g = base + threadIdx.x;
         bool hit = false;
@@ -205,6 +208,7 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
     const int HW = (one_cell ? CELL : TILE) + 2 * ri;
     const int ox = (one_cell ? x & ~(CELL - 1) : tx * TILE) - ri, oy = (one_cell ? y & ~(CELL - 1) : ty * TILE) - ri;
     if (use_sm)
+#pragma unroll 1
         for (int i = threadIdx.x; i < HW * HW * 5; i += blockDim.x) sm[i] = 0.0f;
     __syncthreads();
     const bool valid = x < S.width && y < S.height;
@@ -225,6 +229,7 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
                            (pt.y / (float)S.height) * (float)S.height == pt.y;
         int nf = 0;
         acc = background_premul(S, y * S.width + x);
+#pragma unroll 1
         for (int k = 0; k < walk.n; ++k) {
             // stroke first, then fill; one paint call site for both
             const int4 A = cell_entry(S, walk, k);
@@ -279,7 +284,9 @@ __global__ void __launch_bounds__(256) k_weights(DevScene S, SampleParams sp, fl
     const int ri = S.filter_ri;
     const int sx = sub % sp.sxn, sy = sub / sp.sxn;
     const float2 pt = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, S.width, sp.seed, sp.jitter);
+#pragma unroll 1
     for (int dy = -ri; dy <= ri; ++dy)
+#pragma unroll 1
         for (int dx = -ri; dx <= ri; ++dx) {
             int xx = x + dx, yy = y + dy;
             if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
@@ -367,6 +374,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
         CellWalk walk{};
         if constexpr (!LEAN) walk = cell_walk(S, tile, cell_of_pix(pix));
         const int steps = LEAN ? cn : walk.n;
+#pragma unroll 1
         for (int k = 0; k < steps; ++k) {
             int e, hitp[2];
             if constexpr (LEAN) {
@@ -568,6 +576,7 @@ __device__ float4 edge_color(const DevScene& S, int tile, int cell, float2 pt, f
     const CellWalk walk = cell_walk(S, tile, cell);
     float4 acc = bg;
     int nfrag = 0, ev = 0;  // ev: 0 none, 1 last event sets the hit, 2 last event clears it
+#pragma unroll 1
     for (int k = 0; k < walk.n; ++k) {
         // stroke first, then fill; one paint call site for both
         const int4 A = cell_entry(S, walk, k);
@@ -752,6 +761,7 @@ __device__ float2 sample_join_cap(const DevScene& S, int path, float t, float2* 
         }
     }
     float len[3], total = 0.0f;
+#pragma unroll 1
     for (int i = 0; i < ne; ++i) {
         len[i] = len2(e[i + 1].x - e[i].x, e[i + 1].y - e[i].y);
         total += len[i];
@@ -941,6 +951,7 @@ __device__ float2 sample_boundary_path(const DevScene& S, int shape, float path_
         *pdf = 0.0f;
         return make_float2(0, 0);
     }
+#pragma unroll 1
     for (int k = 0; k < np; ++k) {
         long idx = (k == np - 1) ? nxt(pid + k) : (long)(pid + k);
         if (!path_pt_r(S, po, pc, closed, thick, idx, srad, &q[k], &r[k])) {
@@ -1396,7 +1407,9 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
     float4 dc = make_float4(0, 0, 0, 0);
     {
         const int px = f2i(floorf(sb.x)), py = f2i(floorf(sb.y)), ri = S.filter_ri;
+#pragma unroll 1
         for (int dy = -ri; dy <= ri; ++dy)
+#pragma unroll 1
             for (int dx = -ri; dx <= ri; ++dx) {
                 int xx = px + dx, yy = py + dy;
                 if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
@@ -1692,6 +1705,7 @@ __global__ void k_fill_background(DevScene S, float* out) {
 __global__ void k_l2(const float* img, const float* target, size_t n, float* d_render, float* loss) {
     __shared__ float red[8];
     float s = 0.0f;
+#pragma unroll 1
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float d = img[i] - target[i];
         d_render[i] = 2.0f * d;
@@ -1702,6 +1716,7 @@ __global__ void k_l2(const float* img, const float* target, size_t n, float* d_r
     __syncthreads();
     if (threadIdx.x == 0 && loss) {
         float t = 0.0f;
+#pragma unroll 1
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
         atomicAdd(loss, t);
     }
@@ -1733,6 +1748,7 @@ __global__ void k_l2_batch(const BatchEntry* __restrict__ B) {
     const BatchEntry& E = B[blockIdx.y];
     const size_t n = (size_t)E.S.width * E.S.height * 4;
     float s = 0.0f;
+#pragma unroll 1
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float d = E.image[i] - E.target[i];
         E.d_render[i] = 2.0f * d;
@@ -1743,6 +1759,7 @@ __global__ void k_l2_batch(const BatchEntry* __restrict__ B) {
     __syncthreads();
     if (threadIdx.x == 0) {
         float t = 0.0f;
+#pragma unroll 1
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
         atomicAdd(E.loss, t);
     }
@@ -1848,6 +1865,7 @@ int launch_boundary(const DevScene& S, const BoundaryParams& bp, const float* d_
     const int tiles = S.tiles_x * S.tiles_y * bnd_buckets(bp.cell);  // sort buckets
     const int segs = S.num_segs + S.num_shapes;
     int launches = 0;
+#pragma unroll 1
     for (uint64_t base = bp.sample_base; base < n; base += capacity) {
         const uint64_t cnt = base + capacity < n ? capacity : n - base;
         BoundaryParams b = bp;

@@ -74,6 +74,7 @@ static __device__ bool closest_path_bvh(const DevScene& S, int path, float2 p, f
         const int4 m = __ldg(&S.pn_meta[n]);
         if (box_distance(__ldg(&S.pn_bounds[n]), p) > best) continue;
         if (m.z > 0) {
+#pragma unroll 1
             for (int k = m.y; k < m.y + m.z; ++k) {
                 const int sidx = __ldg(&S.pl_segs[k]);
                 SegGeom sg;
@@ -153,6 +154,7 @@ static __device__ bool closest_shape(const DevScene& S, int s, float2 lp, float2
         float best = INF_F, bt = 0.0f;
         float2 bp = make_float2(0.0f, 0.0f);
         int bseg = 0;
+#pragma unroll 1
         for (int k = 0; k < pi.y; ++k) {
             SegGeom sg;
             load_seg(S, pi.x + k, sg);
@@ -182,6 +184,7 @@ static __device__ bool compute_distance_group(const DevScene& S, int g, float2 p
     const float2 lp = xf9(S.g_c2s + 9 * g, pt);
     if (gb.y == 0) {
         bool have = false;
+#pragma unroll 1
         for (int k = 0; k < gb.w; ++k) {
             const int s = __ldg(&S.g_shape_list[gb.z + k]);
             float2 lc;
@@ -208,6 +211,7 @@ static __device__ bool compute_distance_group(const DevScene& S, int g, float2 p
         const int4 m = __ldg(&S.gn_meta[n]);
         if (box_distance(__ldg(&S.gn_bounds[n]), lp) > best_dist) continue;
         if (m.z > 0) {
+#pragma unroll 1
             for (int k = m.y; k < m.y + m.z; ++k) {
                 const int s = __ldg(&S.gl_shapes[k]);
                 const int4 si = __ldg(&S.s_info[s]);
@@ -362,6 +366,7 @@ static __device__ __noinline__ bool styled_end_sd(const DevScene& S, int g, int 
     }
     // squared distance to the closest outer edge e[i] -> e[i + 1]
     Dl best = dl_const(0.0f);
+#pragma unroll 1
     for (int i = 0; i < ne; ++i) {
         const DV ex = dv_sub(e[i + 1], e[i]);
         const Dl ee = ex.x * ex.x + ex.y * ex.y;
@@ -382,6 +387,7 @@ static __device__ __noinline__ bool styled_end_sd(const DevScene& S, int g, int 
     const float2 v0 = make_float2(V.x.v, V.y.v);
     auto val = [](const DV& a) { return make_float2(a.x.v, a.y.v); };
     if (fan)
+#pragma unroll 1
         for (int i = 0; i < ne; ++i) inside = inside || in_triangle(pt, v0, val(e[i]), val(e[i + 1]));
     if (rect)
         inside = in_triangle(pt, val(e[0]), val(e[1]), val(e[2])) || in_triangle(pt, val(e[0]), val(e[2]), val(e[3]));
@@ -459,6 +465,7 @@ __device__ __forceinline__ bool pf_group_reaches(const DevScene& S, int tile, in
     float reach = 1.0f;
     if (gi.y >= 0) {
         const int4 gb = __ldg(&S.g_bvh[g]);
+#pragma unroll 1
         for (int k = 0; k < gb.w; ++k)
             reach = fmaxf(reach, 1.0f + fabsf(__ldg(&S.s_stroke[__ldg(&S.g_shape_list[gb.z + k])])));
     }
@@ -506,6 +513,7 @@ __device__ __forceinline__ void forward_prefilter_body(const DevScene& S, const 
     const int x = tx * TILE + (pix % TILE), y = ty * TILE + (pix / TILE);
     __shared__ int list[256], warp_cnt[8];
     if (use_sm)
+#pragma unroll 1
         for (int i = threadIdx.x; i < HW * HW * 5; i += blockDim.x) sm[i] = 0.0f;
     const bool valid = x < S.width && y < S.height;
     float2 pt = make_float2(0.0f, 0.0f);
@@ -515,9 +523,11 @@ __device__ __forceinline__ void forward_prefilter_body(const DevScene& S, const 
         pt = sample_pos(x, y, sx, sy, sp.sxn, sp.syn, S.width, sp.seed, false);
         acc = background_premul(S, y * S.width + x);
     }
+#pragma unroll 1
     for (int base = 0; base < S.num_groups; base += 256) {
         const int n = pf_bin_chunk(S, tile, base, list, warp_cnt);  // also orders the smem clear above
         if (!valid) continue;
+#pragma unroll 1
         for (int e = 0; e < n; ++e) {
             const int g = list[e];
             const int4 gi = __ldg(&S.g_info[g]);
@@ -790,6 +800,7 @@ static __device__ void d_closest_point_ellipse(float4 prm, float2 pt, float2 d_c
     float x = fabsf(lx), y = fabsf(ly);
     float t = dvg_atan2f(y * rx, x * ry);
     float g_t = 0.0f;
+#pragma unroll 1
     for (int i = 0; i < 20; ++i) {
         float sn = dvg_sinf(t), cs = dvg_cosf(t);
         float gg = rx * x * sn - ry * y * cs + (ry * ry - rx * rx) * sn * cs;
@@ -1032,9 +1043,11 @@ __device__ __forceinline__ void interior_prefilter_body(const DevScene& S, const
     int nf = 0;
     bool overflow = false;
     float4 acc = bg;
+#pragma unroll 1
     for (int base = 0; base < S.num_groups; base += 256) {
         const int n = pf_bin_chunk(S, tile, base, list, warp_cnt);
         if (!valid) continue;
+#pragma unroll 1
         for (int e = 0; e < n; ++e) {
             const int g = list[e];
             const int4 gi = __ldg(&S.g_info[g]);
@@ -1300,7 +1313,9 @@ __global__ void DVG_SDF_BOUNDS k_render_sdf(DevScene S, SampleParams sp, float* 
     if (x >= S.width || y >= S.height) return;
     const float inv_sx = 1.0f / (float)sp.sxn, inv_sy = 1.0f / (float)sp.syn;
     float acc = 0.0f;
+#pragma unroll 1
     for (int sy = 0; sy < sp.syn; ++sy)
+#pragma unroll 1
         for (int sx = 0; sx < sp.sxn; ++sx) {
             float rx = 0.5f, ry = 0.5f;
             if (sp.jitter) {

@@ -129,10 +129,10 @@ extern "C" void cell_winding_stress(int kind, int mode, uint64_t seed, uint64_t 
                 const float y = l + (rng.next() % 2 ? 1.0f : -1.0f) * r.tol * rng.range(1.0f, 1.5f);
                 if (y >= b.y0 && y <= b.y1) pt.y = y;
             }
-            if (r.nc && rng.next() % 2) {  // just outside the band of a parabola
+            if (r.nc && rng.next() % 2) {  // just outside the band of a curve
                 const dvgb::CellCurve& c = r.curve[rng.next() % (uint64_t)r.nc];
                 const float v = pt.y - dvgb::cc_row_centre(b);
-                const float x = c.c0 + (c.c1 + c.c2 * v) * v + (rng.next() % 2 ? 1.0f : -1.0f) * c.band * rng.range(1.0f, 1.5f);
+                const float x = c.c0 + (c.c1 + (c.c2 + c.c3 * v) * v) * v + (rng.next() % 2 ? 1.0f : -1.0f) * c.band * rng.range(1.0f, 1.5f);
                 if (x >= b.x0 && x <= b.x1) pt.x = x;
             }
             bool close = false;
@@ -140,7 +140,7 @@ extern "C" void cell_winding_stress(int kind, int mode, uint64_t seed, uint64_t 
             int w = r.base;
             for (int j = 0; j < r.nc; ++j) {
                 const float v = pt.y - dvgb::cc_row_centre(b);
-                const float dx = pt.x - (r.curve[j].c0 + (r.curve[j].c1 + r.curve[j].c2 * v) * v);
+                const float dx = pt.x - (r.curve[j].c0 + (r.curve[j].c1 + (r.curve[j].c2 + r.curve[j].c3 * v) * v) * v);
                 close = close || std::fabs(dx) <= r.curve[j].band;
                 if (dx < 0.0f) w += r.curve[j].sign;
             }
@@ -154,6 +154,38 @@ extern "C" void cell_winding_stress(int kind, int mode, uint64_t seed, uint64_t 
             const int ref = culled(p, pt) ? 0 : winding_number_segment((uint8_t)kind, p[0], p[1], p[2], p[3], pt);
             out[3] += 1;
             if (ref != w) out[5] += 1;
+        }
+    }
+}
+
+// The one-point version: points, points decided, decided with a crossing, decided and different
+// from the crate's winding.
+extern "C" void cell_point_stress(int kind, int mode, uint64_t seed, uint64_t n, int points, unsigned long long* out) {
+    SplitMix rng{seed * 0x2545f4914f6cdd1dull + (uint64_t)(mode * 3 + kind) + 177};
+    for (int k = 0; k < 4; ++k) out[k] = 0;
+    for (uint64_t i = 0; i < n; ++i) {
+        V2 p[4];
+        random_segment(rng, kind, mode, p);
+        const dvgb::CellBox b = random_box(rng, kind, p);
+        const float q[8] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y, p[3].x, p[3].y};
+        float e1, e2;
+        dvgb::cell_extrema(kind, q, dvgb::cc_max8(q), &e1, &e2);
+        for (int k = 0; k < points; ++k) {
+            V2 pt = random_point(rng, b, p);
+            if (rng.next() % 2) {  // near the curve or near an end's row
+                const float t = (float)rng.uni(), u = 1.0f - t, mag = (float)std::pow(10.0, -6.0 + 6.0 * rng.uni());
+                V2 on = kind == 0 ? p[0] * u + p[1] * t
+                        : kind == 1 ? p[0] * (u * u) + p[1] * (2 * u * t) + p[2] * (t * t)
+                                    : p[0] * (u * u * u) + p[1] * (3 * u * u * t) + p[2] * (3 * u * t * t) + p[3] * (t * t * t);
+                pt = on + mk(rng.range(-mag, mag), rng.range(-mag, mag));
+                if (rng.next() % 4 == 0) pt.y = (rng.next() % 2 ? p[0].y : p[3].y) + rng.range(-mag, mag);
+            }
+            out[0] += 1;
+            int w = 0;
+            if (!(e1 >= 0.0f) || !dvgb::cell_winding_point(kind, q, e1, e2, pt.x, pt.y, &w)) continue;
+            out[1] += 1;
+            if (w) out[2] += 1;
+            if (w != winding_number_segment((uint8_t)kind, p[0], p[1], p[2], p[3], pt)) out[3] += 1;
         }
     }
 }

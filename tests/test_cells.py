@@ -22,7 +22,7 @@ MODES = ("uniform", "integer", "near-degenerate", "large coordinates", "small an
 def stress():
     subprocess.run(["make", "-s", "-C", ORACLE], check=True)
     L = C.CDLL(LIB)
-    for f in (L.cell_winding_stress, L.cell_stroke_stress):
+    for f in (L.cell_winding_stress, L.cell_point_stress, L.cell_stroke_stress):
         f.argtypes = [C.c_int, C.c_int, C.c_uint64, C.c_uint64, C.c_int, C.POINTER(C.c_ulonglong)]
         f.restype = None
 
@@ -41,6 +41,14 @@ def test_cell_winding_never_disagrees(stress, kind, mode):
     assert wrong == 0, f"{wrong} of {tested} points differ from the crate's winding"
     # near-degenerate cubics are left to the per-sample test wherever they are ill conditioned
     assert decided >= (0.5 if mode == 2 and kind == 2 else 0.7) * boxes
+
+
+@pytest.mark.parametrize("mode", range(len(MODES)), ids=MODES)
+@pytest.mark.parametrize("kind", range(3), ids=KINDS)
+def test_point_winding_never_disagrees(stress, kind, mode):
+    points, decided, crossing, wrong, *_ = stress("cell_point_stress", kind, mode, 100_000)
+    assert wrong == 0, f"{wrong} of {points} points differ from the crate's winding"
+    assert crossing > 0 and decided >= (0.4 if mode in (1, 2, 5) else 0.55) * points  # half of them lie on or near the curve
 
 
 @pytest.mark.parametrize("mode", range(len(MODES)), ids=MODES)
