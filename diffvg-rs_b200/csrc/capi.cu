@@ -483,7 +483,7 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
     const HostScene& h = sc->host;
     Blob b;
     size_t o_g_c2s = b.add(h.g_c2s), o_g_s2c = b.add(h.g_s2c), o_g_info = b.add(h.g_info), o_g_bvh = b.add(h.g_bvh),
-           o_g_bbox = b.add(h.g_bbox), o_g_list = b.add(h.g_shape_list), o_gn_b = b.add(h.gn_bounds),
+           o_g_bbox = b.add(h.g_bbox), o_g_isig = b.add(h.g_isig), o_g_list = b.add(h.g_shape_list), o_gn_b = b.add(h.gn_bounds),
            o_gn_m = b.add(h.gn_meta), o_gl = b.add(h.gl_shapes), o_s_info = b.add(h.s_info),
            o_s_prm = b.add(h.s_params), o_s_inv = b.add(h.s_inv), o_s_x = b.add(h.s_xform),
            o_s_sw = b.add(h.s_stroke), o_s_box = b.add(h.s_box), o_s_pm = b.add(h.s_padmul),
@@ -562,6 +562,7 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
     S.path_len = (const float*)(base + o_plen);
     sc->g_bbox = (const float4*)(base + o_g_bbox);
     S.g_bbox = sc->g_bbox;
+    S.g_isig = (const float*)(base + o_g_isig);
     // tile binning
     S.tiles_x = (S.width + TILE - 1) / TILE;
     S.tiles_y = (S.height + TILE - 1) / TILE;

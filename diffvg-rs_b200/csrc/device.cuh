@@ -97,6 +97,7 @@ struct DevScene {
     const float* path_pmf;
     const int* path_pid;
     const float* path_len;
+    const float* g_isig;   // 1 / smallest stretch of a one-shape group's shape-to-canvas map, 0: unknown
     const float4* g_bbox;  // conservative canvas-space group boxes (binning, distance search skips)
     // tile binning
     int tiles_x, tiles_y;

@@ -56,15 +56,17 @@ struct ClosestD {
     float t;
 };
 
-// closest_point_path_bvh (closest.rs:104-199); cp in shape space.
-static __device__ bool closest_path_bvh(const DevScene& S, int path, float2 p, float2* cp, int* seg, float* tt,
-                                 unsigned* status) {
+// closest_point_path_bvh (closest.rs:104-199); cp in shape space.  `reach`: only a point nearer
+// than this is wanted (infinity: the crate's search); with it the walk starts from that bound,
+// so a path that is farther away costs its box tests, and the point found is the same.
+static __device__ bool closest_path_bvh(const DevScene& S, int path, float2 p, float reach, float2* cp, int* seg,
+                                 float* tt, unsigned* status) {
     const int4 pi = __ldg(&S.p_info[2 * path]);
     if (pi.w == 0) return false;
     const bool approx = __ldg(&S.p_info[2 * path + 1].w) & PF_APPROX;
-    float best = INF_F, bt = 0.0f;
+    float best = reach, bt = 0.0f;
     float2 bp = make_float2(0.0f, 0.0f);
-    int bseg = 0;
+    int bseg = -1;
     int stk[BVH_STACK];
     int sp = 0;
     stk[sp++] = pi.z;
@@ -105,7 +107,7 @@ static __device__ bool closest_path_bvh(const DevScene& S, int path, float2 p, f
             }
         }
     }
-    if (!isfinite(best)) return false;
+    if (bseg < 0 || !isfinite(best)) return false;
     *cp = bp;
     *seg = bseg;
     *tt = bt;
@@ -176,9 +178,17 @@ static __device__ bool closest_shape(const DevScene& S, int s, float2 lp, float2
     return true;
 }
 
+// Shape-space reach for a canvas distance `want` around p: a point of the shape that is farther
+// from p than this is farther than `want` on the canvas (S.g_isig: the map's smallest stretch;
+// the slack covers its 0.01 pixel and the f32 maps).
+__device__ __forceinline__ float shape_reach(const DevScene& S, int g, float want, float2 p) {
+    const float k = __ldg(&S.g_isig[g]);
+    return k > 0.0f ? (want + 0.03f) * k * 1.001f + 1.0e-4f * (1.0f + fabsf(p.x) + fabsf(p.y)) : INF_F;
+}
 // compute_distance_bvh (api.rs:138-236) with the brute-force fallback compute_distance (api.rs:36-76).
-static __device__ bool compute_distance_group(const DevScene& S, int g, float2 pt, float max_radius, ClosestD* best,
-                                       unsigned* status) {
+// `want`: the caller has no use for a canvas distance beyond it.
+static __device__ bool compute_distance_group(const DevScene& S, int g, float2 pt, float max_radius, float want,
+                                       ClosestD* best, unsigned* status) {
     const int4 gb = __ldg(&S.g_bvh[g]);
     const float* s2c = S.g_s2c + 9 * g;
     const float2 lp = xf9(S.g_c2s + 9 * g, pt);
@@ -221,7 +231,8 @@ static __device__ bool compute_distance_group(const DevScene& S, int g, float2 p
                 bool ok;
                 if (si.x == K_PATH && si.z >= 0 && __ldg(&S.p_info[2 * si.z].w) > 0) {
                     float2 scp;
-                    ok = closest_path_bvh(S, si.z, shape_local_dist(S, s, lp), &scp, &seg, &t, status);
+                    const float2 p = shape_local_dist(S, s, lp);
+                    ok = closest_path_bvh(S, si.z, p, shape_reach(S, g, want, p), &scp, &seg, &t, status);
                     if (ok) lc = xf9(S.s_xform + 9 * s, scp);
                 } else {
                     ok = closest_shape(S, s, lp, &lc, &seg, &t);
@@ -402,6 +413,15 @@ __device__ __forceinline__ bool maybe_styled_end(const DevScene& S, int s, int s
     return path >= 0 && (__ldg(&S.p_info[2 * path + 1].w) & PF_STYLED);
 }
 
+// Canvas distance beyond which a one-shape group's stroke has no coverage: its width + 1; a
+// styled one's join and cap regions reach farther.
+__device__ __forceinline__ float pf_stroke_reach(const DevScene& S, int g) {
+    const int s = __ldg(&S.gl_shapes[__ldg(&S.gn_meta[__ldg(&S.g_bvh[g].x)].y)]);
+    const int path = __ldg(&S.s_info[s].z);
+    if (path >= 0 && (__ldg(&S.p_info[2 * path + 1].w) & PF_STYLED)) return INF_F;
+    return fabsf(__ldg(&S.s_stroke[s])) + 1.0f;
+}
+
 // One prefiltered fragment (sampling.rs:240-300).
 struct PFragD {
     bool hit;
@@ -420,7 +440,10 @@ __device__ __forceinline__ PFragD prefilter_frag(const DevScene& S, int g, int w
     PFragD f;
     f.hit = false;
     ClosestD h;
-    const bool have = compute_distance_group(S, g, pt, which == 0 ? INF_F : 1.0f, &h, status);
+    // a fill takes distances up to 1, a round stroke changes up to its width + 1
+    float want = 1.0f;
+    if (which == 0) want = S.g_isig[g] > 0.0f ? pf_stroke_reach(S, g) : INF_F;
+    const bool have = compute_distance_group(S, g, pt, which == 0 ? INF_F : 1.0f, want, &h, status);
     float d, w;
     if (which == 0) {
         if (!have) return f;
@@ -1285,7 +1308,7 @@ static __device__ bool sdf_closest(const DevScene& S, const float4* g_bbox, floa
     for (int g = S.num_groups - 1; g >= 0; --g) {
         if (box_distance(__ldg(&g_bbox[g]), pt) > best_dist) continue;
         ClosestD h;
-        if (compute_distance_group(S, g, pt, best_dist, &h, status) && h.dist < best_dist) {
+        if (compute_distance_group(S, g, pt, best_dist, best_dist, &h, status) && h.dist < best_dist) {
             best_dist = h.dist;
             *best = h;
             *group = g;

@@ -529,6 +529,43 @@ dvg_status prepare_scene(const dvg_scene_desc* d, HostScene* out, std::string* e
         }
     }
 
+    // ---- distance bounds: 1 / the smallest singular value of a one-shape group's map from shape
+    // to canvas space (rounded up), where that map undoes canvas_to_shape and the shape's
+    // inverse over the canvas to 0.01 pixel; 0: no bound is known.
+    h.g_isig.assign(G, 0.0f);
+    for (uint32_t g = 0; g < G; ++g) {
+        const int32_t n0 = h.g_bvh[4 * (size_t)g], nn = h.g_bvh[4 * (size_t)g + 1];
+        if (nn != 1 || h.gn_meta[4 * (size_t)n0 + 2] != 1) continue;
+        const int32_t s = h.gl_shapes[h.gn_meta[4 * (size_t)n0 + 1]];
+        const int32_t fl = h.s_info[4 * (size_t)s + 1];
+        const float* c2s = &h.g_c2s[9 * (size_t)g];
+        const float* s2c = &h.g_s2c[9 * (size_t)g];
+        const float* X = &h.s_xform[9 * (size_t)s];
+        const float* iv = &h.s_inv[6 * (size_t)s];
+        double worst = 0.0;
+        for (int k = 0; k < 4; ++k) {
+            const double px = k & 1 ? (double)d->width + 2.0 : -2.0, py = k & 2 ? (double)d->height + 2.0 : -2.0;
+            double x = c2s[0] * px + c2s[1] * py + c2s[2], y = c2s[3] * px + c2s[4] * py + c2s[5];
+            if (!(fl & SF_IDENTITY) && (fl & SF_INVERTIBLE)) {
+                const double a = iv[0] * x + iv[1] * y + iv[2], b = iv[3] * x + iv[4] * y + iv[5];
+                x = a;
+                y = b;
+            }
+            const double u = X[0] * x + X[1] * y + X[2], v = X[3] * x + X[4] * y + X[5];
+            const double cx = s2c[0] * u + s2c[1] * v + s2c[2], cy = s2c[3] * u + s2c[4] * v + s2c[5];
+            const double e = std::fmax(std::fabs(cx - px), std::fabs(cy - py));
+            worst = e >= worst ? e : (e < worst ? worst : kInf);  // NaN: no bound
+        }
+        if (!(worst <= 0.01)) continue;
+        const double a = (double)s2c[0] * X[0] + (double)s2c[1] * X[3], b = (double)s2c[0] * X[1] + (double)s2c[1] * X[4];
+        const double c = (double)s2c[3] * X[0] + (double)s2c[4] * X[3], e = (double)s2c[3] * X[1] + (double)s2c[4] * X[4];
+        const double q = 0.5 * (a * a + b * b + c * c + e * e), det = a * e - b * c;
+        const double lo = q - std::sqrt(std::fmax(q * q - det * det, 0.0));  // smaller eigenvalue of M^T M
+        if (!(lo > 1.0e-12 * q && q > 0.0)) continue;
+        const float r = (float)(1.0001 / std::sqrt(lo));
+        if (std::isfinite(r)) h.g_isig[g] = r;
+    }
+
     // ---- boundary-sampling tables (src/backward/boundary.rs:46-451)
     h.shape_len.assign(S, 0.0f);
     auto seg_len = [&](uint32_t po, uint32_t pc, bool closed, size_t pid, int nc, bool* ok) -> float {

@@ -35,6 +35,7 @@ struct HostScene {
     std::vector<int32_t> g_info;       // 4 per group: fill paint, stroke paint, fill rule, 0
     std::vector<int32_t> g_bvh;        // 4 per group: node offset, node count, shape-list offset, shape-list count
     std::vector<float> g_bbox;         // 4 per group: canvas-space conservative bounds
+    std::vector<float> g_isig;         // per group: 1 / smallest stretch, shape to canvas (0: unknown)
     std::vector<int32_t> g_shape_list; // flat ShapeGroup::shape_indices (valid ids only)
     // group BVH nodes (global), preorder with skip links
     std::vector<float> gn_bounds;      // 4 per node

@@ -110,3 +110,37 @@ def test_edge_sample_counts(renderer, samples):
         a, b = g.buffers[name], gref[name]
         scale = float(np.max(np.abs(b))) + 1e-6
         assert float(np.max(np.abs(a - b))) <= 1e-4 * scale + 1e-6, name
+
+
+@pytest.mark.parametrize("how", ["scale 0.02", "scale 50", "skewed", "not the inverse", "singular", "two shapes"])
+def test_distance_reach(renderer, how):
+    """Searches that start from the distance they are asked for: prefiltered image and gradients
+    and the signed distance against the oracle's unbounded searches."""
+    import pyoracle
+
+    k = {"scale 0.02": 0.02, "scale 50": 50.0}.get(how, 1.0)
+    sc = _scene(45, 33, [_ring(7, 2, 0.0, 0.0, 3.0 / k, 14.0 / k, 8), _ring(6, 1, 20.0, 15.0, 3.0, 12.0, 9),
+                         _ring(5, 0, 30.0, 12.0, 2.0, 8.0, 10)], 0.0)
+    g = sc.groups[0]
+    g.set_shape_to_canvas(Mat3.translate(22.0, 16.0).mul(Mat3.rotate(0.7)).mul(Mat3.scale(k, k)))
+    sc.shapes[1].stroke_width = 1.5
+    sc.groups[1].stroke = Color(0.9, 0.1, 0.2, 0.8)
+    if how == "skewed":
+        g.set_shape_to_canvas(Mat3.translate(22.0, 16.0).mul(Mat3.rotate(0.7)).mul(Mat3.scale(3.0, 0.2)))
+    if how == "not the inverse":
+        g.canvas_to_shape = Mat3.scale(0.9, 1.1).mul(g.canvas_to_shape)
+    if how == "singular":
+        sc.shapes[1].transform = Mat3.scale(0.0, 1.0)
+    if how == "two shapes":
+        sc.groups[1].shape_indices = [1, 2]
+    opts = RenderOptions(samples_x=2, samples_y=2, seed=3, jitter=True, use_prefiltering=True)
+    assert float(np.max(np.abs(renderer.render(sc, opts).pixels - pyoracle.render(sc, opts)))) <= 1e-5
+    a, b = renderer.render_sdf(sc, opts).values, pyoracle.render_sdf(sc, opts).reshape(33, 45)
+    assert float(np.max(np.abs(a - b) / (1.0 + np.abs(b)))) <= 1e-5
+    d = np.random.default_rng(1).uniform(-1.0, 1.0, (33, 45, 4)).astype(np.float32)
+    gr = renderer.render_backward(sc, opts, BackwardOptions(), d)
+    _, ref = pyoracle.render_backward(sc, opts, BackwardOptions(), d)
+    for name in ("d_points", "d_paint_params", "d_shape_stroke_width"):
+        x, y = gr.buffers[name], ref[name]
+        scale = float(np.max(np.abs(y))) + 1e-6
+        assert float(np.max(np.abs(x - y))) <= 1e-4 * scale + 1e-6, name
