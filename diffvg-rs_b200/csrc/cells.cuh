@@ -9,7 +9,6 @@
 // do not describe (several shapes, styled strokes, strokes of ellipses and rectangles) keep the
 // full query.
 #pragma once
-#include "cell_classify.cuh"
 #include "device.cuh"
 
 namespace dvgb {

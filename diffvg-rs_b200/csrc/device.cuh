@@ -22,6 +22,7 @@
 #ifndef DVG_EXACT_CLOSEST_QUAD
 #define DVG_EXACT_CLOSEST_QUAD DVG_EXACT_ROOT_SOLVES
 #endif
+#include "cell_classify.cuh"
 #include "winding_newton.cuh"
 
 namespace dvgb {
@@ -861,13 +862,26 @@ __device__ __forceinline__ int seg_slot_point(int4 meta, int j, bool closed, int
     return closed ? idx % pc : idx;
 }
 
-// Nearest-segment searches keep a segment only when its distance is strictly below
-// the best so far; a cubic whose lower bound exceeds that by the culling margin
-// cannot be kept, so its exact solve is skipped (same argument as above).
-__device__ __forceinline__ bool cubic_cannot_beat(const SegGeom& s, float2 p, bool approx, float best) {
-    if (s.kind != 2 || approx || !(best < INFINITY)) return false;
-    return cubic_dist_lower(p.x, p.y, s.q[0], s.q[1], s.q[2], s.q[3], s.q[4], s.q[5], s.q[6], s.q[7]) >
-           best + cull_margin(s, p);
+// Nearest-segment searches keep a segment only when its distance is strictly below the best so
+// far: one whose control box, or whose chord polyline less its deviation, is farther than that
+// by the culling margin cannot be kept, so its exact solve is skipped.
+static __device__ __noinline__ float chord_dist_lower(int kind, float px, float py, float a0, float a1, float a2, float a3,
+                                                      float a4, float a5, float a6, float a7) {
+    const float q[8] = {a0, a1, a2, a3, a4, a5, a6, a7};
+    const CellChords c = cell_chords(kind, q);
+    return sqrtf(cell_chords_d2(c, px, py, 0, c.n)) - c.dev;
+}
+__device__ __forceinline__ bool segment_cannot_beat(const SegGeom& s, float2 p, bool approx, float best) {
+    if (!(best < INFINITY)) return false;
+    const float far = best + cull_margin(s, p);
+    const float xmin = fminf(fminf(s.q[0], s.q[2]), fminf(s.q[4], s.q[6]));
+    const float xmax = fmaxf(fmaxf(s.q[0], s.q[2]), fmaxf(s.q[4], s.q[6]));
+    const float ymin = fminf(fminf(s.q[1], s.q[3]), fminf(s.q[5], s.q[7]));
+    const float ymax = fmaxf(fmaxf(s.q[1], s.q[3]), fmaxf(s.q[5], s.q[7]));
+    const float dx = fmaxf(fmaxf(xmin - p.x, p.x - xmax), 0.0f), dy = fmaxf(fmaxf(ymin - p.y, p.y - ymax), 0.0f);
+    if (dx * dx + dy * dy > far * far) return true;
+    if (s.kind == 0 || approx) return false;
+    return chord_dist_lower(s.kind, p.x, p.y, s.q[0], s.q[1], s.q[2], s.q[3], s.q[4], s.q[5], s.q[6], s.q[7]) > far;
 }
 
 // ------------------------------------------------------------------ path queries

@@ -20,7 +20,7 @@
 // Minimum resident CTAs per SM for the scene-evaluation kernels (register cap =
 // 65536 / (threads * value)); chosen by measurement on B200.
 #ifndef DVG_MINB_FWD
-#define DVG_MINB_FWD 4
+#define DVG_MINB_FWD 5  // 48 registers: mixed 512x512 forward 0.82 -> 0.78 ms against 4 (3: 0.90, 6: 0.78, 8: 0.85)
 #endif
 #ifndef DVG_MINB_INT
 #define DVG_MINB_INT 2
@@ -568,6 +568,22 @@ static __device__ __noinline__ bool within_shape_any(const DevScene& S, int s, f
 static __device__ __noinline__ int winding_shape_any(const DevScene& S, int s, float2 sp) {
     return winding_shape(S, s, sp, true);
 }
+// Whether the group tests above, which found no hit of the queried group, are the queried
+// shape's own tests at lp: the group has no other shape, lp lies in its box (so the tests were
+// made) and both take the same point (shape_local_dist's identity shortcut is exact).  Half of
+// the samples' points end here, each with a walk over the whole path: 128x128 adjoint scene,
+// edge evaluation 0.32 -> 0.18 ms.
+__device__ __forceinline__ bool edge_tests_done(const DevScene& S, int g, int s, float2 lp) {
+    const int4 gb = __ldg(&S.g_bvh[g]);
+    if (gb.y != 1 || __ldg(&S.gn_meta[gb.x].z) != 1) return false;
+    const float4 b = __ldg(&S.gn_bounds[gb.x]);
+    if (!(lp.x >= b.x && lp.x <= b.z && lp.y >= b.y && lp.y <= b.w)) return false;
+    const int4 si = __ldg(&S.s_info[s]);
+    if (si.x == K_PATH && (si.z < 0 || (__ldg(&S.p_info[2 * si.z + 1].w) & PF_STYLED))) return false;
+    if (!(si.y & SF_IDENTITY)) return true;
+    const float* v = S.s_inv + 6 * s;
+    return v[0] == 1.0f && v[1] == 0.0f && v[2] == 0.0f && v[3] == 0.0f && v[4] == 1.0f && v[5] == 0.0f;
+}
 // sample_color with an EdgeQuery (sampling.rs:76-224, 485-552) at canvas point pt.
 // Returns the un-premultiplied colour (or the premultiplied background when no
 // fragment covers pt) and whether the queried shape is the visible boundary.
@@ -599,13 +615,15 @@ __device__ float4 edge_color(const DevScene& S, int tile, int cell, float2 pt, f
         bool hit0 = false;
         const int4 gi = __ldg(&S.g_info[eq_group]);
         const float2 lp = xf9(S.g_c2s + 9 * eq_group, pt);
-        if (gi.y >= 0) {
-            float sw = __ldg(&S.s_stroke[eq_shape]);
-            if (sw > 0.0f && within_shape_any(S, eq_shape, lp, sw)) hit0 = true;
-        }
-        if (gi.x >= 0) {
-            float2 sp = shape_local_bwd(S, eq_shape, lp);
-            if (fill_hit(gi.z, winding_shape_any(S, eq_shape, sp))) hit0 = true;
+        if (!edge_tests_done(S, eq_group, eq_shape, lp)) {
+            if (gi.y >= 0) {
+                float sw = __ldg(&S.s_stroke[eq_shape]);
+                if (sw > 0.0f && within_shape_any(S, eq_shape, lp, sw)) hit0 = true;
+            }
+            if (gi.x >= 0) {
+                float2 sp = shape_local_bwd(S, eq_shape, lp);
+                if (fill_hit(gi.z, winding_shape_any(S, eq_shape, sp))) hit0 = true;
+            }
         }
         *hit_out = hit0;
     }
@@ -1241,7 +1259,7 @@ __device__ void accumulate_boundary(const DevScene& S, const GradPtrs& G, int sh
 __device__ __forceinline__ void boundary_gen_one(const DevScene& S, uint64_t idx, uint64_t slot, uint32_t seed,
                                                  int rng_kind, int tile_off, int seg_off, int scene, int cell,
                                                  float pdf_scale, BSample* out, int2* key, int* tile_counts,
-                                                 int* seg_counts) {
+                                                 int* seg_bucket) {
     key[slot] = make_int2(-1, -1);
     float u, t;
     if (rng_kind == 1) {
@@ -1314,45 +1332,136 @@ __device__ __forceinline__ void boundary_gen_one(const DevScene& S, uint64_t idx
     const int seg = bd.base_point_id >= 0 && bd.base_point_id < ps.y ? ps.x + bd.base_point_id : S.num_segs + shape;
     key[slot] = make_int2(bucket, seg_off + seg);
     atomicAdd(tile_counts + bucket, 1);
-    atomicAdd(seg_counts + seg_off + seg, 1);
+    *seg_bucket = seg_off + seg;
+}
+// Counts of the segment buckets that a CTA's samples fall in, in shared memory while they span
+// at most SEG_SPAN buckets (a scene of few shapes has all its samples in a few dozen, and L2
+// serialises their atomics: 128x128 adjoint scene, drawing and scatter 0.145 -> 0.055 ms).
+constexpr int SEG_SPAN = 4096;
+constexpr int GEN_ITEMS = 4;  // samples per thread
+struct SegSpan {
+    int lo, hi;
+};
+__device__ __forceinline__ SegSpan seg_span(const int* bucket, int2* range) {
+    if (threadIdx.x == 0) *range = make_int2(0x7fffffff, -1);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < GEN_ITEMS; ++k)
+        if (bucket[k] >= 0) {
+            atomicMin(&range->x, bucket[k]);
+            atomicMax(&range->y, bucket[k]);
+        }
+    __syncthreads();
+    return SegSpan{range->x, range->y};
+}
+// Adds the CTA's buckets (-1: none) to the counts.
+__device__ __forceinline__ void seg_count(const int* bucket, int* seg_counts, int* hist, int2* range) {
+    const SegSpan sp = seg_span(bucket, range);
+    const int n = sp.hi - sp.lo + 1;
+    if (sp.hi < 0) return;
+    if (n > SEG_SPAN) {
+#pragma unroll
+        for (int k = 0; k < GEN_ITEMS; ++k)
+            if (bucket[k] >= 0) atomicAdd(seg_counts + bucket[k], 1);
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) hist[i] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < GEN_ITEMS; ++k)
+        if (bucket[k] >= 0) atomicAdd(hist + (bucket[k] - sp.lo), 1);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        if (hist[i]) atomicAdd(seg_counts + sp.lo + i, hist[i]);
 }
 __global__ void __launch_bounds__(256) k_boundary_gen(const __grid_constant__ DevScene S, BoundaryParams bp, BSample* out,
                                                       int2* key, int* tile_counts, int* seg_counts) {
-    const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x + bp.sample_base;
-    if (idx >= bp.num_samples) return;
-    boundary_gen_one(S, idx, idx - bp.slot_base, bp.seed, bp.rng, 0, 0, 0, bp.cell, bp.pdf_scale, out, key,
-                     tile_counts, seg_counts);
+    __shared__ int hist[SEG_SPAN];
+    __shared__ int2 range;
+    int bucket[GEN_ITEMS];
+#pragma unroll 1
+    for (int k = 0; k < GEN_ITEMS; ++k) {
+        const uint64_t idx = ((uint64_t)blockIdx.x * GEN_ITEMS + k) * blockDim.x + threadIdx.x + bp.sample_base;
+        int b = -1;
+        if (idx < bp.num_samples)
+            boundary_gen_one(S, idx, idx - bp.slot_base, bp.seed, bp.rng, 0, 0, 0, bp.cell, bp.pdf_scale, out, key,
+                             tile_counts, &b);
+#pragma unroll
+        for (int j = 0; j < GEN_ITEMS; ++j)
+            if (j == k) bucket[j] = b;
+    }
+    seg_count(bucket, seg_counts, hist, &range);
 }
 // Batched stage 1: one flat index over all scenes' boundary samples; the scene is
 // found by binary search over the per-scene sample offsets.
 __global__ void __launch_bounds__(256) k_boundary_gen_batch(const BatchEntry* __restrict__ B, int nscenes,
                                                             uint64_t total, int cell, BSample* out, int2* key,
                                                             int* tile_counts, int* seg_counts) {
-    const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int lo = 0, hi = nscenes - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (B[mid].b_off <= g)
-            lo = mid;
-        else
-            hi = mid - 1;
+    __shared__ int hist[SEG_SPAN];
+    __shared__ int2 range;
+    int bucket[GEN_ITEMS];
+#pragma unroll 1
+    for (int k = 0; k < GEN_ITEMS; ++k) {
+        const uint64_t g = ((uint64_t)blockIdx.x * GEN_ITEMS + k) * blockDim.x + threadIdx.x;
+        int b = -1;
+        if (g < total) {
+            int lo = 0, hi = nscenes - 1;
+            while (lo < hi) {
+                int mid = (lo + hi + 1) >> 1;
+                if (B[mid].b_off <= g)
+                    lo = mid;
+                else
+                    hi = mid - 1;
+            }
+            const BatchEntry& E = B[lo];
+            key[g] = make_int2(-1, -1);
+            if (E.S.boundary_ok && g - E.b_off < E.nb)
+                boundary_gen_one(E.S, g - E.b_off, g, E.bseed, E.rng, E.tile_off, E.seg_off, lo, cell, E.bscale, out,
+                                 key, tile_counts, &b);
+        }
+#pragma unroll
+        for (int j = 0; j < GEN_ITEMS; ++j)
+            if (j == k) bucket[j] = b;
     }
-    const BatchEntry& E = B[lo];
-    key[g] = make_int2(-1, -1);
-    if (!E.S.boundary_ok || g - E.b_off >= E.nb) return;
-    boundary_gen_one(E.S, g - E.b_off, g, E.bseed, E.rng, E.tile_off, E.seg_off, lo, cell, E.bscale, out, key,
-                     tile_counts, seg_counts);
+    seg_count(bucket, seg_counts, hist, &range);
 }
-// Stage 2: counting-sort scatter of sample slots, by cell and by segment.
-__global__ void k_boundary_scatter(const int2* key, uint64_t n, int* cursor, int* order, int* seg_cursor,
-                                   int* seg_order) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int2 k = key[i];
-    if (k.x < 0) return;
-    order[atomicAdd(cursor + k.x, 1)] = (int)i;
-    seg_order[atomicAdd(seg_cursor + k.y, 1)] = (int)i;
+// Stage 2: counting-sort scatter of sample slots, by cell and by segment (the latter through a
+// CTA's own counts, as in stage 1: one cursor atomic per bucket and CTA).
+__global__ void __launch_bounds__(256) k_boundary_scatter(const int2* key, uint64_t n, int* cursor, int* order,
+                                                          int* seg_cursor, int* seg_order) {
+    __shared__ int hist[SEG_SPAN];
+    __shared__ int2 range;
+    int bucket[GEN_ITEMS];
+    const uint64_t first = (uint64_t)blockIdx.x * GEN_ITEMS * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < GEN_ITEMS; ++k) {
+        const uint64_t i = first + (uint64_t)k * blockDim.x;
+        const int2 q = i < n ? key[i] : make_int2(-1, -1);
+        bucket[k] = q.y;
+        if (q.x >= 0) order[atomicAdd(cursor + q.x, 1)] = (int)i;
+    }
+    const SegSpan sp = seg_span(bucket, &range);
+    const int w = sp.hi - sp.lo + 1;
+    if (sp.hi < 0) return;
+    if (w > SEG_SPAN) {
+#pragma unroll
+        for (int k = 0; k < GEN_ITEMS; ++k)
+            if (bucket[k] >= 0) seg_order[atomicAdd(seg_cursor + bucket[k], 1)] = (int)(first + (uint64_t)k * blockDim.x);
+        return;
+    }
+    for (int i = threadIdx.x; i < w; i += blockDim.x) hist[i] = 0;
+    __syncthreads();
+    int rank[GEN_ITEMS];
+#pragma unroll
+    for (int k = 0; k < GEN_ITEMS; ++k)
+        rank[k] = bucket[k] >= 0 ? atomicAdd(hist + (bucket[k] - sp.lo), 1) : 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < w; i += blockDim.x)
+        if (hist[i]) hist[i] = atomicAdd(seg_cursor + sp.lo + i, hist[i]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < GEN_ITEMS; ++k)
+        if (bucket[k] >= 0) seg_order[hist[bucket[k] - sp.lo] + rank[k]] = (int)(first + (uint64_t)k * blockDim.x);
 }
 // Stage 3: evaluate both sides of every edge sample in tile order, so that the
 // lanes of a warp share one group list (render_edge_sample, boundary.rs:845-967).
@@ -1841,6 +1950,7 @@ int launch_interior(const DevScene& S, const SampleParams& sp, const float* d_re
     k_interior<<<grid, 256, 0, stream>>>(S, sp, d_render, wsum, G, status);
     return sp.frag ? 2 : 1;
 }
+static unsigned gen_grid(uint64_t n) { return (unsigned)((n + 256 * GEN_ITEMS - 1) / (256 * GEN_ITEMS)); }
 // Stages 2 to 4 for the n drawn samples in sc (counts filled by stage 1).
 template <typename Eval, typename Accum>
 static int boundary_stages(const BoundaryScratch& sc, uint64_t n, int tiles, int segs, cudaStream_t stream, Eval eval,
@@ -1853,7 +1963,7 @@ static int boundary_stages(const BoundaryScratch& sc, uint64_t n, int tiles, int
     // reuse the count arrays as the scatter cursors (copies of the exclusive offsets)
     cudaMemcpyAsync(sc.counts, offsets, sizeof(int) * (size_t)tiles, cudaMemcpyDeviceToDevice, stream);
     cudaMemcpyAsync(seg_counts, seg_offsets, sizeof(int) * (size_t)segs, cudaMemcpyDeviceToDevice, stream);
-    k_boundary_scatter<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(sc.key, n, sc.counts, sc.order, seg_counts,
+    k_boundary_scatter<<<gen_grid(n), 256, 0, stream>>>(sc.key, n, sc.counts, sc.order, seg_counts,
                                                                        sc.seg_order);
     eval(offsets, (unsigned)((2 * n + 127) / 128));
     accum(seg_offsets + segs, (unsigned)((n + 8 * ACC_SAMPLES - 1) / (8 * ACC_SAMPLES)));
@@ -1874,7 +1984,7 @@ int launch_boundary(const DevScene& S, const BoundaryParams& bp, const float* d_
         b.num_samples = base + cnt;
         cudaMemsetAsync(sc.counts, 0, sizeof(int) * (2 * (size_t)tiles + 1), stream);
         cudaMemsetAsync(sc.seg_counts, 0, sizeof(int) * (2 * (size_t)segs + 1), stream);
-        k_boundary_gen<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(S, b, sc.samples, sc.key, sc.counts,
+        k_boundary_gen<<<gen_grid(cnt), 256, 0, stream>>>(S, b, sc.samples, sc.key, sc.counts,
                                                                          sc.seg_counts);
         launches += 1 + boundary_stages(
             sc, cnt, tiles, segs, stream,
@@ -1953,7 +2063,7 @@ int launch_boundary_batch(const BatchEntry* B, int nscenes, uint64_t total, int 
     total_tiles *= bnd_buckets(cell);  // sort buckets
     cudaMemsetAsync(sc.counts, 0, sizeof(int) * (2 * (size_t)total_tiles + 1), stream);
     cudaMemsetAsync(sc.seg_counts, 0, sizeof(int) * (2 * (size_t)total_segs + 1), stream);
-    k_boundary_gen_batch<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(B, nscenes, total, cell, sc.samples,
+    k_boundary_gen_batch<<<gen_grid(total), 256, 0, stream>>>(B, nscenes, total, cell, sc.samples,
                                                                               sc.key, sc.counts, sc.seg_counts);
     return 1 + boundary_stages(
         sc, total, total_tiles, total_segs, stream,

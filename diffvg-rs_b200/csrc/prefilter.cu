@@ -20,11 +20,11 @@
 #include "device.cuh"
 #include "kernels.cuh"
 // Minimum resident CTAs per SM of the prefiltered forward and interior kernels, by
-// measurement on B200 (mixed 512x512 scene, 4x4 spp): the forward at 4 (64 registers,
-// spilling) 42.0 -> 36.4 ms against 2; the interior at 1 (168 registers, no spills)
-// 64.7 -> 62.6 ms against the compiler's own choice of 128.
+// measurement on B200 (mixed 512x512 scene): the forward at 6 (40 registers, 2x2 spp) 4.03 ->
+// 3.80 ms against 4 (5: 3.94, 3: 4.16); the interior at 1 (168 registers, no spills)
+// 9.18 ms (2: 10.3, 3: 10.2, 4: 9.8).
 #ifndef DVG_MINB_PF_FWD
-#define DVG_MINB_PF_FWD 4
+#define DVG_MINB_PF_FWD 6
 #endif
 #ifndef DVG_MINB_PF_INT
 #define DVG_MINB_PF_INT 1
@@ -81,7 +81,7 @@ static __device__ bool closest_path_bvh(const DevScene& S, int path, float2 p, f
                 const int sidx = __ldg(&S.pl_segs[k]);
                 SegGeom sg;
                 load_seg(S, sidx, sg);
-                if (cubic_cannot_beat(sg, p, approx, best)) continue;
+                if (segment_cannot_beat(sg, p, approx, best)) continue;
                 CPRes c = seg_closest(sg, p, approx);
                 if (c.dist < best) {
                     best = c.dist;
@@ -160,7 +160,7 @@ static __device__ bool closest_shape(const DevScene& S, int s, float2 lp, float2
         for (int k = 0; k < pi.y; ++k) {
             SegGeom sg;
             load_seg(S, pi.x + k, sg);
-            if (cubic_cannot_beat(sg, p, approx, best)) continue;
+            if (segment_cannot_beat(sg, p, approx, best)) continue;
             CPRes cc = seg_closest(sg, p, approx);
             if (cc.dist < best) {
                 best = cc.dist;
@@ -533,7 +533,8 @@ __device__ __forceinline__ void forward_prefilter_body(const DevScene& S, const 
     const int spp = sp.sxn * sp.syn;
     const int s_in_tile = round * 256 + (int)threadIdx.x;
     const int pix = sp.layout ? s_in_tile / spp : (int)threadIdx.x, sub = sp.layout ? s_in_tile % spp : round;
-    const int x = tx * TILE + (pix % TILE), y = ty * TILE + (pix / TILE);
+    const int2 pxy = pix_xy(pix);
+    const int x = tx * TILE + pxy.x, y = ty * TILE + pxy.y;
     __shared__ int list[256], warp_cnt[8];
     if (use_sm)
 #pragma unroll 1
@@ -564,7 +565,10 @@ __device__ __forceinline__ void forward_prefilter_body(const DevScene& S, const 
         }
     }
     __syncthreads();  // the splat tile is cleared even without groups
-    if (valid) splat_sample(S, x, y, tx * TILE - ri, ty * TILE - ri, ri, HW, use_sm, pt, acc, sm, accum, wsum);
+    if (use_sm && sp.layout && spp == 4)  // (the crate's default 2x2 samples)
+        splat_group<4>(S, x, y, tx * TILE - ri, ty * TILE - ri, ri, HW, valid, pt, acc, sm);
+    else if (valid)
+        splat_sample(S, x, y, tx * TILE - ri, ty * TILE - ri, ri, HW, use_sm, pt, acc, sm, accum, wsum);
     if (!use_sm) return;
     __syncthreads();
     flush_splat(S, tx * TILE - ri, ty * TILE - ri, HW, sm, accum, wsum);
@@ -1043,7 +1047,8 @@ __device__ __forceinline__ void interior_prefilter_body(const DevScene& S, const
     const int spp = sp.sxn * sp.syn;
     const int s_in_tile = round * 256 + (int)threadIdx.x;
     const int pix = sp.layout ? s_in_tile / spp : (int)threadIdx.x, sub = sp.layout ? s_in_tile % spp : round;
-    const int x = tx * TILE + (pix % TILE), y = ty * TILE + (pix / TILE);
+    const int2 pxy = pix_xy(pix);
+    const int x = tx * TILE + pxy.x, y = ty * TILE + pxy.y;
     const bool valid = x < S.width && y < S.height;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __shared__ int list[256], warp_cnt[8];
