@@ -636,6 +636,59 @@ __device__ __forceinline__ void d_xform_pt(const float* m, float2 p, float2 d_ou
     d_p->x += d0 * m[0] + d1 * m[3] + d2 * m[6];
     d_p->y += d0 * m[1] + d1 * m[4] + d2 * m[7];
 }
+// The same, dm as its left factor: dm = row (p.x, p.y, 1).
+__device__ __forceinline__ float3 d_xform_row(const float* m, float2 p, float2 d_out, float2* d_p) {
+    const float t0 = m[0] * p.x + m[1] * p.y + m[2];
+    const float t1 = m[3] * p.x + m[4] * p.y + m[5];
+    const float t2 = m[6] * p.x + m[7] * p.y + m[8];
+    const float ox = t0 / t2, oy = t1 / t2;
+    const float3 d = make_float3(d_out.x / t2, d_out.y / t2, -(d_out.x * ox + d_out.y * oy) / t2);
+    d_p->x += d.x * m[0] + d.y * m[3] + d.z * m[6];
+    d_p->y += d.x * m[1] + d.y * m[4] + d.z * m[7];
+    return d;
+}
+// out = row0 p0^T - (A^T row1) (A p1)^T, points homogeneous.
+__device__ __forceinline__ void transform_grad(float3 row0, float2 p0, const float* A, float3 row1, float2 p1, float* out) {
+    const float u[3] = {A[0] * row1.x + A[3] * row1.y + A[6] * row1.z, A[1] * row1.x + A[4] * row1.y + A[7] * row1.z,
+                        A[2] * row1.x + A[5] * row1.y + A[8] * row1.z};
+    const float v[3] = {A[0] * p1.x + A[1] * p1.y + A[2], A[3] * p1.x + A[4] * p1.y + A[5],
+                        A[6] * p1.x + A[7] * p1.y + A[8]};
+    const float r[3] = {row0.x, row0.y, row0.z}, q[3] = {p0.x, p0.y, 1.0f};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) out[3 * i + j] = r[i] * q[j] - u[i] * v[j];
+}
+// Adds the transform and stroke width gradients of a warp's samples: of those with `have`, tg
+// (as above; [18]: the stroke width's) goes to group g (uniform) and shape s.  The nineteen
+// sums over the warp's samples of one shape take 31 exchanges (each halves the values a lane
+// keeps) and leave sum k in lane k, so one add instruction reaches memory per warp and shape.
+__device__ __forceinline__ void add_transform_grads(const GradPtrs& G, int g, int s, bool have, const float* tg) {
+    const int lane = threadIdx.x & 31;
+    unsigned left = __ballot_sync(0xffffffffu, have);
+#pragma unroll 1
+    while (left) {
+        const int s0 = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+        const bool mine = have && s == s0;
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float a = mine ? tg[k] : 0.0f, b = k + 16 < 19 && mine ? tg[k + 16 < 19 ? k + 16 : 0] : 0.0f;
+            v[k] = (lane & 16 ? b : a) + __shfl_xor_sync(0xffffffffu, lane & 16 ? a : b, 16);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < o; ++k) {
+                const float a = v[k], b = v[k + o];
+                v[k] = (lane & o ? b : a) + __shfl_xor_sync(0xffffffffu, lane & o ? a : b, o);
+            }
+        float* d = lane < 9 ? G.d_group_transform + 9 * g + lane
+                            : (lane < 18 ? G.d_shape_transform + 9 * s0 + lane - 9 : G.d_shape_stroke_width + s0);
+        if (lane < 19) add_if(d, v[0]);
+        left &= ~__ballot_sync(0xffffffffu, mine);
+    }
+}
 __device__ __forceinline__ float2 d_length2(float2 v, float d_l) {
     float l = sqrtf(v.x * v.x + v.y * v.y);
     if (l == 0.0f) return make_float2(0.0f, 0.0f);
@@ -954,12 +1007,17 @@ static __device__ __noinline__ float2 d_styled_end(const DevScene& S, const Grad
     }
     return make_float2(-sum.x, -sum.y);
 }
-// d_compute_distance (distance.rs:50-136): geometry, shape and group transform
-// gradients by atomics; returns d_pt (for the translation adjoint).
+// d_compute_distance (distance.rs:50-136): geometry gradients by atomics; returns d_pt (for the
+// translation adjoint) and the gradients of the group's transform in tg[0..9) and of the shape's
+// in tg[9..18) for the caller to add: every sample of a group goes to these eighteen numbers.
 static __device__ float2 d_compute_distance(const DevScene& S, const GradPtrs& G, int g, int s, float2 pt, float2 cp,
-                                     int seg, float seg_t, float d_dist) {
+                                     int seg, float seg_t, float d_dist, float* tg) {
     float dx = pt.x - cp.x, dy = pt.y - cp.y;
-    if (dx * dx + dy * dy < 1.0e-10f) return make_float2(0.0f, 0.0f);
+    if (dx * dx + dy * dy < 1.0e-10f) {
+#pragma unroll
+        for (int k = 0; k < 18; ++k) tg[k] = 0.0f;
+        return make_float2(0.0f, 0.0f);
+    }
     const float* c2s = S.g_c2s + 9 * g;
     const float* s2c = S.g_s2c + 9 * g;
     const float* X = S.s_xform + 9 * s;
@@ -971,10 +1029,9 @@ static __device__ float2 d_compute_distance(const DevScene& S, const GradPtrs& G
     float2 dl = d_length2(make_float2(pt.x - cp.x, pt.y - cp.y), d_dist);
     float2 d_pt = dl;
     float2 d_closest = make_float2(-dl.x, -dl.y);
-    float d_s2c[9] = {0}, d_st[9] = {0}, d_sinv[9] = {0}, d_c2s[9] = {0};
     float2 d_lcg = make_float2(0, 0), d_lcs = make_float2(0, 0), d_lps = make_float2(0, 0), d_lpg = make_float2(0, 0);
-    d_xform_pt(s2c, lcg, d_closest, d_s2c, &d_lcg);
-    d_xform_pt(X, lcs, d_lcg, d_st, &d_lcs);
+    const float3 r_s2c = d_xform_row(s2c, lcg, d_closest, &d_lcg);
+    const float3 r_st = d_xform_row(X, lcs, d_lcg, &d_lcs);
     // d_closest_point (distance.rs:139-187)
     const int4 si = __ldg(&S.s_info[s]);
     const float4 prm = __ldg(&S.s_params[s]);
@@ -1014,26 +1071,13 @@ static __device__ float2 d_compute_distance(const DevScene& S, const GradPtrs& G
     } else if (si.x == K_PATH && seg >= 0 && si.z >= 0) {
         d_closest_point_path(S, G, s, lps, d_lcs, seg, seg_t, &d_lps);
     }
-    d_xform_pt(inv, lpg, d_lps, d_sinv, &d_lpg);
-    d_xform_pt(c2s, pt, d_lpg, d_c2s, &d_pt);
-    // d_group += d_s2c + (-c2s^T) d_c2s c2s^T ; d_shape += (-inv^T) d_sinv inv^T + d_st
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            float cg = 0.0f, cs = 0.0f;
-            for (int k = 0; k < 3; ++k) {
-                // (-A^T M)[r][k] summed against A^T[k][c] = A[c][k]
-                float mg = (-c2s[0 * 3 + r]) * d_c2s[0 * 3 + k] + (-c2s[1 * 3 + r]) * d_c2s[1 * 3 + k] +
-                           (-c2s[2 * 3 + r]) * d_c2s[2 * 3 + k];
-                float ms = (-inv[0 * 3 + r]) * d_sinv[0 * 3 + k] + (-inv[1 * 3 + r]) * d_sinv[1 * 3 + k] +
-                           (-inv[2 * 3 + r]) * d_sinv[2 * 3 + k];
-                cg += mg * c2s[3 * c + k];
-                cs += ms * inv[3 * c + k];
-            }
-            add_if(G.d_group_transform + 9 * g + 3 * r + c, (0.0f + d_s2c[3 * r + c]) + cg);
-            add_if(G.d_shape_transform + 9 * s + 3 * r + c, (0.0f + cs) + d_st[3 * r + c]);
-        }
+    const float3 r_sinv = d_xform_row(inv, lpg, d_lps, &d_lpg);
+    const float3 r_c2s = d_xform_row(c2s, pt, d_lpg, &d_pt);
+    // d_group = d_s2c - c2s^T d_c2s c2s^T ; d_shape = d_st - inv^T d_sinv inv^T.  Each d_M is the
+    // outer product of its row factor with the homogeneous point, so A^T d_M A^T is the one of
+    // A^T row and A point.
+    transform_grad(r_s2c, lcg, c2s, r_c2s, pt, tg);
+    transform_grad(r_st, lcs, inv, r_sinv, lpg, tg + 9);
     return d_pt;
 }
 
@@ -1200,42 +1244,53 @@ __device__ __forceinline__ void interior_prefilter_body(const DevScene& S, const
             }
             float2 tdelta = make_float2(0.0f, 0.0f);
             if (kind != P_SOLID) d_gradient_paint_warp(S, G, p, pt, dv, has && w != 0.0f, &tdelta);
-            if (!has || w == 0.0f) continue;
-            const float d = fdist[i];
-            float d_d;
-            bool geom = true;
-            if (which == 0 && styled) {
-                const float sw = __ldg(&S.s_stroke[fshape[i]]);
-                const float dp = d_smoothstep(sd.v + 2.0f * sw, d_w), dm = d_smoothstep(sd.v, d_w);
-                const float d_s = dp - dm;
-                add_if(G.d_shape_stroke_width + fshape[i], 2.0f * dp + d_s * sd.d[6]);
-                const float2 dpt = d_styled_end(S, G, g, fshape[i], sd, d_s, sids, sq);
-                tdelta.x += -dpt.x;
-                tdelta.y += -dpt.y;
-                d_d = 0.0f;
-                geom = false;
-            } else if (which == 0) {
-                const float sw = __ldg(&S.s_stroke[fshape[i]]);
-                const float ap = fabsf(d) + sw, am = fabsf(d) - sw;
-                const float dap = d_smoothstep(ap, d_w), dam = -d_smoothstep(am, d_w);
-                d_d = dap + dam;
-                if (d < 0.0f) d_d = -d_d;
-                add_if(G.d_shape_stroke_width + fshape[i], dap - dam);
-            } else {
-                d_d = d_smoothstep(d, d_w);
-                if (d < 0.0f) d_d = -d_d;
-                geom = fwithin[i];
+            float tg[19];
+#pragma unroll
+            for (int k = 0; k < 19; ++k) tg[k] = 0.0f;
+            const bool reached = has && w != 0.0f;
+            const int shape = reached ? fshape[i] : -1;
+            if (reached) {
+                const float d = fdist[i];
+                float d_d;
+                bool geom = true;
+                if (which == 0 && styled) {
+                    const float sw = __ldg(&S.s_stroke[shape]);
+                    const float dp = d_smoothstep(sd.v + 2.0f * sw, d_w), dm = d_smoothstep(sd.v, d_w);
+                    const float d_s = dp - dm;
+                    tg[18] = 2.0f * dp + d_s * sd.d[6];
+                    const float2 dpt = d_styled_end(S, G, g, shape, sd, d_s, sids, sq);
+                    tdelta.x += -dpt.x;
+                    tdelta.y += -dpt.y;
+                    d_d = 0.0f;
+                    geom = false;
+                } else if (which == 0) {
+                    const float sw = __ldg(&S.s_stroke[shape]);
+                    const float ap = fabsf(d) + sw, am = fabsf(d) - sw;
+                    const float dap = d_smoothstep(ap, d_w), dam = -d_smoothstep(am, d_w);
+                    d_d = dap + dam;
+                    if (d < 0.0f) d_d = -d_d;
+                    tg[18] = dap - dam;
+                } else {
+                    d_d = d_smoothstep(d, d_w);
+                    if (d < 0.0f) d_d = -d_d;
+                    geom = fwithin[i];
+                }
+                if (fabsf(d_d) > 1.0e-10f && geom) {
+                    float2 dpt = d_compute_distance(S, G, g, shape, pt, make_float2(fcx[i], fcy[i]), fseg[i], ft[i],
+                                                    d_d, tg);
+                    tdelta.x += -dpt.x;
+                    tdelta.y += -dpt.y;
+                }
+                if (G.d_translation) {
+                    add_if(G.d_translation + 2 * (size_t)pixel, tdelta.x);
+                    add_if(G.d_translation + 2 * (size_t)pixel + 1, tdelta.y);
+                }
             }
-            if (fabsf(d_d) > 1.0e-10f && geom) {
-                float2 dpt = d_compute_distance(S, G, g, fshape[i], pt, make_float2(fcx[i], fcy[i]), fseg[i], ft[i],
-                                                d_d);
-                tdelta.x += -dpt.x;
-                tdelta.y += -dpt.y;
-            }
-            if (G.d_translation) {
-                add_if(G.d_translation + 2 * (size_t)pixel, tdelta.x);
-                add_if(G.d_translation + 2 * (size_t)pixel + 1, tdelta.y);
-            }
+            bool some = tg[18] != 0.0f;
+#pragma unroll
+            for (int k = 0; k < 18; ++k) some = some || tg[k] != 0.0f;
+            __syncwarp();
+            add_transform_grads(G, g, shape, some, tg);
         }
     }
     float dradius = 0.0f;
@@ -1373,7 +1428,13 @@ __device__ __forceinline__ void sdf_adjoint(const DevScene& S, const GradPtrs& G
     int g = 0;
     if (!sdf_closest(S, S.g_bbox, pt, INF_F, &b, &g, status)) return;
     const float d_abs = sdf_inside(S, g, pt) ? -d_dist : d_dist;
-    const float2 dpt = d_compute_distance(S, G, g, b.shape, pt, b.point, b.seg, b.t, d_abs);
+    float tg[18];
+    const float2 dpt = d_compute_distance(S, G, g, b.shape, pt, b.point, b.seg, b.t, d_abs, tg);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        add_if(G.d_group_transform + 9 * g + k, tg[k]);
+        add_if(G.d_shape_transform + 9 * b.shape + k, tg[9 + k]);
+    }
     if (translation_pixel >= 0 && G.d_translation) {
         add_if(G.d_translation + 2 * (size_t)translation_pixel, -dpt.x);
         add_if(G.d_translation + 2 * (size_t)translation_pixel + 1, -dpt.y);
