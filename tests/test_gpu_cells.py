@@ -144,3 +144,32 @@ def test_distance_reach(renderer, how):
         x, y = gr.buffers[name], ref[name]
         scale = float(np.max(np.abs(y))) + 1e-6
         assert float(np.max(np.abs(x - y))) <= 1e-4 * scale + 1e-6, name
+
+
+@pytest.mark.parametrize("how", ["plain", "scale 0.02", "scale 50", "even odd", "no stroke width", "crowded",
+                                 "two shapes", "past the canvas"])
+def test_prefiltered_fill_and_stroke(renderer, how):
+    """One search for a group's fill and stroke, and the fill's inside test from the cell lists:
+    prefiltered image and gradients against the oracle, which searches and tests for each."""
+    import pyoracle
+
+    k = {"scale 0.02": 0.02, "scale 50": 50.0}.get(how, 1.0)
+    n = 300 if how == "crowded" else 9
+    rule = FillRule.EVEN_ODD if how == "even odd" else FillRule.NON_ZERO
+    sc = _scene(45, 33, [_ring(n, 2, 0.0, 0.0, 3.0 / k, 14.0 / k, 8), _ring(6, 1, 20.0, 15.0, 3.0, 12.0, 9),
+                         _ring(5, 0, 30.0, 12.0, 2.0, 8.0, 10)], 1.5, rule)
+    x, y = (2.0, 30.0) if how == "past the canvas" else (22.0, 16.0)
+    sc.groups[0].set_shape_to_canvas(Mat3.translate(x, y).mul(Mat3.rotate(0.7)).mul(Mat3.scale(k, k)))
+    if how == "no stroke width":
+        sc.shapes[1].stroke_width = 0.0
+    if how == "two shapes":
+        sc.groups[1].shape_indices = [1, 2]
+    opts = RenderOptions(samples_x=2, samples_y=2, seed=3, jitter=True, use_prefiltering=True)
+    assert float(np.max(np.abs(renderer.render(sc, opts).pixels - pyoracle.render(sc, opts)))) <= 1e-5
+    d = np.random.default_rng(1).uniform(-1.0, 1.0, (33, 45, 4)).astype(np.float32)
+    gr = renderer.render_backward(sc, opts, BackwardOptions(), d)
+    _, ref = pyoracle.render_backward(sc, opts, BackwardOptions(), d)
+    for name in ("d_points", "d_paint_params", "d_shape_stroke_width", "d_group_transform", "d_shape_transform"):
+        a, b = gr.buffers[name], ref[name]
+        scale = float(np.max(np.abs(b))) + 1e-6
+        assert float(np.max(np.abs(a - b))) <= 1e-4 * scale + 1e-6, name
