@@ -54,7 +54,7 @@ __device__ __forceinline__ int coded_curve(const CellCurve& q, int step) {
 
 __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene S, const CellTable T) {
     __shared__ CellBox cbox[CELLS], pbox[CELLS];
-    __shared__ int state[CELLS], base[CELLS], kept[CELLS], ent_base;
+    __shared__ int state[CELLS], base[CELLS], kept[CELLS], steps[CELLS], ent_base;
     __shared__ short leaf_of[CELL_MAX_SEGS];  // from the path's first node
     __shared__ uint8_t levels_of[CELL_MAX_SEGS][CELLS];
     // an entry's items, per cell (segments as leaf slots; stroke segments with their distance)
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
         const float px = 1.01e-4f * (float)S.width + 0.01f, py = 1.01e-4f * (float)S.height + 0.01f;
         cbox[tid] = CellBox{(float)x0 - px - (x0 == 0 ? 1.0f : 0.0f), (float)y0 - py - (y0 == 0 ? 1.0f : 0.0f),
                             (float)(x0 + CELL) + px, (float)(y0 + CELL) + py};
-        kept[tid] = 0;
+        kept[tid] = steps[tid] = 0;
     }
     __syncthreads();
     if (ent_base < 0) {
@@ -314,9 +314,10 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
         E[1] = make_int4(s, (base[c] & 0xffff) | (base_slow[c] << 16), at,
                          nl | (nc << 6) | (nh << 12) | (nf << 18) | (ns << 24));
         kept[c] += 1;
+        steps[c] += nl + nc + nh + ns;
     }
     __syncthreads();
-    if (tid < CELLS) T.info[tile * CELLS + tid] = make_int2(ent_base + tid * n, kept[tid]);
+    if (tid < CELLS) T.info[tile * CELLS + tid] = make_int2(ent_base + tid * n, kept[tid] | (steps[tid] >= CELL_HEAVY ? CELL_HEAVY_BIT : 0));
 }
 
 int launch_cells(const DevScene& S, const CellTable& T, cudaStream_t stream) {

@@ -68,11 +68,20 @@ static __device__ __noinline__ bool group_inside_any(const DevScene& S, int g, f
     return group_inside(S, g, lp, __ldg(&S.g_info[g].z));
 }
 
+// A cell is heavy from this many rows, curves and one-point segments in its lists.  The kernels
+// are bound by instruction fetch: where the lists are long, a CTA's warps take them one entry at
+// a time, so that they run the same code together (forward of the large 1024x1024 scene 18.5 ->
+// 14.7 ms, edge pass 62.9 -> 48.0).  From 40: 15.5 and 49.0 ms, from 64: 17.4 and 55.9; short
+// lists lose by it (mixed 512x512 scene, forward 0.81 ms, 0.85 with every list in steps).
+constexpr int CELL_HEAVY = 24;
+constexpr int CELL_HEAVY_BIT = 1 << 30;
+
 // The groups to visit at one cell: the cell's entries, or the tile's whole list.
 struct CellWalk {
     const int4* ent;
     const int* list;
     int n;
+    bool heavy;  // its items take CELL_HEAVY steps or more
 };
 __device__ __forceinline__ CellWalk cell_walk(const DevScene& S, int tile, int cell) {
     CellWalk w;
@@ -80,12 +89,14 @@ __device__ __forceinline__ CellWalk cell_walk(const DevScene& S, int tile, int c
     if (info.y >= 0) {
         w.ent = S.cell_entries + 2 * (size_t)info.x;
         w.list = nullptr;
-        w.n = info.y;
+        w.n = info.y & ~CELL_HEAVY_BIT;
+        w.heavy = info.y & CELL_HEAVY_BIT;
     } else {
         const int off = S.tile_offsets[tile];
         w.ent = nullptr;
         w.list = S.tile_entries + off;
         w.n = S.tile_offsets[tile + 1] - off;
+        w.heavy = false;
     }
     return w;
 }

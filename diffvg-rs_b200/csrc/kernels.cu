@@ -25,8 +25,15 @@
 #ifndef DVG_MINB_INT
 #define DVG_MINB_INT 2
 #endif
+// The edge evaluation is bound by instruction fetch: 512 threads of a CTA that take a heavy cell's
+// entries together, at 40 registers, against 128 threads at 32 that run apart: edge pass of the
+// large 1024x1024 scene 62.0 -> 48.0 ms, mixed 0.43 -> 0.41 (together: 128 threads 59.9 ms, 256
+// 52.4, 512 at 32 registers 49.8 and at 64 51.7, 1024 at 64 59.1).
+#ifndef DVG_BND_THREADS
+#define DVG_BND_THREADS 512
+#endif
 #ifndef DVG_MINB_BND
-#define DVG_MINB_BND 16  // 32 registers: more warps for the two-lane edge evaluation outweigh its spills
+#define DVG_MINB_BND 3
 #endif
 #ifndef DVG_MINB_LEAN
 #define DVG_MINB_LEAN 4
@@ -229,8 +236,11 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
                            (pt.y / (float)S.height) * (float)S.height == pt.y;
         int nf = 0;
         acc = background_premul(S, y * S.width + x);
+        // one list for the CTA, and all of its threads here: entry by entry if the list is heavy
+        const bool step = one_cell && walk.heavy && (tx + 1) * TILE <= S.width && (ty + 1) * TILE <= S.height;
 #pragma unroll 1
         for (int k = 0; k < walk.n; ++k) {
+            if (step) __syncthreads();
             // stroke first, then fill; one paint call site for both
             const int4 A = cell_entry(S, walk, k);
             bool hit[2];
@@ -410,6 +420,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
         atomicOr(status, ST_FRAGMENT_OVERFLOW);
         nf = 0;
     }
+    __syncthreads();  // the CTA's warps fetch one pass's instructions at a time: 0.874 -> 0.836 ms (mixed scene)
     const bool active = valid && !overflow;
     // Final colour and the adjoint at the end of compositing (sampling.rs:161-174).
     float4 ret = bg;
@@ -572,7 +583,7 @@ static __device__ __noinline__ int winding_shape_any(const DevScene& S, int s, f
 // shape's own tests at lp: the group has no other shape, lp lies in its box (so the tests were
 // made) and both take the same point (shape_local_dist's identity shortcut is exact).  Half of
 // the samples' points end here, each with a walk over the whole path: 128x128 adjoint scene,
-// edge evaluation 0.32 -> 0.18 ms.
+// the edge pass 0.53 -> 0.40 ms (256x256 scene of filled outlines, 200,000 samples).
 __device__ __forceinline__ bool edge_tests_done(const DevScene& S, int g, int s, float2 lp) {
     const int4 gb = __ldg(&S.g_bvh[g]);
     if (gb.y != 1 || __ldg(&S.gn_meta[gb.x].z) != 1) return false;
@@ -587,13 +598,17 @@ __device__ __forceinline__ bool edge_tests_done(const DevScene& S, int g, int s,
 // sample_color with an EdgeQuery (sampling.rs:76-224, 485-552) at canvas point pt.
 // Returns the un-premultiplied colour (or the premultiplied background when no
 // fragment covers pt) and whether the queried shape is the visible boundary.
-__device__ float4 edge_color(const DevScene& S, int tile, int cell, float2 pt, float4 bg, int eq_group, int eq_shape,
-                             bool* hit_out) {
-    const CellWalk walk = cell_walk(S, tile, cell);
+// All threads of the CTA call it (`valid` false: no point).
+__device__ __forceinline__ float4 edge_color(const DevScene& S, bool valid, int tile, int cell, float2 pt, float4 bg,
+                                             int eq_group, int eq_shape, bool* hit_out) {
+    CellWalk walk{};
+    if (valid) walk = cell_walk(S, tile, cell);
+    const bool step = __syncthreads_or(walk.heavy);  // (the CTA's samples share a cell or neighbouring ones)
     float4 acc = bg;
     int nfrag = 0, ev = 0;  // ev: 0 none, 1 last event sets the hit, 2 last event clears it
 #pragma unroll 1
-    for (int k = 0; k < walk.n; ++k) {
+    for (int k = 0; step ? __syncthreads_or(k < walk.n) : k < walk.n; ++k) {
+        if (k >= walk.n) continue;
         // stroke first, then fill; one paint call site for both
         const int4 A = cell_entry(S, walk, k);
         bool hit[2];
@@ -608,6 +623,7 @@ __device__ float4 edge_color(const DevScene& S, int tile, int cell, float2 pt, f
             if (A.y == eq_group) ev = 1;
         }
     }
+    if (!valid) return bg;
     if (ev != 0) {
         *hit_out = ev == 1;
     } else {  // no deciding fragment: the edge tests on the queried shape alone
@@ -1336,7 +1352,7 @@ __device__ __forceinline__ void boundary_gen_one(const DevScene& S, uint64_t idx
 }
 // Counts of the segment buckets that a CTA's samples fall in, in shared memory while they span
 // at most SEG_SPAN buckets (a scene of few shapes has all its samples in a few dozen, and L2
-// serialises their atomics: 128x128 adjoint scene, drawing and scatter 0.145 -> 0.055 ms).
+// serialises their atomics: edge pass of the adjoint scene 0.40 -> 0.33 ms).
 constexpr int SEG_SPAN = 4096;
 constexpr int GEN_ITEMS = 4;  // samples per thread
 struct SegSpan {
@@ -1480,15 +1496,17 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
     float4 cs = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     bool hs = false;
     float4 bg = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int tile = 0, cell = 0;
+    float2 q = make_float2(0.0f, 0.0f);
     if (valid) {
         bg = background_premul(S, r.pixel);
         const int bx = r.pixel % S.width, by = r.pixel / S.width;
-        const int tile = (by / TILE) * S.tiles_x + bx / TILE;
-        const int cell = (by % TILE) / CELL * (TILE / CELL) + (bx % TILE) / CELL;
+        tile = (by / TILE) * S.tiles_x + bx / TILE;
+        cell = (by % TILE) / CELL * (TILE / CELL) + (bx % TILE) / CELL;
         const float o = side == 0 ? -1.0e-4f : 1.0e-4f;
-        const float2 q = make_float2(r.bx + r.nx * o, r.by + r.ny * o);
-        cs = edge_color(S, tile, cell, make_float2(q.x * W, q.y * H), bg, r.group, r.shape, &hs);
+        q = make_float2(r.bx + r.nx * o, r.by + r.ny * o);
     }
+    cs = edge_color(S, valid, tile, cell, make_float2(q.x * W, q.y * H), bg, r.group, r.shape, &hs);
     float4 co;
     co.x = __shfl_xor_sync(0xffffffffu, cs.x, 1);
     co.y = __shfl_xor_sync(0xffffffffu, cs.y, 1);
@@ -1552,7 +1570,7 @@ __device__ __forceinline__ void boundary_eval_pair(const DevScene& S, const BSam
     }
 }
 // Two threads per sample (boundary_eval_pair): launch 2 * samples threads.
-__global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval(const __grid_constant__ DevScene S,
+__global__ void __launch_bounds__(DVG_BND_THREADS, DVG_MINB_BND) k_boundary_eval(const __grid_constant__ DevScene S,
                                                                      BSample* samples, const int* order,
                                                                      const int* offsets, int tiles,
                                                                      const float* d_render, const float* wsum,
@@ -1564,7 +1582,7 @@ __global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval(const __gri
     if (valid) r = samples[at];
     boundary_eval_pair(S, r, valid, d_render, wsum, d_translation, samples + at);
 }
-__global__ void __launch_bounds__(128, DVG_MINB_BND) k_boundary_eval_batch(const BatchEntry* __restrict__ B,
+__global__ void __launch_bounds__(DVG_BND_THREADS, DVG_MINB_BND) k_boundary_eval_batch(const BatchEntry* __restrict__ B,
                                                                            BSample* samples, const int* order,
                                                                            const int* offsets, int tiles) {
     const int64_t i = (int64_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1);
@@ -1965,7 +1983,7 @@ static int boundary_stages(const BoundaryScratch& sc, uint64_t n, int tiles, int
     cudaMemcpyAsync(seg_counts, seg_offsets, sizeof(int) * (size_t)segs, cudaMemcpyDeviceToDevice, stream);
     k_boundary_scatter<<<gen_grid(n), 256, 0, stream>>>(sc.key, n, sc.counts, sc.order, seg_counts,
                                                                        sc.seg_order);
-    eval(offsets, (unsigned)((2 * n + 127) / 128));
+    eval(offsets, (unsigned)((2 * n + DVG_BND_THREADS - 1) / DVG_BND_THREADS));
     accum(seg_offsets + segs, (unsigned)((n + 8 * ACC_SAMPLES - 1) / (8 * ACC_SAMPLES)));
     return launches + 3;
 }
@@ -1989,7 +2007,7 @@ int launch_boundary(const DevScene& S, const BoundaryParams& bp, const float* d_
         launches += 1 + boundary_stages(
             sc, cnt, tiles, segs, stream,
             [&](const int* offsets, unsigned grid) {
-                k_boundary_eval<<<grid, 128, 0, stream>>>(S, sc.samples, sc.order, offsets, tiles, d_render, wsum,
+                k_boundary_eval<<<grid, DVG_BND_THREADS, 0, stream>>>(S, sc.samples, sc.order, offsets, tiles, d_render, wsum,
                                                           G.d_translation);
             },
             [&](const int* total, unsigned grid) {
@@ -2068,7 +2086,7 @@ int launch_boundary_batch(const BatchEntry* B, int nscenes, uint64_t total, int 
     return 1 + boundary_stages(
         sc, total, total_tiles, total_segs, stream,
         [&](const int* offsets, unsigned grid) {
-            k_boundary_eval_batch<<<grid, 128, 0, stream>>>(B, sc.samples, sc.order, offsets, total_tiles);
+            k_boundary_eval_batch<<<grid, DVG_BND_THREADS, 0, stream>>>(B, sc.samples, sc.order, offsets, total_tiles);
         },
         [&](const int* tot, unsigned grid) {
             if (styled)

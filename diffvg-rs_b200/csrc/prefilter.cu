@@ -580,9 +580,10 @@ __device__ __forceinline__ void forward_prefilter_body(const DevScene& S, const 
 #pragma unroll 1
     for (int base = 0; base < S.num_groups; base += 256) {
         const int n = pf_bin_chunk(S, tile, base, list, warp_cnt);  // also orders the smem clear above
-        if (!valid) continue;
 #pragma unroll 1
         for (int e = 0; e < n; ++e) {
+            __syncthreads();  // warps search one group at a time, for the instruction cache: 2.75 -> 2.40 ms (mixed scene)
+            if (!valid) continue;
             const int g = list[e];
             const int4 gi = __ldg(&S.g_info[g]);
             ClosestD h;
@@ -1188,6 +1189,7 @@ __device__ __forceinline__ void interior_prefilter_body(const DevScene& S, const
         atomicOr(status, ST_FRAGMENT_OVERFLOW);
         nf = 0;
     }
+    __syncthreads();  // the CTA's warps fetch one pass's instructions at a time: 6.17 -> 4.86 ms (mixed scene)
     const bool active = valid && !overflow;
     float4 ret = bg;
     float dcr = dcol.x, dcg = dcol.y, dcb = dcol.z, dca = dcol.w;

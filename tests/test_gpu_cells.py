@@ -173,3 +173,11 @@ def test_prefiltered_fill_and_stroke(renderer, how):
         a, b = gr.buffers[name], ref[name]
         scale = float(np.max(np.abs(b))) + 1e-6
         assert float(np.max(np.abs(a - b))) <= 1e-4 * scale + 1e-6, name
+
+
+@pytest.mark.parametrize("spp", [(2, 2), (4, 4), (5, 4), (8, 8)])
+def test_long_lists(renderer, spp):
+    """Cells with many groups of many list items, which a CTA takes entry by entry: in whole
+    tiles, in tiles that the canvas cuts, with one cell to a CTA and with several."""
+    paths = [_ring(40, i % 3, 20.0 + i, 18.0, 6.0, 17.0, 20 + i) for i in range(8)]
+    _check(renderer, _scene(53, 41, paths, 0.7), spp)
