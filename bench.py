@@ -41,6 +41,9 @@ UNIT = "Msamples/s"
 LARGE_FIT_LR = 0.1  # Adam step on path points (pixels) and paint parameters of the large fitting loop
 
 
+FORWARD_CTAS_PER_SM = 5  # k_forward's register bound (csrc/kernels.cu)
+
+
 def workload(name: str, seed: int):
     if name == "mixed":
         sc = synth.mixed_scene(seed)
@@ -229,7 +232,7 @@ def compute_roofline(workload, prof, up, W, H, dev, clocks):
     peak = sms * 128 * mhz * 1e6 / 1e12
     achieved = work["total_flops"] / (avg_ms / 1e3) / 1e12 if work and avg_ms > 0 else None
     kernels, fresh, src = ncu_figures(workload)
-    # the forward kernel is a template over its resident CTAs per SM (k_forward<2>, k_forward<3>);
+    # the forward kernel is a template over the lanes that share a pixel (k_forward<4>, k_forward<16>);
     # the captured step ran the shape the autotuner picked
     fk = next((v for k, v in kernels.items() if k == "k_forward" or k.startswith("k_forward<")), {})
     step_ms = sum(v[0] for v in prof.values())
@@ -353,7 +356,7 @@ def large_fit(r, dev, lib_stream, steps, warmup, rank, lr=LARGE_FIT_LR):
             "loss_first": traj[0][1], "loss_last": traj[-1][1], "loss_trajectory": traj,
             "launch_shape": {"sample_layout": tuning[0], "boundary_cell": tuning[1], "fragment_slots": tuning[2],
                              "work_queue": "persistent CTAs" if tuning[3] else "one CTA per item",
-                             "forward_ctas_per_sm": 4 - tuning[4]}}
+                             "forward_ctas_per_sm": FORWARD_CTAS_PER_SM}}
 
 
 def prefiltered_step(r, dev, lib_stream, flush, steps, warmup, rank):
@@ -546,7 +549,7 @@ def batched_vs_plain(r, dev, lib_stream, flush, scenes, steps, label):
                        "fused device call, gradient read-back, host Adam"},
            "workload": label, "launch_shape": {"sample_layout": tuning[0], "boundary_cell": tuning[1], "fragment_slots": tuning[2],
                              "work_queue": "persistent CTAs" if tuning[3] else "one CTA per item",
-                             "forward_ctas_per_sm": 4 - tuning[4]}}
+                             "forward_ctas_per_sm": FORWARD_CTAS_PER_SM}}
     batch.close()
     for u in ups + tgts:
         u.close()
@@ -792,7 +795,7 @@ def main():
         "config": {**cfg, "boundary_samples": bopts.boundary_samples, "l2": "flushed between timed steps "
                    "(256 MiB write outside the timed events)", "parallelism": f"weak, {world} independent scene(s)",
                    "launch_shape": {"sample_layout": tuning[0], "boundary_cell": tuning[1],
-                                    "fragment_slots": tuning[2], "forward_ctas_per_sm": 4 - tuning[4],
+                                    "fragment_slots": tuning[2], "forward_ctas_per_sm": FORWARD_CTAS_PER_SM,
                                     "chosen_by": "dvg_scene_autotune"}},
         "roofline": roofline,
         "kernel_ms_per_step": prof_json,

@@ -196,8 +196,8 @@ dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
     return DVG_OK;
 }
 // Reserves and builds, and waits: the item counter runs on past the room there is, so a scene
-// that needs more than the first guess (three per cell entry; the mixed scene takes 1.7, the
-// large one 4) is built once again with what it counted, times `slack`.
+// that needs more than the first guess (three per cell entry) is built once again with what it
+// counted, times `slack`.
 dvg_status make_cells(dvg_context* ctx, dvg_scene* sc, size_t total, int slack) {
     dvg_status st = reserve_cells(sc, total, 3 * CELLS * total * slack);
     if (st == DVG_OK) st = build_cells(ctx, sc);

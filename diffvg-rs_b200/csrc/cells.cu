@@ -6,9 +6,12 @@
 // 16 * spp sample points.  The sample kernels are bound by instruction issue on those tests
 // (f64 root solves): on the mixed 512x512 scene a sample met 49 segments of 5.3 groups, and
 // with the lists 1.2 segments, 1.5 curves and 2.7 rows of 2.2 groups are left (large
-// 1024x1024 scene: 199 -> 18, 6, 26).  Forward 3.43 -> 1.23 ms and edge pass 1.31 -> 0.81 ms on
-// the mixed scene at 4x4 spp, 76 -> 34 ms and 216 -> 136 ms on the large one.  4x4 pixels: the
-// 16 samples per pixel of a CTA share one list; cells of a whole tile leave 8 segments.
+// 1024x1024 scene: 199 -> 18, 6, 26).  The lists took the forward from 3.43 to 1.23 ms and the
+// edge pass from 1.31 to 0.81 ms on the mixed scene at 4x4 spp, from 76 to 34 ms and from 216 to
+// 136 ms on the large one (with the steps taken since: 0.82, 0.41, 14.6 and 46.9 ms).  4x4
+// pixels: the 16 samples per pixel of a CTA share one list; cells of a whole tile leave 8
+// segments.  The build itself is bound by latency, a few barriers per group at 12-24 % occupancy:
+// 55 us on a 128x128 scene of 8 shapes, 0.22 ms on the mixed scene, 4.2 ms on the large one.
 #include "cells.cuh"
 #include "kernels.cuh"
 

@@ -20,7 +20,7 @@
 // Minimum resident CTAs per SM for the scene-evaluation kernels (register cap =
 // 65536 / (threads * value)); chosen by measurement on B200.
 #ifndef DVG_MINB_FWD
-#define DVG_MINB_FWD 5  // 48 registers: mixed 512x512 forward 0.82 -> 0.78 ms against 4 (3: 0.90, 6: 0.78, 8: 0.85)
+#define DVG_MINB_FWD 5  // 48 registers: mixed 512x512 forward 0.86 -> 0.82 ms against 4 (large scene 14.3 -> 14.7)
 #endif
 #ifndef DVG_MINB_INT
 #define DVG_MINB_INT 2
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) k_bin_write(DevScene S, const float4* g_b
 // accumulator covers that cell and its halo only.  G: the splat's lane groups (splat_group: the
 // samples per pixel, 4 or 16, with layout 1), 0: a shared-memory atomic per sample and value.
 // Gaussian r = 1, 4x4 spp, mixed 512x512 scene: 0.55 of the forward's 1.23 ms were those atomics;
-// 0.93 ms with the groups.
+// 0.93 ms with the groups (0.82 with the steps taken since).
 template <int G>
 __device__ __forceinline__ void forward_body(const DevScene& S, const SampleParams& sp, int tile, int round,
                                              float* accum, float* wsum, float* sm) {
@@ -583,7 +583,7 @@ static __device__ __noinline__ int winding_shape_any(const DevScene& S, int s, f
 // shape's own tests at lp: the group has no other shape, lp lies in its box (so the tests were
 // made) and both take the same point (shape_local_dist's identity shortcut is exact).  Half of
 // the samples' points end here, each with a walk over the whole path: 128x128 adjoint scene,
-// the edge pass 0.53 -> 0.40 ms (256x256 scene of filled outlines, 200,000 samples).
+// the edge pass 0.53 -> 0.40 ms (128x128 scene of 8 outlines, 262,144 samples).
 __device__ __forceinline__ bool edge_tests_done(const DevScene& S, int g, int s, float2 lp) {
     const int4 gb = __ldg(&S.g_bvh[g]);
     if (gb.y != 1 || __ldg(&S.gn_meta[gb.x].z) != 1) return false;
@@ -1352,7 +1352,7 @@ __device__ __forceinline__ void boundary_gen_one(const DevScene& S, uint64_t idx
 }
 // Counts of the segment buckets that a CTA's samples fall in, in shared memory while they span
 // at most SEG_SPAN buckets (a scene of few shapes has all its samples in a few dozen, and L2
-// serialises their atomics: edge pass of the adjoint scene 0.40 -> 0.33 ms).
+// serialises their atomics: edge pass of a 128x128 scene of 8 outlines 0.40 -> 0.33 ms).
 constexpr int SEG_SPAN = 4096;
 constexpr int GEN_ITEMS = 4;  // samples per thread
 struct SegSpan {

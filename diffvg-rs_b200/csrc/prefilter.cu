@@ -20,9 +20,9 @@
 #include "device.cuh"
 #include "kernels.cuh"
 // Minimum resident CTAs per SM of the prefiltered forward and interior kernels, by
-// measurement on B200 (mixed 512x512 scene): the forward at 6 (40 registers, 2x2 spp) 4.03 ->
-// 3.80 ms against 4 (5: 3.94, 3: 4.16); the interior at 1 (168 registers, no spills)
-// 9.18 ms (2: 10.3, 3: 10.2, 4: 9.8).
+// measurement on B200 (mixed 512x512 scene, 2x2 spp): the forward at 6 (40 registers) 4.03 ->
+// 3.80 ms against 4 (5: 3.94, 3: 4.16; 2.36 now); the interior at 1 (168 registers, no spills)
+// 6.17 ms (2: 7.36, 3: 7.59; 4.88 now).
 #ifndef DVG_MINB_PF_FWD
 #define DVG_MINB_PF_FWD 6
 #endif
