@@ -460,16 +460,21 @@ DVG_CC_HD float cell_chords_d2(const CellChords& c, float px, float py, int k0, 
 //   d2 > miss: the crate's closest point is farther than the radius, by the culling margin of
 //     the per-sample tests and the chord deviation;
 //   d2 <= hit: the crate finds a point nearer than the radius (hit < 0: never taken).
-// For `hit` the curve has a point within sqrt(d2) + dev, and the crate's closest point is at
-// most a little farther than the true one.  A quadratic's comes from f64 roots (within 1e-6 of
-// the coordinates).  A cubic's parameter comes from a bracketed Newton iteration that stops at
-// |p(t)| < 1e-5 of the normalised quintic p, and d(dist^2)/dt = 2 a p with a = 3 |A|^2 (A the
-// curve's leading coefficient), so dist^2 is at most 2e-5 a too large, given that the brackets
-// isolate the roots; `hit` is left out for segments where they may not: |A| small against the
-// other coefficients (9 |A|^2 < |B|^2 or |C|^2), nearly straight ones (the sine between A and B
-// or C below 0.1), and those symmetric about t = 1/2 (whose isolating point is a root).
-// oracle/cell_stress.cpp counts no exception on random segments, and one in 10^7 on integer
-// coordinates, where the crate misses its nearest root.
+// `hit` is for quadratics.  There the curve has a point within sqrt(d2) + dev, and the crate's
+// closest point is at most a little farther.  Its candidates are the end points and the roots in
+// [0, 1] of the cubic D'(t) / 4 = A t^3 + B t^2 + C t + D of the squared distance D(t), A = |a|^2
+// with a half the second derivative.  In f64 its formula returns the sign-changing roots of a cubic
+// within E = 500 eps S^3 of the monic one on [0, 1], S = B / A + sqrt(C / A) + cbrt(D / A) from the
+// norms of the coefficients' terms (a double root that it misses changes no sign), and moves
+// them by 1e-6 at most (the term that it drops for |ar| <= 1e-6).  Between candidates D is off by
+// 8 A E, and a moved root adds 4 A (3 + 2 S + S^2) 1e-12; below A = 1e-6 the crate solves the
+// quadratic, which is off by 2 A.  All of that, and the rounding of the coefficients to f32, is
+// taken off r^2.
+// A cubic's closest point comes from brackets that need not part the roots of its quintic: with
+// the control points (-11, -15), (5, 9), (-3, 15), (1, 3) the crate passes over the nearest root
+// for whole areas of points.  No threshold on the chord distance decides as it does, so cubics
+// have no `hit`; their samples run the crate's search, which ends at its first candidate within the
+// radius.  Its first candidates are the end points: a box within r of one is full.
 struct CellStroke {
     bool far;   // no point of the box is in reach
     bool full;  // every point of the box is a hit
@@ -521,15 +526,18 @@ DVG_CC_HD CellStroke cell_stroke(int kind, const float* q, const float* rad, Cel
     s.k1 = k1;
     s.miss = (rm + c.dev) * (rm + c.dev) * 1.00001f;
     if (!(rad[0] > 0.0f && rad[0] == rad[1] && rad[0] == rad[2] && rad[0] == rad[3])) return s;
-    float slack = 2.0e-4f * (1.0f + m) * r;
     if (kind == 2) {
-        const float A = c.ax * c.ax + c.ay * c.ay, B = c.bx * c.bx + c.by * c.by, C = c.cx * c.cx + c.cy * c.cy;
-        const float ab = c.ax * c.by - c.ay * c.bx, ac = c.ax * c.cy - c.ay * c.cx;
-        const float tq = -(c.ax * c.bx + c.ay * c.by) / (3.0f * A);
-        if (!(9.0f * A >= B && 9.0f * A >= C && ab * ab >= 0.01f * A * B && ac * ac >= 0.01f * A * C && C > 0.0f &&
-              B > 0.0f && std::fabs(tq - 0.5f) >= 1.0e-3f))
-            return s;
-        slack += 6.3e-5f * A;
+        const float ex = std::fmin(std::hypot(q[0] - px, q[1] - py), std::hypot(q[6] - px, q[7] - py));
+        s.full = ex + hd <= r - 1.0e-5f * (1.0f + m);
+        return s;
+    }
+    float slack = 2.0e-4f * (1.0f + m) * r + 1.0e-5f;
+    const float A = c.bx * c.bx + c.by * c.by;
+    if (!(A < 0.9e-6f)) {
+        const float a = std::sqrt(A), b = 0.5f * std::sqrt(c.cx * c.cx + c.cy * c.cy);
+        const float R = std::hypot(q[0] - px, q[1] - py) + hd;
+        const float S = 1.001f * (3.0f * b / a + std::sqrt((2.0f * b * b + a * R) / A) + std::cbrt(b * R / A));
+        slack += 1.0e-12f * A * S * S * S + 1.0e-11f * A * (S + 2.0f) * (S + 2.0f);
     }
     const float in = r * r - slack;
     const float h = in > 0.0f ? std::sqrt(in) - c.dev : -1.0f;

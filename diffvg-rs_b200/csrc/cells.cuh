@@ -198,7 +198,9 @@ __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, 
             } else if (stroke_misses_segment(sg, p)) {
                 continue;
             }
-            const CPRes c = seg_closest_plain(sg, p, approx);
+            // one radius: the first candidate within it decides (1e-6 below the rounding of seg_radius)
+            const bool even = sg.r[0] == sg.r[1] && sg.r[0] == sg.r[2] && sg.r[0] == sg.r[3];
+            const CPRes c = seg_closest_plain(sg, p, approx, even ? sg.r[0] * (1.0f - 1.0e-6f) : 0.0f);
             if (c.dist < seg_radius(sg, c.t)) {
                 *stroke = true;
                 break;

@@ -367,11 +367,13 @@ static __device__ __noinline__ CPRes closest_cubic_approx_v(float2 pt, float a0,
     }
     return CPRes{bx, by, best_t, best};
 }
-static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, bool approx);
-__device__ __forceinline__ CPRes closest_cubic(float2 pt, const float* q, bool approx) {
-    return closest_cubic_v(pt, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], approx);
+// `stop`: the first of the crate's candidates that is nearer than this ends the search (0: none
+// does), for callers that only ask whether the distance is below it.
+static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, bool approx, float stop);
+__device__ __forceinline__ CPRes closest_cubic(float2 pt, const float* q, bool approx, float stop = 0.0f) {
+    return closest_cubic_v(pt, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], approx, stop);
 }
-static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, bool approx) {
+static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7, bool approx, float stop) {
     const float q[8] = {a0, a1, a2, a3, a4, a5, a6, a7};  // curve.rs:124-264
     if (approx) return closest_cubic_approx(pt, q);
     float best_t = 0.0f, bx = q[0], by = q[1];
@@ -383,6 +385,7 @@ static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float 
         by = q[7];
         best_t = 1.0f;
     }
+    if (best < stop) return CPRes{bx, by, best_t, best};
     double ax = (double)(-q[0] + 3.0f * q[2] - 3.0f * q[4] + q[6]);
     double ay = (double)(-q[1] + 3.0f * q[3] - 3.0f * q[5] + q[7]);
     double bxx = (double)(3.0f * q[0] - 6.0f * q[2] + 3.0f * q[4]);
@@ -467,6 +470,7 @@ static __device__ __noinline__ CPRes closest_cubic_v(float2 pt, float a0, float 
                 bx = px;
                 by = py;
                 best_t = t32;
+                if (best < stop) break;
             }
         }
         if (upper >= 1.0) break;
@@ -593,12 +597,13 @@ __device__ __forceinline__ int winding_segment(const SegGeom& s, float2 pt) {
 
 // The crate's own formulas for the strokes that the cell lists' chord tests leave open (a few
 // percent of the samples): small code, since every excursion to it displaces the sample loop's
-// from the instruction cache.  Same results as seg_closest.
-__device__ __forceinline__ CPRes seg_closest_plain(const SegGeom& sg, float2 p, bool approx) {
+// from the instruction cache.  Same results as seg_closest (of a cubic, with `stop`, the first
+// candidate nearer than that).
+__device__ __forceinline__ CPRes seg_closest_plain(const SegGeom& sg, float2 p, bool approx, float stop) {
     if (sg.kind == 0) return closest_line(p, sg.q[0], sg.q[1], sg.q[2], sg.q[3]);
     if (sg.kind == 1)
         return closest_quad_v<true>(p, sg.q[0], sg.q[1], sg.q[2], sg.q[3], sg.q[4], sg.q[5], sg.q[6], sg.q[7], approx);
-    return closest_cubic(p, sg.q, approx);
+    return closest_cubic(p, sg.q, approx, stop);
 }
 
 // ------------------------------------------------------------------ exact-result culling

@@ -227,3 +227,33 @@ extern "C" void cell_stroke_stress(int kind, int mode, uint64_t seed, uint64_t n
         }
     }
 }
+
+// One stroke segment (eight coordinates, four radii), one box and one point of it.  out: the
+// decision of the lists (0 left to the crate's search, 1 a miss, 2 a hit, 3 a box that is full),
+// whether the crate's closest point is within its radius.
+extern "C" void cell_stroke_point(int kind, const float* q, const float* rad, const float* box, const float* pt, int approx,
+                                  int* out) {
+    const dvgb::CellBox b{box[0], box[1], box[2], box[3]};
+    const dvgb::CellStroke s = dvgb::cell_stroke(kind, q, rad, b, approx != 0);
+    const V2 p[4] = {mk(q[0], q[1]), mk(q[2], q[3]), mk(q[4], q[5]), mk(q[6], q[7])}, at = mk(pt[0], pt[1]);
+    out[0] = s.full ? 3 : s.far ? 1 : 0;
+    if (!s.full && !s.far && s.k1) {
+        const float d2 = dvgb::cell_chords_d2(dvgb::cell_chords(kind, q), at.x, at.y, s.k0, s.k1);
+        out[0] = d2 > s.miss ? 1 : d2 <= s.hit ? 2 : 0;
+    }
+    CP c;
+    float r;
+    if (kind == 0) {
+        distance_to_segment(at, p[0], p[1], &c.dist, &c.cp, &c.t);
+        r = rad[0] + c.t * (rad[1] - rad[0]);
+    } else if (kind == 1) {
+        c = closest_point_quadratic(at, p[0], p[1], p[2], approx != 0);
+        const float u = 1.0f - c.t;
+        r = u * u * rad[0] + 2.0f * u * c.t * rad[1] + c.t * c.t * rad[2];
+    } else {
+        c = closest_point_cubic(at, p[0], p[1], p[2], p[3], approx != 0);
+        const float u = 1.0f - c.t;
+        r = u * u * u * rad[0] + 3.0f * u * u * c.t * rad[1] + 3.0f * u * c.t * c.t * rad[2] + c.t * c.t * c.t * rad[3];
+    }
+    out[1] = c.dist < r ? 1 : 0;
+}
