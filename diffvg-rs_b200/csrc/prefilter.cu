@@ -413,13 +413,14 @@ __device__ __forceinline__ bool maybe_styled_end(const DevScene& S, int s, int s
     return path >= 0 && (__ldg(&S.p_info[2 * path + 1].w) & PF_STYLED);
 }
 
-// Canvas distance beyond which a one-shape group's stroke has no coverage: its width + 1; a
+// Canvas distance beyond which a one-shape group's stroke has no coverage: its width + 1 (at
+// least the 1 of a fill that shares the search; a width that is no number has no coverage); a
 // styled one's join and cap regions reach farther.
 __device__ __forceinline__ float pf_stroke_reach(const DevScene& S, int g) {
     const int s = __ldg(&S.gl_shapes[__ldg(&S.gn_meta[__ldg(&S.g_bvh[g].x)].y)]);
     const int path = __ldg(&S.s_info[s].z);
     if (path >= 0 && (__ldg(&S.p_info[2 * path + 1].w) & PF_STYLED)) return INF_F;
-    return fabsf(__ldg(&S.s_stroke[s])) + 1.0f;
+    return fmaxf(fabsf(__ldg(&S.s_stroke[s])) + 1.0f, 1.0f);
 }
 
 // One prefiltered fragment (sampling.rs:240-300).
