@@ -1650,6 +1650,7 @@ __device__ __forceinline__ float4 gather_d_color_radius(const DevScene& S, const
             if (w <= 0.0f) continue;
             const float denom = ws * ws;
             const float dw = denom > 0.0f ? (ws - w * (ws - w)) / denom : 0.0f;
+            if (dw == 0.0f) continue;  // (the square of the weights overflows for a radius below 1e-10; g may be NaN)
             const float g = S.filter_type == F_GAUSSIAN
                                 ? (r != 0.0f ? dw * w * (4.0f * (fx * fx + fy * fy) / (r * r * r) - 2.0f / r) : 0.0f)
                                 : d_filter_weight(S.filter_type, r, fx, fy, dw);
