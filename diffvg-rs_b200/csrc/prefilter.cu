@@ -180,10 +180,12 @@ static __device__ bool closest_shape(const DevScene& S, int s, float2 lp, float2
 
 // Shape-space reach for a canvas distance `want` around p: a point of the shape that is farther
 // from p than this is farther than `want` on the canvas (S.g_isig: the map's smallest stretch;
-// the slack covers its 0.01 pixel and the f32 maps).
-__device__ __forceinline__ float shape_reach(const DevScene& S, int g, float want, float2 p) {
+// the slack covers its 0.01 pixel and the f32 maps).  The two maps of a group undo each other to
+// 0.01 pixel over the canvas; elsewhere (positions of a signed distance) no bound is known.
+__device__ __forceinline__ float shape_reach(const DevScene& S, int g, float2 pt, float want, float2 p) {
     const float k = __ldg(&S.g_isig[g]);
-    return k > 0.0f ? (want + 0.03f) * k * 1.001f + 1.0e-4f * (1.0f + fabsf(p.x) + fabsf(p.y)) : INF_F;
+    const bool on = pt.x >= -2.0f && pt.x <= (float)S.width + 2.0f && pt.y >= -2.0f && pt.y <= (float)S.height + 2.0f;
+    return k > 0.0f && on ? (want + 0.03f) * k * 1.001f + 1.0e-4f * (1.0f + fabsf(p.x) + fabsf(p.y)) : INF_F;
 }
 // compute_distance_bvh (api.rs:138-236) with the brute-force fallback compute_distance (api.rs:36-76).
 // `want`: the caller has no use for a canvas distance beyond it.
@@ -232,7 +234,7 @@ static __device__ bool compute_distance_group(const DevScene& S, int g, float2 p
                 if (si.x == K_PATH && si.z >= 0 && __ldg(&S.p_info[2 * si.z].w) > 0) {
                     float2 scp;
                     const float2 p = shape_local_dist(S, s, lp);
-                    ok = closest_path_bvh(S, si.z, p, shape_reach(S, g, want, p), &scp, &seg, &t, status);
+                    ok = closest_path_bvh(S, si.z, p, shape_reach(S, g, pt, want, p), &scp, &seg, &t, status);
                     if (ok) lc = xf9(S.s_xform + 9 * s, scp);
                 } else {
                     ok = closest_shape(S, s, lp, &lc, &seg, &t);

@@ -36,3 +36,20 @@ def test_stroke_width_that_is_no_number(renderer):
     opts = RenderOptions(samples_x=2, samples_y=2, seed=3, jitter=True, use_prefiltering=True)
     a, b = renderer.render(scene(True), opts).pixels, renderer.render(scene(False), opts).pixels
     assert float(np.max(np.abs(a - b))) <= 1e-5
+
+
+@pytest.mark.parametrize("x", [8.0, 10000.0])
+def test_position_off_the_canvas(renderer, x):
+    """Two outlines 1 and 0.3 to the right of a point.  The nearer one's map to its shape space is
+    not quite the inverse of the map back: off by 0.007 pixel over a canvas of 16 and by 4 pixels
+    at x = 10000, where the shape's edge is 3.7 units from the point's image."""
+    sc = Scene(16, 16)
+    sc.background = Color(1.0, 1.0, 1.0, 1.0)
+    for dx in (0.3, 1.0):
+        sc.shapes.append(Shape(PathGeometry(_path([(x + dx, -90.0), (x + dx, 90.0), (x + 110.0, 0.0)]))))
+        sc.groups.append(ShapeGroup([len(sc.shapes) - 1], None, Color(0.2, 0.4, 0.8, 1.0)))
+    m = sc.groups[0].canvas_to_shape.m.copy()
+    m[0, 0] = np.float32(1.0004)
+    sc.groups[0].canvas_to_shape.m = m
+    got = float(renderer.eval_positions(sc, np.array([[x, 8.0]], np.float32))[0])
+    assert abs(abs(got) - 0.3) <= 2e-3  # (an ulp of x is 1e-3 at 10000)
