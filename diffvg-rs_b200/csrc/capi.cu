@@ -1227,7 +1227,8 @@ struct dvg_batch {
     std::vector<size_t> wpix_off;     // float offset of each scene's 1-channel region
     std::vector<size_t> grad_base;    // float offset of each scene's gradient block
     size_t total_pix4 = 0, total_pix = 0, total_grads = 0, max_pixels = 0;
-    int items = 0, total_tiles = 0, total_segs = 0, max_ri = 0;
+    int items = 0, total_tiles = 0, total_segs = 0;
+    SplatPlan splat;  // over the scenes' filter radii
     uint64_t total_bsamples = 0;
     DevBuf entries, work, queue, accum, wsum, image, target, d_render, loss, grads, bsamples, bkey, border, bcounts, bsegs;
     DevBuf frag;  // per-scene fragment caches (forward -> interior)
@@ -1260,10 +1261,10 @@ dvg_status batch_enqueue(dvg_batch* b) {
         queue = b->queue.as<int>();
     }
     if (pre)
-        ctx->launches += launch_forward_prefilter_batch(B, b->work.as<int2>(), b->items, queue, b->max_ri,
+        ctx->launches += launch_forward_prefilter_batch(B, b->work.as<int2>(), b->items, queue, b->splat,
                                                         ctx->status, ctx->stream);
     else
-        ctx->launches += launch_forward_batch(B, b->host_entries[0].sp, b->work.as<int2>(), b->items, queue, b->max_ri,
+        ctx->launches += launch_forward_batch(B, b->host_entries[0].sp, b->work.as<int2>(), b->items, queue, b->splat,
                                               ctx->stream);
     ctx->launches += launch_pixels_batch(B, n, b->max_pixels, 0, ctx->stream);
     ctx->launches += launch_pixels_batch(B, n, b->max_pixels, 1, ctx->stream);
@@ -1366,7 +1367,7 @@ extern "C" dvg_status dvg_batch_create(dvg_context* ctx, dvg_scene* const* scene
         b->max_pixels = std::max(b->max_pixels, npix);
         b->grad_base.push_back(b->total_grads);
         b->total_grads += (sc->grad_floats + 63) & ~(size_t)63;
-        b->max_ri = std::max(b->max_ri, S.filter_ri);
+        b->splat.add(S.filter_ri);
         BatchEntry e{};
         e.S = S;
         e.sp = sp;

@@ -1939,10 +1939,11 @@ static int splat_lanes(const SampleParams& sp) {
     return sp.layout && (spp == 4 || spp == 16) ? spp : 0;
 }
 int launch_forward(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, cudaStream_t stream) {
-    const int hw = TILE + 2 * S.filter_ri;
-    size_t smem = S.filter_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
+    SplatPlan splat;
+    splat.add(S.filter_ri);
+    const size_t smem = splat.bytes();
     dim3 grid(launch_tiles(S, sp), sp.sxn * sp.syn);
-    const int g = smem ? splat_lanes(sp) : 0;
+    const int g = splat.all ? splat_lanes(sp) : 0;
     if (g == 16)
         k_forward<16><<<grid, 256, smem, stream>>>(S, sp, accum, wsum);
     else if (g == 4)
@@ -2035,13 +2036,12 @@ int persistent_grid(K kernel, size_t smem, int items) {
     return std::max(1, std::min(items, std::max(per_sm, 1) * std::max(sms, 1)));
 }
 int launch_forward_batch(const BatchEntry* B, const SampleParams& sp, const int2* work, int items, int* counter,
-                         int max_ri, cudaStream_t stream) {
-    const int hw = TILE + 2 * max_ri;
-    const size_t smem = max_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
+                         const SplatPlan& splat, cudaStream_t stream) {
+    const size_t smem = splat.bytes();
     auto go = [&](auto kernel) {
         kernel<<<counter ? persistent_grid(kernel, smem, items) : items, 256, smem, stream>>>(B, work, items, counter);
     };
-    const int g = smem ? splat_lanes(sp) : 0;  // (one set of options, and of a batch one layout, for all its scenes)
+    const int g = splat.all ? splat_lanes(sp) : 0;  // (one set of options, and of a batch one layout, for all its scenes)
     if (g == 16)
         go(k_forward_batch<16>);
     else if (g == 4)

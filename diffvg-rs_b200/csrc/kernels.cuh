@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "limits.hpp"
 
 namespace dvgb {
 
@@ -12,8 +13,6 @@ namespace dvgb {
 // used 256, src/gpu/kernels/backward.rs:1657-1662).  Exceeding it sets
 // ST_FRAGMENT_OVERFLOW and the call returns DVG_ERR_DEVICE_LIMIT.
 constexpr int MAX_FRAGMENTS = 96;
-// Filter radii up to this (ceil) use the shared-memory tile+halo splat.
-constexpr int MAX_SMEM_RI = 8;
 // Boundary samples are counting-sorted by cell x cell-pixel cells of their tile
 // (cell in {2, 4, 8, 16}) and, inside a cell, by class (fill or stroke, path or other
 // shape: the code they run); bnd_buckets(cell) buckets per tile; scratch counts hold
@@ -188,9 +187,9 @@ int launch_fill_background(const DevScene& S, float* out, cudaStream_t stream);
 // for persistent CTAs (see for_each_item; launch_interior_batch takes two, one per
 // kernel).  which: 0 resolve, 1 L2, 2 background.
 int launch_forward_batch(const BatchEntry* B, const SampleParams& sp, const int2* work, int items, int* counter,
-                         int max_ri, cudaStream_t stream);
-int launch_forward_prefilter_batch(const BatchEntry* B, const int2* work, int items, int* counter, int max_ri,
-                                   unsigned* status, cudaStream_t stream);
+                         const SplatPlan& splat, cudaStream_t stream);
+int launch_forward_prefilter_batch(const BatchEntry* B, const int2* work, int items, int* counter,
+                                   const SplatPlan& splat, unsigned* status, cudaStream_t stream);
 int launch_pixels_batch(const BatchEntry* B, int nscenes, size_t max_pixels, int which, cudaStream_t stream);
 int launch_interior_batch(const BatchEntry* B, const int2* work, int items, int* counters, unsigned* status,
                           cudaStream_t stream);

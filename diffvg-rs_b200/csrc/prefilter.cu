@@ -630,16 +630,16 @@ __global__ void __launch_bounds__(256, DVG_MINB_PF_FWD) k_forward_prefilter_batc
 }
 int launch_forward_prefilter(const DevScene& S, const SampleParams& sp, float* accum, float* wsum, unsigned* status,
                              cudaStream_t stream) {
-    const int hw = TILE + 2 * S.filter_ri;
-    size_t smem = S.filter_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
+    SplatPlan splat;
+    splat.add(S.filter_ri);
+    const size_t smem = splat.bytes();
     dim3 grid(launch_tiles(S, sp), sp.sxn * sp.syn);
     k_forward_prefilter<<<grid, 256, smem, stream>>>(S, sp, accum, wsum, status);
     return 1;
 }
-int launch_forward_prefilter_batch(const BatchEntry* B, const int2* work, int items, int* counter, int max_ri,
-                                   unsigned* status, cudaStream_t stream) {
-    const int hw = TILE + 2 * max_ri;
-    size_t smem = max_ri <= MAX_SMEM_RI ? (size_t)hw * hw * 5 * sizeof(float) : 0;
+int launch_forward_prefilter_batch(const BatchEntry* B, const int2* work, int items, int* counter,
+                                   const SplatPlan& splat, unsigned* status, cudaStream_t stream) {
+    const size_t smem = splat.bytes();
     int grid = items;
     if (counter) {
         int dev = 0, sms = 0, per_sm = 0;

@@ -1,0 +1,12 @@
+// limits.cpp — test infrastructure: the library's sizes and index arithmetic at the limits of a
+// scene (diffvg-rs_b200/csrc/limits.hpp), called by tests/test_limits.py.
+#include "../diffvg-rs_b200/csrc/limits.hpp"
+
+// Shared-memory bytes of a forward launch over scenes of these filter radii; *all: whether every
+// scene accumulates there.
+extern "C" size_t limits_splat(const int* ri, int n, int* all) {
+    dvgb::SplatPlan p;
+    for (int i = 0; i < n; ++i) p.add(ri[i]);
+    *all = p.all;
+    return p.bytes();
+}

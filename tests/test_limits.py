@@ -1,0 +1,57 @@
+"""Sizes and index arithmetic at limits that no test can reach on a device."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ORACLE = os.path.join(os.path.dirname(HERE), "oracle")
+
+
+@pytest.fixture(scope="module")
+def limits():
+    subprocess.run(["make", "-s", "-C", ORACLE], check=True)
+    return C.CDLL(os.path.join(ORACLE, "_build", "liblimits.so"))
+
+
+@pytest.mark.parametrize("radii", [[1], [8], [9], [1, 3, 8], [9, 1], [1, 9, 3], [40, 8, 200], [0], [9, 0, 9]])
+def test_splat_room_for_every_scene(limits, radii):
+    """A batch's scenes whose own radius fits accumulate in shared memory, so there has to be room
+    for the largest of them next to any that does not fit; the lane-group splat needs all to fit."""
+    f = limits.limits_splat
+    f.restype = C.c_size_t
+    all_fit = C.c_int()
+    got = f((C.c_int * len(radii))(*radii), len(radii), C.byref(all_fit))
+    need = max([(16 + 2 * r) ** 2 * 20 for r in radii if r <= 8], default=0)
+    assert got == need
+    assert bool(all_fit.value) == all(r <= 8 for r in radii)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("spp", [(2, 2), (4, 4), (3, 2)])
+@pytest.mark.parametrize("prefilter", [False, True])
+@pytest.mark.parametrize("work_queue", [0, 1])
+def test_batch_of_mixed_filter_radii(work_queue, prefilter, spp):
+    """Radii on both sides of what shared memory holds in one batch, against single renders."""
+    import numpy as np
+    from dvg import Batch, Renderer, RenderOptions, synth
+    from dvg.scene import Filter, FilterType
+
+    scenes = []
+    for i, r in enumerate((0.5, 9.5, 2.5)):
+        sc = synth.plain_scene(i, 40 + 3 * i, 33, 4)
+        sc.filter = Filter(FilterType.GAUSSIAN, r)
+        scenes.append(sc)
+    opts = RenderOptions(samples_x=spp[0], samples_y=spp[1], seed=3, jitter=True, use_prefiltering=prefilter)
+    rn = Renderer(0)
+    ups = [rn.upload(s) for s in scenes]
+    b = Batch(rn, ups, opts)
+    b.set_tuning(1, 4, 16, work_queue)
+    b.step(use_graph=False)
+    b.losses()  # waits
+    for i, s in enumerate(scenes):
+        img = b.buffers(i)[0].cpu().numpy().reshape(s.height, s.width, 4)
+        assert float(np.max(np.abs(img - rn.render(s, opts).pixels))) <= 1e-5
+    b.close()
+    rn.close()
