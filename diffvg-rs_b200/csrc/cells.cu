@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
     const int tx = tile % S.tiles_x, ty = tile / S.tiles_x;
     const int off = S.tile_offsets[tile], n = S.tile_offsets[tile + 1] - off;
     if (tid == 0) {
-        const bool fits = n < (1 << 22);  // list indices share a word with the entry flags
+        const bool fits = n < CELL_LIST_MAX;
         const int b = n > 0 && fits ? atomicAdd(&T.counters[0], CELLS * n) : 0;
         ent_base = fits && b >= 0 && b <= T.cap_entries - CELLS * n ? b : -1;
     }
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
             str_hit[c][best] = str_hit[c][j];
         }
         int4* E = T.entries + 2 * ((size_t)ent_base + (size_t)c * n + kept[c]);
-        E[0] = make_int4((e << 8) | flags, g, gi.x, gi.y);
+        E[0] = make_int4(entry_word(true, e, flags), g, gi.x, gi.y);
         E[1] = make_int4(s, (base[c] & 0xffff) | (base_slow[c] << 16), at,
                          nl | (nc << 6) | (nh << 12) | (nf << 18) | (ns << 24));
         kept[c] += 1;

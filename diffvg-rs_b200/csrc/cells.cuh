@@ -10,6 +10,7 @@
 // full query.
 #pragma once
 #include "device.cuh"
+#include "limits.hpp"
 
 namespace dvgb {
 
@@ -17,7 +18,7 @@ constexpr int CELL = 4;               // cell edge in pixels
 constexpr int CELLS = 16;             // cells per tile
 constexpr int CELL_MAX_SEGS = 512;    // longer paths keep the full query
 
-// Entry flags (low 8 bits of an entry's first word; the tile-list index is above them).
+// Entry flags (low 8 bits of an entry's first word, entry_word).
 enum : int {
     CE_FILL = 1,         // the fill covers every sample point of the cell
     CE_FILL_TEST = 2,    // winding = base + the entry's levels and fill segments
@@ -104,8 +105,11 @@ __device__ __forceinline__ int4 cell_entry(const DevScene& S, const CellWalk& w,
     if (w.ent) return __ldg(&w.ent[2 * k]);
     const int g = __ldg(&w.list[k]);
     const int4 gi = __ldg(&S.g_info[g]);
-    return make_int4((k << 8) | (gi.x >= 0 ? CE_FILL_ANY : 0) | (gi.y >= 0 ? CE_STROKE_ANY : 0), g, gi.x, gi.y);
+    const int flags = (gi.x >= 0 ? CE_FILL_ANY : 0) | (gi.y >= 0 ? CE_STROKE_ANY : 0);
+    return make_int4(entry_word(false, k, flags), g, gi.x, gi.y);
 }
+// The place of entry k (first words A) in the tile list.
+__device__ __forceinline__ int cell_place(const CellWalk& w, int k, int4 A) { return entry_place(w.ent != nullptr, k, A.x); }
 // Whether the stroke and the fill of entry k (first words A) cover canvas point pt: the
 // decisions of group_within / group_inside.
 __device__ __forceinline__ void cell_hits(const DevScene& S, const CellWalk& w, int k, int4 A, float2 pt, bool* stroke,

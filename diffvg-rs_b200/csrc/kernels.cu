@@ -250,7 +250,7 @@ __device__ __forceinline__ void forward_body(const DevScene& S, const SamplePara
                 if (which ? hit[1] : hit[0]) {
                     over(acc, paint_color(S, which ? A.z : A.w, pt));
                     if (cache) {
-                        if (nf < sp.frag_slots) sp.frag[(size_t)nf * fstride + sid] = (uint16_t)(2 * (A.x >> 8) + which);
+                        if (nf < sp.frag_slots) sp.frag[(size_t)nf * fstride + sid] = (uint16_t)(2 * cell_place(walk, k, A) + which);
                         ++nf;
                     }
                 }
@@ -397,7 +397,7 @@ __device__ __forceinline__ void interior_body(const DevScene& S, const SamplePar
                 const int4 A = cell_entry(S, walk, k);
                 bool st, fi;
                 cell_hits(S, walk, k, A, pt, &st, &fi);
-                e = A.x >> 8;
+                e = cell_place(walk, k, A);
                 hitp[0] = st ? A.w : -1;
                 hitp[1] = fi ? A.z : -1;
             }

@@ -3,6 +3,12 @@
 #pragma once
 #include <cstddef>
 
+#ifdef __CUDACC__
+#define DVG_LIM_HD __host__ __device__ __forceinline__
+#else
+#define DVG_LIM_HD inline
+#endif
+
 namespace dvgb {
 
 // Filter radii up to this (ceil) use the shared-memory tile+halo splat.
@@ -25,5 +31,12 @@ struct SplatPlan {
         return ri < 0 ? 0 : w * w * 5 * sizeof(float);
     }
 };
+
+// The word of a cell entry: its group's place in the tile list above eight flags.  Longer tile
+// lists than CELL_LIST_MAX get no cell lists; a walk over the list itself (`listed` false) has
+// any length, and the place is the step of the walk.
+constexpr int CELL_LIST_MAX = 1 << 22;
+DVG_LIM_HD int entry_word(bool listed, int place, int flags) { return listed ? (place << 8) | flags : flags; }
+DVG_LIM_HD int entry_place(bool listed, int step, int word) { return listed ? word >> 8 : step; }
 
 }  // namespace dvgb

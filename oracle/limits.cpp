@@ -10,3 +10,9 @@ extern "C" size_t limits_splat(const int* ri, int n, int* all) {
     *all = p.all;
     return p.bytes();
 }
+
+// The place in the tile list that the kernels read back from entry `place` of a walk.
+extern "C" int limits_place(int listed, int place, int flags) {
+    return dvgb::entry_place(listed != 0, place, dvgb::entry_word(listed != 0, place, flags));
+}
+extern "C" int limits_cell_list_max() { return dvgb::CELL_LIST_MAX; }

@@ -28,6 +28,17 @@ def test_splat_room_for_every_scene(limits, radii):
     assert bool(all_fit.value) == all(r <= 8 for r in radii)
 
 
+def test_place_in_the_tile_list(limits):
+    """Cell entries keep their group's place next to eight flags; a walk over a longer tile list than
+    that leaves room for has to give its own step (2^23 shifted by eight is negative)."""
+    top = limits.limits_cell_list_max()
+    for place in (0, 1, 32767, top - 1):
+        for flags in (0, 1, 20, 255):
+            assert limits.limits_place(1, place, flags) == place
+    for place in (0, top, (1 << 23) - 1, 1 << 23, 9_000_000, (1 << 24) + 5, (1 << 31) - 1):
+        assert limits.limits_place(0, place, 20) == place
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("spp", [(2, 2), (4, 4), (3, 2)])
 @pytest.mark.parametrize("prefilter", [False, True])
