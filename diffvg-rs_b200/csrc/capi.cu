@@ -180,9 +180,10 @@ dvg_status reserve_cells(dvg_scene* sc, size_t total, size_t items) {
     items = std::min<size_t>(std::max<size_t>(items, 1), (size_t)1 << 30);
     const size_t o_ent = (cells * sizeof(int2) + 255) & ~(size_t)255, o_item = o_ent + ents * 2 * sizeof(int4);
     const size_t o_cnt = (o_item + items * sizeof(int4) + 255) & ~(size_t)255;
-    CK(sc->cells.reserve(o_cnt + 2 * sizeof(int)));
+    CK(sc->cells.reserve(o_cnt + 2 * sizeof(unsigned long long)));
     char* b = sc->cells.as<char>();
-    sc->cell_table = CellTable{(int2*)b, (int4*)(b + o_ent), (int4*)(b + o_item), (int*)(b + o_cnt), (int)ents, (int)items};
+    sc->cell_table = CellTable{(int2*)b, (int4*)(b + o_ent), (int4*)(b + o_item),
+                               (unsigned long long*)(b + o_cnt), (int)ents, (int)items};
     S.cell_info = sc->cell_table.info;
     S.cell_entries = sc->cell_table.entries;
     S.cell_items = sc->cell_table.items;
@@ -190,7 +191,7 @@ dvg_status reserve_cells(dvg_scene* sc, size_t total, size_t items) {
 }
 // Builds the lists on the context's stream (after the tile lists).
 dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
-    CK(cudaMemsetAsync(sc->cell_table.counters, 0, 2 * sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(sc->cell_table.counters, 0, 2 * sizeof(unsigned long long), ctx->stream));
     ctx->launches += launch_cells(sc->dev, sc->cell_table, ctx->stream);
     CK(cudaGetLastError());
     return DVG_OK;
@@ -202,10 +203,10 @@ dvg_status make_cells(dvg_context* ctx, dvg_scene* sc, size_t total, int slack) 
     dvg_status st = reserve_cells(sc, total, 3 * CELLS * total * slack);
     if (st == DVG_OK) st = build_cells(ctx, sc);
     if (st != DVG_OK) return st;
-    int used[2] = {0, 0};
+    unsigned long long used[2] = {0, 0};
     CK(cudaMemcpyAsync(used, sc->cell_table.counters, sizeof used, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (used[1] <= sc->cell_table.cap_items / slack) return DVG_OK;
+    if (used[1] <= (unsigned long long)(sc->cell_table.cap_items / slack)) return DVG_OK;
     st = reserve_cells(sc, total, (size_t)used[1] * slack);
     if (st == DVG_OK) st = build_cells(ctx, sc);
     return st;

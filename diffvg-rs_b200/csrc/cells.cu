@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
     const int tx = tile % S.tiles_x, ty = tile / S.tiles_x;
     const int off = S.tile_offsets[tile], n = S.tile_offsets[tile + 1] - off;
     if (tid == 0) {
-        const bool fits = n < CELL_LIST_MAX;
-        const int b = n > 0 && fits ? atomicAdd(&T.counters[0], CELLS * n) : 0;
-        ent_base = fits && b >= 0 && b <= T.cap_entries - CELLS * n ? b : -1;
+        ent_base = n > 0 && n < CELL_LIST_MAX
+                       ? room_at(atomicAdd(&T.counters[0], (unsigned long long)(CELLS * n)), CELLS * n, T.cap_entries)
+                       : (n > 0 ? -1 : 0);
     }
     if (tid < CELLS) {
         // Every point that is looked up in the cell: its pixels' samples, and edge samples,
@@ -265,9 +265,9 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
         }
         const int total = __shfl_sync(0xffffffffu, upto, 15);
         int at = 0;
-        if (tid == 0 && total > 0) at = atomicAdd(&T.counters[1], total);
+        if (tid == 0 && total > 0) at = room_at(atomicAdd(&T.counters[1], (unsigned long long)total), total, T.cap_items);
         at = __shfl_sync(0xffffffffu, at, 0);
-        const bool room = at >= 0 && at <= T.cap_items - total;
+        const bool room = at >= 0;
         at += upto - need;
         if (tid >= CELLS || !flags) continue;
         if (!room && need > 0) {  // no room left: the full queries

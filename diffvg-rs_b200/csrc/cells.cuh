@@ -56,7 +56,7 @@ struct CellTable {
     int2* info;     // per cell: first entry, entries (-1: none were kept, walk the tile's list)
     int4* entries;
     int4* items;
-    int* counters;  // entries and segments taken so far
+    unsigned long long* counters;  // entries and items asked for so far (room_at)
     int cap_entries, cap_items;
 };
 

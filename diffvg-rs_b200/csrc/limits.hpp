@@ -39,4 +39,12 @@ constexpr int CELL_LIST_MAX = 1 << 22;
 DVG_LIM_HD int entry_word(bool listed, int place, int flags) { return listed ? (place << 8) | flags : flags; }
 DVG_LIM_HD int entry_place(bool listed, int step, int word) { return listed ? word >> 8 : step; }
 
+// Where a request for `need` of `cap` places begins when `taken` were asked for before it, or -1:
+// no room.  `taken` goes on counting when the room is used up (the host reads what a scene
+// would have needed), in 64 bits: in 32 it came round to small numbers after 2^28 tile entries, and
+// places were handed out twice.
+DVG_LIM_HD int room_at(unsigned long long taken, int need, int cap) {
+    return taken + (unsigned long long)need <= (unsigned long long)cap ? (int)taken : -1;
+}
+
 }  // namespace dvgb

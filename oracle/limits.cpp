@@ -16,3 +16,19 @@ extern "C" int limits_place(int listed, int place, int flags) {
     return dvgb::entry_place(listed != 0, place, dvgb::entry_word(listed != 0, place, flags));
 }
 extern "C" int limits_cell_list_max() { return dvgb::CELL_LIST_MAX; }
+
+// `tiles` requests of `need` places each of `cap`, as k_cells makes them.  Returns the requests
+// granted; -1 if a grant reaches past `cap` or into an earlier one.
+extern "C" long long limits_room(long long tiles, int need, int cap) {
+    unsigned long long taken = 0;
+    long long granted = 0, end = 0;
+    for (long long i = 0; i < tiles; ++i) {
+        const int at = dvgb::room_at(taken, need, cap);
+        taken += (unsigned long long)need;
+        if (at < 0) continue;
+        if (at < end || (long long)at + need > cap) return -1;
+        end = (long long)at + need;
+        granted += 1;
+    }
+    return granted;
+}

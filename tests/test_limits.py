@@ -39,6 +39,17 @@ def test_place_in_the_tile_list(limits):
         assert limits.limits_place(0, place, 20) == place
 
 
+@pytest.mark.parametrize("tiles, groups", [(512 * 512, 1025), (256 * 256, 4100), (1024, 1 << 21), (64, 3), (1, 0)])
+def test_room_is_given_once(limits, tiles, groups):
+    """Scenes whose cell entries (16 per tile and group) or items pass 2^32: canvases of 8192 and 4096
+    pixels full of groups.  Only the room there is is given, and none of it twice."""
+    f = limits.limits_room
+    f.argtypes, f.restype = [C.c_longlong, C.c_int, C.c_int], C.c_longlong
+    for cap in (1 << 30, (1 << 31) - 1, 1000, 0):
+        need = 16 * groups
+        assert f(tiles, need, cap) == (min(tiles, cap // need) if need else tiles)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("spp", [(2, 2), (4, 4), (3, 2)])
 @pytest.mark.parametrize("prefilter", [False, True])
