@@ -74,18 +74,38 @@ struct SceneBuf {
     cudaStream_t stream = nullptr;
     void* ptr = nullptr;
     size_t bytes = 0;
+    SceneBuf() = default;
+    SceneBuf(SceneBuf&& o) noexcept : pool(o.pool), stream(o.stream), ptr(o.ptr), bytes(o.bytes) {
+        o.ptr = nullptr;
+        o.bytes = 0;
+    }
+    SceneBuf& operator=(SceneBuf&& o) noexcept {
+        std::swap(pool, o.pool);
+        std::swap(stream, o.stream);
+        std::swap(ptr, o.ptr);
+        std::swap(bytes, o.bytes);
+        return *this;
+    }
     ~SceneBuf() {
         if (ptr) cudaFreeAsync(ptr, stream);
     }
-    cudaError_t reserve(size_t n) {
+    // On failure the block that was there stays (and the error is not left behind).  `keep`
+    // takes a block that is replaced, for those who still hold its address.
+    cudaError_t reserve(size_t n, std::vector<SceneBuf>* keep = nullptr) {
         if (n <= bytes) return cudaSuccess;
-        if (ptr) cudaFreeAsync(ptr, stream);
-        ptr = nullptr;
-        bytes = 0;
-        cudaError_t e = cudaMallocFromPoolAsync(&ptr, n, pool, stream);
-        if (e == cudaSuccess) bytes = n;
-        else ptr = nullptr;
-        return e;
+        SceneBuf b;
+        b.pool = pool;
+        b.stream = stream;
+        const cudaError_t e = cudaMallocFromPoolAsync(&b.ptr, n, pool, stream);
+        if (e != cudaSuccess) {
+            b.ptr = nullptr;
+            cudaGetLastError();
+            return e;
+        }
+        b.bytes = n;
+        *this = std::move(b);  // b has the old block now
+        if (keep && b.ptr) keep->push_back(std::move(b));
+        return cudaSuccess;
     }
     template <typename T>
     T* as() const {
@@ -94,6 +114,8 @@ struct SceneBuf {
 };
 // Bytes of freed scene memory that a context keeps for its next uploads.
 constexpr uint64_t kScenePoolKeep = 256ull << 20;
+// Bytes that the cell lists of one scene may take (dvg_context_set_list_memory).
+constexpr uint64_t kListMemory = 4ull << 30;
 
 // Packs several host arrays into one blob with 256-byte aligned offsets.
 struct Blob {
@@ -126,6 +148,7 @@ struct dvg_context {
     std::vector<ProfStat> stats;
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;  // scene memory (SceneBuf)
+    uint64_t list_memory = kListMemory;
     unsigned* status = nullptr;  // device word
     DevBuf accum, wsum, image, d_render, target, loss, bg_grad, trans_grad;
     DevBuf bsamples, bkey, border, bcounts, bsegs;  // boundary-pass scratch
@@ -160,7 +183,8 @@ struct dvg_scene {
     SceneBuf tiles;    // counts, offsets
     SceneBuf entries;  // tile entries
     SceneBuf cells;    // per-cell lists (cell_table)
-    CellTable cell_table{};
+    CellTable cell_table{};          // info NULL: none
+    std::vector<SceneBuf> replaced;  // blocks that a batch or a captured graph may still read
     SceneBuf grads;    // gradient arena (device)
     size_t grad_off[11] = {0};
     size_t grad_floats = 0;
@@ -171,26 +195,25 @@ struct dvg_scene {
 
 namespace {
 
-// Sizes a scene's per-cell lists for `total` tile entries (at most one cell entry per tile entry
-// and cell) and `items` items, and points its tables at them.
-dvg_status reserve_cells(dvg_scene* sc, size_t total, size_t items) {
+// Makes room for a scene's cell lists, of `total` tile entries and `items` items, within the
+// context's limit, and points its tables at it.  The lists are an optimisation: without
+// memory for more, the room and the lists that there are stay (false), or there are none and
+// the kernels walk the tile lists.
+bool reserve_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, uint64_t items, std::vector<SceneBuf>* keep) {
     DevScene& S = sc->dev;
-    const size_t cells = (size_t)S.tiles_x * S.tiles_y * CELLS;
-    const size_t ents = std::min<size_t>(std::max<size_t>(total, 1) * CELLS, (size_t)1 << 30);
-    items = std::min<size_t>(std::max<size_t>(items, 1), (size_t)1 << 30);
-    const size_t o_ent = (cells * sizeof(int2) + 255) & ~(size_t)255, o_item = o_ent + ents * 2 * sizeof(int4);
-    const size_t o_cnt = (o_item + items * sizeof(int4) + 255) & ~(size_t)255;
-    CK(sc->cells.reserve(o_cnt + 2 * sizeof(unsigned long long)));
+    const CellRoom r = cell_room((uint64_t)S.tiles_x * S.tiles_y, total, items, ctx->list_memory);
+    if (r.bytes <= sc->cells.bytes || sc->cells.reserve(r.bytes, keep) != cudaSuccess) return false;
     char* b = sc->cells.as<char>();
-    sc->cell_table = CellTable{(int2*)b, (int4*)(b + o_ent), (int4*)(b + o_item),
-                               (unsigned long long*)(b + o_cnt), (int)ents, (int)items};
+    sc->cell_table = CellTable{(int2*)b, (int4*)(b + r.at_ents), (int4*)(b + r.at_items),
+                               (unsigned long long*)(b + r.at_counters), (int)r.ents, (int)r.items};
     S.cell_info = sc->cell_table.info;
     S.cell_entries = sc->cell_table.entries;
     S.cell_items = sc->cell_table.items;
-    return DVG_OK;
+    return true;
 }
 // Builds the lists on the context's stream (after the tile lists).
 dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
+    if (!sc->cell_table.info) return DVG_OK;
     CK(cudaMemsetAsync(sc->cell_table.counters, 0, 2 * sizeof(unsigned long long), ctx->stream));
     ctx->launches += launch_cells(sc->dev, sc->cell_table, ctx->stream);
     CK(cudaGetLastError());
@@ -199,17 +222,15 @@ dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
 // Reserves and builds, and waits: the item counter runs on past the room there is, so a scene
 // that needs more than the first guess (three per cell entry) is built once again with what it
 // counted, times `slack`.
-dvg_status make_cells(dvg_context* ctx, dvg_scene* sc, size_t total, int slack) {
-    dvg_status st = reserve_cells(sc, total, 3 * CELLS * total * slack);
-    if (st == DVG_OK) st = build_cells(ctx, sc);
+dvg_status make_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, int slack, std::vector<SceneBuf>* keep) {
+    if (!reserve_cells(ctx, sc, total, 3 * CELLS * total * slack, keep)) return DVG_OK;
+    dvg_status st = build_cells(ctx, sc);
     if (st != DVG_OK) return st;
     unsigned long long used[2] = {0, 0};
     CK(cudaMemcpyAsync(used, sc->cell_table.counters, sizeof used, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (used[1] <= (unsigned long long)(sc->cell_table.cap_items / slack)) return DVG_OK;
-    st = reserve_cells(sc, total, (size_t)used[1] * slack);
-    if (st == DVG_OK) st = build_cells(ctx, sc);
-    return st;
+    return reserve_cells(ctx, sc, total, used[1] * slack, keep) ? build_cells(ctx, sc) : DVG_OK;
 }
 
 // Offsets of each gradient part inside the scene's gradient arena (in floats).
@@ -453,6 +474,12 @@ dvg_status dvg_context_set_retain(dvg_context* ctx, int enable) {
     return DVG_OK;
 }
 
+dvg_status dvg_context_set_list_memory(dvg_context* ctx, uint64_t bytes) {
+    if (!ctx) return fail(DVG_ERR_INVALID_ARGUMENT, "null context");
+    ctx->list_memory = bytes;
+    return DVG_OK;
+}
+
 void dvg_context_destroy(dvg_context* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
@@ -582,7 +609,7 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
         S.tile_entries = sc->entries.as<int>();
         ctx->launches += launch_binning(S, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
         CK(cudaGetLastError());
-        st = make_cells(ctx, sc.get(), (size_t)std::max(total, 0), 1);
+        st = make_cells(ctx, sc.get(), (uint64_t)std::max(total, 0), 1, nullptr);
         if (st != DVG_OK) return st;
     }
     layout_grads(sc.get());
@@ -1550,7 +1577,7 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
         if (need > ((size_t)1 << 28))
             return fail(DVG_ERR_DEVICE_LIMIT, "tile lists of an optimised scene would exceed 2^28 entries");
         if (sc->entries.bytes < need * sizeof(int)) {
-            CK(sc->entries.reserve(need * sizeof(int)));
+            CK(sc->entries.reserve(need * sizeof(int), &sc->replaced));
             sc->dev.tile_entries = sc->entries.as<int>();
             int* counts = sc->tiles.as<int>();
             int* offsets = counts + tiles;
@@ -1562,7 +1589,8 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
             int total = 0;
             CK(cudaMemcpyAsync(&total, offsets + tiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
-            const dvg_status st = make_cells(ctx, sc, std::min<size_t>(need, 2 * (size_t)std::max(total, 0) + 1024), 2);
+            const dvg_status st =
+                make_cells(ctx, sc, std::min<uint64_t>(need, 2 * (uint64_t)std::max(total, 0) + 1024), 2, &sc->replaced);
             if (st != DVG_OK) return st;
         }
         b->host_entries[i].S.tile_entries = sc->dev.tile_entries;

@@ -1,7 +1,9 @@
 // limits.hpp — sizes and index arithmetic whose limits no test can reach on a device, in plain
 // functions that oracle/limits.cpp runs on the CPU (tests/test_limits.py).
 #pragma once
+#include <algorithm>
 #include <cstddef>
+#include <cstdint>
 
 #ifdef __CUDACC__
 #define DVG_LIM_HD __host__ __device__ __forceinline__
@@ -45,6 +47,37 @@ DVG_LIM_HD int entry_place(bool listed, int step, int word) { return listed ? wo
 // places were handed out twice.
 DVG_LIM_HD int room_at(unsigned long long taken, int need, int cap) {
     return taken + (unsigned long long)need <= (unsigned long long)cap ? (int)taken : -1;
+}
+
+// The memory of one scene's cell lists: 8 bytes per cell, 32 per entry (at most one per tile-list
+// entry and cell of its tile), 16 per item.  Within `budget` bytes: all that is wanted, or four
+// fifths of the rest for entries at most and what is left for items (a tile without entries is
+// walked, an entry without items keeps the full queries).  bytes 0: no lists.
+constexpr int TILE_CELLS = 16;
+struct CellRoom {
+    size_t ents = 0, items = 0, at_ents = 0, at_items = 0, at_counters = 0, bytes = 0;
+};
+inline CellRoom cell_room(uint64_t tiles, uint64_t tile_entries, uint64_t want_items, uint64_t budget) {
+    constexpr uint64_t most = 1ull << 30, pad = 3 * 256 + 16;
+    const uint64_t info = tiles * TILE_CELLS * 8;
+    CellRoom r;
+    if (tiles == 0 || budget < info + pad + 48) return r;
+    const uint64_t rest = budget - info - pad;
+    const uint64_t want_ents = std::min(std::max<uint64_t>(tile_entries, 1) * TILE_CELLS, most);
+    want_items = std::min(std::max<uint64_t>(want_items, 1), most);
+    uint64_t ents = want_ents, items = want_items;
+    if (ents * 32 + items * 16 > rest) {
+        ents = std::min(want_ents, rest / 5 * 4 / 32);
+        items = std::min(want_items, (rest - ents * 32) / 16);
+    }
+    if (ents == 0 || items == 0) return r;
+    r.ents = (size_t)ents;
+    r.items = (size_t)items;
+    r.at_ents = (size_t)((info + 255) & ~255ull);
+    r.at_items = r.at_ents + (size_t)ents * 32;
+    r.at_counters = (size_t)((r.at_items + items * 16 + 255) & ~255ull);
+    r.bytes = r.at_counters + 16;
+    return r;
 }
 
 }  // namespace dvgb

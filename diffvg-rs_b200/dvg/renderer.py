@@ -129,6 +129,8 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
     L.dvg_context_set_profiling.restype = C.c_int
     L.dvg_context_set_retain.argtypes = [vp, C.c_int]
     L.dvg_context_set_retain.restype = C.c_int
+    L.dvg_context_set_list_memory.argtypes = [vp, C.c_uint64]
+    L.dvg_context_set_list_memory.restype = C.c_int
     Sh = C.POINTER(ShardC)
     L.dvg_scene_tile_count.argtypes = [vp, C.POINTER(C.c_uint32)]
     L.dvg_scene_tile_groups.argtypes = [vp, C.POINTER(C.c_uint32), C.c_uint32]
@@ -414,6 +416,10 @@ class Renderer:
     def set_retain(self, enable: bool) -> None:
         """dvg_context_set_retain: keep the last render for a following render_backward."""
         _check(self.lib.dvg_context_set_retain(self.ctx, 1 if enable else 0))
+
+    def set_list_memory(self, nbytes: int) -> None:
+        """dvg_context_set_list_memory: bytes that the cell lists of a scene uploaded later may take."""
+        _check(self.lib.dvg_context_set_list_memory(self.ctx, nbytes))
 
     def set_profiling(self, enable: bool) -> None:
         _check(self.lib.dvg_context_set_profiling(self.ctx, 1 if enable else 0))

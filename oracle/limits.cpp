@@ -32,3 +32,10 @@ extern "C" long long limits_room(long long tiles, int need, int cap) {
     }
     return granted;
 }
+
+// The room of a scene's cell lists: out = entries, items, their offsets, the counters' offset, bytes.
+extern "C" void limits_cell_room(uint64_t tiles, uint64_t tile_entries, uint64_t items, uint64_t budget, uint64_t* out) {
+    const dvgb::CellRoom r = dvgb::cell_room(tiles, tile_entries, items, budget);
+    const uint64_t v[6] = {r.ents, r.items, r.at_ents, r.at_items, r.at_counters, r.bytes};
+    for (int k = 0; k < 6; ++k) out[k] = v[k];
+}

@@ -50,6 +50,28 @@ def test_room_is_given_once(limits, tiles, groups):
         assert f(tiles, need, cap) == (min(tiles, cap // need) if need else tiles)
 
 
+@pytest.mark.parametrize("tiles, entries", [(0, 0), (1, 0), (16, 40), (4096, 110_700), (16384, 16_400_000),
+                                            (262144, 1 << 31)])
+def test_cell_list_memory_within_its_limit(limits, tiles, entries):
+    """1,000 canvas-wide groups at 2048x2048 wanted 21 GB for lists that are an optimisation."""
+    f = limits.limits_cell_room
+    f.argtypes, f.restype = [C.c_uint64] * 4 + [C.c_void_p], None
+    want = (min(max(entries, 1) * 16, 1 << 30), min(max(48 * entries, 1), 1 << 30))
+    for budget in (0, 1, 1000, 1 << 16, 1 << 20, 1 << 30, 4 << 30, 1 << 40):
+        out = (C.c_uint64 * 6)()
+        f(tiles, entries, 48 * entries, budget, out)
+        ents, items, at_ents, at_items, at_counters, total = out
+        if total == 0:
+            assert tiles == 0 or budget < tiles * 128 + 1000
+            continue
+        assert total <= budget and 1 <= ents <= want[0] and 1 <= items <= want[1]
+        assert at_ents >= tiles * 128 and at_ents % 16 == 0
+        assert at_items >= at_ents + ents * 32 and at_counters >= at_items + items * 16 and at_counters % 8 == 0
+        assert total >= at_counters + 16
+        if budget == 1 << 40:
+            assert (ents, items) == want
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("spp", [(2, 2), (4, 4), (3, 2)])
 @pytest.mark.parametrize("prefilter", [False, True])
