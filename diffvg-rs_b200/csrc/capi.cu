@@ -184,6 +184,7 @@ struct dvg_scene {
     SceneBuf entries;  // tile entries
     SceneBuf cells;    // per-cell lists (cell_table)
     CellTable cell_table{};          // info NULL: none
+    bool lists_for_steps = false;    // they have room for what parameter steps move (dvg_batch_set_adam)
     std::vector<SceneBuf> replaced;  // blocks that a batch or a captured graph may still read
     SceneBuf grads;    // gradient arena (device)
     size_t grad_off[11] = {0};
@@ -1576,22 +1577,26 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
         const size_t need = std::max<size_t>(tiles * (size_t)std::max(sc->dev.num_groups, 1), 1);
         if (need > ((size_t)1 << 28))
             return fail(DVG_ERR_DEVICE_LIMIT, "tile lists of an optimised scene would exceed 2^28 entries");
+        int* counts = sc->tiles.as<int>();
+        int* offsets = counts + tiles;
         if (sc->entries.bytes < need * sizeof(int)) {
             CK(sc->entries.reserve(need * sizeof(int), &sc->replaced));
             sc->dev.tile_entries = sc->entries.as<int>();
-            int* counts = sc->tiles.as<int>();
-            int* offsets = counts + tiles;
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, nullptr, ctx->stream);
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
             CK(cudaGetLastError());
-            // room for twice the entries and items that the present geometry takes: what a step
-            // moves into view beyond that walks the tile lists or keeps the full queries
+        }
+        if (!sc->lists_for_steps) {
+            // room for twice the entries and items that the present geometry takes, whether or not the
+            // tile list had to grow: what a step moves into view beyond that walks the tile
+            // lists or keeps the full queries
             int total = 0;
             CK(cudaMemcpyAsync(&total, offsets + tiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
             const dvg_status st =
                 make_cells(ctx, sc, std::min<uint64_t>(need, 2 * (uint64_t)std::max(total, 0) + 1024), 2, &sc->replaced);
             if (st != DVG_OK) return st;
+            sc->lists_for_steps = true;
         }
         b->host_entries[i].S.tile_entries = sc->dev.tile_entries;
         b->host_entries[i].S.cell_info = sc->dev.cell_info;

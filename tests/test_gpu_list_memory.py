@@ -136,3 +136,19 @@ def test_optimised_scene(renderer, limited, share, step_share):
     other.close()
     up.close()
     fresh.close()
+
+
+def test_room_for_steps_where_the_tile_list_is_full(renderer):
+    """A canvas of one tile has every group in its list from the start; its cell lists are still made
+    anew, with room for what steps move, when the steps are set up (once)."""
+    sc = _scene(16, 16, 3, 10)
+    up = renderer.upload(sc)
+    assert int(up.tile_groups().sum()) == 3  # the list needs no growth
+    b = Batch(renderer, [up], RenderOptions(samples_x=2, samples_y=2, seed=1, use_prefiltering=False))
+    n = [renderer.launch_count]
+    for _ in range(2):
+        b.set_adam(0.1)
+        n.append(renderer.launch_count)
+    assert n[1] > n[0] and n[2] == n[1]
+    b.close()
+    up.close()
