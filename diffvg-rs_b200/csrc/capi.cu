@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -179,6 +180,7 @@ struct dvg_scene {
     dvg_context* ctx = nullptr;
     HostScene host;
     DevScene dev{};
+    std::atomic<bool> shared{false};  // another context has work on it (use_scene)
     SceneBuf arena;
     SceneBuf tiles;    // counts, offsets
     SceneBuf entries;  // tile entries
@@ -196,6 +198,10 @@ struct dvg_scene {
 
 namespace {
 
+// Called before a context enqueues work that reads or writes a scene's memory.
+void use_scene(const dvg_context* ctx, dvg_scene* sc) {
+    if (ctx != sc->ctx) sc->shared = true;
+}
 // Makes room for a scene's cell lists, of `total` tile entries and `items` items, within the
 // context's limit, and points its tables at it.  The lists are an optimisation: without
 // memory for more, the room and the lists that there are stay (false), or there are none and
@@ -623,7 +629,9 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
 void dvg_scene_destroy(dvg_scene* scene) {
     if (!scene) return;
     cudaSetDevice(scene->ctx->device);
-    cudaStreamSynchronize(scene->ctx->stream);
+    // the memory goes back to the pool for the next upload: no stream may still be on it
+    if (scene->shared) cudaDeviceSynchronize();
+    else cudaStreamSynchronize(scene->ctx->stream);
     if (scene->ctx->shard_scene == scene) scene->ctx->shard_scene = nullptr;
     delete scene;
 }
@@ -639,6 +647,7 @@ static dvg_status render_into(dvg_context* ctx, dvg_scene* sc, const dvg_render_
     if (weights_out) *weights_out = false;
     const size_t npix = (size_t)S.width * S.height;
     if (npix == 0) return DVG_OK;
+    use_scene(ctx, sc);
     if (S.num_groups == 0) {  // Image::solid / background image (src/renderer/renderer.rs:57-66)
         {
             Prof prof_(ctx, "fill_background");
@@ -725,6 +734,7 @@ static dvg_status backward_core(dvg_context* ctx, dvg_scene* sc, const dvg_rende
     const DevScene& S = sc->dev;
     const size_t npix = (size_t)S.width * S.height;
     if (npix == 0) return DVG_OK;
+    use_scene(ctx, sc);
     SampleParams sp = sample_params(opts, sc->tune);
     if (frag_ready) attach_frag(sp, ctx->frag.ptr, S.tiles_x * S.tiles_y, (int)sc->tune.fragment_slots);
     const bool run_tiles = !shard || shard->tile_end > shard->tile_begin;  // a shard may hold samples only
@@ -892,6 +902,7 @@ static dvg_status backward_host_impl(dvg_context* ctx, dvg_scene* scene, const d
     CK(cudaSetDevice(ctx->device));
     const HostScene& h = scene->host;
     const size_t npix = (size_t)h.width * h.height;
+    use_scene(ctx, scene);
     GradPtrs G = device_grads(scene);
     CK(cudaMemsetAsync(scene->grads.ptr, 0, scene->grad_floats * sizeof(float), ctx->stream));
     bool want_bg_img = d_render && !h.bg_image.empty() && grads->d_background_image;
@@ -1080,6 +1091,7 @@ dvg_status dvg_shard_forward(dvg_context* ctx, dvg_scene* scene, const dvg_rende
     CK(cudaSetDevice(ctx->device));
     const DevScene& S = scene->dev;
     const size_t npix = (size_t)S.width * S.height;
+    use_scene(ctx, scene);
     ++ctx->gen;
     ctx->shard_scene = nullptr;
     if (npix == 0) return DVG_OK;
@@ -1119,6 +1131,7 @@ dvg_status dvg_shard_resolve(dvg_context* ctx, dvg_scene* scene, const float* ac
     if (!ctx || !scene || !accum_rgba || !wsum || !out_rgba) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     CK(cudaSetDevice(ctx->device));
     const DevScene& S = scene->dev;
+    use_scene(ctx, scene);
     if ((size_t)S.width * S.height == 0) return DVG_OK;
     if (S.num_groups == 0) {
         ctx->launches += launch_fill_background(S, out_rgba, ctx->stream);
@@ -1225,6 +1238,7 @@ extern "C" dvg_status dvg_render_device_noalloc(dvg_context* ctx, dvg_scene* sce
     float* scratch = nullptr;
     st = noalloc_scratch(ctx->device, &scratch);
     if (st != DVG_OK) return st;
+    use_scene(ctx, scene);
     if (S.num_groups == 0) {
         ctx->launches += launch_fill_background(S, out_rgba, ctx->stream);
         CK(cudaGetLastError());
@@ -1725,6 +1739,7 @@ extern "C" dvg_status dvg_render_sdf_device(dvg_context* ctx, dvg_scene* scene, 
     const DevScene& S = scene->dev;
     const size_t npix = (size_t)S.width * S.height;
     if (npix == 0) return DVG_OK;
+    use_scene(ctx, scene);
     if (S.num_groups == 0) {
         CK(cudaMemsetAsync(out, 0, npix * sizeof(float), ctx->stream));
         return DVG_OK;
@@ -1769,6 +1784,7 @@ extern "C" dvg_status dvg_eval_positions_device(dvg_context* ctx, dvg_scene* sce
     if (!ctx || !scene || (count && (!positions || !out))) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     CK(cudaSetDevice(ctx->device));
     if (count == 0) return DVG_OK;
+    use_scene(ctx, scene);
     if (scene->dev.num_groups == 0) {
         CK(cudaMemsetAsync(out, 0, count * sizeof(float), ctx->stream));
         return DVG_OK;
@@ -1822,6 +1838,7 @@ extern "C" dvg_status dvg_eval_positions_backward_device(dvg_context* ctx, dvg_s
     G.d_background_image = nullptr;
     dvg_status st = zero_grads(ctx, scene, grads_from_user(grads));
     if (st != DVG_OK) return st;
+    use_scene(ctx, scene);
     if (count == 0 || scene->dev.num_groups == 0) return DVG_OK;
     {
         Prof prof_(ctx, "positions_backward");
@@ -1840,6 +1857,7 @@ extern "C" dvg_status dvg_eval_positions_backward_host(dvg_context* ctx, dvg_sce
     CK(cudaSetDevice(ctx->device));
     const HostScene& h = scene->host;
     const size_t npix = (size_t)h.width * h.height;
+    use_scene(ctx, scene);
     GradPtrs G = device_grads(scene);
     CK(cudaMemsetAsync(scene->grads.ptr, 0, scene->grad_floats * sizeof(float), ctx->stream));
     const bool want_tr = bopts && bopts->compute_translation && grads->d_translation && npix;
