@@ -148,6 +148,7 @@ struct dvg_context {
     std::vector<ProfEvent> pending;
     std::vector<ProfStat> stats;
     cudaStream_t stream = nullptr;
+    cudaStream_t build = nullptr;  // builds scenes' cell lists, independent of what `stream` waits for
     cudaMemPool_t pool = nullptr;  // scene memory (SceneBuf)
     uint64_t list_memory = kListMemory;
     unsigned* status = nullptr;  // device word
@@ -155,7 +156,7 @@ struct dvg_context {
     DevBuf bsamples, bkey, border, bcounts, bsegs;  // boundary-pass scratch
     DevBuf sdf, positions, dvalues;          // signed-distance host calls
     DevBuf frag;                             // fragment cache of the fused calls
-    uint64_t launches = 0;
+    std::atomic<uint64_t> launches{0};  // (another context's call may build a scene's lists here)
     // Retained render: dvg_render keeps its prepared scene, and its weight image and
     // fragment cache stay valid until the next call that writes them (gen counts
     // those calls), so a dvg_render_backward of the same description and options
@@ -185,15 +186,27 @@ struct dvg_scene {
     SceneBuf tiles;    // counts, offsets
     SceneBuf entries;  // tile entries
     SceneBuf cells;    // per-cell lists (cell_table)
-    CellTable cell_table{};          // info NULL: none
-    bool lists_for_steps = false;    // they have room for what parameter steps move (dvg_batch_set_adam)
-    std::vector<SceneBuf> replaced;  // blocks that a batch or a captured graph may still read
+    // The lists are built by the first call that reads them (scene_with_lists), since
+    // signed-distance calls never do; `lists` and what follows it belong to the mutex.
+    enum class Lists { NONE, RESERVED, BUILDING, READY };
+    std::mutex lists_mutex;
+    Lists lists = Lists::NONE;
+    CellTable cell_table{};
+    cudaEvent_t lists_built = nullptr;  // recorded on ctx->build
+    uint64_t lists_total = 0;           // tile entries at the upload
+    uint64_t lists_items = 0;           // items that the built lists asked for
+    bool lists_passed = false;          // a small render has done without them
+    bool lists_for_steps = false;       // room for what parameter steps move (dvg_batch_set_adam)
+    std::vector<SceneBuf> replaced;     // blocks that a batch or a captured graph may still read
     SceneBuf grads;    // gradient arena (device)
     size_t grad_off[11] = {0};
     size_t grad_floats = 0;
     size_t arena_bytes = 0;  // bytes of prepared tables in `arena`
     const float4* g_bbox = nullptr;
     dvg_tuning tune{1, 4, 16, 0, 0};  // launch shape (dvg_scene_set_tuning / dvg_scene_autotune)
+    ~dvg_scene() {
+        if (lists_built) cudaEventDestroy(lists_built);
+    }
 };
 
 namespace {
@@ -203,43 +216,134 @@ void use_scene(const dvg_context* ctx, dvg_scene* sc) {
     if (ctx != sc->ctx) sc->shared = true;
 }
 // Makes room for a scene's cell lists, of `total` tile entries and `items` items, within the
-// context's limit, and points its tables at it.  The lists are an optimisation: without
-// memory for more, the room and the lists that there are stay (false), or there are none and
-// the kernels walk the tile lists.
-bool reserve_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, uint64_t items, std::vector<SceneBuf>* keep) {
-    DevScene& S = sc->dev;
-    const CellRoom r = cell_room((uint64_t)S.tiles_x * S.tiles_y, total, items, ctx->list_memory);
-    if (r.bytes <= sc->cells.bytes || sc->cells.reserve(r.bytes, keep) != cudaSuccess) return false;
+// context's limit, for use on `stream`.  The lists are an optimisation: without memory for more,
+// the room and the lists that there are stay (false), or there are none and the kernels walk
+// the tile lists.
+bool reserve_cells(dvg_scene* sc, uint64_t total, uint64_t items, cudaStream_t stream, std::vector<SceneBuf>* keep) {
+    const CellRoom r = cell_room((uint64_t)sc->dev.tiles_x * sc->dev.tiles_y, total, items, sc->ctx->list_memory);
+    if (r.bytes <= sc->cells.bytes) return false;
+    sc->cells.stream = stream;
+    if (sc->cells.reserve(r.bytes, keep) != cudaSuccess) return false;
     char* b = sc->cells.as<char>();
     sc->cell_table = CellTable{(int2*)b, (int4*)(b + r.at_ents), (int4*)(b + r.at_items),
                                (unsigned long long*)(b + r.at_counters), (int)r.ents, (int)r.items};
-    S.cell_info = sc->cell_table.info;
-    S.cell_entries = sc->cell_table.entries;
-    S.cell_items = sc->cell_table.items;
     return true;
 }
-// Builds the lists on the context's stream (after the tile lists).
-dvg_status build_cells(dvg_context* ctx, dvg_scene* sc) {
+// Builds the lists on `stream` (after the tile lists).
+dvg_status build_cells(dvg_scene* sc, cudaStream_t stream) {
     if (!sc->cell_table.info) return DVG_OK;
-    CK(cudaMemsetAsync(sc->cell_table.counters, 0, 2 * sizeof(unsigned long long), ctx->stream));
-    ctx->launches += launch_cells(sc->dev, sc->cell_table, ctx->stream);
+    CK(cudaMemsetAsync(sc->cell_table.counters, 0, 2 * sizeof(unsigned long long), stream));
+    sc->ctx->launches += launch_cells(sc->dev, sc->cell_table, stream);
     CK(cudaGetLastError());
     return DVG_OK;
 }
-// Reserves and builds, and waits: the item counter runs on past the room there is, so a scene
-// that needs more than the first guess (three per cell entry) is built once again with what it
-// counted, times `slack`.
-dvg_status make_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, int slack, std::vector<SceneBuf>* keep) {
-    if (!reserve_cells(ctx, sc, total, 3 * CELLS * total * slack, keep)) return DVG_OK;
-    dvg_status st = build_cells(ctx, sc);
-    if (st != DVG_OK) return st;
+// Waits for lists built on `stream` and reads how many items they asked for (the counter runs on
+// past the room there is).
+dvg_status read_cells(dvg_scene* sc, cudaStream_t stream) {
     unsigned long long used[2] = {0, 0};
-    CK(cudaMemcpyAsync(used, sc->cell_table.counters, sizeof used, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (used[1] <= (unsigned long long)(sc->cell_table.cap_items / slack)) return DVG_OK;
-    return reserve_cells(ctx, sc, total, used[1] * slack, keep) ? build_cells(ctx, sc) : DVG_OK;
+    CK(cudaMemcpyAsync(used, sc->cell_table.counters, sizeof used, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    sc->lists_items = used[1];
+    sc->lists = dvg_scene::Lists::READY;
+    return DVG_OK;
+}
+// Builds lists once again with the room that they asked for, times `slack`, where the first guess
+// (three items per cell entry) was short of it.  What reads the old ones may go on.
+dvg_status grow_cells(dvg_scene* sc, uint64_t total, int slack, cudaStream_t stream) {
+    if (sc->lists_items * slack <= (uint64_t)sc->cell_table.cap_items) return DVG_OK;
+    const uint64_t items = sc->lists_items * slack;
+    sc->lists_items = 0;  // one attempt
+    if (!reserve_cells(sc, total, items, stream, &sc->replaced)) return DVG_OK;
+    dvg_status st = build_cells(sc, stream);
+    if (st == DVG_OK) CK(cudaStreamSynchronize(stream));
+    return st;
+}
+// Lists of a scene that a batch holds, made anew on the context's stream with room for `slack` times
+// what they ask for; without memory for them the old ones stay.
+dvg_status remake_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, int slack) {
+    std::lock_guard<std::mutex> lock(sc->lists_mutex);
+    if (!reserve_cells(sc, total, 3 * CELLS * total * slack, ctx->stream, &sc->replaced)) return DVG_OK;
+    dvg_status st = build_cells(sc, ctx->stream);
+    if (st == DVG_OK) st = read_cells(sc, ctx->stream);
+    if (st == DVG_OK) st = grow_cells(sc, total, slack, ctx->stream);
+    sc->lists_items = 0;
+    return st;
+}
+// Lets this thread make calls that a stream capture elsewhere in the process would refuse.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// The scene's tables with its cell lists, for work on ctx->stream.  The first call builds the lists
+// on a stream of their own: it needs nothing that ctx->stream waits for, and the host waits
+// only where ctx->stream is being captured (the lists have to be there when the capture is
+// replayed, on whatever stream) or where the caller keeps the addresses (Reader::BATCH: they do not
+// change after it).  Other calls that come before the lists are complete wait for them on the
+// device, and one that comes later makes room for crowded cells, unless it must not allocate.
+//
+// `ctas`: the CTAs of a point-sampled render that is all the call does (0: anything else).  A first
+// render of up to kWalkCtas walks the tile lists and leaves the lists to a second reader: building
+// them takes about as long as a render without them that fills no more than half of the 148
+// SMs.  Upload and one render, 3 to 100 paths: 4 to 64 CTAs 0.73 to 1.13 times as fast with lists as
+// without (a 64x64 icon of 10 paths at 2x2, 64 CTAs: 215 us with, 207 without), 144 CTAs 0.97 to
+// 1.18, 1024 CTAs 1.15 to 2.6; prefiltered renders 0.98 to 1.2 up to 256 CTAs.
+constexpr uint64_t kWalkCtas = 74;
+enum class Reader { CALL, NO_ALLOC, BATCH };
+dvg_status scene_with_lists(dvg_context* ctx, dvg_scene* sc, DevScene* S, Reader reader = Reader::CALL,
+                            uint64_t ctas = 0) {
+    using Lists = dvg_scene::Lists;
+    const bool grow = reader != Reader::NO_ALLOC;
+    *S = sc->dev;
+    if (S->num_groups == 0) return DVG_OK;
+    std::lock_guard<std::mutex> lock(sc->lists_mutex);
+    if (sc->lists == Lists::NONE) return DVG_OK;
+    const cudaStream_t build = sc->ctx->build;
+    if (sc->lists != Lists::READY || (grow && sc->lists_items > (uint64_t)sc->cell_table.cap_items)) {
+        RelaxedCapture relaxed;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(ctx->stream, &capture));
+        const bool captured = capture != cudaStreamCaptureStatusNone;
+        if (sc->lists == Lists::RESERVED) {
+            if (ctas > 0 && ctas <= kWalkCtas && !captured && !sc->lists_passed) {
+                sc->lists_passed = true;
+                return DVG_OK;
+            }
+            if (!sc->lists_built) CK(cudaEventCreateWithFlags(&sc->lists_built, cudaEventDisableTiming));
+            const dvg_status st = build_cells(sc, build);
+            if (st != DVG_OK) return st;
+            CK(cudaEventRecord(sc->lists_built, build));
+            sc->lists = Lists::BUILDING;
+        }
+        if (sc->lists == Lists::BUILDING) {
+            const cudaError_t e = captured || reader == Reader::BATCH ? cudaEventSynchronize(sc->lists_built)
+                                                                      : cudaEventQuery(sc->lists_built);
+            if (e == cudaErrorNotReady) {
+                cudaGetLastError();  // (not an error)
+                CK(cudaStreamWaitEvent(ctx->stream, sc->lists_built, 0));
+            } else {
+                CK(e);
+                const dvg_status st = read_cells(sc, build);
+                if (st != DVG_OK) return st;
+            }
+        }
+        if (sc->lists == Lists::READY && grow && !captured) {
+            const dvg_status st = grow_cells(sc, sc->lists_total, 1, build);
+            if (st != DVG_OK) return st;
+        }
+    }
+    S->cell_info = sc->cell_table.info;
+    S->cell_entries = sc->cell_table.entries;
+    S->cell_items = sc->cell_table.items;
+    return DVG_OK;
 }
 
+// The CTAs of a point-sampled forward over the whole canvas; 0 for a prefiltered one.
+uint64_t render_ctas(uint64_t width, uint64_t height, const dvg_render_options* o) {
+    if (o->use_prefiltering) return 0;
+    const uint64_t tiles = ((width + TILE - 1) / TILE) * ((height + TILE - 1) / TILE);
+    return tiles * std::max<uint64_t>(o->samples_x, 1) * std::max<uint64_t>(o->samples_y, 1);
+}
 // Offsets of each gradient part inside the scene's gradient arena (in floats).
 void layout_grads(dvg_scene* sc) {
     const HostScene& h = sc->host;
@@ -457,6 +561,7 @@ dvg_status dvg_context_create(int device, dvg_context** out) {
     ctx->device = device;
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&ctx->build, cudaStreamNonBlocking));
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -493,17 +598,26 @@ void dvg_context_destroy(dvg_context* ctx) {
     if (ctx->kept) dvg_scene_destroy(ctx->kept);
     ctx->kept = nullptr;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->build) cudaStreamSynchronize(ctx->build);
     if (ctx->status) cudaFree(ctx->status);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+    if (ctx->build) cudaStreamDestroy(ctx->build);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
 
-uint64_t dvg_context_launch_count(const dvg_context* ctx) { return ctx ? ctx->launches : 0; }
+uint64_t dvg_context_launch_count(const dvg_context* ctx) { return ctx ? ctx->launches.load() : 0; }
 
 void* dvg_context_stream(dvg_context* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
+// When an upload's cell lists are built: at once (the caller renders it next), by the first call
+// that reads them, or not at all (nothing will).
+enum class Build { NOW, FIRST_USE, NEVER };
+static dvg_status upload_scene(dvg_context* ctx, const dvg_scene_desc* desc, Build build, dvg_scene** out);
 dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_scene** out) {
+    return upload_scene(ctx, desc, Build::FIRST_USE, out);
+}
+static dvg_status upload_scene(dvg_context* ctx, const dvg_scene_desc* desc, Build build, dvg_scene** out) {
     if (!ctx || !desc || !out) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     CK(cudaSetDevice(ctx->device));
     std::unique_ptr<dvg_scene> sc(new dvg_scene());
@@ -616,11 +730,20 @@ dvg_status dvg_scene_upload(dvg_context* ctx, const dvg_scene_desc* desc, dvg_sc
         S.tile_entries = sc->entries.as<int>();
         ctx->launches += launch_binning(S, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
         CK(cudaGetLastError());
-        st = make_cells(ctx, sc.get(), (uint64_t)std::max(total, 0), 1, nullptr);
-        if (st != DVG_OK) return st;
+        sc->lists_total = (uint64_t)std::max(total, 0);
+        if (S.num_groups > 0 && build != Build::NEVER &&
+            reserve_cells(sc.get(), sc->lists_total, 3 * CELLS * sc->lists_total,
+                          build == Build::NOW ? ctx->stream : ctx->build, nullptr))
+            sc->lists = dvg_scene::Lists::RESERVED;
     }
     layout_grads(sc.get());
     CK(sc->grads.reserve(sizeof(float) * std::max<size_t>(sc->grad_floats, 64)));
+    if (build == Build::NOW && sc->lists == dvg_scene::Lists::RESERVED) {
+        st = build_cells(sc.get(), ctx->stream);
+        if (st == DVG_OK) st = read_cells(sc.get(), ctx->stream);
+        if (st == DVG_OK) st = grow_cells(sc.get(), sc->lists_total, 1, ctx->stream);
+        if (st != DVG_OK) return st;
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     *out = sc.release();
     return DVG_OK;
@@ -632,6 +755,7 @@ void dvg_scene_destroy(dvg_scene* scene) {
     // the memory goes back to the pool for the next upload: no stream may still be on it
     if (scene->shared) cudaDeviceSynchronize();
     else cudaStreamSynchronize(scene->ctx->stream);
+    if (scene->lists == dvg_scene::Lists::BUILDING) cudaStreamSynchronize(scene->ctx->build);
     if (scene->ctx->shard_scene == scene) scene->ctx->shard_scene = nullptr;
     delete scene;
 }
@@ -640,8 +764,9 @@ void dvg_scene_destroy(dvg_scene* scene) {
 // interior pass that follows (non-prefiltered, cache enabled by the scene's tuning);
 // *frag_out tells whether it did.
 // *weights_out: whether ctx->wsum now holds this scene's weight image.
+// `ctas`: see scene_with_lists.
 static dvg_status render_into(dvg_context* ctx, dvg_scene* sc, const dvg_render_options* opts, float* out_dev,
-                              bool* frag_out = nullptr, bool* weights_out = nullptr) {
+                              uint64_t ctas, bool* frag_out = nullptr, bool* weights_out = nullptr) {
     const DevScene& S = sc->dev;
     if (frag_out) *frag_out = false;
     if (weights_out) *weights_out = false;
@@ -657,6 +782,9 @@ static dvg_status render_into(dvg_context* ctx, dvg_scene* sc, const dvg_render_
         return DVG_OK;
     }
     ++ctx->gen;  // accum, wsum and the fragment cache are rewritten below
+    DevScene L;
+    const dvg_status st = scene_with_lists(ctx, sc, &L, Reader::CALL, ctas);
+    if (st != DVG_OK) return st;
     SampleParams sp = sample_params(opts, sc->tune);
     if (frag_out && !opts->use_prefiltering && sc->tune.fragment_slots > 0) {
         const int tiles = S.tiles_x * S.tiles_y, slots = (int)sc->tune.fragment_slots;
@@ -671,10 +799,10 @@ static dvg_status render_into(dvg_context* ctx, dvg_scene* sc, const dvg_render_
     {
         Prof prof_(ctx, opts->use_prefiltering ? "forward_prefilter" : "forward");
         if (opts->use_prefiltering)
-            ctx->launches += launch_forward_prefilter(S, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->status,
+            ctx->launches += launch_forward_prefilter(L, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->status,
                                                       ctx->stream);
         else
-            ctx->launches += launch_forward(S, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->stream);
+            ctx->launches += launch_forward(L, sp, ctx->accum.as<float>(), ctx->wsum.as<float>(), ctx->stream);
     }
     CK(cudaGetLastError());
     {
@@ -691,7 +819,7 @@ dvg_status dvg_render_device(dvg_context* ctx, dvg_scene* scene, const dvg_rende
     dvg_status st = check_options(opts);
     if (st != DVG_OK) return st;
     CK(cudaSetDevice(ctx->device));
-    return render_into(ctx, scene, opts, out_rgba);
+    return render_into(ctx, scene, opts, out_rgba, render_ctas(scene->dev.width, scene->dev.height, opts));
 }
 
 static dvg_status render_host_impl(dvg_context* ctx, dvg_scene* scene, const dvg_render_options* opts,
@@ -716,7 +844,7 @@ static dvg_status render_host_impl(dvg_context* ctx, dvg_scene* scene, const dvg
         return DVG_OK;
     }
     CK(ctx->image.reserve(npix * 4 * sizeof(float)));
-    st = render_into(ctx, scene, opts, ctx->image.as<float>(), frag_out, weights_out);
+    st = render_into(ctx, scene, opts, ctx->image.as<float>(), render_ctas(h.width, h.height, opts), frag_out, weights_out);
     if (st != DVG_OK) return st;
     CK(cudaMemcpyAsync(out_rgba, ctx->image.ptr, npix * 4 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -745,6 +873,9 @@ static dvg_status backward_core(dvg_context* ctx, dvg_scene* sc, const dvg_rende
     // read at each launch: the weights pass below may (re)allocate ctx->wsum
     auto wsum_now = [&]() -> const float* { return shard ? shard_wsum : ctx->wsum.as<float>(); };
     if (d_render && S.num_groups > 0) {
+        DevScene L;
+        const dvg_status st = scene_with_lists(ctx, sc, &L);
+        if (st != DVG_OK) return st;
         if (!have_weights) {
             ++ctx->gen;
             CK(ctx->wsum.reserve(npix * sizeof(float)));
@@ -757,9 +888,9 @@ static dvg_status backward_core(dvg_context* ctx, dvg_scene* sc, const dvg_rende
             Prof prof_(ctx, opts->use_prefiltering ? "interior_prefilter" : "interior");
             if (opts->use_prefiltering)
                 ctx->launches +=
-                    launch_interior_prefilter(S, sp, d_render, wsum_now(), G, ctx->status, ctx->stream);
+                    launch_interior_prefilter(L, sp, d_render, wsum_now(), G, ctx->status, ctx->stream);
             else
-                ctx->launches += launch_interior(S, sp, d_render, wsum_now(), G, ctx->status, ctx->stream);
+                ctx->launches += launch_interior(L, sp, d_render, wsum_now(), G, ctx->status, ctx->stream);
         }
         CK(cudaGetLastError());
         if (S.boundary_ok && !opts->use_prefiltering) {  // src/backward/render.rs:191
@@ -783,7 +914,7 @@ static dvg_status backward_core(dvg_context* ctx, dvg_scene* sc, const dvg_rende
             const BoundaryScratch sc_{ctx->bsamples.as<BSample>(),   ctx->bkey.as<int2>(),    ctx->border.as<int>(),
                                       ctx->border.as<int>() + cap,   ctx->bcounts.as<int>(), ctx->bsegs.as<int>()};
             Prof prof_(ctx, "boundary");
-            ctx->launches += launch_boundary(S, bp, d_render, wsum_now(), G, sc_, cap, ctx->stream);
+            ctx->launches += launch_boundary(L, bp, d_render, wsum_now(), G, sc_, cap, ctx->stream);
             CK(cudaGetLastError());
         }
     } else if (d_render && S.num_groups == 0) {
@@ -972,7 +1103,8 @@ dvg_status dvg_render(dvg_context* ctx, const dvg_scene_desc* desc, const dvg_re
     dvg_status st = check_options(opts);
     if (st != DVG_OK) return st;
     dvg_scene* sc = nullptr;
-    st = dvg_scene_upload(ctx, desc, &sc);
+    const uint64_t ctas = render_ctas(desc->width, desc->height, opts);
+    st = upload_scene(ctx, desc, ctas > 0 && ctas <= kWalkCtas ? Build::FIRST_USE : Build::NOW, &sc);
     if (st != DVG_OK) return st;
     if (!ctx->retain) {
         st = dvg_render_host(ctx, sc, opts, out_rgba);
@@ -1011,7 +1143,7 @@ dvg_status dvg_render_backward(dvg_context* ctx, const dvg_scene_desc* desc, con
                                       ctx->kept_frag);
     }
     dvg_scene* sc = nullptr;
-    st = dvg_scene_upload(ctx, desc, &sc);
+    st = upload_scene(ctx, desc, d_render ? Build::NOW : Build::NEVER, &sc);
     if (st != DVG_OK) return st;
     st = dvg_render_backward_host(ctx, sc, opts, bopts, d_render, d_sdf, grads);
     dvg_scene_destroy(sc);
@@ -1033,7 +1165,7 @@ dvg_status dvg_fwd_bwd_l2_device(dvg_context* ctx, dvg_scene* scene, const dvg_r
         img = ctx->image.as<float>();
     }
     bool frag = false;
-    st = render_into(ctx, scene, opts, img, &frag);
+    st = render_into(ctx, scene, opts, img, 0, &frag);
     if (st != DVG_OK) return st;
     CK(ctx->d_render.reserve(npix * 4 * sizeof(float)));
     if (loss_out) CK(cudaMemsetAsync(loss_out, 0, sizeof(float), ctx->stream));
@@ -1098,6 +1230,9 @@ dvg_status dvg_shard_forward(dvg_context* ctx, dvg_scene* scene, const dvg_rende
     CK(cudaMemsetAsync(accum_rgba, 0, npix * 4 * sizeof(float), ctx->stream));
     CK(cudaMemsetAsync(wsum, 0, npix * sizeof(float), ctx->stream));
     if (S.num_groups == 0 || shard->tile_end == shard->tile_begin) return DVG_OK;
+    DevScene L;
+    st = scene_with_lists(ctx, scene, &L);
+    if (st != DVG_OK) return st;
     SampleParams sp = sample_params(opts, scene->tune);
     sp.tile_base = (int)shard->tile_begin;
     sp.tile_count = (int)(shard->tile_end - shard->tile_begin);
@@ -1111,9 +1246,9 @@ dvg_status dvg_shard_forward(dvg_context* ctx, dvg_scene* scene, const dvg_rende
     {
         Prof prof_(ctx, opts->use_prefiltering ? "forward_prefilter" : "forward");
         if (opts->use_prefiltering)
-            ctx->launches += launch_forward_prefilter(S, sp, accum_rgba, wsum, ctx->status, ctx->stream);
+            ctx->launches += launch_forward_prefilter(L, sp, accum_rgba, wsum, ctx->status, ctx->stream);
         else
-            ctx->launches += launch_forward(S, sp, accum_rgba, wsum, ctx->stream);
+            ctx->launches += launch_forward(L, sp, accum_rgba, wsum, ctx->stream);
     }
     CK(cudaGetLastError());
     ctx->shard_scene = scene;
@@ -1244,14 +1379,17 @@ extern "C" dvg_status dvg_render_device_noalloc(dvg_context* ctx, dvg_scene* sce
         CK(cudaGetLastError());
         return DVG_OK;
     }
+    DevScene L;
+    st = scene_with_lists(ctx, scene, &L, Reader::NO_ALLOC, render_ctas(S.width, S.height, opts));
+    if (st != DVG_OK) return st;
     float* accum = scratch;            // 4 floats per pixel (float4 aligned: 256-byte base)
     float* wsum = scratch + 4 * npix;  // 1 float per pixel
     CK(cudaMemsetAsync(scratch, 0, 5 * npix * sizeof(float), ctx->stream));
     const SampleParams sp = sample_params(opts, scene->tune);
     if (opts->use_prefiltering)
-        ctx->launches += launch_forward_prefilter(S, sp, accum, wsum, ctx->status, ctx->stream);
+        ctx->launches += launch_forward_prefilter(L, sp, accum, wsum, ctx->status, ctx->stream);
     else
-        ctx->launches += launch_forward(S, sp, accum, wsum, ctx->stream);
+        ctx->launches += launch_forward(L, sp, accum, wsum, ctx->stream);
     ctx->launches += launch_resolve(S, accum, wsum, out_rgba, ctx->stream);
     CK(cudaGetLastError());
     return DVG_OK;
@@ -1335,7 +1473,7 @@ dvg_status batch_enqueue(dvg_batch* b) {
             int* offsets = counts + sc->dev.tiles_x * sc->dev.tiles_y;
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, nullptr, ctx->stream);
             ctx->launches += launch_binning(sc->dev, sc->g_bbox, counts, offsets, sc->entries.as<int>(), ctx->stream);
-            const dvg_status st = build_cells(ctx, sc);
+            const dvg_status st = build_cells(sc, ctx->stream);
             if (st != DVG_OK) return st;
         }
     }
@@ -1397,7 +1535,9 @@ extern "C" dvg_status dvg_batch_create(dvg_context* ctx, dvg_scene* const* scene
     for (uint32_t i = 0; i < count; ++i) {
         dvg_scene* sc = scenes[i];
         if (!sc || sc->ctx != ctx) return fail(DVG_ERR_INVALID_ARGUMENT, "batch scene is null or from another context");
-        const DevScene& S = sc->dev;
+        DevScene S;
+        st = scene_with_lists(ctx, sc, &S, Reader::BATCH);
+        if (st != DVG_OK) return st;
         const size_t npix = (size_t)S.width * S.height;
         if (npix == 0 || S.num_groups == 0)
             return fail(DVG_ERR_INVALID_ARGUMENT, "batch scenes need a non-empty canvas and at least one group");
@@ -1608,14 +1748,14 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
             CK(cudaMemcpyAsync(&total, offsets + tiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
             const dvg_status st =
-                make_cells(ctx, sc, std::min<uint64_t>(need, 2 * (uint64_t)std::max(total, 0) + 1024), 2, &sc->replaced);
+                remake_cells(ctx, sc, std::min<uint64_t>(need, 2 * (uint64_t)std::max(total, 0) + 1024), 2);
             if (st != DVG_OK) return st;
             sc->lists_for_steps = true;
         }
         b->host_entries[i].S.tile_entries = sc->dev.tile_entries;
-        b->host_entries[i].S.cell_info = sc->dev.cell_info;
-        b->host_entries[i].S.cell_entries = sc->dev.cell_entries;
-        b->host_entries[i].S.cell_items = sc->dev.cell_items;
+        b->host_entries[i].S.cell_info = sc->cell_table.info;
+        b->host_entries[i].S.cell_entries = sc->cell_table.entries;
+        b->host_entries[i].S.cell_items = sc->cell_table.items;
     }
     // Adam moments and sort scratch, one block per scene.
     std::vector<size_t> st_off(n), so_off(n);
@@ -1772,7 +1912,7 @@ extern "C" dvg_status dvg_render_sdf(dvg_context* ctx, const dvg_scene_desc* des
     dvg_status st = check_options(opts);
     if (st != DVG_OK) return st;
     dvg_scene* sc = nullptr;
-    st = dvg_scene_upload(ctx, desc, &sc);
+    st = upload_scene(ctx, desc, Build::NEVER, &sc);
     if (st != DVG_OK) return st;
     st = dvg_render_sdf_host(ctx, sc, opts, out);
     dvg_scene_destroy(sc);
@@ -1819,7 +1959,7 @@ extern "C" dvg_status dvg_eval_positions(dvg_context* ctx, const dvg_scene_desc*
     if (!ctx || !desc) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     if (count == 0) return DVG_OK;
     dvg_scene* sc = nullptr;
-    dvg_status st = dvg_scene_upload(ctx, desc, &sc);
+    dvg_status st = upload_scene(ctx, desc, Build::NEVER, &sc);
     if (st != DVG_OK) return st;
     st = dvg_eval_positions_host(ctx, sc, positions, count, out);
     dvg_scene_destroy(sc);
@@ -1913,7 +2053,7 @@ extern "C" dvg_status dvg_eval_positions_backward(dvg_context* ctx, const dvg_sc
                                                   uint64_t count, const float* d_values, dvg_grads* grads) {
     if (!ctx || !desc || !grads) return fail(DVG_ERR_INVALID_ARGUMENT, "null argument");
     dvg_scene* sc = nullptr;
-    dvg_status st = dvg_scene_upload(ctx, desc, &sc);
+    dvg_status st = upload_scene(ctx, desc, Build::NEVER, &sc);
     if (st != DVG_OK) return st;
     st = dvg_eval_positions_backward_host(ctx, sc, bopts, positions, count, d_values, grads);
     dvg_scene_destroy(sc);
