@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
         E[1] = make_int4(s, (base[c] & 0xffff) | (base_slow[c] << 16), at,
                          nl | (nc << 6) | (nh << 12) | (nf << 18) | (ns << 24));
         kept[c] += 1;
-        steps[c] += nl + nc + nh + ns;
+        steps[c] += entry_steps(nl, nc, nh, ns);
     }
     __syncthreads();
     if (tid < CELLS) T.info[tile * CELLS + tid] = make_int2(ent_base + tid * n, kept[tid] | (steps[tid] >= CELL_HEAVY ? CELL_HEAVY_BIT : 0));

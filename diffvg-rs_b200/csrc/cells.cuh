@@ -46,7 +46,6 @@ enum : int {
 // counts: level pairs, curves, hard segments, segments, stroke segments, six bits each; hard =
 // CELL_PRIMITIVE: the shape is a circle, an ellipse or a rectangle.
 constexpr int CELL_MAX_ITEMS = 48;  // of each kind
-constexpr int CELL_PRIMITIVE = 63;
 struct CellCounts {
     int pairs, curves, hard, segs, strokes;
     __device__ __forceinline__ explicit CellCounts(int w)
@@ -69,11 +68,11 @@ static __device__ __noinline__ bool group_inside_any(const DevScene& S, int g, f
     return group_inside(S, g, lp, __ldg(&S.g_info[g].z));
 }
 
-// A cell is heavy from this many rows, curves and one-point segments in its lists.  The kernels
-// are bound by instruction fetch: where the lists are long, a CTA's warps take them one entry at
-// a time, so that they run the same code together (forward of the large 1024x1024 scene 18.5 ->
-// 14.7 ms, edge pass 62.9 -> 48.0).  From 40: 15.5 and 49.0 ms, from 64: 17.4 and 55.9; short
-// lists lose by it (mixed 512x512 scene, forward 0.81 ms, 0.85 with every list in steps).
+// A cell is heavy from this many steps in its lists (entry_steps).  The kernels are bound by
+// instruction fetch: where the lists are long, a CTA's warps take them one entry at a time, so that
+// they run the same code together (forward of the large 1024x1024 scene 18.5 -> 14.7 ms, edge pass
+// 62.9 -> 48.0 when it came in).  Against 24, from 12 on: batch of 64 icons 5.25 -> 5.58 ms, large
+// render 15.9 -> 15.7; from 40 on: large render 16.7, its step 69.6 -> 71.5 ms.
 constexpr int CELL_HEAVY = 24;
 constexpr int CELL_HEAVY_BIT = 1 << 30;
 

@@ -41,6 +41,13 @@ constexpr int CELL_LIST_MAX = 1 << 22;
 DVG_LIM_HD int entry_word(bool listed, int place, int flags) { return listed ? (place << 8) | flags : flags; }
 DVG_LIM_HD int entry_place(bool listed, int step, int word) { return listed ? word >> 8 : step; }
 
+// Steps that an entry adds to its cell: pairs of rows, curves, one-point segments and stroke
+// segments.  `hard` also says that the shape is a primitive (one formula, no segments).
+constexpr int CELL_PRIMITIVE = 63;
+DVG_LIM_HD int entry_steps(int pairs, int curves, int hard, int strokes) {
+    return pairs + curves + (hard == CELL_PRIMITIVE ? 1 : hard) + strokes;
+}
+
 // Where a request for `need` of `cap` places begins when `taken` were asked for before it, or -1:
 // no room.  `taken` goes on counting when the room is used up (the host reads what a scene
 // would have needed), in 64 bits: in 32 it came round to small numbers after 2^28 tile entries, and

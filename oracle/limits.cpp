@@ -39,3 +39,7 @@ extern "C" void limits_cell_room(uint64_t tiles, uint64_t tile_entries, uint64_t
     const uint64_t v[6] = {r.ents, r.items, r.at_ents, r.at_items, r.at_counters, r.bytes};
     for (int k = 0; k < 6; ++k) out[k] = v[k];
 }
+
+extern "C" int limits_entry_steps(int pairs, int curves, int hard, int strokes) {
+    return dvgb::entry_steps(pairs, curves, hard, strokes);
+}

@@ -72,6 +72,14 @@ def test_cell_list_memory_within_its_limit(limits, tiles, entries):
             assert (ents, items) == want
 
 
+def test_steps_of_an_entry(limits):
+    """The count that makes a cell heavy: a circle's edge is one step, not the 63 that mark it in the
+    place of a number of segments."""
+    assert limits.limits_entry_steps(2, 3, 4, 5) == 14
+    assert limits.limits_entry_steps(0, 0, 63, 0) == 1
+    assert limits.limits_entry_steps(0, 0, 48, 2) == 50
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("spp", [(2, 2), (4, 4), (3, 2)])
 @pytest.mark.parametrize("prefilter", [False, True])
