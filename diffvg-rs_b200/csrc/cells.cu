@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) k_cells(const __grid_constant__ DevScene 
         const int g = __ldg(&S.tile_entries[off + e]);
         const int4 gi = __ldg(&S.g_info[g]);
         const int4 gb = __ldg(&S.g_bvh[g]);
-        if (gb.y == 0) continue;  // no bounds, no binning: not reached
+        if (gb.y == 0) continue;  // no shape with points: nothing to cover (an empty box is in the list of a one-tile canvas)
         const int4 root = __ldg(&S.gn_meta[gb.x]);
         const bool single = gb.y == 1 && root.z == 1;
         const int s = single ? __ldg(&S.gl_shapes[root.y]) : 0;

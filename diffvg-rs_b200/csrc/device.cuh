@@ -1596,35 +1596,11 @@ __device__ __forceinline__ void flush_splat(const DevScene& S, int ox, int oy, i
         atomicAdd(wsum + p, c[4]);
     }
 }
-// gather_d_color (src/backward/filters.rs:70-103)
-__device__ __forceinline__ float4 gather_d_color(const DevScene& S, const float* d_render, const float* wsum,
-                                                 float2 ps) {
-    float4 out = make_float4(0, 0, 0, 0);
-    const int px = f2i(floorf(ps.x)), py = f2i(floorf(ps.y)), ri = S.filter_ri;
-#pragma unroll 1
-    for (int dy = -ri; dy <= ri; ++dy)
-#pragma unroll 1
-        for (int dx = -ri; dx <= ri; ++dx) {
-            int xx = px + dx, yy = py + dy;
-            if (xx < 0 || yy < 0 || xx >= S.width || yy >= S.height) continue;
-            float w = filter_weight(S.filter_type, S.filter_radius, (float)xx + 0.5f - ps.x, (float)yy + 0.5f - ps.y);
-            size_t q = (size_t)yy * S.width + xx;
-            float ws = wsum[q];
-            if (ws > 0.0f) {
-                float4 d = reinterpret_cast<const float4*>(d_render)[q];
-                float k = w / ws;
-                out.x += k * d.x;
-                out.y += k * d.y;
-                out.z += k * d.z;
-                out.w += k * d.w;
-            }
-        }
-    return out;
-}
-// gather_d_color, and in the same pass over the footprint the vector whose dot product with the
-// sample's colour is the filter-radius adjoint (accumulate_filter_gradient below is linear in
-// the colour, and d_filter_weight in its return's adjoint, for every filter but the
-// parabolic one, whose adjoint the crate does not scale): one weight per pixel instead of three.
+// gather_d_color (src/backward/filters.rs:70-103), and in the same pass over the footprint the
+// vector whose dot product with the sample's colour is the filter-radius adjoint
+// (accumulate_filter_gradient below is linear in the colour, and d_filter_weight in its return's
+// adjoint, for every filter but the parabolic one, whose adjoint the crate does not scale): one
+// weight per pixel instead of three.
 __device__ __forceinline__ float4 gather_d_color_radius(const DevScene& S, const float* d_render, const float* wsum,
                                                         float2 ps, float4* rad) {
     float4 out = make_float4(0, 0, 0, 0), r4 = out;

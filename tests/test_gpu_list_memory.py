@@ -78,7 +78,7 @@ def test_results_do_not_depend_on_the_room(renderer, limited, share, prefilter):
         assert float(np.max(np.abs(a - b))) <= 1e-4 * scale + 1e-6, name
 
 
-@pytest.mark.parametrize("share", SHARES)
+@pytest.mark.parametrize("share", SHARES + [8.0])  # (the last: whole lists, taken in step where they are heavy)
 @pytest.mark.parametrize("work_queue", [0, 1])
 def test_batch(renderer, limited, share, work_queue):
     scenes = [_scene(), synth.plain_scene(3, 64, 48, 9), _scene(45, 70, 3, 25)]
