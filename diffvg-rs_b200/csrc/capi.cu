@@ -115,6 +115,10 @@ struct SceneBuf {
 };
 // Bytes of freed scene memory that a context keeps for its next uploads.
 constexpr uint64_t kScenePoolKeep = 256ull << 20;
+// Items per cell entry that lists have room for at first.  Scenes of icons, outlines and mixed shapes
+// ask for 0.6 to 1.5, the 1024x1024 scene of 4096 16-segment paths for 3.2 (with room for 3 its first
+// render ran with full queries in what was left over, 24.3 ms, and its second made room).
+constexpr uint64_t kItemGuess = 4;
 // Bytes that the cell lists of one scene may take (dvg_context_set_list_memory).
 constexpr uint64_t kListMemory = 4ull << 30;
 
@@ -248,7 +252,7 @@ dvg_status read_cells(dvg_scene* sc, cudaStream_t stream) {
     return DVG_OK;
 }
 // Builds lists once again with the room that they asked for, times `slack`, where the first guess
-// (three items per cell entry) was short of it.  What reads the old ones may go on.
+// was short of it.  What reads the old ones may go on.
 dvg_status grow_cells(dvg_scene* sc, uint64_t total, int slack, cudaStream_t stream) {
     if (sc->lists_items * slack <= (uint64_t)sc->cell_table.cap_items) return DVG_OK;
     const uint64_t items = sc->lists_items * slack;
@@ -262,7 +266,7 @@ dvg_status grow_cells(dvg_scene* sc, uint64_t total, int slack, cudaStream_t str
 // what they ask for; without memory for them the old ones stay.
 dvg_status remake_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, int slack) {
     std::lock_guard<std::mutex> lock(sc->lists_mutex);
-    if (!reserve_cells(sc, total, 3 * CELLS * total * slack, ctx->stream, &sc->replaced)) return DVG_OK;
+    if (!reserve_cells(sc, total, kItemGuess * CELLS * total * slack, ctx->stream, &sc->replaced)) return DVG_OK;
     dvg_status st = build_cells(sc, ctx->stream);
     if (st == DVG_OK) st = read_cells(sc, ctx->stream);
     if (st == DVG_OK) st = grow_cells(sc, total, slack, ctx->stream);
@@ -732,7 +736,7 @@ static dvg_status upload_scene(dvg_context* ctx, const dvg_scene_desc* desc, Bui
         CK(cudaGetLastError());
         sc->lists_total = (uint64_t)std::max(total, 0);
         if (S.num_groups > 0 && build != Build::NEVER &&
-            reserve_cells(sc.get(), sc->lists_total, 3 * CELLS * sc->lists_total,
+            reserve_cells(sc.get(), sc->lists_total, kItemGuess * CELLS * sc->lists_total,
                           build == Build::NOW ? ctx->stream : ctx->build, nullptr))
             sc->lists = dvg_scene::Lists::RESERVED;
     }

@@ -164,7 +164,7 @@ def test_crowded_cells_get_their_room_later(renderer):
     later ones with all, and a batch made in between keeps the tables that it was made with."""
     import test_gpu_list_memory as lm
 
-    sc = lm._scene()
+    sc = lm._scene(rings=8, segs=90)
     ref = renderer.render(sc, OPTS).pixels.reshape(-1)
     up = renderer.upload(sc)
     out = torch.empty(ref.size, device="cuda")
