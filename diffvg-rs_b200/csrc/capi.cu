@@ -736,8 +736,7 @@ static dvg_status upload_scene(dvg_context* ctx, const dvg_scene_desc* desc, Bui
         CK(cudaGetLastError());
         sc->lists_total = (uint64_t)std::max(total, 0);
         if (S.num_groups > 0 && build != Build::NEVER &&
-            reserve_cells(sc.get(), sc->lists_total, kItemGuess * CELLS * sc->lists_total,
-                          build == Build::NOW ? ctx->stream : ctx->build, nullptr))
+            reserve_cells(sc.get(), sc->lists_total, kItemGuess * CELLS * sc->lists_total, ctx->stream, nullptr))
             sc->lists = dvg_scene::Lists::RESERVED;
     }
     layout_grads(sc.get());

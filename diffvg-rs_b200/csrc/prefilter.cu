@@ -181,14 +181,13 @@ static __device__ bool closest_shape(const DevScene& S, int s, float2 lp, float2
 // Shape-space reach for a canvas distance `want` around p: a point of the shape that is farther
 // from p than this is farther than `want` on the canvas (S.g_isig: the map's smallest stretch;
 // the slack covers its 0.01 pixel and the f32 maps).  The two maps of a group undo each other to
-// 0.01 pixel over the canvas; elsewhere (positions of a signed distance) no bound is known.
-__device__ __forceinline__ float shape_reach(const DevScene& S, int g, float2 pt, float want, float2 p) {
+// 0.01 pixel over the canvas; no bound is known elsewhere, and callers there want infinity.
+__device__ __forceinline__ float shape_reach(const DevScene& S, int g, float want, float2 p) {
     const float k = __ldg(&S.g_isig[g]);
-    const bool on = pt.x >= -2.0f && pt.x <= (float)S.width + 2.0f && pt.y >= -2.0f && pt.y <= (float)S.height + 2.0f;
-    return k > 0.0f && on ? (want + 0.03f) * k * 1.001f + 1.0e-4f * (1.0f + fabsf(p.x) + fabsf(p.y)) : INF_F;
+    return k > 0.0f ? (want + 0.03f) * k * 1.001f + 1.0e-4f * (1.0f + fabsf(p.x) + fabsf(p.y)) : INF_F;
 }
 // compute_distance_bvh (api.rs:138-236) with the brute-force fallback compute_distance (api.rs:36-76).
-// `want`: the caller has no use for a canvas distance beyond it.
+// `want`: the caller has no use for a canvas distance beyond it (points off the canvas: infinity).
 static __device__ bool compute_distance_group(const DevScene& S, int g, float2 pt, float max_radius, float want,
                                        ClosestD* best, unsigned* status) {
     const int4 gb = __ldg(&S.g_bvh[g]);
@@ -234,7 +233,7 @@ static __device__ bool compute_distance_group(const DevScene& S, int g, float2 p
                 if (si.x == K_PATH && si.z >= 0 && __ldg(&S.p_info[2 * si.z].w) > 0) {
                     float2 scp;
                     const float2 p = shape_local_dist(S, s, lp);
-                    ok = closest_path_bvh(S, si.z, p, shape_reach(S, g, pt, want, p), &scp, &seg, &t, status);
+                    ok = closest_path_bvh(S, si.z, p, shape_reach(S, g, want, p), &scp, &seg, &t, status);
                     if (ok) lc = xf9(S.s_xform + 9 * s, scp);
                 } else {
                     ok = closest_shape(S, s, lp, &lc, &seg, &t);
@@ -1405,12 +1404,14 @@ int launch_interior_prefilter_batch(const BatchEntry* B, const int2* work, int i
 // return a point within the bound, which is all the crate's search would accept).
 static __device__ bool sdf_closest(const DevScene& S, const float4* g_bbox, float2 pt, float init, ClosestD* best,
                             int* group, unsigned* status) {
+    // (positions may lie anywhere: see shape_reach)
+    const bool on = pt.x >= -2.0f && pt.x <= (float)S.width + 2.0f && pt.y >= -2.0f && pt.y <= (float)S.height + 2.0f;
     float best_dist = init;
     bool found = false;
     for (int g = S.num_groups - 1; g >= 0; --g) {
         if (box_distance(__ldg(&g_bbox[g]), pt) > best_dist) continue;
         ClosestD h;
-        if (compute_distance_group(S, g, pt, best_dist, best_dist, &h, status) && h.dist < best_dist) {
+        if (compute_distance_group(S, g, pt, best_dist, on ? best_dist : INF_F, &h, status) && h.dist < best_dist) {
             best_dist = h.dist;
             *best = h;
             *group = g;
