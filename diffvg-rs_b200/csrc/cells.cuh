@@ -68,12 +68,7 @@ static __device__ __noinline__ bool group_inside_any(const DevScene& S, int g, f
     return group_inside(S, g, lp, __ldg(&S.g_info[g].z));
 }
 
-// A cell is heavy from this many steps in its lists (entry_steps).  The kernels are bound by
-// instruction fetch: where the lists are long, a CTA's warps take them one entry at a time, so that
-// they run the same code together (forward of the large 1024x1024 scene 18.5 -> 14.7 ms, edge pass
-// 62.9 -> 48.0 when it came in).  Against 24, from 12 on: batch of 64 icons 5.25 -> 5.58 ms, large
-// render 15.9 -> 15.7; from 40 on: large render 16.7, its step 69.6 -> 71.5 ms.
-constexpr int CELL_HEAVY = 24;
+// A heavy cell (CELL_HEAVY) is marked next to its number of entries.
 constexpr int CELL_HEAVY_BIT = 1 << 30;
 
 // The groups to visit at one cell: the cell's entries, or the tile's whole list.

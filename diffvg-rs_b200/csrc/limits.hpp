@@ -41,11 +41,20 @@ constexpr int CELL_LIST_MAX = 1 << 22;
 DVG_LIM_HD int entry_word(bool listed, int place, int flags) { return listed ? (place << 8) | flags : flags; }
 DVG_LIM_HD int entry_place(bool listed, int step, int word) { return listed ? word >> 8 : step; }
 
-// Steps that an entry adds to its cell: pairs of rows, curves, one-point segments and stroke
-// segments.  `hard` also says that the shape is a primitive (one formula, no segments).
+// A cell is heavy from this many steps in its lists: pairs of rows, curves, one-point segments and
+// stroke segments.  The kernels are bound by instruction fetch: where the lists are long, a CTA's
+// warps take them one entry at a time, so that they run the same code together (forward of the
+// large 1024x1024 scene 18.5 -> 14.7 ms, edge pass 62.9 -> 48.0 when it came in).  Against 24, from
+// 12 on: batch of 64 icons 5.25 -> 5.58 ms, large render 15.9 -> 15.7; from 40 on: large render
+// 16.7, its step 69.6 -> 71.5 ms.
+constexpr int CELL_HEAVY = 24;
+// A primitive whose edge crosses the cell (`hard` says so: one formula, no segments) makes it heavy
+// by itself: its code is a detour from the segments' that the warps had better take together.
+// Mixed 512x512 step: edge pass 0.432 ms against 0.476 where it counts as one step, forward
+// 0.846 against 0.831.
 constexpr int CELL_PRIMITIVE = 63;
 DVG_LIM_HD int entry_steps(int pairs, int curves, int hard, int strokes) {
-    return pairs + curves + (hard == CELL_PRIMITIVE ? 1 : hard) + strokes;
+    return pairs + curves + (hard == CELL_PRIMITIVE ? CELL_HEAVY : hard) + strokes;
 }
 
 // Where a request for `need` of `cap` places begins when `taken` were asked for before it, or -1:

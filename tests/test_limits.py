@@ -73,10 +73,10 @@ def test_cell_list_memory_within_its_limit(limits, tiles, entries):
 
 
 def test_steps_of_an_entry(limits):
-    """The count that makes a cell heavy: a circle's edge is one step, not the 63 that mark it in the
-    place of a number of segments."""
+    """The count that makes a cell heavy (from 24 steps): a primitive's edge, marked by 63 in the place of
+    a number of segments, does so by itself and no more than that."""
     assert limits.limits_entry_steps(2, 3, 4, 5) == 14
-    assert limits.limits_entry_steps(0, 0, 63, 0) == 1
+    assert limits.limits_entry_steps(0, 0, 63, 0) == 24
     assert limits.limits_entry_steps(0, 0, 48, 2) == 50
 
 
