@@ -151,6 +151,7 @@ struct dvg_context {
     bool profiling = false;
     std::vector<ProfEvent> pending;
     std::vector<ProfStat> stats;
+    std::vector<dvg_batch*> batches;  // alive (dvg_batch_set_adam tells them where a scene's lists are)
     cudaStream_t stream = nullptr;
     cudaStream_t build = nullptr;  // builds scenes' cell lists, independent of what `stream` waits for
     cudaMemPool_t pool = nullptr;  // scene memory (SceneBuf)
@@ -1637,6 +1638,7 @@ extern "C" dvg_status dvg_batch_create(dvg_context* ctx, dvg_scene* const* scene
     CK(cudaMemcpyAsync(b->work.ptr, work2.data(), work2.size() * sizeof(int2), cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    ctx->batches.push_back(b.get());
     *out = b.release();
     return DVG_OK;
 }
@@ -1645,6 +1647,8 @@ extern "C" void dvg_batch_destroy(dvg_batch* b) {
     if (!b) return;
     cudaSetDevice(b->ctx->device);
     cudaStreamSynchronize(b->ctx->stream);
+    auto& all = b->ctx->batches;
+    all.erase(std::remove(all.begin(), all.end(), b), all.end());
     batch_drop_graph(b);
     delete b;
 }
@@ -1709,6 +1713,27 @@ extern "C" dvg_status dvg_batch_losses(dvg_batch* b, float* host_losses) {
     return check_status(ctx);
 }
 
+// Points a batch's entries, on the host and on the device, at the present lists of those of its
+// scenes that are among `scenes`.
+static dvg_status batch_refresh_lists(dvg_batch* b, const std::vector<dvg_scene*>& scenes) {
+    const cudaStream_t stream = b->ctx->stream;
+    const size_t bytes = b->host_entries.size() * sizeof(BatchEntry);
+    // start from the device entries: the optimisation step updates some of their fields
+    CK(cudaMemcpyAsync(b->host_entries.data(), b->entries.ptr, bytes, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    for (size_t i = 0; i < b->scenes.size(); ++i) {
+        if (std::find(scenes.begin(), scenes.end(), b->scenes[i]) == scenes.end()) continue;
+        DevScene& S = b->host_entries[i].S;
+        S.tile_entries = b->scenes[i]->dev.tile_entries;
+        S.cell_info = b->scenes[i]->cell_table.info;
+        S.cell_entries = b->scenes[i]->cell_table.entries;
+        S.cell_items = b->scenes[i]->cell_table.items;
+    }
+    CK(cudaMemcpyAsync(b->entries.ptr, b->host_entries.data(), bytes, cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    return DVG_OK;
+}
+
 extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o) {
     if (!b) return fail(DVG_ERR_INVALID_ARGUMENT, "null batch");
     dvg_context* ctx = b->ctx;
@@ -1728,6 +1753,7 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
                   (o->params & DVG_OPT_PAINTS) ? 1 : 0};
     // Tile lists must hold any binning the moved geometry can produce: every group in
     // every tile at worst.
+    dvg_status st = DVG_OK;
     for (int i = 0; i < n; ++i) {
         dvg_scene* sc = b->scenes[i];
         const size_t tiles = (size_t)sc->dev.tiles_x * sc->dev.tiles_y;
@@ -1750,16 +1776,20 @@ extern "C" dvg_status dvg_batch_set_adam(dvg_batch* b, const dvg_adam_options* o
             int total = 0;
             CK(cudaMemcpyAsync(&total, offsets + tiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
-            const dvg_status st =
-                remake_cells(ctx, sc, std::min<uint64_t>(need, 2 * (uint64_t)std::max(total, 0) + 1024), 2);
+            st = remake_cells(ctx, sc, std::min<uint64_t>(need, 2 * (uint64_t)std::max(total, 0) + 1024), 2);
             if (st != DVG_OK) return st;
             sc->lists_for_steps = true;
         }
-        b->host_entries[i].S.tile_entries = sc->dev.tile_entries;
-        b->host_entries[i].S.cell_info = sc->cell_table.info;
-        b->host_entries[i].S.cell_entries = sc->cell_table.entries;
-        b->host_entries[i].S.cell_items = sc->cell_table.items;
     }
+    // This batch's entries, and those of other batches of the same scenes: the steps write a scene's
+    // tile offsets in place, which belong to the lists that it has now.
+    for (dvg_batch* o : ctx->batches)
+        if (std::any_of(o->scenes.begin(), o->scenes.end(), [&](dvg_scene* sc) {
+                return std::find(b->scenes.begin(), b->scenes.end(), sc) != b->scenes.end();
+            })) {
+            st = batch_refresh_lists(o, b->scenes);
+            if (st != DVG_OK) return st;
+        }
     // Adam moments and sort scratch, one block per scene.
     std::vector<size_t> st_off(n), so_off(n);
     size_t st_total = 0, so_total = 0;

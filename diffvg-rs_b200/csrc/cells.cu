@@ -1,4 +1,5 @@
-// cells.cu — builds the per-cell lists (cells.cuh).  Built with -fmad=false like kernels.cu.
+// cells.cu — builds the per-cell lists (cells.cuh), for the first call that reads a scene's and
+// after each on-device parameter step.  Built with -fmad=false like kernels.cu.
 //
 // One CTA per tile walks the tile's groups; for a path group its 256 threads take the
 // (cell, segment) pairs, sixteen cells of one segment next to each other, so a pair costs one
@@ -8,7 +9,7 @@
 // with the lists 1.2 segments, 1.5 curves and 2.7 rows of 2.2 groups are left (large
 // 1024x1024 scene: 199 -> 18, 6, 26).  The lists took the forward from 3.43 to 1.23 ms and the
 // edge pass from 1.31 to 0.81 ms on the mixed scene at 4x4 spp, from 76 to 34 ms and from 216 to
-// 136 ms on the large one (with the steps taken since: 0.82, 0.41, 14.6 and 46.9 ms).  4x4
+// 136 ms on the large one (with the steps taken since: 0.83, 0.43, 15.9 and 49.2 ms).  4x4
 // pixels: the 16 samples per pixel of a CTA share one list; cells of a whole tile leave 8
 // segments.  The build itself is bound by latency, a few barriers per group at 12-24 % occupancy:
 // 55 us on a 128x128 scene of 8 shapes, 0.22 ms on the mixed scene, 4.2 ms on the large one.

@@ -595,9 +595,9 @@ __device__ __forceinline__ int winding_segment(const SegGeom& s, float2 pt) {
     return winding_segment_v(s.kind, s.q[0], s.q[1], s.q[2], s.q[3], s.q[4], s.q[5], s.q[6], s.q[7], pt);
 }
 
-// The crate's own formulas for the strokes that the cell lists' chord tests leave open (a few
-// percent of the samples): small code, since every excursion to it displaces the sample loop's
-// from the instruction cache.  Same results as seg_closest (of a cubic, with `stop`, the first
+// The crate's own formulas for the strokes that the cell lists' chord tests leave open (of lines and
+// quadratics a few percent of the samples, of cubics all that may be within): small code, since
+// every excursion to it displaces the sample loop's from the instruction cache.  Same results as seg_closest (of a cubic, with `stop`, the first
 // candidate nearer than that).
 __device__ __forceinline__ CPRes seg_closest_plain(const SegGeom& sg, float2 p, bool approx, float stop) {
     if (sg.kind == 0) return closest_line(p, sg.q[0], sg.q[1], sg.q[2], sg.q[3]);

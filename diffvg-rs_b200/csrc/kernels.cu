@@ -27,7 +27,7 @@
 #endif
 // The edge evaluation is bound by instruction fetch: 512 threads of a CTA that take a heavy cell's
 // entries together, at 40 registers, against 128 threads at 32 that run apart: edge pass of the
-// large 1024x1024 scene 62.0 -> 48.0 ms, mixed 0.43 -> 0.41 (together: 128 threads 59.9 ms, 256
+// large 1024x1024 scene 62.0 -> 48.0 ms, mixed 0.43 -> 0.41 (49.2 and 0.43 now; together: 128 threads 59.9 ms, 256
 // 52.4, 512 at 32 registers 49.8 and at 64 51.7, 1024 at 64 59.1).
 #ifndef DVG_BND_THREADS
 #define DVG_BND_THREADS 512

@@ -21,8 +21,8 @@
 #include "kernels.cuh"
 // Minimum resident CTAs per SM of the prefiltered forward and interior kernels, by
 // measurement on B200 (mixed 512x512 scene, 2x2 spp): the forward at 6 (40 registers) 4.03 ->
-// 3.80 ms against 4 (5: 3.94, 3: 4.16; 2.36 now); the interior at 1 (168 registers, no spills)
-// 6.17 ms (2: 7.36, 3: 7.59; 4.88 now).
+// 3.80 ms against 4 (5: 3.94, 3: 4.16; 2.53 now); the interior at 1 (168 registers, no spills)
+// 6.17 ms (2: 7.36, 3: 7.59; 5.20 now).
 #ifndef DVG_MINB_PF_FWD
 #define DVG_MINB_PF_FWD 6
 #endif

@@ -196,8 +196,7 @@ typedef struct dvg_scene dvg_scene;
  *                1 = they launch as many persistent CTAs as the GPU holds at once, which
  *                take the items from a device counter in the same order.
  * forward_occupancy: 0, 1 or 2; accepted and kept, without effect on the launches: the
- *                forward runs at 4 CTAs of 256 threads per SM (64 registers), which measured
- *                faster than 3 or 2 on every scene since the per-cell lists. */
+ *                forward runs at 5 CTAs of 256 threads per SM (48 registers). */
 typedef struct dvg_tuning {
     uint32_t sample_layout;
     uint32_t boundary_cell;

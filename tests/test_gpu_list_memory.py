@@ -152,3 +152,35 @@ def test_room_for_steps_where_the_tile_list_is_full(renderer):
     assert n[1] > n[0] and n[2] == n[1]
     b.close()
     up.close()
+
+
+@pytest.mark.parametrize("share", [0.0, 0.3, 8.0])
+def test_two_batches_of_one_scene(renderer, limited, share):
+    """A batch made before another one optimises its scene: its steps render the geometry of now, from
+    the lists of now (the tile offsets that it reads are written in place)."""
+    sc = _scene()
+    opts = RenderOptions(samples_x=2, samples_y=2, seed=3, jitter=True, use_prefiltering=False)
+    probe = renderer.upload(sc)
+    nbytes = _bytes(probe, share) if share else 0
+    probe.close()
+    limited(nbytes)
+    up, more = renderer.upload(sc), renderer.upload(synth.plain_scene(3, 64, 48, 9))
+    plain = Batch(renderer, [more, up], opts, BackwardOptions(boundary_samples=500))
+    plain.step(True)
+    b = Batch(renderer, [up], opts, BackwardOptions(boundary_samples=500))
+    b.set_adam(2.0)
+    for _ in range(4):
+        b.step(True)
+    b.losses()
+    pts, _ = b.scene_params(0)
+    limited(ALL)
+    want = renderer.render(scene_with_params(sc, up.packed, pts), opts).pixels.reshape(-1)
+    plain.step(True)
+    plain.losses()
+    assert float(np.max(np.abs(plain.buffers(1)[0].cpu().numpy() - want))) <= 1e-5
+    other = renderer.render(more.scene, opts).pixels.reshape(-1)
+    assert float(np.max(np.abs(plain.buffers(0)[0].cpu().numpy() - other))) <= 1e-5
+    b.close()
+    plain.close()
+    up.close()
+    more.close()
