@@ -12,7 +12,7 @@
 // 136 ms on the large one (with the steps taken since: 0.83, 0.43, 15.9 and 49.2 ms).  4x4
 // pixels: the 16 samples per pixel of a CTA share one list; cells of a whole tile leave 8
 // segments.  The build itself is bound by latency, a few barriers per group at 12-24 % occupancy:
-// 55 us on a 128x128 scene of 8 shapes, 0.22 ms on the mixed scene, 4.2 ms on the large one.
+// 55 us on a 128x128 scene of 8 shapes, 0.23 ms on the mixed scene, 3.0 ms on the large one.
 #include "cells.cuh"
 #include "kernels.cuh"
 
