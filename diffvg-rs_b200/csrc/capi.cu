@@ -252,6 +252,11 @@ dvg_status read_cells(dvg_scene* sc, cudaStream_t stream) {
     sc->lists = dvg_scene::Lists::READY;
     return DVG_OK;
 }
+// After a failure between a table's room and its lists: the scene has none.
+void drop_cells(dvg_scene* sc) {
+    sc->cell_table = CellTable{};
+    sc->lists = dvg_scene::Lists::NONE;
+}
 // Builds lists once again with the room that they asked for, times `slack`, where the first guess
 // was short of it.  What reads the old ones may go on.
 dvg_status grow_cells(dvg_scene* sc, uint64_t total, int slack, cudaStream_t stream) {
@@ -260,7 +265,8 @@ dvg_status grow_cells(dvg_scene* sc, uint64_t total, int slack, cudaStream_t str
     sc->lists_items = 0;  // one attempt
     if (!reserve_cells(sc, total, items, stream, &sc->replaced)) return DVG_OK;
     dvg_status st = build_cells(sc, stream);
-    if (st == DVG_OK) CK(cudaStreamSynchronize(stream));
+    if (st == DVG_OK && cudaStreamSynchronize(stream) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "cell lists");
+    if (st != DVG_OK) drop_cells(sc);
     return st;
 }
 // Lists of a scene that a batch holds, made anew on the context's stream with room for `slack` times
@@ -271,6 +277,7 @@ dvg_status remake_cells(dvg_context* ctx, dvg_scene* sc, uint64_t total, int sla
     dvg_status st = build_cells(sc, ctx->stream);
     if (st == DVG_OK) st = read_cells(sc, ctx->stream);
     if (st == DVG_OK) st = grow_cells(sc, total, slack, ctx->stream);
+    if (st != DVG_OK) drop_cells(sc);
     sc->lists_items = 0;
     return st;
 }

@@ -221,9 +221,10 @@ void dvg_context_destroy(dvg_context* ctx);
 dvg_status dvg_context_set_retain(dvg_context* ctx, int enable);
 /* Device memory that the per-cell lists of one scene may take (4 GiB by default; 0: no
  * lists).  A scene's lists take up to 1,536 bytes per tile-list entry (a group on a 16x16 tile)
- * at first and more where its cells are crowded; dvg_batch_set_adam makes room for twice that.
- * They make rendering faster and change no result: with less memory than they want, or none, the
- * tiles and entries left over are searched without them.  Applies to later uploads. */
+ * at first and more where its cells are crowded; dvg_batch_set_adam makes room for twice the
+ * entries and four times the items (up to 5 KiB per tile-list entry).  They make rendering
+ * faster and change no result: with less memory than they want, or none, the tiles and
+ * entries left over are searched without them.  Applies to later uploads. */
 dvg_status dvg_context_set_list_memory(dvg_context* ctx, uint64_t bytes);
 
 /* Host preparation + upload.  Replaces prepare_scene / prepare_scene_backward and the
